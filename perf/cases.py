@@ -93,7 +93,7 @@ def draw(rng) -> dict:
     edits = rng.choice(EDITS)
     cap = rng.choice([64, 1024, 4096, 65_536])
     if api in ("device", "host"):
-        n = _log_uniform(rng, 700, 1_200_000 if genome == "large" else 2_400_000 if api == "device" else 1_500_000)
+        n = _log_uniform(rng, 700, 1_100_000 if genome == "large" else 2_400_000 if api == "device" else 1_500_000)
         return dict(api=api, genome=genome, mode="search1", form="batched", reads=n, lo=lo, hi=hi, edits=edits,
                     max_results=cap)
     if api == "plain":
