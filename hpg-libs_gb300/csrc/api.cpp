@@ -352,6 +352,16 @@ int bwt_gpu_start_table(bwt_index_t* index) {
   return e ? engine_kmer(e) : -1;
 }
 
+int bwt_gpu_set_full_rows(bwt_index_t* index, int on) {
+  Engine* e = engine_of(index);
+  return e ? engine_set_full_rows(e, on) : 0;
+}
+
+int bwt_gpu_full_rows(bwt_index_t* index) {
+  Engine* e = engine_of(index);
+  return e ? engine_full_rows(e) : 0;
+}
+
 void bwt_gpu_set_pipeline_chunk(bwt_index_t* index, size_t reads) {
   Engine* e = engine_of(index);
   if (e) engine_set_pipeline_chunk(e, reads);

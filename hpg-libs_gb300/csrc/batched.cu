@@ -4,6 +4,8 @@
 #include <cooperative_groups/scan.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "batched.cuh"
 #include "batched_dev.cuh"
 #include "kernels.cuh"
@@ -1043,6 +1045,100 @@ __global__ void __launch_bounds__(kExpandTpb)
   }
 }
 
+// Key, chromosome and position of one located row (bwt.c:2025-2036,2158-2166).
+__device__ __forceinline__ hpg_loc_t located(const DevIndex& X, uint32_t sa, uint32_t phys_len, uint32_t hit) {
+  const uint32_t phys = phys_len >> 31;
+  const uint64_t len_calc = phys_len & kRowLenMask;
+  uint64_t key = sa;
+  if (phys && (phys_len & kRowKey32))  // an int length: the SA_TYPE (32-bit) difference wraps
+    key = (uint32_t)((X.top + 1u) - sa - (uint32_t)len_calc - 1u);
+  else if (phys)
+    key = (uint64_t)((X.top + 1u) - sa) - len_calc - 1u;
+  const uint32_t id = kar_search(X, key);
+  hpg_loc_t o;
+  o.key = key;
+  o.hit = hit;
+  o.pad = 0;
+  if (key + len_calc <= X.kar_offset[id]) {
+    o.valid = 1;
+    o.chrom = id - 1;
+    o.position = X.kar_start[id - 1] + (key - X.kar_offset[id - 1]);
+  } else {
+    o.valid = 0;
+    o.chrom = 0;
+    o.position = 0;
+  }
+  return o;
+}
+
+// Locate with the whole suffix array: a thread per hit locates the hit's rows,
+// one gather each; hits of more than 4 rows (repeats, up to the locate limit)
+// are shared by the warp, 32 rows a round.  No row items: a hit's rows land at
+// loc_off[hit] in row order.  Bound by random 32-byte sectors, one a row, and
+// the records streamed through: 2M one-row hits at 100 Mbp in 80 us, against
+// 406 us for the row items and the LF walks.
+__global__ void __launch_bounds__(kExpandTpb)
+    locate_hits_kernel(DevIndex X, const hpg_hit_t* __restrict__ hits, const uint64_t* __restrict__ loc_off,
+                       uint32_t n_hits, uint64_t n_locs, const uint64_t* __restrict__ read_offs,
+                       hpg_loc_t* __restrict__ out, unsigned long long* census, LocateSizes z) {
+  if (z.status) {  // graph form: sizes from device memory, rows checked against the output's capacity
+    if (*z.status) return;
+    n_hits = (uint32_t)*z.n_hits;
+    n_locs = *z.n_locs;
+    if (n_locs > z.locs_cap) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(z.status, kStatusLocFull);
+      return;
+    }
+  }
+  const uint32_t lane = threadIdx.x & 31;
+  unsigned long long rows = 0;
+  for (uint64_t h0 = (uint64_t)blockIdx.x * kExpandTpb; h0 < n_hits; h0 += (uint64_t)gridDim.x * kExpandTpb) {
+    const uint64_t h = h0 + threadIdx.x;
+    uint32_t cnt = 0, k = 0, phys_len = 0;
+    uint64_t b = 0;
+    if (h < n_hits) {
+      b = loc_off[h];
+      cnt = (uint32_t)(loc_off[h + 1] - b);
+      if (cnt) {
+        const hpg_hit_t x = hits[h];
+        const uint64_t len = read_offs[x.read + 1] - read_offs[x.read];
+        const uint32_t err = x.nm ? x.err_kind : 0u;
+        const uint32_t phys = (uint32_t)x.dir ^ (uint32_t)x.strand;  // direction = type ? dir : !dir, type = !strand
+        phys_len = (phys << 31) | (uint32_t)(len - (err == 1 ? 1 : 0) + (err == 3 ? 1 : 0));
+        k = (uint32_t)x.k;
+      }
+    }
+    rows += cnt;
+    if (cnt <= 4) {
+      const uint32_t* sa = (phys_len >> 31) ? X.dir[1].sa : X.dir[0].sa;
+      for (uint32_t i = 0; i < cnt; ++i) out[b + i] = located(X, load_row_word(sa + k + i), phys_len, (uint32_t)h);
+    }
+    unsigned big = __ballot_sync(0xFFFFFFFFu, cnt > 4);
+    while (big) {
+      const int j = __ffs(big) - 1;
+      big &= big - 1;
+      const uint32_t cj = __shfl_sync(0xFFFFFFFFu, cnt, j), kj = __shfl_sync(0xFFFFFFFFu, k, j);
+      const uint32_t pj = __shfl_sync(0xFFFFFFFFu, phys_len, j);
+      const uint64_t bj = __shfl_sync(0xFFFFFFFFu, b, j);
+      const uint32_t hj = (uint32_t)__shfl_sync(0xFFFFFFFFu, h, j);
+      const uint32_t* sa = (pj >> 31) ? X.dir[1].sa : X.dir[0].sa;
+      for (uint32_t i = lane; i < cj; i += 32) out[bj + i] = located(X, load_row_word(sa + kj + i), pj, hj);
+    }
+  }
+  if (census && rows) atomicAdd(census, rows);
+}
+
+// The same for caller-built rows: a thread per item.
+__global__ void __launch_bounds__(kExpandTpb)
+    locate_items_kernel(DevIndex X, const RowItem* __restrict__ items, uint64_t n_items, hpg_loc_t* __restrict__ out) {
+  for (uint64_t i = (uint64_t)blockIdx.x * kExpandTpb + threadIdx.x; i < n_items;
+       i += (uint64_t)gridDim.x * kExpandTpb) {
+    const RowItem it = items[i];
+    const uint32_t* sa = (it.phys_len >> 31) ? X.dir[1].sa : X.dir[0].sa;
+    out[it.out] = located(X, load_row_word(sa + it.row), it.phys_len, it.hit);
+  }
+}
+
 constexpr unsigned kRowsPerClaim = 4;
 // Lanes whose walk reached a sampled row (or that hold no row) wait, masked,
 // until this many lanes of their converged group have (or all have), and then
@@ -1073,29 +1169,7 @@ __global__ void __launch_bounds__(kBlock)
   bool active = false, reached = false;
   uint32_t sectors = 0;
   auto finish = [&]() {  // the pending walk's key and chromosome
-    const uint32_t sa = (ps + pj) % X.walk_mod;
-    const uint32_t phys = pit.phys_len >> 31;
-    const uint64_t len_calc = pit.phys_len & kRowLenMask;
-    uint64_t key = sa;
-    if (phys && (pit.phys_len & kRowKey32))  // an int length: the SA_TYPE (32-bit) difference wraps
-      key = (uint32_t)((X.top + 1u) - sa - (uint32_t)len_calc - 1u);
-    else if (phys)
-      key = (uint64_t)((X.top + 1u) - sa) - len_calc - 1u;
-    const uint32_t id = kar_search(X, key);
-    hpg_loc_t o;
-    o.key = key;
-    o.hit = pit.hit;
-    o.pad = 0;
-    if (key + len_calc <= X.kar_offset[id]) {
-      o.valid = 1;
-      o.chrom = id - 1;
-      o.position = X.kar_start[id - 1] + (key - X.kar_offset[id - 1]);
-    } else {
-      o.valid = 0;
-      o.chrom = 0;
-      o.position = 0;
-    }
-    out[pit.out] = o;
+    out[pit.out] = located(X, (ps + pj) % X.walk_mod, pit.phys_len, pit.hit);
     pending = false;
   };
   for (;;) {
@@ -1352,6 +1426,14 @@ void launch_locate_persistent(const DevIndex& X, const hpg_hit_t* hits, const ui
                               unsigned int* row_ctr, unsigned long long* census, int num_sms, cudaStream_t s,
                               const LocateSizes& z) {
   if (!n_locs) return;
+  if (X.text) {
+    count_launches(1);
+    // graph form: grid-stride over the hits, 8 blocks per SM
+    const uint64_t grid = z.status ? 8ull * num_sms : ((uint64_t)n_hits + kExpandTpb - 1) / kExpandTpb;
+    locate_hits_kernel<<<(unsigned)(grid ? grid : 1), kExpandTpb, 0, s>>>(X, hits, loc_off, n_hits, n_locs, read_offs,
+                                                                          out, census, z);
+    return;
+  }
   RowItem* items = static_cast<RowItem*>(row_items);
   unsigned int* side = row_ctr + 1;  // two counters after the row claim counter
   cudaMemsetAsync(side, 0, 8, s);
@@ -1373,6 +1455,12 @@ void launch_locate_persistent(const DevIndex& X, const hpg_hit_t* hits, const ui
 void launch_locate_items(const DevIndex& X, const RowItem* items, uint64_t n_items, hpg_loc_t* out,
                          unsigned int* row_ctr, int num_sms, cudaStream_t s) {
   if (!n_items) return;
+  if (X.text) {
+    const uint64_t blocks = std::min<uint64_t>((n_items + kExpandTpb - 1) / kExpandTpb, 16ull * num_sms);
+    count_launches(1);
+    locate_items_kernel<<<(unsigned)blocks, kExpandTpb, 0, s>>>(X, items, n_items, out);
+    return;
+  }
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, locate_persistent_kernel, kBlock, 0);
   if (per_sm < 1) per_sm = 1;
@@ -1447,6 +1535,18 @@ void launch_search_stage(const DevIndex& X, const BatchedParams& p, const Batche
     pw.blocks = blocks;
     pw.block_n = ctr + 13;
     pw.block_cap = block_cap;
+    BatchedTuning tl = t;
+    tl.split = 0;
+    tl.dir_split = 0;
+    if (X.text && p.fin) {
+      // the text on the device: one-row searches by comparison (the queue's
+      // counters take the place of the warp form's)
+      pw.rest_head = ctr + 0;
+      pw.fin_n = ctr + 9;
+      pw.rest_n = ctr + 10;
+      launch_text_search(X, pw, num_sms, s);
+      mark();
+    } else {
     if (t.dir_split == 2) {
       pw.dir_split = 2;
       launch_wave_search(X, pw, t, num_sms, s);
@@ -1457,9 +1557,6 @@ void launch_search_stage(const DevIndex& X, const BatchedParams& p, const Batche
       launch_wave_search(X, pw, t, num_sms, s);
     }
     BatchedParams pl = p;
-    BatchedTuning tl = t;
-    tl.split = 0;
-    tl.dir_split = 0;
     // reads above kWaveLongMin bases are at most 1/4000 of the bases: two
     // blocks per SM serve them, and an empty list costs a short launch
     tl.blocks_per_sm = 2;
@@ -1473,6 +1570,7 @@ void launch_search_stage(const DevIndex& X, const BatchedParams& p, const Batche
     // queued change points' branches, eight per change point; the blocks among
     // them join the block list, which the fused kernel's drain then empties
     launch_wave_branches(X, p, blocks, ctr + 13, block_cap, num_sms, s);
+    }
     BatchedParams pb = p;
     pb.spill = blocks;
     pb.spill_head = ctr + 12;

@@ -78,6 +78,17 @@ struct BatchedParams {
   SpillEntry* blocks = nullptr;
   unsigned int* block_n = nullptr;
   uint32_t block_cap = 0;
+  // text form (text_search.cu): the bases as 2-bit codes, 32 to a word, a word of
+  // padding before and two after; the queue of one-row searches (fin_n written, of
+  // fin_cap) and the chains its head leaves to the rest kernel (rest_n of them)
+  const uint64_t* packed = nullptr;
+  uint64_t packed_len = 0;  // bases it holds room for
+  uint4* fin = nullptr;
+  unsigned int* fin_n = nullptr;
+  uint32_t fin_cap = 0;
+  uint4* rest = nullptr;
+  unsigned int* rest_n = nullptr;
+  unsigned int* rest_head = nullptr;
   // fused form: when set, claim i runs read read_list[i], for i < *read_list_n
   const uint32_t* read_list = nullptr;
   const unsigned int* read_list_n = nullptr;
@@ -148,6 +159,12 @@ int wave_max_blocks_per_sm(const BatchedTuning& t);
 // entries are copied to `blocks` (count in *block_n) for the fused drain.
 void launch_wave_branches(const DevIndex& X, const BatchedParams& p, SpillEntry* blocks, unsigned int* block_n,
                           uint32_t block_cap, int num_sms, cudaStream_t s);
+// The search with the text on the device (text_search.cu); the blocks go to p.blocks.
+// Queues for n_reads reads: text_fin_cap entries of p.fin and 4 n_reads of p.rest, up to
+// kTextMaxReads reads (their counters and packed chunk states are below 2^28).
+constexpr size_t kTextMaxReads = 1u << 25;
+size_t text_fin_cap(size_t n_reads, int num_sms);
+void launch_text_search(const DevIndex& X, const BatchedParams& p, int num_sms, cudaStream_t s);
 // The whole search stage of a tuning: the search launches, then (after `mid`,
 // recorded when not null) the drain of queued change points.  `ctr` is the
 // counter block (16 words, zeroed); the warp-cooperative form also needs

@@ -197,6 +197,7 @@ Engine* engine_create(const HostIndex& h, int device, std::string* err) {
     en->X.comp[b] = a.comp[b];
     en->X.comp_packed |= (a.comp[b] & 3u) << (2 * b);
   }
+  en->X.comp_xor = a.comp[0];  // A-T and C-G pair the codes, so comp[b] = b ^ comp[0]
   en->X.ratio = h.S.ratio;
   en->X.ratio_shift = 0xFFFFFFFFu;
   for (uint32_t s = 0; s < 32; ++s)
@@ -216,7 +217,12 @@ Engine* engine_create(const HostIndex& h, int device, std::string* err) {
       engine_destroy(en);
       return nullptr;
     }
-    for (int d = 0; d < 2; ++d) {  // the row samples served only the derivation
+    if (build_full_rows(en, n_samples, &terr) != 0) {
+      *err = terr;
+      engine_destroy(en);
+      return nullptr;
+    }
+    for (int d = 0; d < 2; ++d) {  // the row samples served only the derivations
       cudaFree(en->d_S[d]);
       en->d_S[d] = nullptr;
       en->X.dir[d].S = nullptr;
@@ -239,7 +245,7 @@ void engine_release_workspace(Engine* e, uint64_t keep_n_cap) {
   DevBuf* bufs[] = {&e->seqs, &e->offs, &e->codes, &e->ok, &e->rs_count, &e->rs_trunc, &e->vecs, &e->slots,
                     &e->ovf, &e->ovf_count, &e->hit_off, &e->scan_part, &e->hits, &e->rows, &e->loc_off, &e->locs,
                     &e->b_res, &e->b_sorted, &e->b_spill, &e->b_arr, &e->b_seg, &e->b_rowhit, &e->b_long,
-                    &e->b_blocks, &e->b_bovf, &e->m_hitoff, &e->m_part, &e->m_offs, &e->m_rows, &e->m_pflag,
+                    &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_fin, &e->b_rest, &e->m_hitoff, &e->m_part, &e->m_offs, &e->m_rows, &e->m_pflag,
                     &e->m_rowoff, &e->m_nrec, &e->m_flags, &e->m_rec};
   for (DevBuf* b : bufs) {
     cudaFree(b->p);
@@ -266,6 +272,7 @@ void engine_destroy(Engine* e) {
     cudaFree(e->d_mark[d]);
     cudaFree(e->d_T[d]);
   }
+  free_full_rows(e);
   cudaFree(e->d_kar_off);
   cudaFree(e->d_kar_start);
   cudaFree(e->d_table);
@@ -275,7 +282,7 @@ void engine_destroy(Engine* e) {
   DevBuf* bufs[] = {&e->seqs, &e->offs, &e->codes, &e->ok, &e->rs_count, &e->rs_trunc, &e->vecs, &e->slots,
                     &e->ovf, &e->ovf_count, &e->hit_off, &e->scan_part, &e->hits, &e->rows, &e->loc_off, &e->locs,
                     &e->census, &e->b_ctr, &e->b_res, &e->b_sorted, &e->b_spill, &e->b_arr, &e->b_seg,
-                    &e->b_rowhit, &e->b_long, &e->b_blocks, &e->b_bovf, &e->m_hitoff, &e->m_part, &e->m_offs,
+                    &e->b_rowhit, &e->b_long, &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_fin, &e->b_rest, &e->m_hitoff, &e->m_part, &e->m_offs,
                     &e->m_rows, &e->m_pflag, &e->m_rowoff, &e->m_nrec, &e->m_flags, &e->m_rec};
   for (DevBuf* b : bufs) cudaFree(b->p);
   for (int i = 0; i <= kStageCount; ++i)
@@ -310,10 +317,9 @@ namespace {
 
 // Batched form: persistent search (+ drain of spilled change points), ordered
 // finalize, persistent locate.  Grows its pools and reruns on overflow.
-int run_batched(Engine* e, const uint8_t* d_offs_u8, const uint64_t* d_offs, uint32_t n, uint32_t max_results,
+int run_batched(Engine* e, uint64_t total_bases, const uint64_t* d_offs, uint32_t n, uint32_t max_results,
                 unsigned long long* census, size_t* n_hits_out, size_t* n_locs_out, float* t_search, float* t_final,
                 float* t_loc, std::string* err) {
-  (void)d_offs_u8;
   cudaStream_t s = e->stream;
   const size_t T = 2ull * n;
   // reads too long for a warp group buffer of the warp-cooperative form (at most one per kWaveLongMin bases)
@@ -322,6 +328,13 @@ int run_batched(Engine* e, const uint8_t* d_offs_u8, const uint64_t* d_offs, uin
       !ensure(e, e->hit_off, (T + 1) * 8) || !ensure(e, e->scan_part, scan_parts(T) * 8) ||
       !ensure(e, e->b_long, (size_t)long_cap * 4)) {
     *err = "out of device memory (batched counters)";
+    return -1;
+  }
+  const bool text = text_form(e, n);
+  const uint32_t fin_cap = text ? (uint32_t)text_fin_cap(n, e->num_sms) : 0u;
+  if (text && (!ensure(e, e->b_fin, (size_t)fin_cap * sizeof(uint4)) ||
+               !ensure(e, e->b_rest, 4 * (size_t)n * sizeof(uint4) + 16))) {
+    *err = "out of device memory (batched queues)";
     return -1;
   }
   if (e->b_res_cap < 4 * (size_t)n + 4096) e->b_res_cap = (uint32_t)std::min<size_t>(4 * (size_t)n + 4096, 0xFFFFFFF0u);
@@ -365,6 +378,13 @@ int run_batched(Engine* e, const uint8_t* d_offs_u8, const uint64_t* d_offs, uin
     p.rs_count = ptr<uint32_t>(e->b_arr);
     p.status = ctr + 4;
     p.census = census;
+    if (text) {
+      p.packed = ptr<uint64_t>(e->b_packed) + kPackedPad;
+      p.packed_len = total_bases;
+      p.fin = ptr<uint4>(e->b_fin);
+      p.fin_cap = fin_cap;
+      p.rest = ptr<uint4>(e->b_rest);
+    }
     cudaEventRecord(e->cev[0], s);
     launch_search_stage(e->X, p, e->tuning, e->num_sms, ctr, ptr<uint32_t>(e->b_long), long_cap,
                         wave ? ptr<SpillEntry>(e->b_blocks) : nullptr, wave ? e->b_spill_cap : 0u, e->dev_mid, false,
@@ -803,7 +823,15 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
   chunk = std::max<size_t>(1, std::min(chunk, std::max<size_t>(n_reads, 1)));
 
   cudaEventRecord(e->ev[0], s);
-  launch_encode(d_seqs, total_bases, d_offs, n, e->d_table, ptr<uint8_t>(e->codes), ptr<uint8_t>(e->ok), s);
+  uint64_t* packed = nullptr;
+  if (form == kFormBatched && text_form(e, n)) {
+    if (!ensure(e, e->b_packed, packed_words(total_bases) * 8)) {
+      *err = "out of device memory (packed reads)";
+      return -1;
+    }
+    packed = ptr<uint64_t>(e->b_packed) + kPackedPad;
+  }
+  launch_encode(d_seqs, total_bases, d_offs, n, e->d_table, ptr<uint8_t>(e->codes), ptr<uint8_t>(e->ok), s, packed);
   cudaEventRecord(e->ev[1], s);
 
   size_t n_hits = 0, n_locs = 0;
@@ -811,7 +839,7 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
   cudaEvent_t a = e->cev[0], b = e->cev[1], c = e->cev[2], d = e->cev[3];
   e->drain_ms = 0;
   if (form == kFormBatched) {
-    if (run_batched(e, d_seqs, d_offs, n, max_results, census, &n_hits, &n_locs, &t_search, &t_final, &t_loc, err) !=
+    if (run_batched(e, total_bases, d_offs, n, max_results, census, &n_hits, &n_locs, &t_search, &t_final, &t_loc, err) !=
         0)
       return -1;
     chunk = n_reads;  // skip the plain chunk loop

@@ -87,6 +87,10 @@ void engine_set_graph(Engine* e, int on);
 // begin with one lookup instead of their first L steps (0 = no table).
 constexpr int kDefaultKmer = 0;
 int engine_set_kmer(Engine* e, int L, std::string* err);
+// Use the whole suffix arrays and the text, where the index has them (1, the
+// default), or the sampled arrays (0); returns what is in use.
+int engine_set_full_rows(Engine* e, int on);
+int engine_full_rows(Engine* e);
 int engine_kmer(Engine* e);
 // Host-buffer batches of at least two chunks run pipelined; reads per chunk (0 automatic, SIZE_MAX off).
 void engine_set_pipeline_chunk(Engine* e, size_t reads);

@@ -44,12 +44,17 @@ struct GraphPlan {
   bool skip_locate = false;  // hits only (the alignment-list layer locates the rows it needs)
   uint32_t kmer_len = 0;     // start table captured with the kernels (length and address)
   const void* kmer0 = nullptr;
+  const void* text = nullptr;  // the packed text the kernels were captured with (null: sampled arrays only)
   // device buffers
   uint8_t* seqs = nullptr;
   uint64_t* offs = nullptr;
   uint32_t* hdr = nullptr;  // [0] reads in this batch, [1] max_results, [2..3] locate limit (u64),
                             // [4..5] source of the bases (u64, 0 = seqs), [6..7] its bytes
   uint8_t* codes = nullptr;
+  uint64_t* packed = nullptr;  // text form: packed codes (with padding), finish queue, rest list
+  uint4* fin = nullptr;
+  uint4* rest = nullptr;
+  uint32_t fin_cap = 0;
   uint8_t* ok = nullptr;
   unsigned* ctr = nullptr;  // as the direct form: [0] chains [1] spill head [2] spill tail [3] results [4] status
                             // [5..7] locate [8] phase-1 chains [9] forward-index reads [10] long reads
@@ -94,6 +99,9 @@ struct Engine {
   uint32_t* d_S[2] = {nullptr, nullptr};  // freed once the text-sampled arrays are built
   uint4* d_mark[2] = {nullptr, nullptr};
   uint32_t* d_T[2] = {nullptr, nullptr};
+  uint32_t* d_sa[2] = {nullptr, nullptr};  // whole suffix arrays, inverses and text (full_rows.cu), or null
+  uint32_t* d_isa[2] = {nullptr, nullptr};
+  uint64_t* d_text = nullptr;
   uint64_t* d_kar_off = nullptr;
   uint64_t* d_kar_start = nullptr;
   uint8_t* d_table = nullptr;
@@ -106,6 +114,7 @@ struct Engine {
       loc_off, locs, census;
   // batched form
   DevBuf b_ctr, b_res, b_sorted, b_spill, b_arr, b_seg, b_rowhit, b_long, b_blocks;
+  DevBuf b_packed, b_fin, b_rest;  // text form (text_search.cu)
   DevBuf b_bovf;  // block search: results past a block's slots, in chunks
   // alignment-list records (map_device.cu)
   DevBuf m_hitoff, m_part, m_offs, m_rows, m_pflag, m_rowoff, m_nrec, m_flags, m_rec;
@@ -181,6 +190,11 @@ inline T* ptr(DevBuf& b) {
 }
 
 
+// Whether a batch of n reads runs the search with the text on the device (text_search.cu).
+inline bool text_form(const Engine* e, uint64_t n) {
+  return e->tuning.split == 3 && e->X.text && n <= kTextMaxReads;
+}
+
 // Reads to the engine's device buffers, encoded (codes + validity flags);
 // offsets may start anywhere (map_device.cu).
 int upload_reads(Engine* e, const char* seqs, const uint64_t* offs, size_t n, std::string* err);
@@ -224,5 +238,10 @@ int run_graph_pipelined(Engine* e, const char* seqs, const uint64_t* offs, size_
 // The text-sampled suffix array of both directions (mark + T), derived from the
 // row samples already on the device (text_samples.cu); called once at open.
 int build_text_samples(Engine* en, const uint32_t n_samples[2], std::string* err);
+// The whole suffix arrays, their inverses and the text, where they fit the
+// device and are consistent with the index (full_rows.cu); called once at open,
+// while the row samples are on the device.  Not having them is no error.
+int build_full_rows(Engine* en, const uint32_t n_samples[2], std::string* err);
+void free_full_rows(Engine* en);
 
 }  // namespace hpgbwt

@@ -17,6 +17,10 @@
 //                        one entry per 64 rows: x = such rows before the block,
 //                        y/z = their bits for rows 0..31 / 32..63
 //   uint32 T[]           SA values of the text-sampled rows, in row order
+//   uint32 sa[], isa[]   the whole suffix array and its inverse, and
+//   uint64 text[]        the text as 2-bit codes, 32 to a word (one for both
+//                        directions): where the device has room for them
+//                        (full_rows.cu), 8.1 bytes per base and direction
 //
 // A locate walk (LF until a sampled row) therefore ends within ratio - 1 steps
 // instead of after a geometric number of them (text_samples.cu).
@@ -46,6 +50,8 @@ struct DevDir {
   const uint32_t* S;
   const uint4* mark;
   const uint32_t* T;
+  const uint32_t* sa;   // SA value of every row, or null
+  const uint32_t* isa;  // row of every SA value, or null
   uint32_t dollar;  // BWT row holding '$'
   uint32_t nblk;
 };
@@ -71,6 +77,10 @@ struct DevIndex {
   // no table.
   const uint2* kmer[2];
   uint32_t kmer_len;
+  // The text's codes, base i at bits 2(i & 31) of word i >> 5, two words of
+  // padding on either side; set when dir[].sa and dir[].isa are.
+  const uint64_t* text;
+  uint32_t comp_xor;  // comp[b] = b ^ comp_xor (the complement pairs the four codes)
 };
 
 constexpr uint32_t kErrWalk = 1u;
@@ -174,6 +184,8 @@ __device__ __forceinline__ DevDir dir_of(const DevIndex& X, uint32_t d) {
   D.S = d ? X.dir[1].S : X.dir[0].S;
   D.mark = d ? X.dir[1].mark : X.dir[0].mark;
   D.T = d ? X.dir[1].T : X.dir[0].T;
+  D.sa = d ? X.dir[1].sa : X.dir[0].sa;
+  D.isa = d ? X.dir[1].isa : X.dir[0].isa;
   D.dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
   D.nblk = d ? X.dir[1].nblk : X.dir[0].nblk;
   return D;
@@ -270,11 +282,24 @@ __device__ __forceinline__ bool text_sampled(const uint4& m, uint32_t i, uint32_
   return (w >> (r & 31)) & 1u;
 }
 
-// getScompValue (csafm.h:208-235): walk LF to a sampled row, add the steps;
+// One gather from the whole suffix array or its inverse: no neighbour of the
+// entry is wanted, so the line is not kept in L1.
+__device__ __forceinline__ uint32_t load_row_word(const uint32_t* p) {
+  uint32_t v;
+  asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+// getScompValue (csafm.h:208-235).  With the whole suffix array on the device,
+// one gather; else walk LF to a sampled row and add the steps;
 // here to a text-sampled row, so at most ratio - 1 steps (a longer walk means
 // a corrupt index: the error bit is set and slot 0 taken).  The row's mark
 // entry and block are fetched together; `sectors` counts them and the sample.
 __device__ __forceinline__ uint32_t sa_value(const DevIndex& X, const DevDir& D, uint32_t m, uint32_t* sectors) {
+  if (D.sa) {
+    *sectors = 1;
+    return load_row_word(D.sa + m);
+  }
   uint32_t i = m, j = 0, slot = 0;
   for (;;) {
     uint32_t cnt[4];

@@ -71,7 +71,7 @@ bool same_settings(const GraphPlan* g, const Engine* e) {
          a.batch_idle == b.batch_idle && a.group == b.group &&
          g->load_mode == e->X.load_mode &&
          g->census == e->census_on && g->skip_locate == e->skip_locate && g->kmer_len == e->X.kmer_len &&
-         g->kmer0 == (const void*)e->X.kmer[0];
+         g->kmer0 == (const void*)e->X.kmer[0] && g->text == (const void*)e->X.text;
 }
 
 void record(cudaEvent_t ev, cudaStream_t s) { cudaEventRecordWithFlags(ev, s, cudaEventRecordExternal); }
@@ -80,6 +80,8 @@ void record(cudaEvent_t ev, cudaStream_t s) { cudaEventRecordWithFlags(ev, s, cu
 int capture(Engine* e, GraphPlan* g, std::string* err) {
   const size_t T = 2ull * g->n_cap;
   const size_t parts = std::max(scan_parts(T), scan_parts(g->res_cap));
+  const bool text = text_form(e, g->n_cap);
+  g->fin_cap = text ? (uint32_t)text_fin_cap(g->n_cap, e->num_sms) : 0u;
   if (!grab(g, &g->seqs, g->bases_cap + 64) || !grab(g, &g->offs, ((size_t)g->n_cap + 1) * 8) ||
       !grab(g, &g->hdr, 32) || !grab(g, &g->codes, g->bases_cap + 64) || !grab(g, &g->ok, (size_t)g->n_cap + 16) ||
       !grab(g, &g->ctr, 64) || !grab(g, &g->arr, T * 4 + 16) || !grab(g, &g->seg, (T + 1) * 8) ||
@@ -89,10 +91,13 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
       !grab(g, &g->spill, (size_t)g->spill_cap * sizeof(SpillEntry)) ||
       !grab(g, &g->hits, ((size_t)g->res_cap + 1) * sizeof(hpg_hit_t)) ||
       !grab(g, &g->rows, ((size_t)g->res_cap + 1) * 4) || !grab(g, &g->loc_off, ((size_t)g->res_cap + 2) * 8) ||
-      !grab(g, &g->items, (g->locs_cap + 1) * locate_row_item_bytes()) ||
+      (!e->X.text && !grab(g, &g->items, (g->locs_cap + 1) * locate_row_item_bytes())) ||
       !grab(g, &g->locs, (g->locs_cap + 1) * sizeof(hpg_loc_t)) || !grab(g, &g->census_d, 16) ||
       !grab(g, &g->long_list, (size_t)g->long_cap * 4) || !grab(g, &g->longs, long_lists_cap(g->res_cap) * 4) ||
       (g->tuning.split == 3 && !grab(g, &g->blocks, (size_t)g->spill_cap * sizeof(SpillEntry))) ||
+      (text && (!grab(g, &g->packed, packed_words(g->bases_cap) * 8) ||
+                !grab(g, &g->fin, (size_t)g->fin_cap * sizeof(uint4)) ||
+                !grab(g, &g->rest, 4ull * g->n_cap * sizeof(uint4)))) ||
       !grab(g, &g->summary_d, 64)) {
     *err = "out of device memory (graph plan)";
     return -1;
@@ -113,7 +118,7 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
   cudaMemsetAsync(g->arr, 0, T * 4, s);
   if (census) cudaMemsetAsync(census, 0, 8, s);
   launch_encode_dev(g->seqs, g->bases_cap, g->offs, g->hdr, g->n_cap, e->d_table, g->codes, g->ok, s,
-                    reinterpret_cast<const uint64_t*>(g->hdr + 4));
+                    reinterpret_cast<const uint64_t*>(g->hdr + 4), text ? g->packed + kPackedPad : nullptr);
   launch_check_offsets(g->offs, g->hdr, g->n_cap, g->bases_cap, g->ok, status, s);
   record(g->ev[1], s);
 
@@ -140,6 +145,13 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
   p.rs_count = g->arr;
   p.status = status;
   p.census = census;
+  if (text) {
+    p.packed = g->packed + kPackedPad;
+    p.packed_len = g->bases_cap;
+    p.fin = g->fin;
+    p.fin_cap = g->fin_cap;
+    p.rest = g->rest;
+  }
   launch_search_stage(e->X, p, g->tuning, e->num_sms, ctr, g->long_list, g->long_cap, g->blocks,
                       g->blocks ? g->spill_cap : 0u, g->ev[2], true, s);
   record(g->ev[3], s);
@@ -278,6 +290,7 @@ GraphPlan* graph_plan_for(Engine* e, uint32_t n, uint64_t total, const GraphPlan
   g->skip_locate = e->skip_locate;
   g->kmer_len = e->X.kmer_len;
   g->kmer0 = e->X.kmer[0];
+  g->text = e->X.text;
   if (old) {  // no stream may still read the old plan's buffers
     cudaStreamSynchronize(e->stream);
     for (cudaStream_t x : e->xs)

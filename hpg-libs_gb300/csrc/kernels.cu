@@ -30,7 +30,8 @@ inline unsigned grid_for(size_t n, int tpb) { return (unsigned)((n + tpb - 1) / 
 // is offs[n] (graph replays); the grid is then sized for the capacity.
 __global__ void encode_kernel(const uint8_t* __restrict__ ascii, uint64_t total, const uint64_t* __restrict__ offs,
                               uint32_t n_reads, const uint8_t* __restrict__ table, uint8_t* __restrict__ codes,
-                              uint8_t* __restrict__ ok, const uint32_t* n_dev, const uint64_t* src_dev) {
+                              uint8_t* __restrict__ ok, const uint32_t* n_dev, const uint64_t* src_dev,
+                              uint32_t* __restrict__ packed) {
   if (n_dev) {
     n_reads = *n_dev;
     const uint64_t t = offs[n_reads];
@@ -66,6 +67,12 @@ __global__ void encode_kernel(const uint8_t* __restrict__ ascii, uint64_t total,
       *reinterpret_cast<uint4*>(codes + b) = *reinterpret_cast<const uint4*>(out);
     } else {
       for (uint64_t i = 0; i < m; ++i) codes[b + i] = out[i];
+    }
+    if (packed) {
+      uint32_t w = 0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) w |= (i < (int)m ? out[i] & 3u : 0u) << (2 * i);
+      packed[c] = w;
     }
     while (bad) {
       const int i = __ffs(bad) - 1;
@@ -415,14 +422,15 @@ __global__ void __launch_bounds__(kTpb)
 }  // namespace
 
 void launch_encode(const uint8_t* ascii, uint64_t total, const uint64_t* offs, uint32_t n_reads,
-                   const uint8_t* d_table, uint8_t* codes, uint8_t* ok, cudaStream_t s) {
+                   const uint8_t* d_table, uint8_t* codes, uint8_t* ok, cudaStream_t s, uint64_t* packed) {
   if (!n_reads) return;
   cudaMemsetAsync(ok, 1, n_reads, s);
   if (!total) return;
   const uint64_t chunks = (total + 15) / 16;
   const unsigned grid = (unsigned)(chunks < 152ull * 32 * 8 ? (chunks + 255) / 256 : 152ull * 32);
   count_launches(1);
-  encode_kernel<<<grid, 256, 0, s>>>(ascii, total, offs, n_reads, d_table, codes, ok, nullptr, nullptr);
+  encode_kernel<<<grid, 256, 0, s>>>(ascii, total, offs, n_reads, d_table, codes, ok, nullptr, nullptr,
+                                       reinterpret_cast<uint32_t*>(packed));
 }
 
 namespace {
@@ -454,12 +462,13 @@ void launch_check_offsets(const uint64_t* offs, const uint32_t* n_dev, uint32_t 
 
 void launch_encode_dev(const uint8_t* ascii, uint64_t bases_cap, const uint64_t* offs, const uint32_t* n_dev,
                        uint32_t n_cap, const uint8_t* d_table, uint8_t* codes, uint8_t* ok, cudaStream_t s,
-                       const uint64_t* src_dev) {
+                       const uint64_t* src_dev, uint64_t* packed) {
   cudaMemsetAsync(ok, 1, n_cap, s);
   const uint64_t chunks = (bases_cap + 15) / 16;
   const unsigned grid = (unsigned)(chunks < 152ull * 32 * 8 ? (chunks + 255) / 256 : 152ull * 32);
   count_launches(1);
-  encode_kernel<<<grid ? grid : 1, 256, 0, s>>>(ascii, bases_cap, offs, 0, d_table, codes, ok, n_dev, src_dev);
+  encode_kernel<<<grid ? grid : 1, 256, 0, s>>>(ascii, bases_cap, offs, 0, d_table, codes, ok, n_dev, src_dev,
+                                                   reinterpret_cast<uint32_t*>(packed));
 }
 
 void launch_exact(const DevIndex& X, const uint8_t* codes, const uint64_t* offs, const uint8_t* ok, uint32_t r0,

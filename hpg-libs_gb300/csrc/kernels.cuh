@@ -24,9 +24,10 @@ unsigned long long launch_count();
 void count_launches(unsigned n);
 void uncount_launches(unsigned long long n);  // launches recorded while capturing a graph
 
-// ASCII -> 2-bit codes (0xFF outside the alphabet) and a per-read validity flag.
+// ASCII -> 2-bit codes (0xFF outside the alphabet) and a per-read validity flag; with
+// `packed` also the codes 32 to a word, base i at bits 2(i & 31) of word i >> 5.
 void launch_encode(const uint8_t* ascii, uint64_t total, const uint64_t* offs, uint32_t n_reads,
-                   const uint8_t* d_table, uint8_t* codes, uint8_t* ok, cudaStream_t s);
+                   const uint8_t* d_table, uint8_t* codes, uint8_t* ok, cudaStream_t s, uint64_t* packed = nullptr);
 
 // Graph form of launch_encode: n_reads read from device memory, byte count
 // offs[n] (at most bases_cap), flags cleared over n_cap reads.  src_dev (device
@@ -34,7 +35,10 @@ void launch_encode(const uint8_t* ascii, uint64_t total, const uint64_t* offs, u
 // pointer is not 0 (a caller's device buffer, read in place), else `ascii`.
 void launch_encode_dev(const uint8_t* ascii, uint64_t bases_cap, const uint64_t* offs, const uint32_t* n_dev,
                        uint32_t n_cap, const uint8_t* d_table, uint8_t* codes, uint8_t* ok, cudaStream_t s,
-                       const uint64_t* src_dev = nullptr);
+                       const uint64_t* src_dev = nullptr, uint64_t* packed = nullptr);
+// Words to allocate for the packed codes of `total` bases, and the words of padding before the first.
+constexpr size_t kPackedPad = 2;
+constexpr size_t packed_words(uint64_t total) { return total / 32 + 1 + 2 * kPackedPad; }
 
 // Graph form: reads whose offsets are decreasing, longer than 32767 bases or
 // past the staged bases get ok = 0 and set bit 8 of *status.

@@ -148,6 +148,8 @@ def load() -> ctypes.CDLL:
     lib.bwt_gpu_graph.argtypes = [vp]
     lib.bwt_gpu_set_pipeline_chunk.argtypes = [vp, sz]
     lib.bwt_gpu_set_start_table.argtypes = [vp, ctypes.c_int]
+    lib.bwt_gpu_set_full_rows.argtypes = [vp, ctypes.c_int]
+    lib.bwt_gpu_full_rows.argtypes = [vp]
     lib.bwt_gpu_set_direction_split.argtypes = [vp, ctypes.c_int]
     lib.bwt_gpu_direction_split.argtypes = [vp]
     lib.bwt_gpu_map_device_seconds.restype = ctypes.c_double
@@ -509,6 +511,13 @@ class GpuIndex:
 
     def start_table(self) -> int:
         return int(self.lib.bwt_gpu_start_table(self.handle))
+
+    def set_full_rows(self, on: bool) -> bool:
+        """Whole suffix arrays and text where the index has them (default), or the sampled arrays; which are in use."""
+        return bool(self.lib.bwt_gpu_set_full_rows(self.handle, 1 if on else 0))
+
+    def full_rows(self) -> bool:
+        return bool(self.lib.bwt_gpu_full_rows(self.handle))
 
     def set_pipeline_chunk(self, reads: int) -> None:
         """Reads per chunk of pipelined host batches (0 or -1: not pipelined, the default)."""
