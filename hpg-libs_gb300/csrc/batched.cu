@@ -1538,12 +1538,14 @@ void launch_search_stage(const DevIndex& X, const BatchedParams& p, const Batche
     BatchedTuning tl = t;
     tl.split = 0;
     tl.dir_split = 0;
-    if (X.text && p.fin) {
+    if (X.text && p.walk) {
       // the text on the device: one-row searches by comparison (the queue's
       // counters take the place of the warp form's)
       pw.rest_head = ctr + 0;
-      pw.fin_n = ctr + 9;
+      pw.rows_head = ctr + 8;
+      pw.walk_n = ctr + 9;
       pw.rest_n = ctr + 10;
+      pw.rows_n = ctr + 11;
       launch_text_search(X, pw, num_sms, s);
       mark();
     } else {

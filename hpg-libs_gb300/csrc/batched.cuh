@@ -78,17 +78,21 @@ struct BatchedParams {
   SpillEntry* blocks = nullptr;
   unsigned int* block_n = nullptr;
   uint32_t block_cap = 0;
-  // text form (text_search.cu): the bases as 2-bit codes, 32 to a word, a word of
-  // padding before and two after; the queue of one-row searches (fin_n written, of
-  // fin_cap) and the chains its head leaves to the rest kernel (rest_n of them)
+  // text form (text_search.cu): the bases as 2-bit codes, 32 to a word, padded on both
+  // sides; per chain the alignment of a one-row chain (4 x n_reads words); the queue of
+  // chains of a few rows, the list of those of more, and the queue of one-row walks
   const uint64_t* packed = nullptr;
   uint64_t packed_len = 0;  // bases it holds room for
-  uint4* fin = nullptr;
-  unsigned int* fin_n = nullptr;
-  uint32_t fin_cap = 0;
+  uint32_t* diag = nullptr;
+  uint4* rows = nullptr;    // 4 x n_reads, as rest
+  unsigned int* rows_n = nullptr;
+  unsigned int* rows_head = nullptr;
   uint4* rest = nullptr;
   unsigned int* rest_n = nullptr;
   unsigned int* rest_head = nullptr;
+  uint4* walk = nullptr;
+  unsigned int* walk_n = nullptr;
+  uint32_t walk_cap = 0;
   // fused form: when set, claim i runs read read_list[i], for i < *read_list_n
   const uint32_t* read_list = nullptr;
   const unsigned int* read_list_n = nullptr;
@@ -160,10 +164,11 @@ int wave_max_blocks_per_sm(const BatchedTuning& t);
 void launch_wave_branches(const DevIndex& X, const BatchedParams& p, SpillEntry* blocks, unsigned int* block_n,
                           uint32_t block_cap, int num_sms, cudaStream_t s);
 // The search with the text on the device (text_search.cu); the blocks go to p.blocks.
-// Queues for n_reads reads: text_fin_cap entries of p.fin and 4 n_reads of p.rest, up to
-// kTextMaxReads reads (their counters and packed chunk states are below 2^28).
+// Up to kTextMaxReads reads a batch (the queues' counters and packed chunk states stay below
+// 2^28); text_queue_bytes is what its buffers take for a capacity of n_reads, set by text_queues.
 constexpr size_t kTextMaxReads = 1u << 25;
-size_t text_fin_cap(size_t n_reads, int num_sms);
+size_t text_queue_bytes(size_t n_reads, int num_sms);
+void text_queues(BatchedParams& p, void* buffer, size_t n_reads, int num_sms);
 void launch_text_search(const DevIndex& X, const BatchedParams& p, int num_sms, cudaStream_t s);
 // The whole search stage of a tuning: the search launches, then (after `mid`,
 // recorded when not null) the drain of queued change points.  `ctr` is the

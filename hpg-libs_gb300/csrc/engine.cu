@@ -245,7 +245,7 @@ void engine_release_workspace(Engine* e, uint64_t keep_n_cap) {
   DevBuf* bufs[] = {&e->seqs, &e->offs, &e->codes, &e->ok, &e->rs_count, &e->rs_trunc, &e->vecs, &e->slots,
                     &e->ovf, &e->ovf_count, &e->hit_off, &e->scan_part, &e->hits, &e->rows, &e->loc_off, &e->locs,
                     &e->b_res, &e->b_sorted, &e->b_spill, &e->b_arr, &e->b_seg, &e->b_rowhit, &e->b_long,
-                    &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_fin, &e->b_rest, &e->m_hitoff, &e->m_part, &e->m_offs, &e->m_rows, &e->m_pflag,
+                    &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->m_hitoff, &e->m_part, &e->m_offs, &e->m_rows, &e->m_pflag,
                     &e->m_rowoff, &e->m_nrec, &e->m_flags, &e->m_rec};
   for (DevBuf* b : bufs) {
     cudaFree(b->p);
@@ -282,7 +282,7 @@ void engine_destroy(Engine* e) {
   DevBuf* bufs[] = {&e->seqs, &e->offs, &e->codes, &e->ok, &e->rs_count, &e->rs_trunc, &e->vecs, &e->slots,
                     &e->ovf, &e->ovf_count, &e->hit_off, &e->scan_part, &e->hits, &e->rows, &e->loc_off, &e->locs,
                     &e->census, &e->b_ctr, &e->b_res, &e->b_sorted, &e->b_spill, &e->b_arr, &e->b_seg,
-                    &e->b_rowhit, &e->b_long, &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_fin, &e->b_rest, &e->m_hitoff, &e->m_part, &e->m_offs,
+                    &e->b_rowhit, &e->b_long, &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->m_hitoff, &e->m_part, &e->m_offs,
                     &e->m_rows, &e->m_pflag, &e->m_rowoff, &e->m_nrec, &e->m_flags, &e->m_rec};
   for (DevBuf* b : bufs) cudaFree(b->p);
   for (int i = 0; i <= kStageCount; ++i)
@@ -331,9 +331,7 @@ int run_batched(Engine* e, uint64_t total_bases, const uint64_t* d_offs, uint32_
     return -1;
   }
   const bool text = text_form(e, n);
-  const uint32_t fin_cap = text ? (uint32_t)text_fin_cap(n, e->num_sms) : 0u;
-  if (text && (!ensure(e, e->b_fin, (size_t)fin_cap * sizeof(uint4)) ||
-               !ensure(e, e->b_rest, 4 * (size_t)n * sizeof(uint4) + 16))) {
+  if (text && !ensure(e, e->b_text, text_queue_bytes(n, e->num_sms))) {
     *err = "out of device memory (batched queues)";
     return -1;
   }
@@ -381,9 +379,7 @@ int run_batched(Engine* e, uint64_t total_bases, const uint64_t* d_offs, uint32_
     if (text) {
       p.packed = ptr<uint64_t>(e->b_packed) + kPackedPad;
       p.packed_len = total_bases;
-      p.fin = ptr<uint4>(e->b_fin);
-      p.fin_cap = fin_cap;
-      p.rest = ptr<uint4>(e->b_rest);
+      text_queues(p, e->b_text.p, n, e->num_sms);
     }
     cudaEventRecord(e->cev[0], s);
     launch_search_stage(e->X, p, e->tuning, e->num_sms, ctr, ptr<uint32_t>(e->b_long), long_cap,

@@ -51,10 +51,8 @@ struct GraphPlan {
   uint32_t* hdr = nullptr;  // [0] reads in this batch, [1] max_results, [2..3] locate limit (u64),
                             // [4..5] source of the bases (u64, 0 = seqs), [6..7] its bytes
   uint8_t* codes = nullptr;
-  uint64_t* packed = nullptr;  // text form: packed codes (with padding), finish queue, rest list
-  uint4* fin = nullptr;
-  uint4* rest = nullptr;
-  uint32_t fin_cap = 0;
+  uint64_t* packed = nullptr;  // text form: packed codes (with padding) and its queues
+  uint8_t* queues = nullptr;
   uint8_t* ok = nullptr;
   unsigned* ctr = nullptr;  // as the direct form: [0] chains [1] spill head [2] spill tail [3] results [4] status
                             // [5..7] locate [8] phase-1 chains [9] forward-index reads [10] long reads
@@ -102,6 +100,7 @@ struct Engine {
   uint32_t* d_sa[2] = {nullptr, nullptr};  // whole suffix arrays, inverses and text (full_rows.cu), or null
   uint32_t* d_isa[2] = {nullptr, nullptr};
   uint64_t* d_text = nullptr;
+  uint2* d_tmer[2] = {nullptr, nullptr};  // wide start tables, or null
   uint64_t* d_kar_off = nullptr;
   uint64_t* d_kar_start = nullptr;
   uint8_t* d_table = nullptr;
@@ -114,7 +113,7 @@ struct Engine {
       loc_off, locs, census;
   // batched form
   DevBuf b_ctr, b_res, b_sorted, b_spill, b_arr, b_seg, b_rowhit, b_long, b_blocks;
-  DevBuf b_packed, b_fin, b_rest;  // text form (text_search.cu)
+  DevBuf b_packed, b_text;  // text form (text_search.cu)
   DevBuf b_bovf;  // block search: results past a block's slots, in chunks
   // alignment-list records (map_device.cu)
   DevBuf m_hitoff, m_part, m_offs, m_rows, m_pflag, m_rowoff, m_nrec, m_flags, m_rec;

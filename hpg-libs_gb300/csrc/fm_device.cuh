@@ -80,6 +80,9 @@ struct DevIndex {
   // The text's codes, base i at bits 2(i & 31) of word i >> 5, two words of
   // padding on either side; set when dir[].sa and dir[].isa are.
   const uint64_t* text;
+  // Start table of the search with the text (full_rows.cu), as kmer; set when text is.
+  const uint2* tmer[2];
+  uint32_t tmer_len;
   uint32_t comp_xor;  // comp[b] = b ^ comp_xor (the complement pairs the four codes)
 };
 

@@ -8,10 +8,15 @@
 // located by one gather, and once a search's interval is a single row the rest
 // of the match is a comparison of the read with the text: SA of the row, the
 // text (25 bytes per 100 bases), SA^-1 of the position reached.  16.25 bytes
-// per base for both directions: 1.6 GB at 100 Mbp, 50 GB at 3.1 Gbp of the
-// device's 284 GB.  Measured on 2M x 100 bp reads, 100 Mbp: the locate stage
+// per base for both directions, and a start table of log4(n) symbols, 14 at
+// most, per direction (8 bytes an entry): 2.7 GB at 100 Mbp, 54 GB at 3.1 Gbp of
+// the device's 284 GB.  Measured on 2M x 100 bp reads, 100 Mbp: the locate stage
 // takes 406 us per 2M rows with LF walks (16 sectors a row), 80 us with the gather;
-// the search 3704 us with rank steps only, 1165 us with the text.
+// the search 3704 us with rank steps only, 880 us with the text.
+//
+// Table length (search stage there / on 2M x 150 bp, 600 Mbp): 11 symbols 903 /
+// 7783 us, 12: 903 / 7570, 13: 891 / 7550, 14: 864 / 7392; a table longer than
+// log4(n) is mostly empty intervals and four times the memory.
 //
 // They are kept when they take at most a quarter of the device's free memory
 // (several indexes and batch workspaces share the rest) and the derivation
@@ -99,6 +104,13 @@ __global__ void full_rows_kernel(DevIndex X, uint32_t d, uint32_t n_samples, uin
 
 }  // namespace
 
+// Symbols of the start table of the search with the text.
+uint32_t tmer_symbols(const Engine* en) {
+  uint32_t L = 1;
+  while (L < 14 && (1ull << (2 * (L + 1))) <= en->X.walk_mod) ++L;
+  return L;
+}
+
 constexpr size_t kTextPad = 2;  // words of padding on either side of the text
 
 void free_full_rows(Engine* en) {
@@ -106,6 +118,10 @@ void free_full_rows(Engine* en) {
     cudaFree(en->d_sa[d]);
     cudaFree(en->d_isa[d]);
     en->d_sa[d] = en->d_isa[d] = nullptr;
+  }
+  for (uint2*& m : en->d_tmer) {
+    cudaFree(m);
+    m = nullptr;
   }
   cudaFree(en->d_text);
   en->d_text = nullptr;
@@ -118,7 +134,9 @@ int engine_set_full_rows(Engine* en, int on) {
   for (int d = 0; d < 2; ++d) {
     en->X.dir[d].sa = use ? en->d_sa[d] : nullptr;
     en->X.dir[d].isa = use ? en->d_isa[d] : nullptr;
+    en->X.tmer[d] = use ? en->d_tmer[d] : nullptr;
   }
+  en->X.tmer_len = use ? tmer_symbols(en) : 0;
   en->X.text = use ? en->d_text + kTextPad : nullptr;
   return use ? 1 : 0;
 }
@@ -128,7 +146,9 @@ int engine_full_rows(Engine* en) { return en->X.text ? 1 : 0; }
 int build_full_rows(Engine* en, const uint32_t n_samples[2], std::string* err) {
   const size_t n_rows = en->X.walk_mod;
   const size_t words = n_rows / 32 + 1 + 2 * kTextPad;
-  const size_t need = 4 * n_rows * sizeof(uint32_t) + words * sizeof(uint64_t);
+  const uint32_t L = tmer_symbols(en);
+  const size_t tmer_bytes = ((size_t)1 << (2 * L)) * sizeof(uint2);
+  const size_t need = 4 * n_rows * sizeof(uint32_t) + words * sizeof(uint64_t) + 2 * tmer_bytes;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || need > free_b / 4) {
     cudaGetLastError();
@@ -137,6 +157,7 @@ int build_full_rows(Engine* en, const uint32_t n_samples[2], std::string* err) {
   bool ok = cudaMalloc(&en->d_text, words * sizeof(uint64_t)) == cudaSuccess;
   for (int d = 0; d < 2 && ok; ++d)
     ok = cudaMalloc(&en->d_sa[d], n_rows * 4) == cudaSuccess && cudaMalloc(&en->d_isa[d], n_rows * 4) == cudaSuccess;
+  for (int d = 0; d < 2 && ok; ++d) ok = cudaMalloc(&en->d_tmer[d], tmer_bytes) == cudaSuccess;
   unsigned long long* bad = nullptr;
   ok = ok && cudaMalloc(&bad, 4 * sizeof(*bad)) == cudaSuccess;
   if (!ok) {
@@ -156,7 +177,7 @@ int build_full_rows(Engine* en, const uint32_t n_samples[2], std::string* err) {
                                                          en->d_text + kTextPad, bad + 2 * d);
   }
   unsigned long long h[4] = {0, 0, 0, 0};
-  const cudaError_t ce = cudaMemcpy(h, bad, sizeof h, cudaMemcpyDeviceToHost);
+  cudaError_t ce = cudaMemcpy(h, bad, sizeof h, cudaMemcpyDeviceToHost);
   cudaFree(bad);
   if (ce != cudaSuccess) {
     *err = std::string("full suffix arrays: ") + cudaGetErrorString(ce);
@@ -165,6 +186,11 @@ int build_full_rows(Engine* en, const uint32_t n_samples[2], std::string* err) {
   if (h[0] || h[2] || h[1] != n_rows || h[3] != n_rows) {  // not consistent: the sampled arrays serve this index
     free_full_rows(en);
     return 0;
+  }
+  for (uint32_t d = 0; d < 2; ++d) launch_build_kmer(en->X, d, L, en->d_tmer[d], 0);
+  if ((ce = cudaDeviceSynchronize()) != cudaSuccess) {
+    *err = std::string("full suffix arrays: ") + cudaGetErrorString(ce);
+    return -1;
   }
   engine_set_full_rows(en, 1);
   return 0;

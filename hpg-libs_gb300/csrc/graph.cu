@@ -81,7 +81,6 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
   const size_t T = 2ull * g->n_cap;
   const size_t parts = std::max(scan_parts(T), scan_parts(g->res_cap));
   const bool text = text_form(e, g->n_cap);
-  g->fin_cap = text ? (uint32_t)text_fin_cap(g->n_cap, e->num_sms) : 0u;
   if (!grab(g, &g->seqs, g->bases_cap + 64) || !grab(g, &g->offs, ((size_t)g->n_cap + 1) * 8) ||
       !grab(g, &g->hdr, 32) || !grab(g, &g->codes, g->bases_cap + 64) || !grab(g, &g->ok, (size_t)g->n_cap + 16) ||
       !grab(g, &g->ctr, 64) || !grab(g, &g->arr, T * 4 + 16) || !grab(g, &g->seg, (T + 1) * 8) ||
@@ -96,8 +95,7 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
       !grab(g, &g->long_list, (size_t)g->long_cap * 4) || !grab(g, &g->longs, long_lists_cap(g->res_cap) * 4) ||
       (g->tuning.split == 3 && !grab(g, &g->blocks, (size_t)g->spill_cap * sizeof(SpillEntry))) ||
       (text && (!grab(g, &g->packed, packed_words(g->bases_cap) * 8) ||
-                !grab(g, &g->fin, (size_t)g->fin_cap * sizeof(uint4)) ||
-                !grab(g, &g->rest, 4ull * g->n_cap * sizeof(uint4)))) ||
+                !grab(g, &g->queues, text_queue_bytes(g->n_cap, e->num_sms)))) ||
       !grab(g, &g->summary_d, 64)) {
     *err = "out of device memory (graph plan)";
     return -1;
@@ -148,9 +146,7 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
   if (text) {
     p.packed = g->packed + kPackedPad;
     p.packed_len = g->bases_cap;
-    p.fin = g->fin;
-    p.fin_cap = g->fin_cap;
-    p.rest = g->rest;
+    text_queues(p, g->queues, g->n_cap, e->num_sms);
   }
   launch_search_stage(e->X, p, g->tuning, e->num_sms, ctr, g->long_list, g->long_cap, g->blocks,
                       g->blocks ? g->spill_cap : 0u, g->ev[2], true, s);

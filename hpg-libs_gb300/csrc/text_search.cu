@@ -12,16 +12,22 @@
 // whose interval is one row are comparisons too, and only three of them can
 // match: the deletion, and insertion and mismatch of the one base the text has.
 //
-// Three launches:
+// Launches:
 //   text_head_kernel    a thread per chain: start table, then rank steps until
-//                       the interval is empty, has stayed one row for a step
-//                       (-> finish queue), or is still several rows where the
-//                       helper branches or after kHeadSymbols (-> rest list)
-//   text_rest_kernel    persistent warps: the chains still several rows wide and
-//                       their change points, one rank step per lane and
-//                       iteration; what narrows to one row -> finish queue
-//   text_finish_kernel  a thread per queued one-row search: SA, comparison,
-//                       inverse SA, hits
+//                       the interval is empty or has stayed one row for a step
+//                       (its SA value, as an alignment, to `diag`), or is still
+//                       several rows where the helper branches or after
+//                       kHeadSteps steps (up to 32 rows -> row queue, else rest list)
+//   text_read_kernel    a thread per read: its one-row chains compared with the
+//                       text, hits
+//   text_wide_kernel    persistent lanes: the chains more than 32 rows wide until
+//                       they are not (-> row queue); their change points queued
+//   text_branch_kernel  persistent lanes: a queued change point's continuations,
+//                       one rank step per lane and iteration; walks that narrow
+//                       to one row -> walk queue
+//   text_rows_kernel    a lane per row of the queued chains, all their change
+//                       points from one comparison of each row's text
+//   text_walk_kernel    a thread per queued walk
 //
 // Positions are counted in search order: symbol i of a chain is W[len-1-i]
 // (backward) or W[i] (forward), complemented on the '-' strand, so both
@@ -29,13 +35,15 @@
 // (backward) or t - 1 (forward) for an interval of t matched symbols, and its
 // order key's t field is len - t in both.
 //
-// Bound by random 32-byte sectors, as rank walks are, but about 26 a read of
-// 100 bp at 100 Mbp against 180.  Search stage there on 2M reads 3704 -> 1165 us;
-// 4M reads of 36-250 bp 12570 -> 2333 us; 1000 reads of 50-300 bp 510 -> 98 us (a
-// chain is some 8 dependent accesses, whatever its length); 2M x 150 bp on a
-// 600 Mbp genome with 45 % repeats 9809 -> 8390 us, most of it the rest kernel's
-// change points.  Indexes without the arrays, and batches above kTextMaxReads
-// (the queues' counters), take the warp-cooperative form (wave.cu).
+// Bound by random sectors, as rank walks are, but about 20 a read of 100 bp at 100
+// Mbp against 180, and by the latency of some 8 dependent accesses a chain, whatever
+// the read's length.  Search stage, rank walks (wave.cu) -> here:
+//   2M x 100 bp, 100 Mbp                          3704 ->  880 us
+//   4M x 36-250 bp, 100 Mbp                      12570 -> 1965 us
+//   1000 x 50-300 bp, 100 Mbp                      510 ->   92 us
+//   2M x 150 bp, 600 Mbp with 45 % repeats        9809 -> 4087 us
+// Indexes without the arrays, and batches above kTextMaxReads (the queues'
+// counters), take the warp-cooperative form.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -50,12 +58,18 @@ namespace {
 
 using namespace bdev;
 
-constexpr int kHeadTpb = 256, kFinishTpb = 256, kRestTpb = 128;
-constexpr int kRestWarps = kRestTpb / 32;
-constexpr uint32_t kRestStack = 64;   // change points per warp
-constexpr uint32_t kHeadSymbols = 28; // symbols a head matches at most (it holds 32)
+constexpr int kHeadTpb = 256, kReadTpb = 256, kWalkTpb = 256, kWideTpb = 128, kRowsTpb = 128;
+constexpr int kRowsWarps = kRowsTpb / 32;
+// Rank steps of a head past its start table: nearly all chains are empty or one row
+// by then (search stage at 4 / 5 / 6 / 8 steps, 2M x 100 bp, 100 Mbp: 899 / 884 / 891 /
+// 901 us; the lanes of the others, some in most warps, would hold their warps longer).
+constexpr int kHeadSteps = 6;
+constexpr uint32_t kRows = 32;       // rows of a chain in the row queue at most
+// A chain's entry of `diag` that is no alignment: its first symbols (kHeadSteps past the
+// table at most) do not occur, or it was left to the row queue or the rest list.
+constexpr uint32_t kAbsent = 0xFFFFFFFFu, kMany = 0xFFFFFFFEu;
+__device__ __forceinline__ bool is_diag(uint32_t x) { return x < kMany; }
 constexpr unsigned kFull = 0xFFFFFFFFu;
-constexpr uint32_t kNoKey = 0xFFFFFFFFu;  // of a queue entry: a chain, not a branch walk
 
 // 32 symbols of a 2-bit stream from symbol i on (i may be -31 or reach past the
 // end by as much: the streams are padded), symbol i in the low bits.
@@ -136,6 +150,15 @@ __device__ __forceinline__ int branch_from(int len, bool fwd) {
   return fwd ? half : len - half;
 }
 
+// What the head found of the strand's chain on the other index (an entry of `diag`),
+// which reads the symbols from t on from their other end; kMany where they do not
+// reach past its head.
+__device__ __forceinline__ uint32_t other_chain(const DevIndex& X, const BatchedParams& p, uint32_t rs, uint32_t d,
+                                                int len, int t) {
+  if (len - t < (int)X.tmer_len + kHeadSteps || len < 2 * (int)X.tmer_len + 2) return kMany;
+  return p.diag[(uint64_t)((d ^ 1u) * 2u + (rs & 1u)) * p.n_reads + (rs >> 1)];
+}
+
 // The block entry (j = 1 / j = n-1) for the fused drain.
 __device__ __forceinline__ void push_block(const BatchedParams& p, uint32_t k, uint32_t l, uint32_t rs, int len,
                                            bool fwd) {
@@ -149,8 +172,8 @@ __device__ __forceinline__ uint32_t branch_meta(bool fwd, int len, int t, uint32
   return pack_meta(fwd ? 1u : 0u, 1, kind, base, fwd ? t : len - t - 1);
 }
 
-// Queue entries: x = row (finish) or k (rest), y = l (rest) or order key (finish),
-// z = rs, w = symbols matched | forward << 16.
+// Entries of the row queue and the rest list: x = k, y = l, z = rs, w = symbols matched |
+// forward << 16; of the walk queue: x = row, y = order key, z = rs, w the same.
 
 // blockIdx.y 0, 1: the chains on the backward index ('+' backward, '-' forward),
 // 2, 3: those on the forward index ('+' forward, '-' backward), so that the
@@ -163,7 +186,8 @@ __global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, Batched
   const uint32_t read = blockIdx.x * kHeadTpb + threadIdx.x;
   const uint32_t d = blockIdx.y >> 1, strand = blockIdx.y & 1u;
   const bool fwd = (d ^ strand) != 0;
-  uint32_t dest = 0, sectors = 0;  // 1: finish queue, 2: rest list
+  uint32_t dest = 0, sectors = 0;  // 1: row queue, 2: rest list
+  uint32_t diag = kAbsent;
   uint4 e = make_uint4(0, 0, 0, 0);
   if (read < n_reads && p.ok[read]) {
     const uint64_t b0 = p.offs[read], b1 = p.offs[read + 1];
@@ -172,13 +196,13 @@ __global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, Batched
       const OccBlock* occ = d ? X.dir[1].occ : X.dir[0].occ;
       const uint32_t dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
       uint64_t q = query32(X, p.packed, b0, len, fwd, strand, 0);
-      const int L = (int)X.kmer_len;
       uint32_t k = 0, l = X.top;
       int t = 0;
-      if (L && len >= 2 * L + 2) {
-        // the first L steps from the full interval reach no branching position: one lookup
+      // the first L steps from the full interval reach no branching position: one lookup
+      const int L = (int)X.tmer_len;
+      if (len >= 2 * L + 2) {
         const uint32_t r = __brev((uint32_t)q) >> (32 - 2 * L);
-        const uint2 s = __ldg((d ? X.kmer[1] : X.kmer[0]) +
+        const uint2 s = __ldg((d ? X.tmer[1] : X.tmer[0]) +
                               (((r & 0x55555555u) << 1) | ((r >> 1) & 0x55555555u)));
         if (CENSUS) ++sectors;
         k = s.x;
@@ -186,35 +210,48 @@ __global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, Batched
         t = L;
         q >>= 2 * L;
       }
-      const int ts = branch_from(len, fwd);
+      const int ts = branch_from(len, fwd), stop = min(t + kHeadSteps, len - 1);
+      bool one = false;
       while (k <= l) {
-        if (t == len - 1 || t >= (int)kHeadSymbols) {  // the last symbol, or still several rows
-          dest = 2;
+        if (t == stop) {
+          one = k == l;
+          dest = one ? 0 : (l - k < kRows ? 1 : 2);
           e = make_uint4(k, l, 0, (uint32_t)t);
           break;
         }
         const uint32_t pk = k, pl = l;
         if (CENSUS) sectors += (k >> 6) == (l >> 6) ? 1u : 2u;
         rank_step(X, occ, dollar, (uint32_t)q & 3u, k, l);
-        if (t >= ts && l - k != pl - pk) {  // a change point
-          dest = pk == pl ? 1 : 2;
-          e = make_uint4(pk, pk == pl ? kNoKey : pl, 0, (uint32_t)t);
+        if (t >= ts && l - k != pl - pk) {  // a change point: the interval before it
+          one = pk == pl;
+          dest = one ? 0 : (pl - pk < kRows ? 1 : 2);
+          e = make_uint4(pk, pl, 0, (uint32_t)t);
           break;
         }
         ++t;
         q >>= 2;
         if (k == l && pk == pl) {  // one row that has matched on: not a chance match about to end
-          dest = 1;
-          e = make_uint4(k, kNoKey, 0, (uint32_t)t);
+          one = true;
+          e = make_uint4(k, l, 0, (uint32_t)t);
           break;
         }
       }
+      if (one) {  // symbol i of the chain lies at T_d[diag - 1 - i]
+        diag = load_row_word((d ? X.dir[1].sa : X.dir[0].sa) + e.x) + e.w;
+        if (CENSUS) ++sectors;
+      }
+      if (dest) diag = kMany;
       e.z = (read << 1) | strand;
       e.w |= fwd ? 1u << 16 : 0u;
     }
   }
+  if (read < n_reads) __stcs(p.diag + (uint64_t)blockIdx.y * p.n_reads + read, diag);
   // the block's entries appended with one atomic per queue
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (!__syncthreads_or(dest)) {
+    if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
+    return;
+  }
   const unsigned m1 = __ballot_sync(kFull, dest == 1), m2 = __ballot_sync(kFull, dest == 2);
   if (lane == 0) {
     s_cnt[0][warp] = (uint32_t)__popc(m1);
@@ -228,222 +265,461 @@ __global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, Batched
       s_cnt[threadIdx.x][w] = tot;
       tot += c;
     }
-    s_base[threadIdx.x] = tot ? atomicAdd(threadIdx.x ? p.rest_n : p.fin_n, tot) : 0u;
+    s_base[threadIdx.x] = tot ? atomicAdd(threadIdx.x ? p.rest_n : p.rows_n, tot) : 0u;
   }
   __syncthreads();
-  if (dest == 1) {  // (the queue holds one entry per chain and more: no bound to check)
-    p.fin[s_base[0] + s_cnt[0][warp] + (uint32_t)__popc(m1 & ((1u << lane) - 1u))] = e;
-  } else if (dest == 2) {
-    p.rest[s_base[1] + s_cnt[1][warp] + (uint32_t)__popc(m2 & ((1u << lane) - 1u))] = e;
-  }
+  // (either holds one entry per chain: no bound to check)
+  if (dest == 1) p.rows[s_base[0] + s_cnt[0][warp] + (uint32_t)__popc(m1 & ((1u << lane) - 1u))] = e;
+  else if (dest == 2) p.rest[s_base[1] + s_cnt[1][warp] + (uint32_t)__popc(m2 & ((1u << lane) - 1u))] = e;
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
 
-struct RestShared {
-  uint4 stk[kRestStack];  // change points: k, l, rs, t | forward << 16
-  unsigned top;
+// The hits of a change point whose interval is one row, at T_d[Q - 1] for symbol te: bit 0
+// the deletion, 1 the insertion and 2 the mismatch of the text's next symbol, `base` as a query base.
+__device__ __forceinline__ uint32_t one_row_branches(const DevIndex& X, const uint64_t* packed, uint64_t b0, int len,
+                                                     bool fwd, uint32_t strand, uint32_t d, int te, uint32_t Q,
+                                                     uint32_t& base) {
+  const int after = len - te - 1;  // symbols after the failing one
+  uint32_t mask = 0;
+  if (Q >= (uint32_t)after && agree(X, packed, b0, len, fwd, strand, d, te + 1, Q, after) == after) mask = 1;
+  if (Q >= 1) {
+    const uint64_t tw = d ? load32(X.text, (int64_t)(X.top - Q)) : load32(X.text, (int64_t)Q - 1);
+    base = ((uint32_t)tw & 3u) ^ (strand ? X.comp_xor : 0u);
+    const uint32_t R = Q - 1;
+    if (R >= (uint32_t)after + 1 && agree(X, packed, b0, len, fwd, strand, d, te, R, after + 1) == after + 1)
+      mask |= 2;
+    if (R >= (uint32_t)after && agree(X, packed, b0, len, fwd, strand, d, te + 1, R, after) == after) mask |= 4;
+  }
+  return mask;
+}
+
+// Sum over the block of v before this thread, plus *ctr advanced by the block's total.
+template <int TPB>
+__device__ __forceinline__ uint32_t block_slots(uint32_t v, unsigned int* ctr, uint32_t* s_cnt, uint32_t* s_base) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(kFull, incl, o);
+    if (lane >= (uint32_t)o) incl += x;
+  }
+  if (lane == 31) s_cnt[warp] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t tot = 0;
+    for (int w = 0; w < TPB / 32; ++w) {
+      const uint32_t c = s_cnt[w];
+      s_cnt[w] = tot;
+      tot += c;
+    }
+    *s_base = tot ? atomicAdd(ctr, tot) : 0u;
+  }
+  __syncthreads();
+  return *s_base + s_cnt[warp] + incl - v;
+}
+
+// The one-row chains of a read, a strand at a time.  With R the read ('+') or
+// its reverse complement ('-'), the strand's chain on the forward index reads R
+// from its left end and the one on the backward index from its right end; where
+// both lie on the same alignment (all but the reads with an indel) one pass over
+// the text serves both.  Up to seven hits a strand: the exact one, three a chain.
+__global__ void __launch_bounds__(kReadTpb) text_read_kernel(DevIndex X, BatchedParams p) {
+  __shared__ uint32_t s_cnt[kReadTpb / 32], s_base;
+  const uint32_t n_reads = p.n_reads_dev ? *p.n_reads_dev : p.n_reads;
+  if ((uint64_t)blockIdx.x * kReadTpb >= n_reads) return;
+  const uint32_t read = blockIdx.x * kReadTpb + threadIdx.x;
+  uint32_t dg[4] = {kAbsent, kAbsent, kAbsent, kAbsent};  // '+' right, '-' right, '+' left, '-' left
+  uint64_t b0 = 0;
+  int len = 0;
+  if (read < n_reads) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) dg[c] = __ldcs(p.diag + (uint64_t)c * p.n_reads + read);
+    b0 = p.offs[read];
+    len = (int)(p.offs[read + 1] - b0);
+  }
+  const uint32_t n = X.top;
+  uint32_t turns = (is_diag(dg[0]) || is_diag(dg[2]) ? 1u : 0u) | (is_diag(dg[1]) || is_diag(dg[3]) ? 2u : 0u);
+  while (__syncthreads_or((int)turns)) {
+    // bits 0: exact; 1..3: deletion, insertion, mismatch of the right chain's change point; 4..6: the left chain's
+    uint32_t mask = 0, base_r = 0, base_l = 0, strand = 0, right = 0, left = 0;
+    int te_r = 0, te_l = 0;
+    if (turns) {
+      strand = (turns & 1u) ? 0u : 1u;
+      turns &= turns - 1;
+      right = strand ? dg[1] : dg[0];
+      left = strand ? dg[3] : dg[2];
+      const uint64_t cw = comp_word(X, strand);
+      auto R32 = [&](int j) -> uint64_t {  // symbols j .. j+31 of R
+        return strand ? rev32(load32(p.packed, (int64_t)b0 + len - 32 - j)) ^ cw : load32(p.packed, (int64_t)b0 + j);
+      };
+      // the alignment: R[j] at text[a + j]
+      const int64_t a_r = (int64_t)right - len, a_l = (int64_t)n - left;
+      te_r = te_l = len;
+      if (is_diag(left)) {  // from the left; past the text's end nothing matches
+        const int hi = (int)min((int64_t)len, (int64_t)left);
+        int j = 0;
+        for (; j < hi; j += 32) {
+          const uint64_t x = load32(X.text, a_l + j) ^ R32(j);
+          if (x) {
+            j += (__ffsll((long long)x) - 1) >> 1;
+            break;
+          }
+        }
+        if (j < hi) te_l = j;
+        else if (hi < len) te_l = hi;
+      }
+      if (is_diag(right) && !(is_diag(left) && a_l == a_r && te_l == len)) {  // from the right, down to the text's start
+        const int lo = a_r < 0 ? (int)-a_r : 0;
+        int top = len;  // R[top .. len-1] matches
+        for (; top > lo; top -= 32) {
+          const uint64_t x = load32(X.text, a_r + top - 32) ^ R32(top - 32);
+          if (x) {
+            top -= __clzll((long long)x) >> 1;
+            break;
+          }
+        }
+        if (top > lo) te_r = len - top;
+        else if (lo > 0) te_r = len - lo;
+      }
+      // the chain on the right is the backward one of '+', the forward one of '-'
+      if (is_diag(strand ? left : right) && (strand ? te_l : te_r) == len) mask = 1;
+#pragma unroll
+      for (int side = 0; side < 2; ++side) {  // 0: right (backward index), 1: left (forward index)
+        const uint32_t dgs = side ? left : right;
+        const int te = side ? te_l : te_r;
+        const bool fwd = (side != 0) == (strand == 0);
+        if (!is_diag(dgs) || te >= len || te < branch_from(len, fwd)) continue;
+        const uint32_t Q = dgs - (uint32_t)te;
+        if (te == len - 1) {
+          const uint32_t r = load_row_word((side ? X.dir[1].isa : X.dir[0].isa) + Q);
+          push_block(p, r, r, (read << 1) | strand, len, fwd);
+        } else {
+          uint32_t base = 0;
+          const uint32_t m = one_row_branches(X, p.packed, b0, len, fwd, strand, (uint32_t)side, te, Q, base);
+          if (side) {
+            mask |= m << 4;
+            base_l = base;
+          } else {
+            mask |= m << 1;
+            base_r = base;
+          }
+        }
+      }
+    }
+    uint32_t slot = block_slots<kReadTpb>((uint32_t)__popc(mask), p.res_total, s_cnt, &s_base);
+    while (mask) {
+      const int h = __ffs(mask) - 1;
+      mask &= mask - 1;
+      uint32_t key, meta, at;
+      uint32_t side;
+      if (h == 0) {  // the backward chain's
+        side = strand;
+        at = (side ? left : right) - (uint32_t)len;
+        key = order_key(0, 0, 0);
+        meta = pack_meta(0, 0, 0, 0, 0);
+      } else {
+        side = h >= 4 ? 1u : 0u;
+        const int te = side ? te_l : te_r, item = (h - 1) % 3;
+        const uint32_t b = side ? base_l : base_r;
+        const bool fwd = (side != 0) == (strand == 0);
+        // symbols taken from the text: one fewer for the deletion, one more for the insertion
+        at = (side ? left : right) - (uint32_t)(len + (item == 0 ? -1 : (item == 1 ? 1 : 0)));
+        key = order_key(fwd ? 4u : 2u, (uint32_t)(len - te), item == 0 ? 0u : (item == 1 ? 1 + 2 * b : 2 + 2 * b));
+        meta = branch_meta(fwd, len, te, item == 0 ? 1u : (item == 1 ? 3u : 2u), item == 0 ? 0xFFu : b);
+      }
+      const uint32_t row = load_row_word((side ? X.dir[1].isa : X.dir[0].isa) + at);
+      write_hit(p, slot++, (read << 1) | strand, key, row, row, meta);
+    }
+    // (the loop's barrier is passed before s_cnt and s_base are rewritten)
+  }
+}
+
+// A lane per row of the queued chains.  Row r of a chain, matched for t symbols,
+// lies on an alignment: symbol i at T_r(i) = T_d[P - 1 - i], P = SA[r] + t.  With
+//   te_r  the first symbol that disagrees,
+//   D_r   the least i from which on symbol i+1 agrees with T_r(i)   (deletion),
+//   I_r   the least i from which on symbol i agrees with T_r(i+1)   (insertion),
+//   M_r   the least i from which on symbol i agrees with T_r(i)     (mismatch),
+// all by comparing words, the chain's interval at t is the rows with te_r >= t;
+// it changes at each te_r, and the helper's continuations at such a te keep the
+// rows of that interval with D_r <= te; with I_r <= te and T_r(te) = b; with
+// te_r = te, M_r <= te + 1 and T_r(te) = b.  Extending rows by the same symbols
+// keeps their order, so the first and the last row kept give the hit's interval.
+struct RowsShared {
+  uint4 item[32];
+  uint32_t n, next;
 };
 
-// Persistent: a lane runs one chain or one branch walk, a rank step per
-// iteration.  Idle lanes wait, masked, until `batch_idle` of the warp are idle
-// and are handed work together: eight lanes per stacked change point (its eight
-// continuations share the interval's one or two blocks, so their first step is
-// one or two sectors for all), then chains of the rest list; with `spilled` set
-// the change points of the spill queue instead of chains.
-template <bool CENSUS>
-__global__ void __launch_bounds__(kRestTpb, 8) text_rest_kernel(DevIndex X, BatchedParams p, int spilled) {
-  __shared__ RestShared rsh[kRestWarps];
-  __shared__ uint32_t c_res[kRestTpb], c_spl[kRestTpb], c_fin[kRestTpb];
+__global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, BatchedParams p) {
+  __shared__ RowsShared rsh[kRowsWarps];
+  __shared__ uint32_t c_res[kRowsTpb];
   const int tid = threadIdx.x;
   const uint32_t lane = tid & 31;
-  RestShared& ws = rsh[tid >> 5];
-  const uint32_t n_src = spilled ? min(*(volatile unsigned int*)p.spill_tail, p.spill_cap)
-                                 : *(volatile unsigned int*)p.rest_n;
-  unsigned int* src_ctr = spilled ? p.spill_head : p.rest_head;
-  c_res[tid] = c_spl[tid] = c_fin[tid] = 0;
-  if (lane == 0) ws.top = 0;
+  RowsShared& ws = rsh[tid >> 5];
+  const uint32_t n_items = *(volatile unsigned int*)p.rows_n;
+  // eight chains a claim, fewer when every warp then still has some
+  const uint32_t per_claim = min(max(n_items / (gridDim.x * kRowsWarps), 1u), 8u);
+  c_res[tid] = 0;
+  if (lane == 0) ws.n = ws.next = 0;
   __syncwarp();
-  bool active = false, exhausted = false, fin_full = false;
-  uint32_t k = 0, l = 0, rs = 0, key = kNoKey;
-  int t = 0, len = 0;
+  bool exhausted = false;
+  for (;;) {
+    if (ws.next == ws.n) {  // claim the next chains
+      if (exhausted) break;
+      uint32_t c0 = 0;
+      if (lane == 0) c0 = atomicAdd(p.rows_head, per_claim);
+      c0 = __shfl_sync(kFull, c0, 0);
+      if (c0 + per_claim >= n_items) exhausted = true;
+      const uint32_t got = c0 < n_items ? min(per_claim, n_items - c0) : 0u;
+      if (lane < got) ws.item[lane] = p.rows[c0 + lane];
+      __syncwarp();
+      if (lane == 0) {
+        ws.n = got;
+        ws.next = 0;
+      }
+      __syncwarp();
+      if (!got) break;
+    }
+    // as many of the held chains as 32 lanes hold rows of
+    const uint32_t first = ws.next, held = ws.n - first;
+    uint32_t rows = 0;
+    if (lane < held) rows = min(ws.item[first + lane].y - ws.item[first + lane].x + 1u, kRows);
+    uint32_t incl = rows;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(kFull, incl, o);
+      if (lane >= (uint32_t)o) incl += v;
+    }
+    const unsigned fit = __ballot_sync(kFull, lane < held && incl <= 32);
+    const uint32_t take = (uint32_t)__popc(fit);  // (sizes are positive: the fitting ones are the first ones)
+    // this lane's chain and its lanes
+    uint32_t mine = 0xFFFFFFFFu, j = 0;
+    unsigned seg = 0;
+    for (uint32_t i = 0; i < take; ++i) {
+      const uint32_t end = __shfl_sync(kFull, incl, i), len_i = __shfl_sync(kFull, rows, i);
+      if (lane < end && lane >= end - len_i) {
+        mine = i;
+        j = lane - (end - len_i);
+        seg = (end == 32 ? kFull : (1u << end) - 1u) & ~((1u << (end - len_i)) - 1u);
+      }
+    }
+    uint32_t rs = 0, d = 0, P = 0, strand = 0;
+    bool fwd = false;
+    int len = 0, t0 = 0, ts = 0, te = -1, D = 0x7FFFFFFF, I = 0x7FFFFFFF, M = 0x7FFFFFFF;
+    uint64_t b0 = 0;
+    if (mine != 0xFFFFFFFFu) {
+      const uint4 e = ws.item[first + mine];
+      rs = e.z;
+      strand = rs & 1u;
+      fwd = (e.w >> 16) & 1u;
+      d = (fwd ? 1u : 0u) ^ strand;
+      t0 = (int)(e.w & 0xFFFFu);
+      b0 = p.offs[rs >> 1];
+      len = (int)(p.offs[(rs >> 1) + 1] - b0);
+      ts = max(t0, branch_from(len, fwd));  // change points before it are not the helper's
+      const uint32_t sa = __ldg((d ? X.dir[1].sa : X.dir[0].sa) + e.x + j);
+      P = sa + (uint32_t)t0;
+      te = t0 + agree(X, p.packed, b0, len, fwd, strand, d, t0, sa, (int)min((uint32_t)(len - t0), sa));
+    }
+    __syncwarp();
+    if (lane == 0) ws.next = first + take;
+    if (te >= ts) {  // of use to the helper: where the three shifted alignments begin to agree for good
+      auto from_end = [&](int shift) -> int {  // symbols i agree with T(i + shift) down to the returned i, at least ts
+        const int64_t need = (int64_t)len + shift;  // text symbols the read takes
+        if (need > (int64_t)P) return 0x7FFFFFFF;
+        int hi = len;  // symbols hi .. len-1 agree
+        const int lo = shift < 0 ? ts + 1 : ts;  // the deletion's first symbol is te + 1
+        while (hi > lo) {
+          // symbols hi-32 .. hi-1 against T(hi-32+shift) .. T(hi-1+shift), the last symbol in the top bits
+          uint64_t qw = fwd ? load32(p.packed, (int64_t)b0 + hi - 32) : load32(p.packed, (int64_t)b0 + len - hi);
+          qw ^= comp_word(X, strand);
+          uint64_t tw = d ? load32(X.text, (int64_t)(X.top - P) + hi - 32 + shift)
+                          : load32(X.text, (int64_t)P - hi - shift);
+          if (!fwd) qw = rev32(qw);
+          if (!d) tw = rev32(tw);
+          const uint64_t x = qw ^ tw;
+          const int same = x ? __clzll((long long)x) >> 1 : 32;
+          hi -= same;
+          if (same < 32) break;
+        }
+        return max(hi, lo);
+      };
+      D = from_end(-1) - 1;
+      I = from_end(1);
+      M = from_end(0);
+    }
+    // the row each alignment ends in, where it may be asked for
+    const uint32_t* isa = d ? X.dir[1].isa : X.dir[0].isa;
+    const int last = min(te, len - 2);  // the last change point whose interval holds this row
+    uint32_t row_d = 0, row_i = 0, row_m = 0;
+    // a change at the last symbol: the interval before it goes to the block list
+    const unsigned ends = __ballot_sync(kFull, mine != 0xFFFFFFFFu && te == len - 1) & seg;
+    const bool block = ends && te >= len - 1;
+    if (te >= ts) {
+      if (D <= last || block) row_d = load_row_word(isa + P - (uint32_t)(len - 1));
+      if (I <= last) row_i = load_row_word(isa + P - (uint32_t)(len + 1));
+      if (te == len || (te <= len - 2 && M <= te + 1)) row_m = load_row_word(isa + P - (uint32_t)len);
+    }
+    auto emit = [&](uint32_t key, uint32_t k, uint32_t l, uint32_t meta) {
+      uint32_t r = c_res[tid];
+      const unsigned slot = res_slot(p, r);
+      c_res[tid] = r;
+      write_hit(p, slot, rs, key, k, l, meta);
+    };
+    auto interval = [&](bool in, uint32_t row, bool& lead, uint32_t& k, uint32_t& l) {  // of the chain's lanes with `in`
+      const unsigned m = __ballot_sync(kFull, in) & seg;
+      lead = m && lane == (uint32_t)__ffs(m) - 1u;
+      k = row;
+      l = __shfl_sync(kFull, row, m ? 31 - __clz(m) : (int)lane);
+    };
+    bool lead;
+    uint32_t k, l;
+    // the whole read: the backward chain's exact hit
+    interval(te == len, row_m, lead, k, l);
+    if (lead && !fwd) emit(order_key(0, 0, 0), k, l, pack_meta(0, 0, 0, 0, 0));
+    interval(block, row_d, lead, k, l);
+    if (lead) push_block(p, k, l, rs, len, fwd);
+    // the other change points, in order
+    bool todo = te >= ts && te <= len - 2;
+    while (__ballot_sync(kFull, todo)) {
+      int cp = 0x7FFFFFFF;  // the least te left among the chain's lanes
+      for (uint32_t i = 0; i < take; ++i) {
+        const int v = __reduce_min_sync(kFull, mine == i && todo ? te : 0x7FFFFFFF);
+        if (mine == i) cp = v;
+      }
+      const bool live = cp != 0x7FFFFFFF;
+      const bool in = live && te >= cp;
+      uint32_t b = 0;  // the row's text symbol at cp, as a query base
+      if (in && P > (uint32_t)cp) {
+        const uint64_t tw = d ? load32(X.text, (int64_t)(X.top - P) + cp) : load32(X.text, (int64_t)P - 1 - cp);
+        b = ((uint32_t)tw & 3u) ^ (strand ? X.comp_xor : 0u);
+      }
+      const uint32_t tf = (uint32_t)(len - cp);
+      const uint32_t sec = fwd ? 4u : 2u;
+      interval(in && D <= cp, row_d, lead, k, l);
+      if (lead) emit(order_key(sec, tf, 0), k, l, branch_meta(fwd, len, cp, 1, 0xFFu));
+      const bool ins = in && I <= cp, mis = in && te == cp && M <= cp + 1;
+      if (__ballot_sync(kFull, ins || mis)) {
+#pragma unroll
+        for (uint32_t v = 0; v < 4; ++v) {
+          interval(ins && b == v, row_i, lead, k, l);
+          if (lead) emit(order_key(sec, tf, 1 + 2 * v), k, l, branch_meta(fwd, len, cp, 3, v));
+          interval(mis && b == v, row_m, lead, k, l);
+          if (lead) emit(order_key(sec, tf, 2 + 2 * v), k, l, branch_meta(fwd, len, cp, 2, v));
+        }
+      }
+      if (te == cp) todo = false;
+    }
+    __syncwarp();
+  }
+  {
+    const uint32_t r = c_res[tid];
+    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
+      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
+  }
+}
+
+// A slot of a queue written in per-lane chunks: state = next slot | slots left << 28,
+// counters below 2^28.  Past `cap` the slot is not there: returns cap.
+__device__ __forceinline__ unsigned chunk_slot(unsigned int* ctr, uint32_t cap, uint32_t& state) {
+  if ((state >> 28) == 0) {
+    const unsigned c = claim(ctr, kResChunk);
+    if (c >= (1u << 28) - kResChunk || c + kResChunk > cap) {
+      state = 0;
+      return cap;
+    }
+    state = c | (kResChunk << 28);
+  }
+  const unsigned slot = state & 0x0FFFFFFFu;
+  state = (slot + 1) | (((state >> 28) - 1) << 28);
+  return slot;
+}
+
+// Persistent: the chains still more than kRows rows wide, a lane each, one rank
+// step per iteration until they are not (-> row queue); the change points they
+// pass inside the helper's window go to the spill queue.  Idle lanes wait,
+// masked, until `batch_idle` of the warp are idle and claim chains together.
+template <bool CENSUS>
+__global__ void __launch_bounds__(kWideTpb) text_wide_kernel(DevIndex X, BatchedParams p) {
+  __shared__ uint32_t c_res[kWideTpb], c_spl[kWideTpb];
+  const int tid = threadIdx.x;
+  const uint32_t lane = tid & 31;
+  const uint32_t n_src = *(volatile unsigned int*)p.rest_n;
+  c_res[tid] = c_spl[tid] = 0;
+  bool active = false, exhausted = false;
+  uint32_t k = 0, l = 0, rs = 0;
+  int t = 0, len = 0, ts = 0;
   bool fwd = false;
   uint64_t q = 0;  // the next symbols
   int ql = 0;      // how many q holds
   const OccBlock* occ = nullptr;
   uint32_t dollar = 0, sectors = 0;
-
-  // The item's read, direction and symbols from symbol t on.
-  auto open_item = [&](uint32_t rs_, bool fwd_, int t_) {
-    rs = rs_;
-    fwd = fwd_;
-    t = t_;
-    const uint64_t b0 = p.offs[rs >> 1];
-    len = (int)(p.offs[(rs >> 1) + 1] - b0);
-    const uint32_t strand = rs & 1u, d = (fwd ? 1u : 0u) ^ strand;
-    occ = d ? X.dir[1].occ : X.dir[0].occ;
-    dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
-    q = query32(X, p.packed, b0, len, fwd, strand, t);
-    ql = 32;
-    active = true;
-  };
-  // Continuation `item` (0..7) of change point e, as listed at wave_branch_kernel.
-  auto start_walk = [&](const uint4& e, uint32_t item) {
-    const int te = (int)(e.w & 0xFFFFu);
-    k = e.x;
-    l = e.y;
-    // deletion and mismatch go on after symbol te, the insertion with it
-    const bool ins = item >= 1 && item <= 4;
-    open_item(e.z, (e.w >> 16) & 1u, ins ? te : te + 1);
-    uint32_t slot = 0;
-    if (item) {
-      uint32_t b;
-      const uint32_t cx = (rs & 1u) ? X.comp_xor : 0u;
-      if (ins) {
-        b = item - 1;
-        slot = 1 + 2 * b;
-      } else {
-        const uint64_t b0 = p.offs[rs >> 1];
-        const uint32_t w = (uint32_t)load32(p.packed, fwd ? (int64_t)b0 + te : (int64_t)b0 + len - 1 - te) & 3u;
-        b = (item - 5) + ((item - 5) >= w ? 1u : 0u);
-        slot = 2 + 2 * b;
-      }
-      // b is stepped first, in the place of the symbol before t (the symbol that
-      // falls out of q is fetched again when q runs out)
-      q = (q << 2) | (b ^ cx);
-      --t;
-    }
-    key = order_key(fwd ? 4u : 2u, (uint32_t)(len - te), slot);
-  };
-  auto refill = [&]() {
-    for (;;) {
-      __syncwarp();
-      const unsigned nd = __ballot_sync(kFull, !active);
-      if (!nd) return;
-      const uint32_t rank = (uint32_t)__popc(nd & ((1u << lane) - 1u));
-      const uint32_t n_nd = (uint32_t)__popc(nd);
-      const unsigned top = min(ws.top, kRestStack);  // pushes past the end went to the spill queue
-      if (top && n_nd >= 8) {
-        const uint32_t take = min(n_nd >> 3, top);
-        __syncwarp();
-        if (!active && (rank >> 3) < take) start_walk(ws.stk[top - 1 - (rank >> 3)], rank & 7u);
-        __syncwarp();
-        if (lane == 0) ws.top = top - take;
-        __syncwarp();
-        continue;
-      }
-      if (exhausted || (spilled && n_nd < 8)) return;
-      const uint32_t want = spilled ? n_nd >> 3 : n_nd;
+  const uint32_t bi = p.batch_idle < 1 ? 1u : p.batch_idle;
+  for (;;) {
+    const unsigned idle = __ballot_sync(kFull, !active);  // every lane, every iteration
+    if (!exhausted && (idle == kFull || (uint32_t)__popc(idle) >= bi)) {
+      const uint32_t want = (uint32_t)__popc(idle), rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
       uint32_t c0 = 0;
-      if (lane == 0) c0 = atomicAdd(src_ctr, want);
+      if (lane == 0) c0 = atomicAdd(p.rest_head, want);
       c0 = __shfl_sync(kFull, c0, 0);
       if (c0 + want >= n_src) exhausted = true;
-      if (spilled) {
-        if (!active && (rank >> 3) < want && c0 + (rank >> 3) < n_src) {
-          const SpillEntry s = p.spill[c0 + (rank >> 3)];
-          if (s.rs != 0xFFFFFFFFu) start_walk(make_uint4(s.k, s.l, s.rs, s.jtype), rank & 7u);
-        }
-      } else if (!active && c0 + rank < n_src) {
+      if (!active && c0 + rank < n_src) {
         const uint4 e = p.rest[c0 + rank];
         k = e.x;
         l = e.y;
-        key = kNoKey;
-        open_item(e.z, (e.w >> 16) & 1u, (int)(e.w & 0xFFFFu));
+        rs = e.z;
+        t = (int)(e.w & 0xFFFFu);
+        fwd = (e.w >> 16) & 1u;
+        const uint64_t b0 = p.offs[rs >> 1];
+        len = (int)(p.offs[(rs >> 1) + 1] - b0);
+        const uint32_t strand = rs & 1u, d = (fwd ? 1u : 0u) ^ strand;
+        ts = branch_from(len, fwd);
+        // change points whose remaining symbols hold a head that does not occur have no hits
+        if (other_chain(X, p, rs, d, len, ts + 1) == kAbsent) ts = len - (int)X.tmer_len - kHeadSteps;
+        occ = d ? X.dir[1].occ : X.dir[0].occ;
+        dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
+        q = query32(X, p.packed, b0, len, fwd, strand, t);
+        ql = 32;
+        active = true;
       }
-      __syncwarp();
-      // (one claim a pass: lanes left idle by holes or by the list's end wait for the next)
-      return;
-    }
-  };
-
-  const uint32_t bi = p.batch_idle < 8 ? 8u : p.batch_idle;
-  for (;;) {
-    const unsigned idle = __ballot_sync(kFull, !active);  // every lane, every iteration
-    if (idle == kFull || (uint32_t)__popc(idle) >= bi) {
-      refill();
-      __syncwarp();
-      if (__ballot_sync(kFull, !active) == kFull && exhausted && ws.top == 0) break;
+      if (__ballot_sync(kFull, active) == 0) break;
+    } else if (exhausted && idle == kFull) {
+      break;
     }
     if (!active) continue;
     const uint32_t pk = k, pl = l;
     if (CENSUS) sectors += (k >> 6) == (l >> 6) ? 1u : 2u;
     rank_step(X, occ, dollar, (uint32_t)q & 3u, k, l);
-    const bool walk = key != kNoKey;
-    if (!walk && l - k != pl - pk && t >= branch_from(len, fwd)) {  // a change point
+    if (t >= ts && l - k != pl - pk) {  // a change point
       if (t == len - 1) {
         push_block(p, pk, pl, rs, len, fwd);
       } else {
-        const uint32_t w = (uint32_t)t | (fwd ? 1u << 16 : 0u);
-        const unsigned at = atomicAdd(&ws.top, 1u);
-        if (at < kRestStack) {
-          ws.stk[at] = make_uint4(pk, pl, rs, w);
-        } else {  // in chunks of slots
-          uint32_t cs = c_spl[tid];
-          unsigned slot;
-          if ((cs >> 28) == 0) {
-            cs = claim(p.spill_tail, kResChunk);
-            if (cs >= (1u << 28) - kResChunk) {  // beyond what the packed form holds
-              slot = cs;
-              cs = 0;
-              for (unsigned i = 1; i < kResChunk; ++i)
-                if (slot + i < p.spill_cap) p.spill[slot + i].rs = 0xFFFFFFFFu;
-            } else {
-              slot = cs;
-              cs = (cs + 1) | ((kResChunk - 1) << 28);
-            }
-          } else {
-            slot = cs & 0x0FFFFFFFu;
-            cs = (slot + 1) | (((cs >> 28) - 1) << 28);
-          }
-          c_spl[tid] = cs;
-          if (slot < p.spill_cap) p.spill[slot] = SpillEntry{pk, pl, rs, w};
-          else atomicOr(p.status, kStatusSpillFull);
-        }
+        uint32_t cs = c_spl[tid];
+        const unsigned slot = chunk_slot(p.spill_tail, p.spill_cap, cs);
+        c_spl[tid] = cs;
+        if (slot < p.spill_cap) p.spill[slot] = SpillEntry{pk, pl, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u)};
+        else atomicOr(p.status, kStatusSpillFull);
       }
     }
     if (k <= l && t + 1 < len) {
       ++t;
-      q >>= 2;
-      if (k == l && pk == pl && !fin_full) {  // one row that has matched on: the text tells the rest
-        uint32_t cs = c_fin[tid];
-        if ((cs >> 28) == 0) {
-          cs = claim(p.fin_n, kResChunk);
-          if (cs >= (1u << 28) - kResChunk || cs + kResChunk > p.fin_cap) {
-            for (unsigned i = 0; i < kResChunk; ++i)
-              if (cs + i < p.fin_cap) p.fin[cs + i].z = 0xFFFFFFFFu;
-            fin_full = true;  // this lane's searches go on by rank steps
-            cs = 0;
-          } else {
-            cs |= kResChunk << 28;
-          }
-        }
-        if (!fin_full) {
-          const unsigned slot = cs & 0x0FFFFFFFu;
-          p.fin[slot] = make_uint4(k, key, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u));
-          cs = (slot + 1) | (((cs >> 28) - 1) << 28);
-          active = false;
-        }
-        c_fin[tid] = cs;
-        if (!active) continue;
+      if (l - k < kRows) {  // few enough rows for a lane each
+        p.rows[claim(p.rows_n, 1)] = make_uint4(k, l, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u));
+        active = false;
+        continue;
       }
+      q >>= 2;
       if (--ql == 0) {  // 32 symbols on
-        const uint64_t b0 = p.offs[rs >> 1];
-        q = query32(X, p.packed, b0, len, fwd, rs & 1u, t);
+        q = query32(X, p.packed, p.offs[rs >> 1], len, fwd, rs & 1u, t);
         ql = 32;
       }
       continue;
     }
-    if (k <= l && (walk || !fwd)) {  // matched to the read end: a branch's hit, or the exact hit
+    if (k <= l && !fwd) {  // the whole read: the exact hit
       uint32_t r = c_res[tid];
       const unsigned slot = res_slot(p, r);
       c_res[tid] = r;
-      if (walk) {
-        const uint32_t s = key & 0xFFu;
-        const int te = len - (int)((key >> 8) & 0xFFFFu);
-        const uint32_t kind = s == 0 ? 1u : ((s & 1u) ? 3u : 2u);
-        write_hit(p, slot, rs, key, k, l, branch_meta(fwd, len, te, kind, s == 0 ? 0xFFu : (s - 1) >> 1));
-      } else {
-        write_hit(p, slot, rs, order_key(0, 0, 0), k, l, pack_meta(0, 0, 0, 0, 0));
-      }
+      write_hit(p, slot, rs, order_key(0, 0, 0), k, l, pack_meta(0, 0, 0, 0, 0));
     }
     active = false;
   }
@@ -454,120 +730,241 @@ __global__ void __launch_bounds__(kRestTpb, 8) text_rest_kernel(DevIndex X, Batc
     const uint32_t cs = c_spl[tid];
     for (unsigned i = 0, left = cs >> 28, s = cs & 0x0FFFFFFFu; i < left; ++i)
       if (s + i < p.spill_cap) p.spill[s + i].rs = 0xFFFFFFFFu;
-    const uint32_t cf = c_fin[tid];
-    for (unsigned i = 0, left = cf >> 28, s = cf & 0x0FFFFFFFu; i < left; ++i)
-      if (s + i < p.fin_cap) p.fin[s + i].z = 0xFFFFFFFFu;
   }
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
 
-// A thread per queued one-row search; up to three hits each, appended with one
-// atomic per block and round.
+// The interval's steps with all four symbols (physical codes), from its one or two blocks.
+__device__ __forceinline__ void rank_step4(const DevIndex& X, const OccBlock* occ, uint32_t dollar, uint32_t k,
+                                           uint32_t l, uint32_t (&nk)[4], uint32_t (&nl)[4]) {
+  const uint32_t q0 = k >> 6, q1 = l >> 6;
+  uint32_t cnt[4];
+  uint4 bits;
+  load_block_m(occ + q0, X.load_mode, cnt, bits);
+  const uint64_t mk = row_mask(k & 63), ml = row_mask((l & 63) + 1);
+#pragma unroll
+  for (uint32_t b = 0; b < 4; ++b) {
+    const uint64_t mm = match_mask(bits, b);
+    nk[b] = X.C[b] + 1u + cnt[b] + (uint32_t)__popcll(mm & mk);
+    nl[b] = X.C[b] + cnt[b] + (uint32_t)__popcll(mm & ml);
+  }
+  if (q1 != q0) {
+    load_block_m(occ + q1, X.load_mode, cnt, bits);
+#pragma unroll
+    for (uint32_t b = 0; b < 4; ++b)
+      nl[b] = X.C[b] + cnt[b] + (uint32_t)__popcll(match_mask(bits, b) & ml);
+  }
+  // the '$' row is stored as code 0 in its block
+  if (k > dollar && q0 == (dollar >> 6)) nk[0] -= 1;
+  if (l >= dollar && q1 == (dollar >> 6)) nl[0] -= 1;
+}
+
+// Persistent: a lane per spilled change point.  Its eight continuations begin
+// with one step from the same interval (the deletion with the symbol after the
+// failing one, the insertions and mismatches with b), so one or two blocks give
+// all their first intervals; the lane then runs those that are not empty one
+// after the other, one rank step per iteration, without touching memory between
+// them.  What has narrowed to one row and matched on goes to the walk queue.
+//
+// Most wide change points lie in tandem runs whose read goes on into sequence that
+// occurs once, or with an error in its head nowhere: there the strand's other chain
+// decides them without a rank step (2M x 150 bp, 600 Mbp with 45 % repeats: 4095 ->
+// 1367 us; about 100 sectors a change point before, its intervals being thousands of
+// rows wide).
 template <bool CENSUS>
-__global__ void __launch_bounds__(kFinishTpb) text_finish_kernel(DevIndex X, BatchedParams p) {
-  __shared__ uint32_t s_cnt[kFinishTpb / 32], s_base;
-  const uint32_t n = min(*(volatile unsigned int*)p.fin_n, p.fin_cap);
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__global__ void __launch_bounds__(kWideTpb) text_branch_kernel(DevIndex X, BatchedParams p) {
+  __shared__ uint32_t c_res[kWideTpb], c_walk[kWideTpb], s_k[4][kWideTpb], s_l[4][kWideTpb];
+  const int tid = threadIdx.x;
+  const uint32_t lane = tid & 31;
+  const uint32_t n_src = min(*(volatile unsigned int*)p.spill_tail, p.spill_cap);
+  c_res[tid] = c_walk[tid] = 0;
+  bool exhausted = false, walk_full = false;
+  uint32_t todo = 0;    // continuations left: bit 0 deletion, 1 + b insertion, 5 + b mismatch
+  bool stepping = false;
+  uint32_t k = 0, l = 0, rs = 0, key = 0;
+  int t = 0, te = 0, len = 0;
+  bool fwd = false;
+  uint64_t q0 = 0, q = 0;  // symbols from te on; the next symbols
+  int ql = 0;
+  const OccBlock* occ = nullptr;
+  uint32_t dollar = 0, sectors = 0;
+  const uint32_t bi = p.batch_idle < 1 ? 1u : p.batch_idle;
+  auto hit = [&]() {
+    const uint32_t s = key & 0xFFu;
+    uint32_t r = c_res[tid];
+    const unsigned slot = res_slot(p, r);
+    c_res[tid] = r;
+    write_hit(p, slot, rs, key, k, l,
+              branch_meta(fwd, len, te, s == 0 ? 1u : ((s & 1u) ? 3u : 2u), s == 0 ? 0xFFu : (s - 1) >> 1));
+  };
+  for (;;) {
+    const unsigned idle = __ballot_sync(kFull, !stepping && !todo);  // every lane, every iteration
+    if (!exhausted && (idle == kFull || (uint32_t)__popc(idle) >= bi)) {
+      const uint32_t want = (uint32_t)__popc(idle), rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+      uint32_t c0 = 0;
+      if (lane == 0) c0 = atomicAdd(p.spill_head, want);
+      c0 = __shfl_sync(kFull, c0, 0);
+      if (c0 + want >= n_src) exhausted = true;
+      SpillEntry e{0, 0, 0xFFFFFFFFu, 0};
+      if (!stepping && !todo && c0 + rank < n_src) e = p.spill[c0 + rank];
+      if (e.rs != 0xFFFFFFFFu) {  // (a reserved slot nothing was written to)
+        rs = e.rs;
+        te = (int)(e.jtype & 0xFFFFu);
+        fwd = (e.jtype >> 16) & 1u;
+        const uint64_t b0 = p.offs[rs >> 1];
+        len = (int)(p.offs[(rs >> 1) + 1] - b0);
+        const uint32_t strand = rs & 1u, d = (fwd ? 1u : 0u) ^ strand;
+        occ = d ? X.dir[1].occ : X.dir[0].occ;
+        dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
+        q0 = query32(X, p.packed, b0, len, fwd, strand, te);
+        // The symbols after the failing one, read from the other end, begin the strand's
+        // other chain.  Where they reach past its head, its one row is the only place a
+        // continuation can match, and there is none if the head found it absent.
+        const uint32_t other = other_chain(X, p, rs, d, len, te + 1);
+        if (other == kMany) {
+          uint32_t nk[4], nl[4];
+          rank_step4(X, occ, dollar, e.k, e.l, nk, nl);
+          if (CENSUS) sectors += (e.k >> 6) == (e.l >> 6) ? 1u : 2u;
+          const uint32_t w = (uint32_t)q0 & 3u, w1 = (uint32_t)(q0 >> 2) & 3u;
+#pragma unroll
+          for (uint32_t b = 0; b < 4; ++b) {
+            s_k[b][tid] = nk[b];
+            s_l[b][tid] = nl[b];
+            if (nk[b] <= nl[b]) todo |= (b == w1 ? 1u : 0u) | 2u << b | (b != w ? 32u << b : 0u);
+          }
+        } else if (other != kAbsent) {
+          // symbol i at T_d[P - 1 - i] for the symbols after the failing one; the ones
+          // before it one place nearer (deletion), there (mismatch) or one farther (insertion)
+          const int r = len - te - 1;
+          const int64_t P64 = (int64_t)X.top + len - other;
+          if (P64 >= len && P64 <= (int64_t)X.top + 1) {
+            const uint32_t P = (uint32_t)P64;
+            if (agree(X, p.packed, b0, len, fwd, strand, d, te + 1, P - (uint32_t)te - 1, r) == r) {
+              const uint32_t row = load_row_word((d ? X.dir[1].isa : X.dir[0].isa) + (P - (uint32_t)len));
+              const uint32_t cx = strand ? X.comp_xor : 0u, sec = fwd ? 4u : 2u, tf = (uint32_t)(len - te);
+              auto text_at = [&](uint32_t at) -> uint32_t {  // T_d[at]
+                return (uint32_t)load32(X.text, d ? (int64_t)X.top - 1 - at : (int64_t)at) & 3u;
+              };
+              auto found = [&](uint32_t slot_key, uint32_t kind, uint32_t base) {
+                uint32_t c = c_res[tid];
+                const unsigned slot = res_slot(p, c);
+                c_res[tid] = c;
+                write_hit(p, slot, rs, order_key(sec, tf, slot_key), row, row, branch_meta(fwd, len, te, kind, base));
+              };
+              if (agree(X, p.packed, b0, len, fwd, strand, d, 0, P - 1, te) == te) found(0, 1, 0xFFu);
+              if (P <= X.top) {
+                const uint32_t here = text_at(P - 1 - (uint32_t)te);  // beside the failing symbol
+                const uint32_t w = (uint32_t)q0 & 3u;
+                if (here == w && P < X.top && agree(X, p.packed, b0, len, fwd, strand, d, 0, P + 1, te) == te) {
+                  const uint32_t b = text_at(P - (uint32_t)te) ^ cx;
+                  found(1 + 2 * b, 3, b);
+                }
+                if (here != w && agree(X, p.packed, b0, len, fwd, strand, d, 0, P, te) == te)
+                  found(2 + 2 * (here ^ cx), 2, here ^ cx);
+              }
+            }
+          }
+        }
+      }
+      if (__ballot_sync(kFull, stepping || todo) == 0) {
+        if (exhausted) break;
+        continue;  // holes only
+      }
+    } else if (exhausted && idle == kFull) {
+      break;
+    }
+    if (!stepping) {
+      if (!todo) continue;
+      const uint32_t item = (uint32_t)__ffs(todo) - 1u;
+      todo &= todo - 1;
+      // the symbol stepped with, as a physical code; the next symbol; the order key's slot
+      const uint32_t b = item == 0 ? (uint32_t)(q0 >> 2) & 3u : (item - 1) & 3u;
+      const int skip = item == 0 ? 2 : (item <= 4 ? 0 : 1);
+      const uint32_t qb = b ^ ((rs & 1u) ? X.comp_xor : 0u);
+      key = order_key(fwd ? 4u : 2u, (uint32_t)(len - te), item == 0 ? 0u : (item <= 4 ? 1 + 2 * qb : 2 + 2 * qb));
+      k = s_k[b][tid];
+      l = s_l[b][tid];
+      t = te + skip;
+      if (t == len) {  // the deletion of the last symbol but one
+        hit();
+        continue;
+      }
+      q = q0 >> (2 * skip);
+      ql = 32 - skip;
+      stepping = true;
+    }
+    const bool was_one = k == l;
+    if (CENSUS) sectors += (k >> 6) == (l >> 6) ? 1u : 2u;
+    rank_step(X, occ, dollar, (uint32_t)q & 3u, k, l);
+    if (k > l) {
+      stepping = false;
+      continue;
+    }
+    if (++t == len) {  // matched to the read end
+      hit();
+      stepping = false;
+      continue;
+    }
+    q >>= 2;
+    if (was_one && !walk_full) {  // one row that has matched on: the text tells the rest
+      uint32_t cs = c_walk[tid];
+      const unsigned slot = chunk_slot(p.walk_n, p.walk_cap, cs);
+      c_walk[tid] = cs;
+      if (slot < p.walk_cap) {
+        p.walk[slot] = make_uint4(k, key, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u));
+        stepping = false;
+        continue;
+      }
+      walk_full = true;  // this lane's walks go on by rank steps
+    }
+    if (--ql == 0) {  // 32 symbols on
+      q = query32(X, p.packed, p.offs[rs >> 1], len, fwd, rs & 1u, t);
+      ql = 32;
+    }
+  }
+  {  // slots of this lane's last chunks that were reserved but not used
+    const uint32_t r = c_res[tid];
+    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
+      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
+    const uint32_t cw = c_walk[tid];
+    for (unsigned i = 0, left = cw >> 28, s = cw & 0x0FFFFFFFu; i < left; ++i)
+      if (s + i < p.walk_cap) p.walk[s + i].z = 0xFFFFFFFFu;
+  }
+  if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
+}
+
+// A thread per queued branch walk that has narrowed to one row.
+template <bool CENSUS>
+__global__ void __launch_bounds__(kWalkTpb) text_walk_kernel(DevIndex X, BatchedParams p) {
+  __shared__ uint32_t s_cnt[kWalkTpb / 32], s_base;
+  const uint32_t n = min(*(volatile unsigned int*)p.walk_n, p.walk_cap);
   uint32_t sectors = 0;
-  for (uint32_t i0 = blockIdx.x * kFinishTpb; i0 < n; i0 += gridDim.x * kFinishTpb) {
+  for (uint32_t i0 = blockIdx.x * kWalkTpb; i0 < n; i0 += gridDim.x * kWalkTpb) {
     const uint32_t i = i0 + threadIdx.x;
-    uint32_t rs = 0, key = 0, meta = 0;
-    uint32_t at[3] = {0, 0, 0};  // SA^-1 index of: the exact hit, the walk's hit or the deletion; the insertion; the mismatch
-    uint32_t mask = 0;           // which of them match
-    uint32_t d = 0, ins_key = 0, ins_meta = 0, mis_meta = 0;
+    bool hit = false;
+    uint32_t row = 0, meta = 0;
     uint4 e = make_uint4(0, 0, 0xFFFFFFFFu, 0);
-    if (i < n) e = __ldcs(p.fin + i);
+    if (i < n) e = __ldcs(p.walk + i);
     if (e.z != 0xFFFFFFFFu) {  // (a reserved slot nothing was written to)
-      rs = e.z;
-      const uint32_t strand = rs & 1u;
+      const uint32_t strand = e.z & 1u;
       const bool fwd = (e.w >> 16) & 1u;
-      d = (fwd ? 1u : 0u) ^ strand;
+      const uint32_t d = (fwd ? 1u : 0u) ^ strand;
       const uint32_t P = load_row_word((d ? X.dir[1].sa : X.dir[0].sa) + e.x);
-      const uint64_t b0 = p.offs[rs >> 1];
-      const int len = (int)(p.offs[(rs >> 1) + 1] - b0);
+      const uint64_t b0 = p.offs[e.z >> 1];
+      const int len = (int)(p.offs[(e.z >> 1) + 1] - b0);
       const int t = (int)(e.w & 0xFFFFu), left = len - t;
-      const int m = agree(X, p.packed, b0, len, fwd, strand, d, t, P, (int)min((uint32_t)left, P));
-      const uint32_t Q = P - (uint32_t)m;
-      if (CENSUS) sectors += 2u + (uint32_t)(m >> 7);
-      if (e.y != kNoKey) {  // a branch walk
-        if (m == left) {
-          const uint32_t s = e.y & 0xFFu;
-          mask = 1;
-          at[0] = Q;
-          key = e.y;
-          meta = branch_meta(fwd, len, len - (int)((e.y >> 8) & 0xFFFFu), s == 0 ? 1u : ((s & 1u) ? 3u : 2u),
-                             s == 0 ? 0xFFu : (s - 1) >> 1);
-        }
-      } else if (m == left) {  // the whole read: the exact hit, reported by the backward chain
-        if (!fwd) {
-          mask = 1;
-          at[0] = Q;
-          key = order_key(0, 0, 0);
-          meta = pack_meta(0, 0, 0, 0, 0);
-        }
-      } else {
-        const int te = t + m;  // the symbol that fails
-        if (te == len - 1) {
-          const uint32_t r = load_row_word((d ? X.dir[1].isa : X.dir[0].isa) + Q);
-          push_block(p, r, r, rs, len, fwd);
-        } else if (te >= branch_from(len, fwd)) {
-          const int after = len - te - 1;  // symbols after the failing one
-          key = order_key(fwd ? 4u : 2u, (uint32_t)(len - te), 0);
-          if (Q >= (uint32_t)after && agree(X, p.packed, b0, len, fwd, strand, d, te + 1, Q, after) == after) {
-            mask = 1;
-            at[0] = Q - (uint32_t)after;
-            meta = branch_meta(fwd, len, te, 1, 0xFFu);
-          }
-          if (Q >= 1) {
-            // the text's next symbol, as a query base: the one insertion and the one mismatch that match it
-            const uint64_t tw = d ? load32(X.text, (int64_t)(X.top - Q)) : load32(X.text, (int64_t)Q - 1);
-            const uint32_t b = ((uint32_t)tw & 3u) ^ (strand ? X.comp_xor : 0u);
-            const uint32_t R = Q - 1;
-            ins_key = key + 1 + 2 * b;
-            ins_meta = branch_meta(fwd, len, te, 3, b);
-            mis_meta = branch_meta(fwd, len, te, 2, b);
-            if (R >= (uint32_t)after + 1 &&
-                agree(X, p.packed, b0, len, fwd, strand, d, te, R, after + 1) == after + 1) {
-              mask |= 2;
-              at[1] = R - (uint32_t)after - 1;
-            }
-            if (R >= (uint32_t)after && agree(X, p.packed, b0, len, fwd, strand, d, te + 1, R, after) == after) {
-              mask |= 4;
-              at[2] = R - (uint32_t)after;
-            }
-          }
-        }
+      if (CENSUS) sectors += 2;
+      if (P >= (uint32_t)left && agree(X, p.packed, b0, len, fwd, strand, d, t, P, left) == left) {
+        const uint32_t s = e.y & 0xFFu;
+        hit = true;
+        row = load_row_word((d ? X.dir[1].isa : X.dir[0].isa) + P - (uint32_t)left);
+        meta = branch_meta(fwd, len, len - (int)((e.y >> 8) & 0xFFFFu), s == 0 ? 1u : ((s & 1u) ? 3u : 2u),
+                           s == 0 ? 0xFFu : (s - 1) >> 1);
+        if (CENSUS) ++sectors;
       }
     }
-    uint32_t row[3];
-    const uint32_t* isa = d ? X.dir[1].isa : X.dir[0].isa;
-#pragma unroll
-    for (int h = 0; h < 3; ++h) row[h] = (mask >> h) & 1u ? load_row_word(isa + at[h]) : 0u;
-    const uint32_t n_hits = (uint32_t)__popc(mask);
-    if (CENSUS) sectors += n_hits;
-    // slots of the block's hits
-    uint32_t incl = n_hits;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(kFull, incl, o);
-      if (lane >= (uint32_t)o) incl += v;
-    }
-    if (lane == 31) s_cnt[warp] = incl;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t tot = 0;
-      for (int w = 0; w < kFinishTpb / 32; ++w) {
-        const uint32_t c = s_cnt[w];
-        s_cnt[w] = tot;
-        tot += c;
-      }
-      s_base = tot ? atomicAdd(p.res_total, tot) : 0u;
-    }
-    __syncthreads();
-    uint32_t slot = s_base + s_cnt[warp] + incl - n_hits;
-    if (mask & 1u) write_hit(p, slot++, rs, key, row[0], row[0], meta);
-    if (mask & 2u) write_hit(p, slot++, rs, ins_key, row[1], row[1], ins_meta);
-    if (mask & 4u) write_hit(p, slot, rs, ins_key + 1, row[2], row[2], mis_meta);
+    const uint32_t slot = block_slots<kWalkTpb>(hit ? 1u : 0u, p.res_total, s_cnt, &s_base);
+    if (hit) write_hit(p, slot, e.z, e.y, row, row, meta);
     __syncthreads();  // s_cnt and s_base are rewritten next round
   }
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
@@ -577,24 +974,38 @@ template <bool CENSUS>
 void launch_text_stage(const DevIndex& X, const BatchedParams& p, int num_sms, cudaStream_t s) {
   const uint32_t cap = p.n_reads;
   if (!cap) return;
-  count_launches(4);
+  count_launches(6);
   text_head_kernel<CENSUS><<<dim3((cap + kHeadTpb - 1) / kHeadTpb, 4), kHeadTpb, 0, s>>>(X, p);
+  text_read_kernel<<<(cap + kReadTpb - 1) / kReadTpb, kReadTpb, 0, s>>>(X, p);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, text_rest_kernel<CENSUS>, kRestTpb, 0);
-  const unsigned rest_grid = (unsigned)(num_sms * std::max(per_sm, 1));
-  text_rest_kernel<CENSUS><<<rest_grid, kRestTpb, 0, s>>>(X, p, 0);
-  text_rest_kernel<CENSUS><<<rest_grid, kRestTpb, 0, s>>>(X, p, 1);
-  text_finish_kernel<CENSUS><<<(unsigned)std::min<uint64_t>((4ull * cap + kFinishTpb - 1) / kFinishTpb,
-                                                            8ull * num_sms),
-                               kFinishTpb, 0, s>>>(X, p);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, text_wide_kernel<CENSUS>, kWideTpb, 0);
+  text_wide_kernel<CENSUS><<<(unsigned)(num_sms * std::max(per_sm, 1)), kWideTpb, 0, s>>>(X, p);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, text_branch_kernel<CENSUS>, kWideTpb, 0);
+  text_branch_kernel<CENSUS><<<(unsigned)(num_sms * std::max(per_sm, 1)), kWideTpb, 0, s>>>(X, p);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, text_rows_kernel, kRowsTpb, 0);
+  text_rows_kernel<<<(unsigned)(num_sms * std::max(per_sm, 1)), kRowsTpb, 0, s>>>(X, p);
+  text_walk_kernel<CENSUS><<<(unsigned)std::min<uint64_t>((4ull * cap + kWalkTpb - 1) / kWalkTpb, 8ull * num_sms),
+                             kWalkTpb, 0, s>>>(X, p);
 }
 
 }  // namespace
 
-// Entries of the finish queue: one per chain, as many again for branch walks, and the chunk
-// tails of the rest kernel's lanes.
-size_t text_fin_cap(size_t n_reads, int num_sms) {
-  return std::min<size_t>(8 * n_reads + (size_t)num_sms * 2048 * kResChunk, (1u << 28) - 1);
+// Entries of the walk queue: four a read and the chunk tails of the branch kernel's lanes; walks
+// that find it full go on by rank steps.
+static size_t text_walk_cap(size_t n_reads, int num_sms) {
+  return std::min<size_t>(4 * n_reads + (size_t)num_sms * 2048 * kResChunk, (1u << 28) - 1);
+}
+
+size_t text_queue_bytes(size_t n_reads, int num_sms) {
+  return (8 * n_reads + text_walk_cap(n_reads, num_sms)) * sizeof(uint4) + 4 * n_reads * sizeof(uint32_t);
+}
+
+void text_queues(BatchedParams& p, void* buffer, size_t n_reads, int num_sms) {
+  p.rows = static_cast<uint4*>(buffer);
+  p.rest = p.rows + 4 * n_reads;
+  p.walk = p.rest + 4 * n_reads;
+  p.walk_cap = (uint32_t)text_walk_cap(n_reads, num_sms);
+  p.diag = reinterpret_cast<uint32_t*>(p.walk + p.walk_cap);
 }
 
 void launch_text_search(const DevIndex& X, const BatchedParams& p, int num_sms, cudaStream_t s) {

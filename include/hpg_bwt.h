@@ -261,8 +261,8 @@ int bwt_gpu_set_start_table(bwt_index_t *index, int symbols);
 int bwt_gpu_start_table(bwt_index_t *index);
 /* Whole suffix arrays: an index that finds room (at most a quarter of the
  * device's free memory) keeps the suffix array, its inverse and the packed text
- * beside the sampled arrays, 16.25 bytes per base in all, and locates rows and
- * finishes one-row searches with them.  set: 0 uses the sampled arrays only, 1
+ * beside the sampled arrays, 16.25 bytes per base in all (and start tables of
+ * up to 4.3 GB), and locates rows and finishes one-row searches with them.  set: 0 uses the sampled arrays only, 1
  * (the default) the whole ones where the index has them; returns which are in
  * use.  Results are identical. */
 int bwt_gpu_set_full_rows(bwt_index_t *index, int on);
