@@ -780,36 +780,111 @@ __global__ void scatter_hits_kernel(const PendingHit* __restrict__ res, const un
 constexpr uint32_t kLongList = 32;  // longer lists are sorted by a whole block (sort_long_lists_kernel)
 constexpr int kRankTpb = 512, kRankTile = 2048;
 
-__global__ void sort_truncate_kernel(PendingHit* __restrict__ sorted, const uint64_t* __restrict__ seg_off,
-                                     uint32_t n_rs, uint32_t max_results, uint32_t* __restrict__ kept,
-                                     uint8_t* __restrict__ trunc, const uint32_t* max_dev, const unsigned* gate,
-                                     uint32_t* __restrict__ longs, unsigned* n_longs, uint32_t longs_cap) {
-  const uint32_t rs = blockIdx.x * blockDim.x + threadIdx.x;
-  if (rs >= n_rs) return;
-  if (gate && *gate) return;
-  if (max_dev) max_results = *max_dev;
-  const uint64_t b = seg_off[rs], e = seg_off[rs + 1];
-  const uint64_t cnt = e - b;
-  const uint32_t keep = (uint32_t)(cnt < max_results ? cnt : max_results);
-  kept[rs] = keep;
-  trunc[rs] = cnt > max_results ? 1 : 0;
-  if (keep == 0) return;
-  if (cnt > kLongList) {  // the long sort's work (the list holds enough room for every such list)
-    if (longs) {
-      const unsigned q = atomicAdd(n_longs, 1u);
-      if (q < longs_cap) longs[q] = rs;
-    }
-    return;
+// Lists are taken a tile at a time: `tile` of them (a multiple of 256) per block of the
+// order and emit kernels, whose per-tile sums of kept hits and rows give every list's
+// place in the outputs without a pass over per-list offsets.
+__host__ __device__ constexpr uint32_t finalize_tile(uint32_t n_rs) { return n_rs <= (1u << 20) ? 256u : 1024u; }
+
+// Lists of more hits or rows than these are emitted by a block each (emit_big_kernel).
+constexpr uint32_t kBigHits = 32, kBigRows = 256;
+
+__device__ __forceinline__ uint32_t rows_of(const PendingHit& x) { return x.k <= x.l ? x.l - x.k + 1 : 0u; }
+
+// The list's rows to locate: none when they pass the limit (0: no limit), which sets bit 1 of its flag.
+__device__ __forceinline__ uint32_t limited(uint64_t rows, uint64_t limit, uint8_t& flag) {
+  if (limit && rows > limit) {
+    flag |= 2;
+    return 0;
   }
-  // insertion sort by key (short list; keys are unique within a list)
-  for (uint64_t i = b + 1; i < e; ++i) {
-    const PendingHit x = sorted[i];
-    uint64_t j = i;
-    while (j > b && sorted[j - 1].key > x.key) {
-      sorted[j] = sorted[j - 1];
-      --j;
+  return rows > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)rows;  // beyond kMaxLocateRows either way
+}
+
+__device__ __forceinline__ uint64_t warp_sum64(uint64_t v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+  return v;
+}
+
+// Sorts every (read, strand) list of up to kLongList entries by emission key, in
+// place, and decides its kept count, flag and rows.  A lane per list; a list of more
+// than one entry is sorted by the whole warp, a lane per entry: the entry's place is
+// the number of smaller keys.  (One lane inserting entry by entry held its warp for
+// the longest list, every move a round trip to memory: 209 us on 2M x 150 bp, 600
+// Mbp, of which 2 % of the lists are longer than one.)  Longer lists go to `longs`.
+__global__ void __launch_bounds__(256)
+    order_lists_kernel(PendingHit* __restrict__ sorted, const uint64_t* __restrict__ seg_off, FinalizeLists f,
+                       const unsigned* gate) {
+  __shared__ uint64_t s_rows[8];
+  __shared__ uint32_t s_kept[8];
+  if (gate && *gate) return;
+  const uint32_t max_results = f.max_dev ? *f.max_dev : f.max_results;
+  const uint64_t limit = f.limit_dev ? *f.limit_dev : f.limit;
+  const uint32_t n_rs = f.n_reads_dev ? min(f.n_rs, 2u * *f.n_reads_dev) : f.n_rs;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t sum_rows = 0;
+  uint32_t sum_kept = 0;
+  for (uint32_t r0 = 0; r0 < f.tile; r0 += 256) {
+    const uint64_t rs64 = (uint64_t)blockIdx.x * f.tile + r0 + threadIdx.x;
+    if ((uint64_t)blockIdx.x * f.tile + r0 >= n_rs) break;  // uniform over the block
+    const uint32_t rs = (uint32_t)rs64;
+    const bool live = rs64 < n_rs;
+    uint64_t b = 0;
+    uint32_t cnt = 0;
+    if (live) {
+      b = seg_off[rs];
+      cnt = (uint32_t)(seg_off[rs + 1] - b);
     }
-    sorted[j] = x;
+    const uint32_t keep = min(cnt, max_results);
+    uint64_t rows = 0;
+    if (cnt == 1 && keep) {
+      const uint2 kl = *reinterpret_cast<const uint2*>(&sorted[b].k);
+      rows = kl.x <= kl.y ? (uint64_t)(kl.y - kl.x) + 1 : 0;
+    }
+    if (cnt > kLongList && keep) {  // the long sort's work (the list holds enough room for every such list)
+      const unsigned q = atomicAdd(f.n_longs, 1u);
+      if (q < f.longs_cap) f.longs[q] = rs;
+    }
+    unsigned some = __ballot_sync(0xFFFFFFFFu, cnt > 1 && cnt <= kLongList && keep);
+    while (some) {
+      const int j = __ffs(some) - 1;
+      some &= some - 1;
+      const uint64_t bj = __shfl_sync(0xFFFFFFFFu, b, j);
+      const uint32_t cj = __shfl_sync(0xFFFFFFFFu, cnt, j), kj = __shfl_sync(0xFFFFFFFFu, keep, j);
+      PendingHit x;
+      x.key = 0xFFFFFFFFu;
+      if (lane < cj) x = sorted[bj + lane];
+      uint32_t rank = 0;
+      for (uint32_t i = 0; i < cj; ++i) rank += __shfl_sync(0xFFFFFFFFu, x.key, i) < x.key ? 1u : 0u;
+      __syncwarp();
+      const bool kept = lane < cj && rank < kj;
+      if (kept) sorted[bj + rank] = x;
+      const uint64_t sum = warp_sum64(kept ? rows_of(x) : 0u);
+      if ((int)lane == j) rows = sum;
+    }
+    if (live) {
+      uint8_t flag = cnt > max_results ? 1 : 0;
+      const uint32_t lim = limited(rows, limit, flag);
+      f.kept[rs] = keep;
+      f.trunc[rs] = flag;
+      f.list_rows[rs] = lim;
+      sum_kept += keep;
+      sum_rows += lim ? rows : 0;
+    }
+  }
+  sum_rows = warp_sum64(sum_rows);
+  sum_kept = __reduce_add_sync(0xFFFFFFFFu, sum_kept);
+  if (lane == 0) {
+    s_rows[warp] = sum_rows;
+    s_kept[warp] = sum_kept;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint64_t k = 0, r = 0;
+    for (int w = 0; w < 8; ++w) {
+      k += s_kept[w];
+      r += s_rows[w];
+    }
+    f.part[blockIdx.x] = make_ulonglong2(k, r);
   }
 }
 
@@ -818,66 +893,43 @@ __global__ void sort_truncate_kernel(PendingHit* __restrict__ sorted, const uint
 // sort of the (key, position) pairs in shared memory, O(m log^2 m / 512).
 // Longer: the rank of an entry is the number of entries of its list with a
 // smaller pair, counted against tiles of the list's keys in shared memory,
-// O(m^2 / 512).  Entries placed below the kept count are written to `scratch`
-// (the unsorted pending array, dead after the scatter) and copied back.
+// O(m^2 / 512).
+// Entries placed below the kept count are written to `scratch` (the unsorted pending
+// array, dead after the scatter) and copied back; then the list's rows, as above.
 __global__ void __launch_bounds__(kRankTpb)
     sort_long_lists_kernel(PendingHit* __restrict__ sorted, PendingHit* __restrict__ scratch,
-                           const uint64_t* __restrict__ seg_off, uint32_t n_rs, const uint32_t* __restrict__ kept,
-                           const unsigned* gate, const uint32_t* __restrict__ work, const unsigned* n_work,
-                           uint32_t work_cap) {
+                           const uint64_t* __restrict__ seg_off, FinalizeLists f, const unsigned* gate) {
   if (gate && *gate) return;
   __shared__ uint64_t tile[kRankTile];
-  __shared__ uint32_t longs[kRankTpb];
-  __shared__ uint32_t n_long;
-  // with a work list: its entries, a block each in turn; else every list, found by a scan
-  const uint64_t n_items = work ? min(*n_work, work_cap) : n_rs;
-  const uint64_t per_round = work ? 1 : kRankTpb;
-  for (uint64_t base = (uint64_t)blockIdx.x * per_round; base < n_items; base += (uint64_t)gridDim.x * per_round) {
-    if (threadIdx.x == 0) n_long = 0;
-    __syncthreads();
-    if (work) {
-      if (threadIdx.x == 0) {
-        longs[0] = work[base];
-        n_long = 1;
-      }
-    } else {
-      const uint64_t rs = base + threadIdx.x;
-      if (rs < n_rs && seg_off[rs + 1] - seg_off[rs] > kLongList && kept[rs] > 0)
-        longs[atomicAdd(&n_long, 1u)] = (uint32_t)rs;
-    }
-    __syncthreads();
-    const uint32_t nl = n_long;
-    for (uint32_t q = 0; q < nl; ++q) {
-      const uint32_t r = longs[q];
-      const uint64_t b = seg_off[r];
-      const uint32_t m = (uint32_t)(seg_off[r + 1] - b), keep = kept[r];
-      if (m <= kRankTile) {
-        // bitonic sort of (key, position) pairs in shared memory, padded to a power of two
-        uint32_t P = 64;
-        while (P < m) P <<= 1;
-        __syncthreads();  // the previous list's tile is no longer read
-        for (uint32_t t = threadIdx.x; t < P; t += kRankTpb)
-          tile[t] = t < m ? ((uint64_t)sorted[b + t].key << 32 | t) : ~0ull;
-        __syncthreads();
-        for (uint32_t k = 2; k <= P; k <<= 1) {
-          for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t t = threadIdx.x; t < P / 2; t += kRankTpb) {
-              const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), q2 = i + j;
-              const uint64_t x = tile[i], y = tile[q2];
-              if ((x > y) == ((i & k) == 0)) {
-                tile[i] = y;
-                tile[q2] = x;
-              }
+  __shared__ uint64_t s_rows[kRankTpb / 32];
+  const uint64_t limit = f.limit_dev ? *f.limit_dev : f.limit;
+  const uint32_t n_items = min(*f.n_longs, f.longs_cap);
+  for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const uint32_t r = f.longs[item];
+    const uint64_t b = seg_off[r];
+    const uint32_t m = (uint32_t)(seg_off[r + 1] - b), keep = f.kept[r];
+    if (m <= kRankTile) {
+      // bitonic sort of (key, position) pairs in shared memory, padded to a power of two
+      uint32_t P = 64;
+      while (P < m) P <<= 1;
+      for (uint32_t t = threadIdx.x; t < P; t += kRankTpb)
+        tile[t] = t < m ? ((uint64_t)sorted[b + t].key << 32 | t) : ~0ull;
+      __syncthreads();
+      for (uint32_t k = 2; k <= P; k <<= 1) {
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+          for (uint32_t t = threadIdx.x; t < P / 2; t += kRankTpb) {
+            const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), q2 = i + j;
+            const uint64_t x = tile[i], y = tile[q2];
+            if ((x > y) == ((i & k) == 0)) {
+              tile[i] = y;
+              tile[q2] = x;
             }
-            __syncthreads();
           }
+          __syncthreads();
         }
-        for (uint32_t t = threadIdx.x; t < keep; t += kRankTpb) scratch[b + t] = sorted[b + (uint32_t)tile[t]];
-        __syncthreads();  // every entry written before the copy back
-        for (uint32_t i = threadIdx.x; i < keep; i += kRankTpb) sorted[b + i] = scratch[b + i];
-        __syncthreads();  // the list is final before the next one reuses the tile
-        continue;
       }
+      for (uint32_t t = threadIdx.x; t < keep; t += kRankTpb) scratch[b + t] = sorted[b + (uint32_t)tile[t]];
+    } else {
       for (uint32_t i0 = 0; i0 < m; i0 += kRankTpb) {
         const uint32_t i = i0 + threadIdx.x;
         const uint64_t mine = i < m ? ((uint64_t)sorted[b + i].key << 32 | i) : ~0ull;
@@ -892,16 +944,31 @@ __global__ void __launch_bounds__(kRankTpb)
         }
         if (i < m && rank < keep) scratch[b + rank] = sorted[b + i];
       }
-      __syncthreads();  // every rank written before the copy back
-      for (uint32_t i = threadIdx.x; i < keep; i += kRankTpb) sorted[b + i] = scratch[b + i];
-      __syncthreads();  // the list is final before the next one reuses the tile
     }
-    __syncthreads();  // n_long and longs are read before they are reset
+    __syncthreads();  // every entry written before the copy back
+    uint64_t rows = 0;
+    for (uint32_t i = threadIdx.x; i < keep; i += kRankTpb) {
+      const PendingHit x = scratch[b + i];
+      sorted[b + i] = x;
+      rows += rows_of(x);
+    }
+    rows = warp_sum64(rows);
+    if ((threadIdx.x & 31) == 0) s_rows[threadIdx.x >> 5] = rows;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint64_t sum = 0;
+      for (int w = 0; w < kRankTpb / 32; ++w) sum += s_rows[w];
+      uint8_t flag = f.trunc[r];
+      const uint32_t lim = limited(sum, limit, flag);
+      f.list_rows[r] = lim;
+      f.trunc[r] = flag;
+      if (lim) atomicAdd(reinterpret_cast<unsigned long long*>(&f.part[r / f.tile].y), (unsigned long long)sum);
+    }
+    __syncthreads();  // s_rows and the tile are rewritten for the next list
   }
 }
 
-__device__ __forceinline__ void write_hit_record(const PendingHit& x, uint32_t rs, hpg_hit_t* __restrict__ hits,
-                                                 uint32_t* __restrict__ rows, uint64_t at) {
+__device__ __forceinline__ hpg_hit_t hit_record(const PendingHit& x, uint32_t rs) {
   hpg_hit_t h;
   h.read = rs >> 1;
   h.strand = (uint8_t)(rs & 1u);
@@ -914,38 +981,48 @@ __device__ __forceinline__ void write_hit_record(const PendingHit& x, uint32_t r
   h.pad1 = 0;
   h.k = (int64_t)x.k;
   h.l = (int64_t)x.l;
-  hits[at] = h;
-  rows[at] = x.k <= x.l ? x.l - x.k + 1 : 0u;
+  return h;
 }
 
-// A thread per (read, strand) list; with skip_long the lists of more than
-// kLongList pending hits are left to expand_long_hits_kernel.
-__global__ void expand_hits_kernel(const PendingHit* __restrict__ sorted, const uint64_t* __restrict__ seg_off,
-                                   const uint64_t* __restrict__ hit_off, const uint32_t* __restrict__ kept,
-                                   uint32_t n_rs, hpg_hit_t* __restrict__ hits, uint32_t* __restrict__ rows,
-                                   const unsigned* gate, int skip_long) {
-  const uint32_t rs = blockIdx.x * blockDim.x + threadIdx.x;
-  if (rs >= n_rs) return;
-  if (gate && *gate) return;
-  const uint32_t m = kept[rs];
-  const uint64_t b = seg_off[rs], o = hit_off[rs];
-  if (skip_long && seg_off[rs + 1] - b > kLongList) return;
-  for (uint32_t i = 0; i < m; ++i) write_hit_record(sorted[b + i], rs, hits, rows, o + i);
-}
-
-// The long lists the short sort collected, a block per list.
-__global__ void expand_long_hits_kernel(const PendingHit* __restrict__ sorted, const uint64_t* __restrict__ seg_off,
-                                        const uint64_t* __restrict__ hit_off, const uint32_t* __restrict__ kept,
-                                        hpg_hit_t* __restrict__ hits, uint32_t* __restrict__ rows,
-                                        const unsigned* gate, const uint32_t* __restrict__ work,
-                                        const unsigned* n_work, uint32_t work_cap) {
-  if (gate && *gate) return;
-  const uint32_t n = min(*n_work, work_cap);
-  for (uint32_t q = blockIdx.x; q < n; q += gridDim.x) {
-    const uint32_t rs = work[q];
-    const uint32_t m = kept[rs];
-    const uint64_t b = seg_off[rs], o = hit_off[rs];
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) write_hit_record(sorted[b + i], rs, hits, rows, o + i);
+// Sums of all tiles (block 0), and of the tiles before each tile in place of the tiles'
+// sums when `excl`: for tile counts that the emit kernel's blocks should not each add up.
+__global__ void __launch_bounds__(1024) tile_sums_kernel(ulonglong2* __restrict__ part, uint32_t n_tiles,
+                                                         uint64_t* __restrict__ totals, int excl) {
+  __shared__ uint64_t s_k[32], s_r[32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t ck = 0, cr = 0;
+  for (uint32_t t0 = 0; t0 < n_tiles; t0 += 1024) {
+    const uint32_t t = t0 + threadIdx.x;
+    const ulonglong2 v = t < n_tiles ? part[t] : make_ulonglong2(0, 0);
+    uint64_t k = v.x, r = v.y;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t a = __shfl_up_sync(0xFFFFFFFFu, k, o), b = __shfl_up_sync(0xFFFFFFFFu, r, o);
+      if (lane >= (uint32_t)o) {
+        k += a;
+        r += b;
+      }
+    }
+    if (lane == 31) {
+      s_k[warp] = k;
+      s_r[warp] = r;
+    }
+    __syncthreads();
+    uint64_t bk = ck, br = cr;
+    for (uint32_t w = 0; w < 32; ++w) {
+      if (w < warp) {
+        bk += s_k[w];
+        br += s_r[w];
+      }
+      ck += s_k[w];
+      cr += s_r[w];
+    }
+    if (excl && t < n_tiles) part[t] = make_ulonglong2(bk + k - v.x, br + r - v.y);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    totals[0] = ck;
+    totals[1] = cr;
   }
 }
 
@@ -1071,61 +1148,262 @@ __device__ __forceinline__ hpg_loc_t located(const DevIndex& X, uint32_t sa, uin
   return o;
 }
 
-// Locate with the whole suffix array: a thread per hit locates the hit's rows,
-// one gather each; hits of more than 4 rows (repeats, up to the locate limit)
-// are shared by the warp, 32 rows a round.  No row items: a hit's rows land at
-// loc_off[hit] in row order.  Bound by random 32-byte sectors, one a row, and
-// the records streamed through: 2M one-row hits at 100 Mbp in 80 us, against
-// 406 us for the row items and the LF walks.
-__global__ void __launch_bounds__(kExpandTpb)
-    locate_hits_kernel(DevIndex X, const hpg_hit_t* __restrict__ hits, const uint64_t* __restrict__ loc_off,
-                       uint32_t n_hits, uint64_t n_locs, const uint64_t* __restrict__ read_offs,
-                       hpg_loc_t* __restrict__ out, unsigned long long* census, LocateSizes z) {
-  if (z.status) {  // graph form: sizes from device memory, rows checked against the output's capacity
-    if (*z.status) return;
-    n_hits = (uint32_t)*z.n_hits;
-    n_locs = *z.n_locs;
-    if (n_locs > z.locs_cap) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(z.status, kStatusLocFull);
-      return;
+// Row item of a hit: direction = type ? dir : !dir, type = !strand; the length by its edit.
+__device__ __forceinline__ uint32_t item_phys_len(uint32_t meta, uint32_t rs, uint32_t len) {
+  const uint32_t err = (meta >> 1) & 1u ? (meta >> 2) & 3u : 0u;
+  return (((meta ^ rs) & 1u) << 31) | (len - (err == 1 ? 1u : 0u) + (err == 3 ? 1u : 0u));
+}
+
+// Hit records and located rows of every list, at the places the tiles' sums and a scan
+// over the tile give.  A lane per list; lists of several hits, and hits of more than 4
+// rows (repeats, up to the locate limit), are shared by the warp.  With the whole
+// suffix array a row costs one gather, so nothing is staged between the lists and the
+// records: one pass over the ordered hits (C2: one hit and one row a read, 64 bytes of
+// records) bound by HBM and one random sector a row.  Without it the hits' row offsets
+// go to loc_off for the LF walks.
+template <bool DIRECT, bool CENSUS>
+__global__ void __launch_bounds__(256)
+    emit_lists_kernel(DevIndex X, const PendingHit* __restrict__ sorted, const uint64_t* __restrict__ seg_off,
+                      FinalizeLists f, const uint64_t* __restrict__ read_offs, hpg_hit_t* __restrict__ hits,
+                      hpg_loc_t* __restrict__ locs, uint64_t* __restrict__ loc_off, uint64_t* __restrict__ totals,
+                      uint2* __restrict__ read_off, int part_is_prefix, int no_locs, unsigned long long* census,
+                      LocateSizes z) {
+  extern __shared__ uint32_t s_off[];  // the tile's first hit and first row per list
+  __shared__ uint64_t s_red[2][8];
+  __shared__ uint32_t s_warp[2][8];
+  if (z.status && *z.status & ~kStatusLocFull) return;
+  const uint32_t tile = f.tile, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t n_rs = f.n_reads_dev ? min(f.n_rs, 2u * *f.n_reads_dev) : f.n_rs;
+  const uint32_t base = blockIdx.x * tile;
+  if (base >= n_rs && base) return;
+  const bool last_tile = n_rs - base <= tile;  // (of an empty batch: the first)
+  // hits and rows before the tile
+  uint64_t h0 = 0, r0 = 0;
+  if (part_is_prefix) {
+    h0 = f.part[blockIdx.x].x;
+    r0 = f.part[blockIdx.x].y;
+  } else {
+    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += 256) {
+      const ulonglong2 v = f.part[t];
+      h0 += v.x;
+      r0 += v.y;
+    }
+    h0 = warp_sum64(h0);
+    r0 = warp_sum64(r0);
+    if (lane == 0) {
+      s_red[0][warp] = h0;
+      s_red[1][warp] = r0;
+    }
+    __syncthreads();
+    h0 = r0 = 0;
+    for (int w = 0; w < 8; ++w) {
+      h0 += s_red[0][w];
+      r0 += s_red[1][w];
     }
   }
-  const uint32_t lane = threadIdx.x & 31;
-  unsigned long long rows = 0;
-  for (uint64_t h0 = (uint64_t)blockIdx.x * kExpandTpb; h0 < n_hits; h0 += (uint64_t)gridDim.x * kExpandTpb) {
-    const uint64_t h = h0 + threadIdx.x;
-    uint32_t cnt = 0, k = 0, phys_len = 0;
-    uint64_t b = 0;
-    if (h < n_hits) {
-      b = loc_off[h];
-      cnt = (uint32_t)(loc_off[h + 1] - b);
-      if (cnt) {
-        const hpg_hit_t x = hits[h];
-        const uint64_t len = read_offs[x.read + 1] - read_offs[x.read];
-        const uint32_t err = x.nm ? x.err_kind : 0u;
-        const uint32_t phys = (uint32_t)x.dir ^ (uint32_t)x.strand;  // direction = type ? dir : !dir, type = !strand
-        phys_len = (phys << 31) | (uint32_t)(len - (err == 1 ? 1 : 0) + (err == 3 ? 1 : 0));
-        k = (uint32_t)x.k;
+  // exclusive scan over the tile's lists (rows saturate per list only past every capacity)
+  uint64_t ch = 0, cr = 0;  // of the rounds before
+  for (uint32_t i0 = 0; i0 < tile; i0 += 256) {
+    const uint32_t i = i0 + threadIdx.x;
+    const bool in = base + i < n_rs;
+    const uint32_t kh = in ? f.kept[base + i] : 0u, kr = in && !no_locs ? f.list_rows[base + i] : 0u;
+    uint32_t a = kh, b = kr;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, a, o), y = __shfl_up_sync(0xFFFFFFFFu, b, o);
+      if (lane >= (uint32_t)o) {
+        a += x;
+        b += y;
       }
     }
-    rows += cnt;
-    if (cnt <= 4) {
-      const uint32_t* sa = (phys_len >> 31) ? X.dir[1].sa : X.dir[0].sa;
-      for (uint32_t i = 0; i < cnt; ++i) out[b + i] = located(X, load_row_word(sa + k + i), phys_len, (uint32_t)h);
+    if (lane == 31) {
+      s_warp[0][warp] = a;
+      s_warp[1][warp] = b;
     }
-    unsigned big = __ballot_sync(0xFFFFFFFFu, cnt > 4);
-    while (big) {
-      const int j = __ffs(big) - 1;
-      big &= big - 1;
-      const uint32_t cj = __shfl_sync(0xFFFFFFFFu, cnt, j), kj = __shfl_sync(0xFFFFFFFFu, k, j);
-      const uint32_t pj = __shfl_sync(0xFFFFFFFFu, phys_len, j);
-      const uint64_t bj = __shfl_sync(0xFFFFFFFFu, b, j);
-      const uint32_t hj = (uint32_t)__shfl_sync(0xFFFFFFFFu, h, j);
-      const uint32_t* sa = (pj >> 31) ? X.dir[1].sa : X.dir[0].sa;
-      for (uint32_t i = lane; i < cj; i += 32) out[bj + i] = located(X, load_row_word(sa + kj + i), pj, hj);
+    __syncthreads();
+    uint32_t pa = 0, pb = 0, ta = 0, tb = 0;
+    for (uint32_t w = 0; w < 8; ++w) {
+      if (w < warp) {
+        pa += s_warp[0][w];
+        pb += s_warp[1][w];
+      }
+      ta += s_warp[0][w];
+      tb += s_warp[1][w];
+    }
+    s_off[i] = (uint32_t)ch + pa + a - kh;
+    s_off[tile + i] = (uint32_t)cr + pb + b - kr;
+    ch += ta;
+    cr += tb;
+    __syncthreads();
+    if (base + i0 + 256 >= n_rs) break;
+  }
+  // (a tile whose rows pass 32 bits lies past locs_cap: found here from the exact sums)
+  bool full = false;
+  if (!no_locs && z.status) {
+    const uint64_t end = !part_is_prefix ? r0 + f.part[blockIdx.x].y
+                                         : (blockIdx.x + 1 < gridDim.x ? f.part[blockIdx.x + 1].y : totals[1]);
+    full = end > z.locs_cap;
+    if (full && threadIdx.x == 0) atomicOr(z.status, kStatusLocFull);
+  }
+  if (last_tile && threadIdx.x == 0) {
+    if (!part_is_prefix) {
+      totals[0] = h0 + f.part[blockIdx.x].x;
+      totals[1] = no_locs ? 0 : r0 + f.part[blockIdx.x].y;
+      if (n_rs == 0) totals[0] = totals[1] = 0;
+    }
+    if (read_off) read_off[n_rs >> 1] = make_uint2((uint32_t)(h0 + ch), (uint32_t)(r0 + cr));
+    if (!DIRECT) loc_off[h0 + ch] = r0 + cr;
+  }
+  unsigned long long sectors = 0;
+  for (uint32_t i0 = 0; i0 < tile && base + i0 < n_rs; i0 += 256) {
+    const uint32_t i = i0 + threadIdx.x, rs = base + i;
+    const bool in = rs < n_rs;
+    uint32_t m = in ? f.kept[rs] : 0u;
+    const uint32_t rows = in && !no_locs && !full ? f.list_rows[rs] : 0u;
+    const uint64_t oh = h0 + s_off[i], orow = r0 + s_off[tile + i];
+    if (m > kBigHits || rows > kBigRows) {  // (the list has room for every such list)
+      const unsigned q = atomicAdd(f.n_bigs, 1u);
+      if (q < f.bigs_cap) f.bigs[q] = make_uint4(rs, (uint32_t)oh, (uint32_t)orow, rows);
+      m = 0;
+    }
+    if (read_off && in && !(rs & 1u)) read_off[rs >> 1] = make_uint2((uint32_t)oh, (uint32_t)orow);
+    uint64_t b = 0;
+    uint32_t len = 0;
+    if (m) {
+      b = seg_off[rs];
+      len = (uint32_t)(read_offs[(rs >> 1) + 1] - read_offs[rs >> 1]);
+    }
+    auto locate = [&](uint64_t at, uint32_t row, uint32_t pl, uint32_t h, uint32_t sa1 = 0) {
+      const uint32_t* sa = (pl >> 31) ? X.dir[1].sa : X.dir[0].sa;
+      locs[at] = located(X, sa1 ? sa1 - 1 : load_row_word(sa + row), pl, h);
+      if (CENSUS) sectors += sa1 ? 0 : 1;
+    };
+    // the rows of 32 hits, one a lane (r rows each from `at` on): up to 4 by the lane, more by the warp
+    auto write_rows = [&](uint64_t at, uint32_t k, uint32_t r, uint32_t pl, uint32_t h, uint32_t sa1) {
+      if (r == 1) locate(at, k, pl, h, sa1);
+      else if (r <= 4)
+        for (uint32_t q = 0; q < r; ++q) locate(at + q, k + q, pl, h);
+      unsigned many = __ballot_sync(0xFFFFFFFFu, r > 4);
+      while (many) {
+        const int j = __ffs(many) - 1;
+        many &= many - 1;
+        const uint32_t rj = __shfl_sync(0xFFFFFFFFu, r, j), kj = __shfl_sync(0xFFFFFFFFu, k, j);
+        const uint32_t pj = __shfl_sync(0xFFFFFFFFu, pl, j), hj = __shfl_sync(0xFFFFFFFFu, h, j);
+        const uint64_t aj = __shfl_sync(0xFFFFFFFFu, at, j);
+        for (uint32_t q = lane; q < rj; q += 32) locate(aj + q, kj + q, pj, hj);
+      }
+    };
+    {  // lists of one hit
+      PendingHit x;
+      x.k = x.l = x.meta = x.sa1 = 0;
+      if (m == 1) {
+        x = sorted[b];
+        hits[oh] = hit_record(x, rs);
+        if (!DIRECT) loc_off[oh] = orow;
+      }
+      if (DIRECT) write_rows(orow, x.k, m == 1 ? rows : 0u, item_phys_len(x.meta, rs, len), (uint32_t)oh, x.sa1);
+    }
+    unsigned some = __ballot_sync(0xFFFFFFFFu, m > 1);
+    while (some) {
+      const int j = __ffs(some) - 1;
+      some &= some - 1;
+      const uint64_t bj = __shfl_sync(0xFFFFFFFFu, b, j), hj = __shfl_sync(0xFFFFFFFFu, oh, j);
+      const uint64_t rj = __shfl_sync(0xFFFFFFFFu, orow, j);
+      const uint32_t mj = __shfl_sync(0xFFFFFFFFu, m, j), lj = __shfl_sync(0xFFFFFFFFu, len, j);
+      const uint32_t sj = __shfl_sync(0xFFFFFFFFu, rs, j);
+      const bool any = __shfl_sync(0xFFFFFFFFu, rows, j) != 0;
+      PendingHit x;
+      x.k = 1;
+      x.l = 0;
+      x.meta = x.sa1 = 0;
+      const bool has = lane < mj;
+      if (has) {
+        x = sorted[bj + lane];
+        hits[hj + lane] = hit_record(x, sj);
+      }
+      const uint32_t r = any && has ? rows_of(x) : 0u;
+      uint32_t incl = r;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+      }
+      if (!DIRECT && has) loc_off[hj + lane] = rj + incl - r;
+      if (DIRECT) write_rows(rj + incl - r, x.k, r, item_phys_len(x.meta, sj, lj), (uint32_t)(hj + lane), x.sa1);
     }
   }
-  if (census && rows) atomicAdd(census, rows);
+  if (CENSUS && census && sectors) atomicAdd(census, sectors);
+}
+
+// The lists the emit kernel left, a block each: 256 hits a round, their rows scanned over
+// the block and shared out evenly, a row a thread, so that neither a list of a thousand
+// hits nor a hit of ten thousand rows holds a warp.
+template <bool DIRECT, bool CENSUS>
+__global__ void __launch_bounds__(256)
+    emit_big_kernel(DevIndex X, const PendingHit* __restrict__ sorted, const uint64_t* __restrict__ seg_off,
+                    FinalizeLists f, const uint64_t* __restrict__ read_offs, hpg_hit_t* __restrict__ hits,
+                    hpg_loc_t* __restrict__ locs, uint64_t* __restrict__ loc_off, unsigned long long* census,
+                    const unsigned* gate) {
+  __shared__ uint32_t s_off[257], s_k[256], s_pl[256], s_warp[8];
+  if (gate && *gate & ~kStatusLocFull) return;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t n = min(*f.n_bigs, f.bigs_cap);
+  unsigned long long sectors = 0;
+  for (uint32_t item = blockIdx.x; item < n; item += gridDim.x) {
+    const uint4 e = f.bigs[item];
+    const uint32_t rs = e.x, m = f.kept[rs];
+    const uint64_t b = seg_off[rs], oh = e.y;
+    uint64_t orow = e.z;
+    const uint32_t len = (uint32_t)(read_offs[(rs >> 1) + 1] - read_offs[rs >> 1]);
+    for (uint32_t q0 = 0; q0 < m; q0 += 256) {
+      const uint32_t q = q0 + threadIdx.x;
+      PendingHit x;
+      x.k = 1;
+      x.l = 0;
+      x.meta = 0;
+      if (q < m) {
+        x = sorted[b + q];
+        hits[oh + q] = hit_record(x, rs);
+      }
+      const uint32_t r = e.w && q < m ? rows_of(x) : 0u;
+      uint32_t incl = r;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+      }
+      if (lane == 31) s_warp[warp] = incl;
+      __syncthreads();
+      uint32_t before = 0, total = 0;
+      for (uint32_t w = 0; w < 8; ++w) {
+        if (w < warp) before += s_warp[w];
+        total += s_warp[w];
+      }
+      const uint32_t first = before + incl - r;
+      if (!DIRECT && q < m) loc_off[oh + q] = orow + first;
+      if (DIRECT) {
+        s_off[threadIdx.x] = first;
+        s_k[threadIdx.x] = x.k;
+        s_pl[threadIdx.x] = item_phys_len(x.meta, rs, len);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < total; i += 256) {
+          uint32_t lo = 0, hi = min(256u, m - q0);  // last hit of the round with s_off <= i
+          while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (s_off[mid] <= i) lo = mid;
+            else hi = mid;
+          }
+          const uint32_t pl = s_pl[lo];
+          const uint32_t* sa = (pl >> 31) ? X.dir[1].sa : X.dir[0].sa;
+          locs[orow + i] = located(X, load_row_word(sa + s_k[lo] + (i - s_off[lo])), pl, (uint32_t)(oh + q0 + lo));
+          if (CENSUS) ++sectors;
+        }
+      }
+      orow += total;
+      __syncthreads();  // s_warp and the round's hits are rewritten
+    }
+  }
+  if (CENSUS && census && sectors) atomicAdd(census, sectors);
 }
 
 // The same for caller-built rows: a thread per item.
@@ -1390,35 +1668,50 @@ void launch_scatter_hits(const PendingHit* res, const unsigned int* res_total, c
 
 size_t long_lists_cap(size_t res_cap) { return res_cap / (kLongList + 1) + 2; }
 
-void launch_sort_truncate(PendingHit* sorted, PendingHit* scratch, const uint64_t* seg_off, uint32_t n_rs,
-                          uint32_t max_results, uint32_t* kept, uint8_t* trunc, int num_sms, cudaStream_t s,
-                          const uint32_t* max_dev, const unsigned* gate, uint32_t* longs, unsigned* n_longs,
-                          uint32_t longs_cap) {
-  if (!n_rs) return;
-  const uint32_t cap = longs ? longs_cap : 0u;
-  count_launches(1);
-  sort_truncate_kernel<<<(n_rs + 255) / 256, 256, 0, s>>>(sorted, seg_off, n_rs, max_results, kept, trunc, max_dev,
-                                                          gate, longs, n_longs, cap);
-  uint64_t blocks = ((uint64_t)n_rs + kRankTpb - 1) / kRankTpb;
-  if (blocks > 2ull * (uint64_t)num_sms) blocks = 2ull * (uint64_t)num_sms;
-  count_launches(1);
-  sort_long_lists_kernel<<<(unsigned)blocks, kRankTpb, 0, s>>>(sorted, scratch, seg_off, n_rs, kept, gate, longs,
-                                                               n_longs, cap);
+size_t big_lists_cap(uint64_t hits, uint64_t rows) { return hits / (kBigHits + 1) + rows / (kBigRows + 1) + 2; }
+
+size_t finalize_tiles(uint32_t n_rs) { return (n_rs + finalize_tile(n_rs) - 1) / finalize_tile(n_rs) + 1; }
+
+void launch_order_lists(PendingHit* sorted, PendingHit* scratch, const uint64_t* seg_off, FinalizeLists& f,
+                        int num_sms, cudaStream_t s, const unsigned* gate) {
+  f.tile = finalize_tile(f.n_rs);
+  if (!f.n_rs) return;
+  count_launches(2);
+  order_lists_kernel<<<(f.n_rs + f.tile - 1) / f.tile, 256, 0, s>>>(sorted, seg_off, f, gate);
+  sort_long_lists_kernel<<<(unsigned)(2 * num_sms), kRankTpb, 0, s>>>(sorted, scratch, seg_off, f, gate);
 }
 
-void launch_expand_hits(const PendingHit* sorted, const uint64_t* seg_off, const uint64_t* hit_off,
-                        const uint32_t* kept, uint32_t n_rs, hpg_hit_t* hits, uint32_t* rows, cudaStream_t s,
-                        const unsigned* gate, const uint32_t* longs, const unsigned* n_longs, uint32_t longs_cap,
-                        int num_sms) {
-  if (!n_rs) return;
+void launch_tile_sums(const FinalizeLists& f, uint64_t* totals, cudaStream_t s) {
   count_launches(1);
-  expand_hits_kernel<<<(n_rs + 255) / 256, 256, 0, s>>>(sorted, seg_off, hit_off, kept, n_rs, hits, rows, gate,
-                                                        longs ? 1 : 0);
-  if (longs) {
-    count_launches(1);
-    expand_long_hits_kernel<<<2 * num_sms, 256, 0, s>>>(sorted, seg_off, hit_off, kept, hits, rows, gate, longs,
-                                                        n_longs, longs_cap);
+  tile_sums_kernel<<<1, 1024, 0, s>>>(f.part, f.n_rs ? (f.n_rs + f.tile - 1) / f.tile : 0, totals, 0);
+}
+
+void launch_emit_lists(const DevIndex& X, const PendingHit* sorted, const uint64_t* seg_off, const FinalizeLists& f,
+                       const uint64_t* read_offs, hpg_hit_t* hits, hpg_loc_t* locs, uint64_t* loc_off,
+                       uint64_t* totals, uint2* read_off, bool no_locs, unsigned long long* census, int num_sms,
+                       cudaStream_t s, const LocateSizes& z) {
+  if (!f.n_rs) {
+    cudaMemsetAsync(totals, 0, 16, s);
+    return;
   }
+  const uint32_t tiles = (f.n_rs + f.tile - 1) / f.tile;
+  const int prefix = tiles > 4096;
+  if (prefix) {  // (fewer: every block adds up the tiles before its own)
+    count_launches(1);
+    tile_sums_kernel<<<1, 1024, 0, s>>>(f.part, tiles, totals, 1);
+  }
+  const size_t smem = 2 * f.tile * sizeof(uint32_t);
+  count_launches(1);
+  count_launches(1);
+  const unsigned big_grid = (unsigned)(4 * num_sms);
+  auto launch = [&](auto lists, auto big) {
+    lists<<<tiles, 256, smem, s>>>(X, sorted, seg_off, f, read_offs, hits, locs, loc_off, totals, read_off, prefix,
+                                   no_locs, census, z);
+    big<<<big_grid, 256, 0, s>>>(X, sorted, seg_off, f, read_offs, hits, locs, loc_off, census, z.status);
+  };
+  if (X.text && census) launch(emit_lists_kernel<true, true>, emit_big_kernel<true, true>);
+  else if (X.text) launch(emit_lists_kernel<true, false>, emit_big_kernel<true, false>);
+  else launch(emit_lists_kernel<false, false>, emit_big_kernel<false, false>);
 }
 
 void launch_locate_persistent(const DevIndex& X, const hpg_hit_t* hits, const uint64_t* loc_off, uint32_t n_hits,
@@ -1426,14 +1719,6 @@ void launch_locate_persistent(const DevIndex& X, const hpg_hit_t* hits, const ui
                               unsigned int* row_ctr, unsigned long long* census, int num_sms, cudaStream_t s,
                               const LocateSizes& z) {
   if (!n_locs) return;
-  if (X.text) {
-    count_launches(1);
-    // graph form: grid-stride over the hits, 8 blocks per SM
-    const uint64_t grid = z.status ? 8ull * num_sms : ((uint64_t)n_hits + kExpandTpb - 1) / kExpandTpb;
-    locate_hits_kernel<<<(unsigned)(grid ? grid : 1), kExpandTpb, 0, s>>>(X, hits, loc_off, n_hits, n_locs, read_offs,
-                                                                          out, census, z);
-    return;
-  }
   RowItem* items = static_cast<RowItem*>(row_items);
   unsigned int* side = row_ctr + 1;  // two counters after the row claim counter
   cudaMemsetAsync(side, 0, 8, s);
@@ -1548,7 +1833,8 @@ void launch_search_stage(const DevIndex& X, const BatchedParams& p, const Batche
       pw.rows_n = ctr + 11;
       launch_text_search(X, pw, num_sms, s);
       mark();
-    } else {
+      return;
+    }
     if (t.dir_split == 2) {
       pw.dir_split = 2;
       launch_wave_search(X, pw, t, num_sms, s);
@@ -1572,7 +1858,6 @@ void launch_search_stage(const DevIndex& X, const BatchedParams& p, const Batche
     // queued change points' branches, eight per change point; the blocks among
     // them join the block list, which the fused kernel's drain then empties
     launch_wave_branches(X, p, blocks, ctr + 13, block_cap, num_sms, s);
-    }
     BatchedParams pb = p;
     pb.spill = blocks;
     pb.spill_head = ctr + 12;

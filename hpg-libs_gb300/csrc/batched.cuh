@@ -28,7 +28,7 @@ struct PendingHit {
   uint32_t key;   // emission order within the (read, strand) list
   uint32_t k, l;
   uint32_t meta;  // packed as pack_meta()
-  uint32_t idx;   // unused (list positions are assigned by the scatter kernel)
+  uint32_t sa1;   // of a one-row hit whose SA value the search came by: that value + 1; else 0
 };
 
 // A spilled change point.
@@ -179,31 +179,53 @@ void launch_search_stage(const DevIndex& X, const BatchedParams& p, const Batche
                          unsigned int* ctr, uint32_t* long_list, uint32_t long_cap, SpillEntry* blocks,
                          uint32_t block_cap, cudaEvent_t mid, bool external, cudaStream_t s);
 
-// Finalize: scatter pending hits into (read, strand) segments, sort each by
-// key, truncate; kept counts to `kept`, truncation flags to `trunc`.
-// In the graph form `gate` (the search status word) skips the stage after a
-// pool overflow and `max_dev` holds max_results.
+// Finalize: scatter pending hits into (read, strand) segments, order each list, emit.
+// In the graph form `gate` (the search status word) skips the stage after a pool overflow.
 void launch_scatter_hits(const PendingHit* res, const unsigned int* res_total, const uint64_t* seg_off,
                          PendingHit* sorted, uint32_t res_cap, uint32_t* cursor, cudaStream_t s,
                          const unsigned* gate = nullptr);
-// Sorts every (read, strand) list by emission key and keeps the first max_results
-// (from max_dev when given); `scratch` holds at least as many entries as
-// `sorted` and its contents are overwritten (the scatter's input is dead by then).
-// With `longs` (longs_cap = long_lists_cap(entries of the pool) entries) and a
-// zeroed counter `n_longs`, the lists above kLongList entries are collected by
-// the short sort and the long sort visits only them; without, it scans every list.
-void launch_sort_truncate(PendingHit* sorted, PendingHit* scratch, const uint64_t* seg_off, uint32_t n_rs,
-                          uint32_t max_results, uint32_t* kept, uint8_t* trunc, int num_sms, cudaStream_t s,
-                          const uint32_t* max_dev = nullptr, const unsigned* gate = nullptr, uint32_t* longs = nullptr,
-                          unsigned* n_longs = nullptr, uint32_t longs_cap = 0);
+// The (read, strand) lists of a batch: what is kept of each, and the sums of their
+// tiles (finalize_tiles entries), which order them in the outputs.
+struct FinalizeLists {
+  uint32_t n_rs = 0;       // lists (of the capacity, when n_reads_dev holds the reads)
+  uint32_t tile = 0;       // set by launch_order_lists
+  uint32_t max_results = 0;
+  uint64_t limit = 0;      // locate limit, 0: none
+  const uint32_t* n_reads_dev = nullptr;  // graph form: read from device memory
+  const uint32_t* max_dev = nullptr;
+  const uint64_t* limit_dev = nullptr;
+  uint32_t* kept = nullptr;
+  uint8_t* trunc = nullptr;
+  uint32_t* list_rows = nullptr;
+  ulonglong2* part = nullptr;
+  // ids of the lists above kLongList entries (long_lists_cap of the pool's entries) and
+  // their number, zeroed by the caller
+  uint32_t* longs = nullptr;
+  unsigned* n_longs = nullptr;
+  uint32_t longs_cap = 0;
+  // lists the emit kernel leaves to a block each (big_lists_cap of the hits and rows), as longs
+  uint4* bigs = nullptr;
+  unsigned* n_bigs = nullptr;
+  uint32_t bigs_cap = 0;
+};
+size_t big_lists_cap(uint64_t hits, uint64_t rows);
+size_t finalize_tiles(uint32_t n_rs);
 // Room for the ids of the lists longer than kLongList entries among res_cap entries.
 size_t long_lists_cap(size_t res_cap);
-// With the long-list work list of launch_sort_truncate, those lists' records are
-// written a block per list.
-void launch_expand_hits(const PendingHit* sorted, const uint64_t* seg_off, const uint64_t* hit_off,
-                        const uint32_t* kept, uint32_t n_rs, hpg_hit_t* hits, uint32_t* rows, cudaStream_t s,
-                        const unsigned* gate = nullptr, const uint32_t* longs = nullptr,
-                        const unsigned* n_longs = nullptr, uint32_t longs_cap = 0, int num_sms = 152);
+// Sorts every list by emission key and keeps the first max_results; `scratch` holds at
+// least as many entries as `sorted` and is overwritten (the scatter's input is dead by then).
+void launch_order_lists(PendingHit* sorted, PendingHit* scratch, const uint64_t* seg_off, FinalizeLists& f,
+                        int num_sms, cudaStream_t s, const unsigned* gate = nullptr);
+// The batch's hits and rows (totals[0], totals[1]) before its outputs are allocated.
+void launch_tile_sums(const FinalizeLists& f, uint64_t* totals, cudaStream_t s);
+// Hit records, and located rows where the index has its whole suffix array; else the
+// hits' row offsets (loc_off, hits + 1 entries) for launch_locate_persistent.  totals as
+// above; read_off (when given) the first hit and row of every read, and the batch's end.
+// no_locs: hits only.
+void launch_emit_lists(const DevIndex& X, const PendingHit* sorted, const uint64_t* seg_off, const FinalizeLists& f,
+                       const uint64_t* read_offs, hpg_hit_t* hits, hpg_loc_t* locs, uint64_t* loc_off,
+                       uint64_t* totals, uint2* read_off, bool no_locs, unsigned long long* census, int num_sms,
+                       cudaStream_t s, const LocateSizes& z = LocateSizes());
 
 // Persistent locate: lanes pull rows from a counter and refill when their walk
 // ends.  In the graph form n_hits / n_locs are capacities and `z` the sizes.

@@ -30,8 +30,9 @@ __device__ __forceinline__ uint32_t order_key(uint32_t section, uint32_t t, uint
 // the list position is assigned later by the scatter kernel.
 constexpr unsigned kResChunk = 8;
 
+// sa1: of a one-row hit whose SA value is known, that value plus one.
 __device__ __forceinline__ void write_hit(const BatchedParams& p, unsigned slot, uint32_t rs, uint32_t key,
-                                          uint32_t k, uint32_t l, uint32_t meta) {
+                                          uint32_t k, uint32_t l, uint32_t meta, uint32_t sa1 = 0) {
   atomicAdd(&p.rs_count[rs], 1u);  // result unused: compiles to a reduction
   if (slot < p.res_cap) {
     PendingHit h;
@@ -40,7 +41,7 @@ __device__ __forceinline__ void write_hit(const BatchedParams& p, unsigned slot,
     h.k = k;
     h.l = l;
     h.meta = meta;
-    h.idx = 0;
+    h.sa1 = sa1;
     p.res[slot] = h;
   } else {
     atomicOr(p.status, kStatusResFull);

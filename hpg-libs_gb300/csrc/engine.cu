@@ -245,7 +245,7 @@ void engine_release_workspace(Engine* e, uint64_t keep_n_cap) {
   DevBuf* bufs[] = {&e->seqs, &e->offs, &e->codes, &e->ok, &e->rs_count, &e->rs_trunc, &e->vecs, &e->slots,
                     &e->ovf, &e->ovf_count, &e->hit_off, &e->scan_part, &e->hits, &e->rows, &e->loc_off, &e->locs,
                     &e->b_res, &e->b_sorted, &e->b_spill, &e->b_arr, &e->b_seg, &e->b_rowhit, &e->b_long,
-                    &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->m_hitoff, &e->m_part, &e->m_offs, &e->m_rows, &e->m_pflag,
+                    &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->b_lists, &e->b_bigs, &e->m_hitoff, &e->m_part, &e->m_offs, &e->m_rows, &e->m_pflag,
                     &e->m_rowoff, &e->m_nrec, &e->m_flags, &e->m_rec};
   for (DevBuf* b : bufs) {
     cudaFree(b->p);
@@ -282,7 +282,7 @@ void engine_destroy(Engine* e) {
   DevBuf* bufs[] = {&e->seqs, &e->offs, &e->codes, &e->ok, &e->rs_count, &e->rs_trunc, &e->vecs, &e->slots,
                     &e->ovf, &e->ovf_count, &e->hit_off, &e->scan_part, &e->hits, &e->rows, &e->loc_off, &e->locs,
                     &e->census, &e->b_ctr, &e->b_res, &e->b_sorted, &e->b_spill, &e->b_arr, &e->b_seg,
-                    &e->b_rowhit, &e->b_long, &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->m_hitoff, &e->m_part, &e->m_offs,
+                    &e->b_rowhit, &e->b_long, &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->b_lists, &e->b_bigs, &e->m_hitoff, &e->m_part, &e->m_offs,
                     &e->m_rows, &e->m_pflag, &e->m_rowoff, &e->m_nrec, &e->m_flags, &e->m_rec};
   for (DevBuf* b : bufs) cudaFree(b->p);
   for (int i = 0; i <= kStageCount; ++i)
@@ -410,46 +410,64 @@ int run_batched(Engine* e, uint64_t total_bases, const uint64_t* d_offs, uint32_
   }
   // ordered finalize
   launch_scan(ptr<uint32_t>(e->b_arr), T, ptr<uint64_t>(e->b_seg), ptr<uint64_t>(e->scan_part), s);
-  cudaMemsetAsync(e->hit_off.p, 0, T * 4, s);  // per-list cursors (hit_off is rewritten below)
+  cudaMemsetAsync(e->hit_off.p, 0, T * 4, s);  // per-list cursors
   launch_scatter_hits(ptr<PendingHit>(e->b_res), ctr + 3, ptr<uint64_t>(e->b_seg), ptr<PendingHit>(e->b_sorted),
                       e->b_res_cap, ptr<uint32_t>(e->hit_off), s);
-  launch_sort_truncate(ptr<PendingHit>(e->b_sorted), ptr<PendingHit>(e->b_res), ptr<uint64_t>(e->b_seg), (uint32_t)T,
-                       max_results, ptr<uint32_t>(e->rs_count), ptr<uint8_t>(e->rs_trunc), e->num_sms, s);
-  launch_scan(ptr<uint32_t>(e->rs_count), T, ptr<uint64_t>(e->hit_off), ptr<uint64_t>(e->scan_part), s);
-  uint64_t h_tot = 0;
-  HPG_CUDA(cudaMemcpyAsync(&h_tot, ptr<uint64_t>(e->hit_off) + T, 8, cudaMemcpyDeviceToHost, s), "hit count");
-  HPG_CUDA(cudaStreamSynchronize(s), "hit scan");
-  if (!ensure(e, e->hits, (h_tot + 1) * sizeof(hpg_hit_t)) || !ensure(e, e->rows, (h_tot + 1) * 4) ||
-      !ensure(e, e->loc_off, (h_tot + 2) * 8) || !ensure(e, e->scan_part, scan_parts(h_tot) * 8)) {
-    *err = "out of device memory (hits)";
+  FinalizeLists f;
+  f.n_rs = (uint32_t)T;
+  f.max_results = max_results;
+  f.limit = e->skip_locate ? 0 : e->locate_limit;
+  f.kept = ptr<uint32_t>(e->rs_count);
+  f.trunc = ptr<uint8_t>(e->rs_trunc);
+  f.longs_cap = (uint32_t)long_lists_cap(e->b_res_cap);
+  const size_t n_tiles = finalize_tiles((uint32_t)T);
+  if (!ensure(e, e->b_lists, n_tiles * sizeof(ulonglong2) + 16 + T * 4 + (size_t)f.longs_cap * 4 + 16)) {
+    *err = "out of device memory (batched lists)";
     return -1;
   }
-  launch_expand_hits(ptr<PendingHit>(e->b_sorted), ptr<uint64_t>(e->b_seg), ptr<uint64_t>(e->hit_off),
-                     ptr<uint32_t>(e->rs_count), (uint32_t)T, ptr<hpg_hit_t>(e->hits), ptr<uint32_t>(e->rows), s);
-  uint64_t l_tot = 0;
-  if (!e->skip_locate) {
-    launch_limit_rows(ptr<uint64_t>(e->hit_off), ptr<uint32_t>(e->rows), (uint32_t)T, e->locate_limit, nullptr,
-                      ptr<uint8_t>(e->rs_trunc), s);
-    launch_scan(ptr<uint32_t>(e->rows), h_tot, ptr<uint64_t>(e->loc_off), ptr<uint64_t>(e->scan_part), s);
-    HPG_CUDA(cudaMemcpyAsync(&l_tot, ptr<uint64_t>(e->loc_off) + h_tot, 8, cudaMemcpyDeviceToHost, s), "loc count");
-  }
-  HPG_CUDA(cudaStreamSynchronize(s), "locate scan");
+  f.part = ptr<ulonglong2>(e->b_lists);
+  uint64_t* totals = reinterpret_cast<uint64_t*>(f.part + n_tiles);
+  f.list_rows = reinterpret_cast<uint32_t*>(totals + 2);
+  f.longs = f.list_rows + T;
+  f.n_longs = ctr + 14;
+  launch_order_lists(ptr<PendingHit>(e->b_sorted), ptr<PendingHit>(e->b_res), ptr<uint64_t>(e->b_seg), f, e->num_sms, s);
+  launch_tile_sums(f, totals, s);
+  uint64_t h_totals[2] = {0, 0};
+  HPG_CUDA(cudaMemcpyAsync(h_totals, totals, 16, cudaMemcpyDeviceToHost, s), "hit count");
+  HPG_CUDA(cudaStreamSynchronize(s), "finalize");
+  const uint64_t h_tot = h_totals[0], l_tot = e->skip_locate ? 0 : h_totals[1];
   cudaEventRecord(e->cev[2], s);
   if (l_tot > kMaxLocateRows) {
     *err = "too many located rows in one batched call (" + std::to_string(l_tot) + ", limit " +
            std::to_string(kMaxLocateRows) + "): split the batch or use the plain form";
     return -1;
   }
-  if (!ensure(e, e->locs, (l_tot + 1) * sizeof(hpg_loc_t)) ||
-      !ensure(e, e->b_rowhit, (l_tot + 1) * locate_row_item_bytes())) {
-    *err = oom_message(("locate output, " + std::to_string(l_tot) + " rows of " + std::to_string(h_tot) + " hits").c_str(),
-                       (l_tot + 1) * (sizeof(hpg_loc_t) + locate_row_item_bytes()));
+  const bool walks = !e->X.text;  // located by LF walks
+  if (!ensure(e, e->hits, (h_tot + 1) * sizeof(hpg_hit_t)) || !ensure(e, e->loc_off, walks ? (h_tot + 2) * 8 : 16)) {
+    *err = "out of device memory (hits)";
     return -1;
   }
+  if (!ensure(e, e->locs, (l_tot + 1) * sizeof(hpg_loc_t)) ||
+      (walks && !ensure(e, e->b_rowhit, (l_tot + 1) * locate_row_item_bytes()))) {
+    *err = oom_message(("locate output, " + std::to_string(l_tot) + " rows of " + std::to_string(h_tot) + " hits").c_str(),
+                       (l_tot + 1) * (sizeof(hpg_loc_t) + (walks ? locate_row_item_bytes() : 0)));
+    return -1;
+  }
+  f.bigs_cap = (uint32_t)big_lists_cap(h_tot, l_tot);
+  if (!ensure(e, e->b_bigs, (size_t)f.bigs_cap * sizeof(uint4))) {
+    *err = "out of device memory (batched lists)";
+    return -1;
+  }
+  f.bigs = ptr<uint4>(e->b_bigs);
+  f.n_bigs = ctr + 15;
   if (census) cudaMemsetAsync(census, 0, 8, s);
-  cudaMemsetAsync(ctr + 5, 0, 12, s);  // row claim counter and the two direction counters
-  launch_locate_persistent(e->X, ptr<hpg_hit_t>(e->hits), ptr<uint64_t>(e->loc_off), (uint32_t)h_tot, l_tot, d_offs,
-                           ptr<hpg_loc_t>(e->locs), e->b_rowhit.p, ctr + 5, census, e->num_sms, s);
+  launch_emit_lists(e->X, ptr<PendingHit>(e->b_sorted), ptr<uint64_t>(e->b_seg), f, d_offs, ptr<hpg_hit_t>(e->hits),
+                    ptr<hpg_loc_t>(e->locs), ptr<uint64_t>(e->loc_off), totals, nullptr, e->skip_locate, census, e->num_sms, s);
+  if (walks && !e->skip_locate) {
+    cudaMemsetAsync(ctr + 5, 0, 12, s);  // row claim counter and the two direction counters
+    launch_locate_persistent(e->X, ptr<hpg_hit_t>(e->hits), ptr<uint64_t>(e->loc_off), (uint32_t)h_tot, l_tot, d_offs,
+                             ptr<hpg_loc_t>(e->locs), e->b_rowhit.p, ctr + 5, census, e->num_sms, s);
+  }
   cudaEventRecord(e->cev[3], s);
   HPG_CUDA(cudaStreamSynchronize(s), "locate kernel");
   if (census) {
@@ -827,7 +845,8 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
     }
     packed = ptr<uint64_t>(e->b_packed) + kPackedPad;
   }
-  launch_encode(d_seqs, total_bases, d_offs, n, e->d_table, ptr<uint8_t>(e->codes), ptr<uint8_t>(e->ok), s, packed);
+  launch_encode(d_seqs, total_bases, d_offs, n, e->d_table, packed ? nullptr : ptr<uint8_t>(e->codes),
+                ptr<uint8_t>(e->ok), s, packed);
   cudaEventRecord(e->ev[1], s);
 
   size_t n_hits = 0, n_locs = 0;
@@ -906,7 +925,7 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
       return -1;
     }
     launch_hit_rows(hits, (uint32_t)h_tot, ptr<uint32_t>(e->rows), s);
-    launch_limit_rows(ptr<uint64_t>(e->hit_off), ptr<uint32_t>(e->rows), (uint32_t)T, e->locate_limit, nullptr,
+    launch_limit_rows(ptr<uint64_t>(e->hit_off), ptr<uint32_t>(e->rows), (uint32_t)T, e->locate_limit,
                       ptr<uint8_t>(e->rs_trunc) + 2 * r0, s);
     launch_scan(ptr<uint32_t>(e->rows), h_tot, ptr<uint64_t>(e->loc_off), ptr<uint64_t>(e->scan_part), s);
     uint64_t l_tot = 0;

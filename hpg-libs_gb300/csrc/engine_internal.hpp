@@ -59,7 +59,7 @@ struct GraphPlan {
                             // [11] long-read claims [12] block head [13] block tail [14] long lists
   uint32_t* arr = nullptr;  // arrivals per (read, strand)
   uint64_t* seg = nullptr;
-  uint64_t* hit_off = nullptr;
+  uint32_t* cursor = nullptr;
   uint32_t* kept = nullptr;
   uint8_t* trunc = nullptr;
   uint64_t* part = nullptr;
@@ -67,8 +67,12 @@ struct GraphPlan {
   PendingHit* sorted = nullptr;
   SpillEntry* spill = nullptr;
   hpg_hit_t* hits = nullptr;
-  uint32_t* rows = nullptr;
-  uint64_t* loc_off = nullptr;
+  uint32_t* list_rows = nullptr;
+  ulonglong2* tiles = nullptr;
+  uint64_t* totals = nullptr;   // hits and located rows of the batch
+  uint4* bigs = nullptr;        // lists of many hits or rows (ctr[15] counts them)
+  uint2* read_off = nullptr;    // first hit and row of each read
+  uint64_t* loc_off = nullptr;  // without the whole suffix array: first row of each hit, and the row items
   void* items = nullptr;
   hpg_loc_t* locs = nullptr;
   unsigned long long* census_d = nullptr;
@@ -112,7 +116,7 @@ struct Engine {
   DevBuf seqs, offs, codes, ok, rs_count, rs_trunc, vecs, slots, ovf, ovf_count, hit_off, scan_part, hits, rows,
       loc_off, locs, census;
   // batched form
-  DevBuf b_ctr, b_res, b_sorted, b_spill, b_arr, b_seg, b_rowhit, b_long, b_blocks;
+  DevBuf b_ctr, b_res, b_sorted, b_spill, b_arr, b_seg, b_rowhit, b_long, b_blocks, b_lists, b_bigs;
   DevBuf b_packed, b_text;  // text form (text_search.cu)
   DevBuf b_bovf;  // block search: results past a block's slots, in chunks
   // alignment-list records (map_device.cu)

@@ -285,11 +285,21 @@ __device__ __forceinline__ bool text_sampled(const uint4& m, uint32_t i, uint32_
   return (w >> (r & 31)) & 1u;
 }
 
-// One gather from the whole suffix array or its inverse: no neighbour of the
-// entry is wanted, so the line is not kept in L1.
+// One gather from an array far larger than the caches: no neighbour of the entry
+// is wanted, so the line is not kept in L1 and a miss takes 64 bytes from DRAM.  A
+// plain load's miss takes the whole 128-byte line (measured: 3.9 sectors per random
+// 4-byte load over 4 GB, 2.0 with the qualifier, at 38.8 G loads/s either way); where
+// other traffic wants the DRAM's bandwidth the difference shows (search stage of 2M x
+// 100 bp, 100 Mbp: 768 -> 721 us).
 __device__ __forceinline__ uint32_t load_row_word(const uint32_t* p) {
   uint32_t v;
-  asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm("ld.global.nc.L1::no_allocate.L2::64B.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ uint2 load_row_pair(const uint2* p) {
+  uint2 v;
+  asm("ld.global.nc.L1::no_allocate.L2::64B.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
 

@@ -79,17 +79,19 @@ void record(cudaEvent_t ev, cudaStream_t s) { cudaEventRecordWithFlags(ev, s, cu
 // Allocate the plan's buffers and capture the pipeline on the engine stream.
 int capture(Engine* e, GraphPlan* g, std::string* err) {
   const size_t T = 2ull * g->n_cap;
-  const size_t parts = std::max(scan_parts(T), scan_parts(g->res_cap));
+  const size_t parts = scan_parts(T);
   const bool text = text_form(e, g->n_cap);
   if (!grab(g, &g->seqs, g->bases_cap + 64) || !grab(g, &g->offs, ((size_t)g->n_cap + 1) * 8) ||
-      !grab(g, &g->hdr, 32) || !grab(g, &g->codes, g->bases_cap + 64) || !grab(g, &g->ok, (size_t)g->n_cap + 16) ||
+      !grab(g, &g->hdr, 32) || (!text && !grab(g, &g->codes, g->bases_cap + 64)) || !grab(g, &g->ok, (size_t)g->n_cap + 16) ||
       !grab(g, &g->ctr, 64) || !grab(g, &g->arr, T * 4 + 16) || !grab(g, &g->seg, (T + 1) * 8) ||
-      !grab(g, &g->hit_off, (T + 1) * 8) || !grab(g, &g->kept, T * 4 + 16) || !grab(g, &g->trunc, T + 16) ||
+      !grab(g, &g->cursor, T * 4 + 16) || !grab(g, &g->kept, T * 4 + 16) || !grab(g, &g->trunc, T + 16) ||
       !grab(g, &g->part, parts * 8) || !grab(g, &g->res, (size_t)g->res_cap * sizeof(PendingHit)) ||
       !grab(g, &g->sorted, (size_t)g->res_cap * sizeof(PendingHit)) ||
       !grab(g, &g->spill, (size_t)g->spill_cap * sizeof(SpillEntry)) ||
       !grab(g, &g->hits, ((size_t)g->res_cap + 1) * sizeof(hpg_hit_t)) ||
-      !grab(g, &g->rows, ((size_t)g->res_cap + 1) * 4) || !grab(g, &g->loc_off, ((size_t)g->res_cap + 2) * 8) ||
+      !grab(g, &g->list_rows, T * 4 + 16) || !grab(g, &g->tiles, finalize_tiles((uint32_t)T) * sizeof(ulonglong2)) ||
+      !grab(g, &g->totals, 16) || !grab(g, &g->bigs, big_lists_cap(g->res_cap, g->locs_cap) * sizeof(uint4)) || !grab(g, &g->read_off, ((size_t)g->n_cap + 1) * sizeof(uint2)) ||
+      (!e->X.text && !grab(g, &g->loc_off, ((size_t)g->res_cap + 2) * 8)) ||
       (!e->X.text && !grab(g, &g->items, (g->locs_cap + 1) * locate_row_item_bytes())) ||
       !grab(g, &g->locs, (g->locs_cap + 1) * sizeof(hpg_loc_t)) || !grab(g, &g->census_d, 16) ||
       !grab(g, &g->long_list, (size_t)g->long_cap * 4) || !grab(g, &g->longs, long_lists_cap(g->res_cap) * 4) ||
@@ -122,7 +124,7 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
 
   BatchedParams p;
   p.codes = g->codes;
-  p.codes_len = g->bases_cap + 64;
+  p.codes_len = g->codes ? g->bases_cap + 64 : 0;
   p.offs = g->offs;
   p.ok = g->ok;
   p.n_reads = g->n_cap;
@@ -154,25 +156,34 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
 
   // ordered finalize over the capacity (lists past the batch are empty)
   launch_scan(g->arr, T, g->seg, g->part, s);
-  cudaMemsetAsync(g->hit_off, 0, T * 4, s);  // per-list cursors (hit_off is rewritten below)
-  launch_scatter_hits(g->res, ctr + 3, g->seg, g->sorted, g->res_cap, reinterpret_cast<uint32_t*>(g->hit_off), s,
-                      status);
-  launch_sort_truncate(g->sorted, g->res, g->seg, (uint32_t)T, 0, g->kept, g->trunc, e->num_sms, s, g->hdr + 1,
-                       status, g->longs, ctr + 14, (uint32_t)long_lists_cap(g->res_cap));
-  launch_scan(g->kept, T, g->hit_off, g->part, s);
-  launch_expand_hits(g->sorted, g->seg, g->hit_off, g->kept, (uint32_t)T, g->hits, g->rows, s, status, g->longs,
-                     ctr + 14, (uint32_t)long_lists_cap(g->res_cap), e->num_sms);
-  launch_limit_rows(g->hit_off, g->rows, (uint32_t)T, 0, reinterpret_cast<const uint64_t*>(g->hdr + 2), g->trunc, s,
-                    status);
-  launch_scan(g->rows, g->res_cap, g->loc_off, g->part, s, g->hit_off + T);  // over the hits found
+  cudaMemsetAsync(g->cursor, 0, T * 4, s);
+  launch_scatter_hits(g->res, ctr + 3, g->seg, g->sorted, g->res_cap, g->cursor, s, status);
+  FinalizeLists f;
+  f.n_rs = (uint32_t)T;
+  f.n_reads_dev = g->hdr;
+  f.max_dev = g->hdr + 1;
+  f.limit_dev = reinterpret_cast<const uint64_t*>(g->hdr + 2);
+  f.kept = g->kept;
+  f.trunc = g->trunc;
+  f.list_rows = g->list_rows;
+  f.part = g->tiles;
+  f.longs = g->longs;
+  f.n_longs = ctr + 14;
+  f.longs_cap = (uint32_t)long_lists_cap(g->res_cap);
+  f.bigs = g->bigs;
+  f.n_bigs = ctr + 15;
+  f.bigs_cap = (uint32_t)big_lists_cap(g->res_cap, g->locs_cap);
+  launch_order_lists(g->sorted, g->res, g->seg, f, e->num_sms, s, status);
   record(g->ev[4], s);
 
   LocateSizes z;
   z.status = status;
-  z.n_hits = g->hit_off + T;
-  z.n_locs = g->loc_off + g->res_cap;
+  z.n_hits = g->totals;
+  z.n_locs = g->totals + 1;
   z.locs_cap = g->locs_cap;
-  if (!g->skip_locate)
+  launch_emit_lists(e->X, g->sorted, g->seg, f, g->offs, g->hits, g->locs, g->loc_off, g->totals, g->read_off,
+                    g->skip_locate, census, e->num_sms, s, z);
+  if (!g->skip_locate && !e->X.text)
     launch_locate_persistent(e->X, g->hits, g->loc_off, g->res_cap, g->locs_cap, g->offs, g->locs, g->items,
                              ctr + 5, census, e->num_sms, s, z);
   record(g->ev[5], s);

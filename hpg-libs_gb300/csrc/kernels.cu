@@ -23,15 +23,67 @@ constexpr int kTpb = 128;
 
 inline unsigned grid_for(size_t n, int tpb) { return (unsigned)((n + tpb - 1) / tpb); }
 
-// Coalesced encoding: each thread translates 16 consecutive bytes; a byte
-// outside the alphabet clears its read's flag (found by binary search over
-// the offsets; such reads are rare).
-// With `n_dev` set the read count comes from device memory and the byte count
-// is offs[n] (graph replays); the grid is then sized for the capacity.
-__global__ void encode_kernel(const uint8_t* __restrict__ ascii, uint64_t total, const uint64_t* __restrict__ offs,
-                              uint32_t n_reads, const uint8_t* __restrict__ table, uint8_t* __restrict__ codes,
-                              uint8_t* __restrict__ ok, const uint32_t* n_dev, const uint64_t* src_dev,
-                              uint32_t* __restrict__ packed) {
+// 16 bases (in w) to their codes, a byte each (in w, 0xFF outside the alphabet) and
+// packed two bits each (returned); bit i of bad: base i is outside the alphabet.
+// Four letters at a time: bits 1-2 of a letter of either case tell A, C, T and G apart
+// (0, 1, 2, 3); a byte permutation by them gives the letter they should be and its code.
+__device__ __forceinline__ uint32_t encode16(uint32_t (&w)[4], uint32_t code4, uint32_t& bad) {
+  const uint32_t letter4 = 'A' | ('C' << 8) | ('T' << 16) | ((uint32_t)'G' << 24);
+  uint32_t pk = 0, any = 0, off[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t x = (w[i] >> 1) & 0x03030303u;
+    const uint32_t pair = (x | (x >> 4)) & 0x00330033u, sel = pair | (pair >> 8);  // a nibble per byte: the selectors
+    off[i] = (w[i] & 0xDFDFDFDFu) ^ __byte_perm(letter4, 0, sel);  // 0 in the bytes of the four letters
+    any |= off[i];
+    w[i] = __byte_perm(code4, 0, sel);
+    const uint32_t two = (w[i] | (w[i] >> 6)) & 0x000F000Fu;  // two codes in each half
+    pk |= ((two | (two >> 12)) & 0xFFu) << (8 * i);
+  }
+  bad = 0;
+  if (any) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if ((off[i >> 2] >> (8 * (i & 3))) & 0xFFu) {
+        bad |= 1u << i;
+        w[i >> 2] |= 0xFFu << (8 * (i & 3));
+      }
+  }
+  return pk;
+}
+
+// The reads of the bases b + i for the bits i of bad are outside the alphabet (binary
+// search over the offsets; such reads are rare).
+__device__ __noinline__ void flag_reads(uint32_t bad, uint64_t b, const uint64_t* __restrict__ offs, uint32_t n_reads,
+                                        uint8_t* __restrict__ ok) {
+  while (bad) {
+    const int i = __ffs(bad) - 1;
+    bad &= bad - 1;
+    const uint64_t at = b + i;
+    if (at < offs[0]) continue;
+    uint32_t lo = 0, hi = n_reads;  // read r with offs[r] <= at < offs[r+1]
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (offs[mid] <= at) lo = mid;
+      else hi = mid;
+    }
+    ok[lo] = 0;
+  }
+}
+
+// Coalesced encoding: a block takes 16 KB of bases a round, a thread 16 bytes of each
+// quarter, all four loaded before the first is used.  Codes mirror the bases byte for
+// byte over [0, total) (null: packed only).  With `n_dev` set the read count comes from
+// device memory and the byte count is offs[n] (graph replays); the grid is then sized
+// for the capacity.  Bound by HBM: 200 MB of reads to packed codes.  A shared-memory
+// lookup a base and one load in flight took 146 us with byte codes besides.
+constexpr int kEncTpb = 256, kEncTile = 4 * kEncTpb;  // 16-byte pieces a round
+
+__global__ void __launch_bounds__(kEncTpb)
+    encode_kernel(const uint8_t* __restrict__ ascii, uint64_t total, const uint64_t* __restrict__ offs,
+                  uint32_t n_reads, const uint8_t* __restrict__ table, uint8_t* __restrict__ codes,
+                  uint8_t* __restrict__ ok, const uint32_t* n_dev, const uint64_t* src_dev,
+                  uint32_t* __restrict__ packed) {
   if (n_dev) {
     n_reads = *n_dev;
     const uint64_t t = offs[n_reads];
@@ -41,51 +93,44 @@ __global__ void encode_kernel(const uint8_t* __restrict__ ascii, uint64_t total,
     ascii = reinterpret_cast<const uint8_t*>(src_dev[0]);
     total = src_dev[1] < total ? src_dev[1] : total;
   }
-  __shared__ uint8_t tab[256];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) tab[i] = table[i];
-  __syncthreads();
-  // codes mirror the bases byte for byte over [0, total), 16 a thread and round
+  const uint64_t pieces = (total + 15) / 16;
+  if ((uint64_t)blockIdx.x * kEncTile >= pieces) return;
+  const uint32_t code4 = table['A'] | ((uint32_t)table['C'] << 8) | ((uint32_t)table['T'] << 16) |
+                         ((uint32_t)table['G'] << 24);
   const bool aligned = ((reinterpret_cast<uintptr_t>(ascii) | reinterpret_cast<uintptr_t>(codes)) & 15) == 0;
-  for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c * 16 < total;
-       c += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t b = c * 16;
-    uint8_t in[16], out[16];
-    const uint64_t m = total - b < 16 ? total - b : 16;
-    const bool full = aligned && m == 16;
-    if (full) {
-      *reinterpret_cast<uint4*>(in) = *reinterpret_cast<const uint4*>(ascii + b);
-    } else {
-      for (uint64_t i = 0; i < m; ++i) in[i] = ascii[b + i];
-    }
-    uint32_t bad = 0;
+  for (uint64_t c0 = (uint64_t)blockIdx.x * kEncTile; c0 < pieces; c0 += (uint64_t)gridDim.x * kEncTile) {
+    if (aligned && (c0 + kEncTile) * 16 <= total) {
+      uint4 v[4];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      out[i] = tab[in[i]];
-      if (i < (int)m && out[i] == 0xFF) bad |= 1u << i;
-    }
-    if (full) {
-      *reinterpret_cast<uint4*>(codes + b) = *reinterpret_cast<const uint4*>(out);
-    } else {
-      for (uint64_t i = 0; i < m; ++i) codes[b + i] = out[i];
-    }
-    if (packed) {
-      uint32_t w = 0;
+      for (int u = 0; u < 4; ++u)
+        v[u] = __ldcs(reinterpret_cast<const uint4*>(ascii) + c0 + u * kEncTpb + threadIdx.x);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) w |= (i < (int)m ? out[i] & 3u : 0u) << (2 * i);
-      packed[c] = w;
-    }
-    while (bad) {
-      const int i = __ffs(bad) - 1;
-      bad &= bad - 1;
-      const uint64_t at = b + i;
-      if (at < offs[0]) continue;
-      uint32_t lo = 0, hi = n_reads;  // read r with offs[r] <= at < offs[r+1]
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (offs[mid] <= at) lo = mid;
-        else hi = mid;
+      for (int u = 0; u < 4; ++u) {
+        const uint64_t c = c0 + u * kEncTpb + threadIdx.x;
+        uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w}, bad;
+        const uint32_t pk = encode16(w, code4, bad);
+        if (codes) reinterpret_cast<uint4*>(codes)[c] = make_uint4(w[0], w[1], w[2], w[3]);
+        if (packed) packed[c] = pk;
+        if (bad) flag_reads(bad, c * 16, offs, n_reads, ok);
       }
-      ok[lo] = 0;
+      continue;
+    }
+    for (int u = 0; u < 4; ++u) {  // the end, or bases that do not start on 16 bytes
+      const uint64_t c = c0 + u * kEncTpb + threadIdx.x, b = c * 16;
+      if (b >= total) break;
+      const int m = (int)(total - b < 16 ? total - b : 16);
+      uint32_t w[4] = {0x41414141u, 0x41414141u, 0x41414141u, 0x41414141u}, bad;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (i < m) w[i >> 2] = (w[i >> 2] & ~(0xFFu << (8 * (i & 3)))) | ((uint32_t)ascii[b + i] << (8 * (i & 3)));
+      const uint32_t pk = encode16(w, code4, bad);
+      if (codes) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (i < m) codes[b + i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
+      }
+      if (packed) packed[c] = pk;
+      if (bad) flag_reads(bad, b, offs, n_reads, ok);
     }
   }
 }
@@ -232,10 +277,7 @@ __device__ __forceinline__ void scan_load8(const uint32_t* __restrict__ in, size
 }
 
 __global__ void __launch_bounds__(kScanTpb) scan_reduce_kernel(const uint32_t* __restrict__ in, size_t n,
-                                                               uint64_t* __restrict__ part,
-                                                               const uint64_t* __restrict__ n_dev) {
-  if (n_dev) n = min((uint64_t)n, *n_dev);
-  if ((size_t)blockIdx.x * kScanTile > n) return;  // past the count (uniform over the block)
+                                                               uint64_t* __restrict__ part) {
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
   scan_load8(in, n, base, v);
@@ -263,11 +305,7 @@ __global__ void __launch_bounds__(1024) scan_parts_kernel(uint64_t* part, size_t
 // (few tiles); else part holds the tiles' exclusive prefixes already.
 __global__ void __launch_bounds__(kScanTpb) scan_apply_kernel(const uint32_t* __restrict__ in, size_t n,
                                                               const uint64_t* __restrict__ part,
-                                                              uint64_t* __restrict__ out, int direct,
-                                                              const uint64_t* __restrict__ n_dev) {
-  const size_t n_cap = n;
-  if (n_dev) n = min((uint64_t)n, *n_dev);
-  if ((size_t)blockIdx.x * kScanTile > n) return;  // past the count (uniform over the block)
+                                                              uint64_t* __restrict__ out, int direct) {
   uint64_t pre;
   if (direct) {
     uint64_t own = 0;
@@ -299,10 +337,7 @@ __global__ void __launch_bounds__(kScanTpb) scan_apply_kernel(const uint32_t* __
     for (int i = 0; i < kScanItems; ++i)
       if (base + i < n) out[base + i] = o[i];
   }
-  if (blockIdx.x == n / kScanTile && threadIdx.x == 0) {  // the tile holding position n: the total
-    out[n] = pre + tot;
-    if (n_cap != n) out[n_cap] = pre + tot;
-  }
+  if (blockIdx.x == n / kScanTile && threadIdx.x == 0) out[n] = pre + tot;  // the tile holding position n: the total
 }
 
 // ---------------------------------------------------------------- gather --
@@ -356,13 +391,9 @@ __global__ void hit_rows_kernel(const hpg_hit_t* __restrict__ hits, uint32_t n, 
 }
 
 __global__ void limit_rows_kernel(const uint64_t* __restrict__ list_off, uint32_t* __restrict__ rows,
-                                  uint32_t n_lists, uint64_t limit, const uint64_t* limit_dev,
-                                  uint8_t* __restrict__ trunc, const unsigned* gate) {
+                                  uint32_t n_lists, uint64_t limit, uint8_t* __restrict__ trunc) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_lists) return;
-  if (gate && *gate) return;
-  if (limit_dev) limit = *limit_dev;
-  if (limit == 0) return;
   const uint64_t b = list_off[t], e = list_off[t + 1];
   uint64_t sum = 0;
   for (uint64_t h = b; h < e; ++h) sum += rows[h];
@@ -421,15 +452,18 @@ __global__ void __launch_bounds__(kTpb)
 
 }  // namespace
 
+static unsigned encode_grid(uint64_t bases) {
+  const uint64_t tiles = (bases + 16ull * kEncTile - 1) / (16ull * kEncTile);
+  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, 152ull * 16));
+}
+
 void launch_encode(const uint8_t* ascii, uint64_t total, const uint64_t* offs, uint32_t n_reads,
                    const uint8_t* d_table, uint8_t* codes, uint8_t* ok, cudaStream_t s, uint64_t* packed) {
   if (!n_reads) return;
   cudaMemsetAsync(ok, 1, n_reads, s);
   if (!total) return;
-  const uint64_t chunks = (total + 15) / 16;
-  const unsigned grid = (unsigned)(chunks < 152ull * 32 * 8 ? (chunks + 255) / 256 : 152ull * 32);
   count_launches(1);
-  encode_kernel<<<grid, 256, 0, s>>>(ascii, total, offs, n_reads, d_table, codes, ok, nullptr, nullptr,
+  encode_kernel<<<encode_grid(total), kEncTpb, 0, s>>>(ascii, total, offs, n_reads, d_table, codes, ok, nullptr, nullptr,
                                        reinterpret_cast<uint32_t*>(packed));
 }
 
@@ -464,10 +498,8 @@ void launch_encode_dev(const uint8_t* ascii, uint64_t bases_cap, const uint64_t*
                        uint32_t n_cap, const uint8_t* d_table, uint8_t* codes, uint8_t* ok, cudaStream_t s,
                        const uint64_t* src_dev, uint64_t* packed) {
   cudaMemsetAsync(ok, 1, n_cap, s);
-  const uint64_t chunks = (bases_cap + 15) / 16;
-  const unsigned grid = (unsigned)(chunks < 152ull * 32 * 8 ? (chunks + 255) / 256 : 152ull * 32);
   count_launches(1);
-  encode_kernel<<<grid ? grid : 1, 256, 0, s>>>(ascii, bases_cap, offs, 0, d_table, codes, ok, n_dev, src_dev,
+  encode_kernel<<<encode_grid(bases_cap), kEncTpb, 0, s>>>(ascii, bases_cap, offs, 0, d_table, codes, ok, n_dev, src_dev,
                                                    reinterpret_cast<uint32_t*>(packed));
 }
 
@@ -493,8 +525,7 @@ void launch_plain_search1(const DevIndex& X, const uint8_t* codes, const uint64_
 
 size_t scan_parts(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
 
-void launch_scan(const uint32_t* in, size_t n, uint64_t* out, uint64_t* part, cudaStream_t s,
-                 const uint64_t* n_dev) {
+void launch_scan(const uint32_t* in, size_t n, uint64_t* out, uint64_t* part, cudaStream_t s) {
   if (n == 0) {
     cudaMemsetAsync(out, 0, sizeof(uint64_t), s);
     return;
@@ -505,13 +536,13 @@ void launch_scan(const uint32_t* in, size_t n, uint64_t* out, uint64_t* part, cu
   // (at most 8 loads a thread); more, and one block scans the tile sums first
   const int direct = nb <= 4096;
   count_launches(1);
-  scan_reduce_kernel<<<nb, kScanTpb, 0, s>>>(in, n, part, n_dev);
+  scan_reduce_kernel<<<nb, kScanTpb, 0, s>>>(in, n, part);
   if (!direct) {
     count_launches(1);
     scan_parts_kernel<<<1, 1024, 0, s>>>(part, nb);
   }
   count_launches(1);
-  scan_apply_kernel<<<nb, kScanTpb, 0, s>>>(in, n, part, out, direct, n_dev);
+  scan_apply_kernel<<<nb, kScanTpb, 0, s>>>(in, n, part, out, direct);
 }
 
 void launch_gather_hits(const uint4* slots, const OvfEntry* ovf, const uint32_t* ovf_count, uint32_t ovf_cap,
@@ -532,11 +563,11 @@ void launch_hit_rows(const hpg_hit_t* hits, uint32_t n_hits, uint32_t* rows, cud
   hit_rows_kernel<<<grid_for(n_hits, 256), 256, 0, s>>>(hits, n_hits, rows);
 }
 
-void launch_limit_rows(const uint64_t* list_off, uint32_t* rows, uint32_t n_lists, uint64_t limit,
-                       const uint64_t* limit_dev, uint8_t* trunc, cudaStream_t s, const unsigned* gate) {
-  if (!n_lists || (!limit_dev && limit == 0)) return;
+void launch_limit_rows(const uint64_t* list_off, uint32_t* rows, uint32_t n_lists, uint64_t limit, uint8_t* trunc,
+                       cudaStream_t s) {
+  if (!n_lists || limit == 0) return;
   count_launches(1);
-  limit_rows_kernel<<<grid_for(n_lists, 256), 256, 0, s>>>(list_off, rows, n_lists, limit, limit_dev, trunc, gate);
+  limit_rows_kernel<<<grid_for(n_lists, 256), 256, 0, s>>>(list_off, rows, n_lists, limit, trunc);
 }
 
 void launch_locate(const DevIndex& X, const hpg_hit_t* hits, const uint64_t* loc_off, uint32_t n_hits,

@@ -58,11 +58,8 @@ void launch_plain_search1(const DevIndex& X, const uint8_t* codes, const uint64_
                           uint32_t* rs_count, uint8_t* rs_trunc, unsigned long long* census, cudaStream_t s);
 
 // Exclusive scan: out[0..n] with out[n] = total.  `part` needs scan_parts(n) entries.
-// With n_dev the scan covers the first min(n, *n_dev) entries (a count found on
-// the device) and writes the total at that position and at out[n].
 size_t scan_parts(size_t n);
-void launch_scan(const uint32_t* in, size_t n, uint64_t* out, uint64_t* part, cudaStream_t s,
-                 const uint64_t* n_dev = nullptr);
+void launch_scan(const uint32_t* in, size_t n, uint64_t* out, uint64_t* part, cudaStream_t s);
 
 // Slots + overflow pool -> ordered hpg_hit_t records, hit i of (read, strand) t at off[t] + i.
 void launch_gather_hits(const uint4* slots, const OvfEntry* ovf, const uint32_t* ovf_count, uint32_t ovf_cap,
@@ -73,10 +70,9 @@ void launch_gather_hits(const uint4* slots, const OvfEntry* ovf, const uint32_t*
 void launch_hit_rows(const hpg_hit_t* hits, uint32_t n_hits, uint32_t* rows, cudaStream_t s);
 
 // Locate limit: a list (read, strand) whose hits list_off[t]..list_off[t+1]
-// cover more than `limit` rows (read from limit_dev when given; 0 = no limit)
-// has its rows set to 0, so nothing of it is located, and trunc[t] |= 2.
-void launch_limit_rows(const uint64_t* list_off, uint32_t* rows, uint32_t n_lists, uint64_t limit,
-                       const uint64_t* limit_dev, uint8_t* trunc, cudaStream_t s, const unsigned* gate = nullptr);
+// cover more than `limit` rows (0 = no limit) has its rows set to 0, so nothing of it is located, and trunc[t] |= 2.
+void launch_limit_rows(const uint64_t* list_off, uint32_t* rows, uint32_t n_lists, uint64_t limit, uint8_t* trunc,
+                       cudaStream_t s);
 
 // Locate every row of every hit (bwt.c:2158-2166); hit ids are offset by hit_base.
 void launch_locate(const DevIndex& X, const hpg_hit_t* hits, const uint64_t* loc_off, uint32_t n_hits,

@@ -46,9 +46,8 @@ double now_ms() {
 // a batch whose pools overflowed is left alone (it runs again and is rebased
 // after its rerun); so the kernel can follow the replay in stream order.
 __global__ void serve_rebase_kernel(hpg_hit_t* __restrict__ hits, uint64_t n_hits, hpg_loc_t* __restrict__ locs,
-                                    uint64_t n_locs, const uint64_t* __restrict__ hit_off,
-                                    const uint64_t* __restrict__ loc_off, const uint32_t* __restrict__ seg_read0,
-                                    uint32_t n_seg, uint64_t* __restrict__ bounds,
+                                    uint64_t n_locs, const uint2* __restrict__ read_off,
+                                    const uint32_t* __restrict__ seg_read0, uint32_t n_seg, uint64_t* __restrict__ bounds,
                                     const uint64_t* __restrict__ summary) {
   if (summary) {
     if ((uint32_t)summary[0] != 0) return;
@@ -57,9 +56,9 @@ __global__ void serve_rebase_kernel(hpg_hit_t* __restrict__ hits, uint64_t n_hit
   }
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t s = tid; s <= n_seg; s += stride) {
-    const uint64_t h0 = hit_off[2ull * seg_read0[s]];
-    bounds[2 * s] = h0;
-    bounds[2 * s + 1] = loc_off[h0];
+    const uint2 first = read_off[seg_read0[s]];
+    bounds[2 * s] = first.x;
+    bounds[2 * s + 1] = first.y;
   }
   for (uint64_t i = tid; i < n_hits; i += stride) {
     const uint32_t r = hits[i].read;
@@ -76,10 +75,10 @@ __global__ void serve_rebase_kernel(hpg_hit_t* __restrict__ hits, uint64_t n_hit
     uint32_t lo = 0, hi = n_seg;
     while (hi - lo > 1) {
       const uint32_t mid = (lo + hi) >> 1;
-      if (hit_off[2ull * seg_read0[mid]] <= h) lo = mid;
+      if (read_off[seg_read0[mid]].x <= h) lo = mid;
       else hi = mid;
     }
-    locs[j].hit = (uint32_t)(h - hit_off[2ull * seg_read0[lo]]);
+    locs[j].hit = (uint32_t)(h - read_off[seg_read0[lo]].x);
   }
 }
 
@@ -118,10 +117,16 @@ struct Batch {
   int slot = 0;  // staging slot of its offsets and segment table
   GraphPlan* g = nullptr;
   ResultBuf* rb = nullptr;  // result set its copies go to, once they are queued
+  int set = -1;             // its index
   double t_launch = 0;
 };
 
-constexpr int kSets = 3;
+constexpr int kSets = 3;  // result sets a server starts with
+// A batch that finds every set held by results its clients have not released waits
+// this long for one, then gets a new set: a client may wait for its requests in any
+// order before it releases one, and a wait without end here would keep the batch it
+// waits for from ever being published (short batches make that many sets' worth).
+constexpr auto kSetWait = std::chrono::milliseconds(20);
 
 template <typename T>
 bool pinned_grow(T** p, size_t* cap, size_t want) {
@@ -158,7 +163,7 @@ struct Server {
   bool stop = false;
   std::thread worker;
 
-  ResultBuf sets[kSets];
+  std::deque<ResultBuf> sets;  // grown by the worker only, under mu; entries stay where they are
   int next_set = 0;
   uint64_t* h_offs[2] = {nullptr, nullptr};
   uint32_t* h_seg[2] = {nullptr, nullptr};
@@ -279,7 +284,7 @@ struct Server {
     GraphPlan* g = b->g;
     count_launches(1);
     serve_rebase_kernel<<<e->num_sms * 2, 256, 0, cs>>>(g->hits, g->res_cap, g->locs, g->skip_locate ? 0 : g->locs_cap,
-                                                       g->hit_off, g->loc_off, d_seg[k], (uint32_t)b->reqs.size(),
+                                                       g->read_off, d_seg[k], (uint32_t)b->reqs.size(),
                                                        d_bounds[k], g->summary_d);
     if (timing) cudaEventRecord(tv1[k], cs);
     HPG_CUDA(cudaEventRecord(ev_run[k], cs), "serving order");
@@ -287,18 +292,29 @@ struct Server {
     return 0;
   }
 
-  ResultBuf* take_set(size_t hits, size_t locs, size_t rs, size_t segs, std::string* err) {
+  ResultBuf* take_set(size_t hits, size_t locs, size_t rs, size_t segs, int* index, std::string* err) {
     int pick = -1;
     {
       std::unique_lock<std::mutex> lk(mu);
-      cv_sets.wait(lk, [&] {
-        for (int k = 0; k < kSets; ++k)
-          if (sets[(next_set + k) % kSets].refs == 0) return true;
+      const int n = (int)sets.size();
+      cv_sets.wait_for(lk, kSetWait, [&] {
+        for (int k = 0; k < n; ++k)
+          if (sets[(next_set + k) % n].refs == 0) return true;
         return false;
       });
-      for (int k = 0; k < kSets && pick < 0; ++k)
-        if (sets[(next_set + k) % kSets].refs == 0) pick = (next_set + k) % kSets;
-      next_set = (pick + 1) % kSets;
+      for (int k = 0; k < n && pick < 0; ++k)
+        if (sets[(next_set + k) % n].refs == 0) pick = (next_set + k) % n;
+      if (pick < 0) {
+        ResultBuf more;
+        if (cudaEventCreateWithFlags(&more.done, cudaEventDisableTiming) != cudaSuccess) {
+          cudaGetLastError();
+          *err = "out of memory (serving results)";
+          return nullptr;
+        }
+        pick = n;
+        sets.push_back(more);
+      }
+      next_set = (pick + 1) % (int)sets.size();
     }
     ResultBuf& rb = sets[pick];
     if (!pinned_grow(&rb.hits, &rb.hits_cap, hits + 1) || !pinned_grow(&rb.locs, &rb.locs_cap, locs + 1) ||
@@ -314,6 +330,7 @@ struct Server {
       }
       rb.rs_cap = std::min(c1, c2);
     }
+    *index = pick;
     return &rb;
   }
 
@@ -376,7 +393,7 @@ struct Server {
     const uint64_t nh = h[2], nl = g->skip_locate ? 0 : h[3];
     const size_t nseg = b->reqs.size();
     const double k0 = now_ms();
-    ResultBuf* rb = take_set(nh, nl, 2ull * b->n, nseg, err);
+    ResultBuf* rb = take_set(nh, nl, 2ull * b->n, nseg, &b->set, err);
     if (!rb) return -1;
     if (timing) note(t_take, m_take, now_ms() - k0);
     HPG_CUDA(cudaStreamWaitEvent(d2h, ev_run[k], 0), "serving order");
@@ -384,7 +401,7 @@ struct Server {
       const uint64_t work = std::max<uint64_t>(std::max<uint64_t>(nh, nl), nseg + 1);
       const unsigned grid = (unsigned)std::min<uint64_t>((work + 255) / 256, (uint64_t)e->num_sms * 8);
       count_launches(1);
-      serve_rebase_kernel<<<grid, 256, 0, d2h>>>(g->hits, nh, g->locs, nl, g->hit_off, g->loc_off, d_seg[k],
+      serve_rebase_kernel<<<grid, 256, 0, d2h>>>(g->hits, nh, g->locs, nl, g->read_off, d_seg[k],
                                                  (uint32_t)nseg, d_bounds[k], nullptr);
     }
     if (nh)
@@ -423,7 +440,7 @@ struct Server {
     uint32_t read0 = 0;  // the slot's staged segment table may already hold the next batch's
     for (size_t q = 0; q < nseg; ++q) {
       ServeReq* r = b->reqs[q];
-      r->set = (int)(rb - sets);
+      r->set = b->set;
       r->read0 = read0;
       read0 += r->n;
       r->hit0 = rb->bounds[2 * q];
@@ -551,6 +568,7 @@ Server* server_create(Engine* e, size_t max_batch_reads, uint64_t max_batch_base
   if (ok && !e->xs[0])
     ok = cudaStreamCreateWithFlags(&e->xs[0], cudaStreamNonBlocking) == cudaSuccess &&
          cudaStreamCreateWithFlags(&e->xs[1], cudaStreamNonBlocking) == cudaSuccess;
+  S->sets.resize(kSets);
   for (int k = 0; k < kSets && ok; ++k) ok = cudaEventCreateWithFlags(&S->sets[k].done, cudaEventDisableTiming) ==
                                             cudaSuccess;
   // result sets sized for two hits and two located rows per read of a full batch up

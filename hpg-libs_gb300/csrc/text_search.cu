@@ -28,6 +28,7 @@
 //   text_rows_kernel    a lane per row of the queued chains, all their change
 //                       points from one comparison of each row's text
 //   text_walk_kernel    a thread per queued walk
+//   text_block_kernel   a thread per j = 1 / j = n-1 block
 //
 // Positions are counted in search order: symbol i of a chain is W[len-1-i]
 // (backward) or W[i] (forward), complemented on the '-' strand, so both
@@ -74,10 +75,9 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 // 32 symbols of a 2-bit stream from symbol i on (i may be -31 or reach past the
 // end by as much: the streams are padded), symbol i in the low bits.
 __device__ __forceinline__ uint64_t load32(const uint64_t* s, int64_t i) {
-  const int64_t w = i >> 5;
+  const uint64_t* w = s + (i >> 5);
   const uint32_t sh = ((uint32_t)i & 31u) << 1;
-  const uint64_t a = __ldg(s + w);
-  return sh ? (a >> sh) | (__ldg(s + w + 1) << (64 - sh)) : a;
+  return (__ldg(w) >> sh) | ((__ldg(w + 1) << 1) << (63u - sh));
 }
 
 // The 32 symbols in reverse order.
@@ -90,29 +90,32 @@ __device__ __forceinline__ uint64_t comp_word(const DevIndex& X, uint32_t strand
   return strand ? 0x5555555555555555ull * X.comp_xor : 0ull;
 }
 
+// (the words below are selected, not branched on, so that a warp's strands and
+// directions stay together)
+
 // Symbols i .. i+31 of a chain (past the read's end: whatever the stream holds), symbol i in the low bits.
 __device__ __forceinline__ uint64_t query32(const DevIndex& X, const uint64_t* packed, uint64_t b0, int len,
                                             bool fwd, uint32_t strand, int i) {
-  const uint64_t x = fwd ? load32(packed, (int64_t)b0 + i) : rev32(load32(packed, (int64_t)b0 + len - 32 - i));
-  return x ^ comp_word(X, strand);
+  const uint64_t x = load32(packed, (int64_t)b0 + (fwd ? i : len - 32 - i));
+  const uint64_t r = rev32(x);
+  return (fwd ? x : r) ^ comp_word(X, strand);
+}
+
+// The text read leftwards from position P of physical direction d, from its m-th symbol on:
+// T_d[P-1-m], T_d[P-2-m], ... (past the text's ends: padding).
+__device__ __forceinline__ uint64_t text32(const DevIndex& X, uint32_t d, uint32_t P, int m) {
+  const uint64_t x = load32(X.text, d ? (int64_t)X.top - P + m : (int64_t)P - 32 - m);
+  const uint64_t r = rev32(x);
+  return d ? x : r;
 }
 
 // How many of the symbols i .. i+want-1 of a chain agree with the text read
-// leftwards from position P of physical direction d (whose next symbol is
-// T_d[P-1]); want <= P.  Text words and query words are taken in the query's
-// order in the stream, so that at most the text word is reversed.
+// leftwards from position P of physical direction d; want <= P.
 __device__ __forceinline__ int agree(const DevIndex& X, const uint64_t* packed, uint64_t b0, int len, bool fwd,
                                      uint32_t strand, uint32_t d, int i, uint32_t P, int want) {
-  const uint64_t cw = comp_word(X, strand);
   for (int m = 0; m < want; m += 32) {
-    // the text's next 32 symbols: text[P-1], text[P-2], ... (d = 0) or text[n-P], text[n-P+1], ... (d = 1)
-    uint64_t tw = d ? load32(X.text, (int64_t)(X.top - P) + m) : load32(X.text, (int64_t)P - 32 - m);
-    const uint64_t qw =
-        (fwd ? load32(packed, (int64_t)b0 + i + m) : load32(packed, (int64_t)b0 + len - 32 - i - m)) ^ cw;
-    if (fwd != (d != 0)) tw = rev32(tw);
-    const uint64_t x = tw ^ qw;
-    const int same = x == 0 ? 32 : (fwd ? __ffsll((long long)x) - 1 : __clzll((long long)x)) >> 1;
-    if (same < 32) return min(want, m + same);
+    const uint64_t x = text32(X, d, P, m) ^ query32(X, packed, b0, len, fwd, strand, i + m);
+    if (x) return min(want, m + ((__ffsll((long long)x) - 1) >> 1));
   }
   return want;
 }
@@ -159,7 +162,7 @@ __device__ __forceinline__ uint32_t other_chain(const DevIndex& X, const Batched
   return p.diag[(uint64_t)((d ^ 1u) * 2u + (rs & 1u)) * p.n_reads + (rs >> 1)];
 }
 
-// The block entry (j = 1 / j = n-1) for the fused drain.
+// An entry of the block list (j = 1 / j = n-1).
 __device__ __forceinline__ void push_block(const BatchedParams& p, uint32_t k, uint32_t l, uint32_t rs, int len,
                                            bool fwd) {
   const unsigned q = atomicAdd(p.block_n, 1u);
@@ -202,8 +205,8 @@ __global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, Batched
       const int L = (int)X.tmer_len;
       if (len >= 2 * L + 2) {
         const uint32_t r = __brev((uint32_t)q) >> (32 - 2 * L);
-        const uint2 s = __ldg((d ? X.tmer[1] : X.tmer[0]) +
-                              (((r & 0x55555555u) << 1) | ((r >> 1) & 0x55555555u)));
+        const uint2 s = load_row_pair((d ? X.tmer[1] : X.tmer[0]) +
+                                      (((r & 0x55555555u) << 1) | ((r >> 1) & 0x55555555u)));
         if (CENSUS) ++sectors;
         k = s.x;
         l = s.y;
@@ -274,21 +277,25 @@ __global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, Batched
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
 
-// The hits of a change point whose interval is one row, at T_d[Q - 1] for symbol te: bit 0
-// the deletion, 1 the insertion and 2 the mismatch of the text's next symbol, `base` as a query base.
+// The hits of a change point whose interval is one row: with the chain's symbol i
+// beside T(i) = T_d[P - 1 - i], symbol te the first that disagrees.  Bit 0 the deletion
+// (symbol i + 1 beside T(i) from te on), 1 the insertion and 2 the mismatch of the
+// text's symbol `base` (as a query base): symbol i beside T(i + 1) from te on, beside T(i)
+// after te.  One pass over the words for all three, 31 places a round.
 __device__ __forceinline__ uint32_t one_row_branches(const DevIndex& X, const uint64_t* packed, uint64_t b0, int len,
-                                                     bool fwd, uint32_t strand, uint32_t d, int te, uint32_t Q,
+                                                     bool fwd, uint32_t strand, uint32_t d, int te, uint32_t P,
                                                      uint32_t& base) {
-  const int after = len - te - 1;  // symbols after the failing one
-  uint32_t mask = 0;
-  if (Q >= (uint32_t)after && agree(X, packed, b0, len, fwd, strand, d, te + 1, Q, after) == after) mask = 1;
-  if (Q >= 1) {
-    const uint64_t tw = d ? load32(X.text, (int64_t)(X.top - Q)) : load32(X.text, (int64_t)Q - 1);
-    base = ((uint32_t)tw & 3u) ^ (strand ? X.comp_xor : 0u);
-    const uint32_t R = Q - 1;
-    if (R >= (uint32_t)after + 1 && agree(X, packed, b0, len, fwd, strand, d, te, R, after + 1) == after + 1)
-      mask |= 2;
-    if (R >= (uint32_t)after && agree(X, packed, b0, len, fwd, strand, d, te + 1, R, after) == after) mask |= 4;
+  // the text has to hold len - 1, len + 1 and len symbols
+  uint32_t mask = (P + 1u >= (uint32_t)len ? 1u : 0u) | (P >= (uint32_t)len + 1u ? 2u : 0u) |
+                  (P >= (uint32_t)len ? 4u : 0u);
+  for (int m = te; mask && m < len; m += 31) {
+    const uint64_t q = query32(X, packed, b0, len, fwd, strand, m), w = text32(X, d, P, m);
+    if (m == te) base = ((uint32_t)w & 3u) ^ (strand ? X.comp_xor : 0u);
+    const int left = len - 1 - m;  // places of the deletion and the mismatch; the insertion has one more
+    const uint64_t some = (1ull << (2 * min(left, 31))) - 1ull, more = (1ull << (2 * min(left + 1, 31))) - 1ull;
+    if (((q >> 2) ^ w) & some) mask &= ~1u;
+    if ((q ^ (w >> 2)) & more) mask &= ~2u;
+    if (((q ^ w) >> 2) & some) mask &= ~4u;
   }
   return mask;
 }
@@ -350,25 +357,35 @@ __global__ void __launch_bounds__(kReadTpb) text_read_kernel(DevIndex X, Batched
       left = strand ? dg[3] : dg[2];
       const uint64_t cw = comp_word(X, strand);
       auto R32 = [&](int j) -> uint64_t {  // symbols j .. j+31 of R
-        return strand ? rev32(load32(p.packed, (int64_t)b0 + len - 32 - j)) ^ cw : load32(p.packed, (int64_t)b0 + j);
+        const uint64_t x = load32(p.packed, (int64_t)b0 + (strand ? len - 32 - j : j));
+        const uint64_t r = rev32(x) ^ cw;
+        return strand ? r : x;
       };
       // the alignment: R[j] at text[a + j]
+      const bool has_r = is_diag(right), has_l = is_diag(left);
       const int64_t a_r = (int64_t)right - len, a_l = (int64_t)n - left;
+      const bool same = has_r && has_l && a_r == a_l;
       te_r = te_l = len;
-      if (is_diag(left)) {  // from the left; past the text's end nothing matches
-        const int hi = (int)min((int64_t)len, (int64_t)left);
-        int j = 0;
-        for (; j < hi; j += 32) {
-          const uint64_t x = load32(X.text, a_l + j) ^ R32(j);
+      {  // one pass for the left chain (or the right one alone): its first and last disagreement
+        const int64_t a = has_l ? a_l : a_r;
+        const int lo = a < 0 ? (int)-a : 0, hi = (int)min((int64_t)len, (int64_t)n - a);  // inside the text
+        int first = -1, last = -1;
+        for (int j = 0; j < len; j += 32) {
+          uint64_t x = 0;
+          if (j + 32 > lo && j < hi) x = load32(X.text, a + j) ^ R32(j);
+          if (j < lo) x |= lo - j >= 32 ? ~0ull : (1ull << (2 * (lo - j))) - 1ull;
+          if (j + 32 > hi) x = (j >= hi ? 0ull : x & ((1ull << (2 * (hi - j))) - 1ull)) |
+                               (j >= hi ? ~0ull : ~0ull << (2 * (hi - j)));
+          if (j + 32 > len) x &= (1ull << (2 * (len - j))) - 1ull;
           if (x) {
-            j += (__ffsll((long long)x) - 1) >> 1;
-            break;
+            if (first < 0) first = j + ((__ffsll((long long)x) - 1) >> 1);
+            last = j + ((63 - __clzll((long long)x)) >> 1);
           }
         }
-        if (j < hi) te_l = j;
-        else if (hi < len) te_l = hi;
+        if (has_l && first >= 0) te_l = first;
+        if ((same || !has_l) && last >= 0) te_r = len - 1 - last;
       }
-      if (is_diag(right) && !(is_diag(left) && a_l == a_r && te_l == len)) {  // from the right, down to the text's start
+      if (has_r && has_l && !same) {  // another alignment: the right chain from its end, down to the text's start
         const int lo = a_r < 0 ? (int)-a_r : 0;
         int top = len;  // R[top .. len-1] matches
         for (; top > lo; top -= 32) {
@@ -395,7 +412,7 @@ __global__ void __launch_bounds__(kReadTpb) text_read_kernel(DevIndex X, Batched
           push_block(p, r, r, (read << 1) | strand, len, fwd);
         } else {
           uint32_t base = 0;
-          const uint32_t m = one_row_branches(X, p.packed, b0, len, fwd, strand, (uint32_t)side, te, Q, base);
+          const uint32_t m = one_row_branches(X, p.packed, b0, len, fwd, strand, (uint32_t)side, te, dgs, base);
           if (side) {
             mask |= m << 4;
             base_l = base;
@@ -428,7 +445,7 @@ __global__ void __launch_bounds__(kReadTpb) text_read_kernel(DevIndex X, Batched
         meta = branch_meta(fwd, len, te, item == 0 ? 1u : (item == 1 ? 3u : 2u), item == 0 ? 0xFFu : b);
       }
       const uint32_t row = load_row_word((side ? X.dir[1].isa : X.dir[0].isa) + at);
-      write_hit(p, slot++, (read << 1) | strand, key, row, row, meta);
+      write_hit(p, slot++, (read << 1) | strand, key, row, row, meta, at + 1);
     }
     // (the loop's barrier is passed before s_cnt and s_base are rewritten)
   }
@@ -560,12 +577,13 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
       if (I <= last) row_i = load_row_word(isa + P - (uint32_t)(len + 1));
       if (te == len || (te <= len - 2 && M <= te + 1)) row_m = load_row_word(isa + P - (uint32_t)len);
     }
-    auto emit = [&](uint32_t key, uint32_t k, uint32_t l, uint32_t meta) {
+    auto emit = [&](uint32_t key, uint32_t k, uint32_t l, uint32_t meta, uint32_t at) {  // at: this lane's SA value
       uint32_t r = c_res[tid];
       const unsigned slot = res_slot(p, r);
       c_res[tid] = r;
-      write_hit(p, slot, rs, key, k, l, meta);
+      write_hit(p, slot, rs, key, k, l, meta, k == l ? at + 1 : 0u);
     };
+    const uint32_t at = P - (uint32_t)len;  // the whole read's and the mismatch's; the deletion ends one on, the insertion one before
     auto interval = [&](bool in, uint32_t row, bool& lead, uint32_t& k, uint32_t& l) {  // of the chain's lanes with `in`
       const unsigned m = __ballot_sync(kFull, in) & seg;
       lead = m && lane == (uint32_t)__ffs(m) - 1u;
@@ -576,7 +594,7 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
     uint32_t k, l;
     // the whole read: the backward chain's exact hit
     interval(te == len, row_m, lead, k, l);
-    if (lead && !fwd) emit(order_key(0, 0, 0), k, l, pack_meta(0, 0, 0, 0, 0));
+    if (lead && !fwd) emit(order_key(0, 0, 0), k, l, pack_meta(0, 0, 0, 0, 0), at);
     interval(block, row_d, lead, k, l);
     if (lead) push_block(p, k, l, rs, len, fwd);
     // the other change points, in order
@@ -597,15 +615,15 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
       const uint32_t tf = (uint32_t)(len - cp);
       const uint32_t sec = fwd ? 4u : 2u;
       interval(in && D <= cp, row_d, lead, k, l);
-      if (lead) emit(order_key(sec, tf, 0), k, l, branch_meta(fwd, len, cp, 1, 0xFFu));
+      if (lead) emit(order_key(sec, tf, 0), k, l, branch_meta(fwd, len, cp, 1, 0xFFu), at + 1);
       const bool ins = in && I <= cp, mis = in && te == cp && M <= cp + 1;
       if (__ballot_sync(kFull, ins || mis)) {
 #pragma unroll
         for (uint32_t v = 0; v < 4; ++v) {
           interval(ins && b == v, row_i, lead, k, l);
-          if (lead) emit(order_key(sec, tf, 1 + 2 * v), k, l, branch_meta(fwd, len, cp, 3, v));
+          if (lead) emit(order_key(sec, tf, 1 + 2 * v), k, l, branch_meta(fwd, len, cp, 3, v), at - 1);
           interval(mis && b == v, row_m, lead, k, l);
-          if (lead) emit(order_key(sec, tf, 2 + 2 * v), k, l, branch_meta(fwd, len, cp, 2, v));
+          if (lead) emit(order_key(sec, tf, 2 + 2 * v), k, l, branch_meta(fwd, len, cp, 2, v), at);
         }
       }
       if (te == cp) todo = false;
@@ -849,7 +867,8 @@ __global__ void __launch_bounds__(kWideTpb) text_branch_kernel(DevIndex X, Batch
                 uint32_t c = c_res[tid];
                 const unsigned slot = res_slot(p, c);
                 c_res[tid] = c;
-                write_hit(p, slot, rs, order_key(sec, tf, slot_key), row, row, branch_meta(fwd, len, te, kind, base));
+                write_hit(p, slot, rs, order_key(sec, tf, slot_key), row, row, branch_meta(fwd, len, te, kind, base),
+                          P - (uint32_t)len + 1);
               };
               if (agree(X, p.packed, b0, len, fwd, strand, d, 0, P - 1, te) == te) found(0, 1, 0xFFu);
               if (P <= X.top) {
@@ -942,7 +961,7 @@ __global__ void __launch_bounds__(kWalkTpb) text_walk_kernel(DevIndex X, Batched
   for (uint32_t i0 = blockIdx.x * kWalkTpb; i0 < n; i0 += gridDim.x * kWalkTpb) {
     const uint32_t i = i0 + threadIdx.x;
     bool hit = false;
-    uint32_t row = 0, meta = 0;
+    uint32_t row = 0, meta = 0, at = 0;
     uint4 e = make_uint4(0, 0, 0xFFFFFFFFu, 0);
     if (i < n) e = __ldcs(p.walk + i);
     if (e.z != 0xFFFFFFFFu) {  // (a reserved slot nothing was written to)
@@ -957,14 +976,80 @@ __global__ void __launch_bounds__(kWalkTpb) text_walk_kernel(DevIndex X, Batched
       if (P >= (uint32_t)left && agree(X, p.packed, b0, len, fwd, strand, d, t, P, left) == left) {
         const uint32_t s = e.y & 0xFFu;
         hit = true;
-        row = load_row_word((d ? X.dir[1].isa : X.dir[0].isa) + P - (uint32_t)left);
+        at = P - (uint32_t)left;
+        row = load_row_word((d ? X.dir[1].isa : X.dir[0].isa) + at);
         meta = branch_meta(fwd, len, len - (int)((e.y >> 8) & 0xFFFFu), s == 0 ? 1u : ((s & 1u) ? 3u : 2u),
                            s == 0 ? 0xFFu : (s - 1) >> 1);
         if (CENSUS) ++sectors;
       }
     }
     const uint32_t slot = block_slots<kWalkTpb>(hit ? 1u : 0u, p.res_total, s_cnt, &s_base);
-    if (hit) write_hit(p, slot, e.z, e.y, row, row, meta);
+    if (hit) write_hit(p, slot, e.z, e.y, row, row, meta, at + 1);
+    __syncthreads();  // s_cnt and s_base are rewritten next round
+  }
+  if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
+}
+
+// A thread per block entry (k, l at the last symbol but one of the chain, as the
+// fused kernel's drain maps them): the deletion is the interval itself; per base b
+// the step with b gives the mismatch, and a further step with the read's end base
+// the insertion.  In the j = 1 block an insertion is reported with base INSERTION
+// and position b, and b stays the position of the block's later mismatches
+// (search.c:1556).
+template <bool CENSUS>
+__global__ void __launch_bounds__(kWalkTpb) text_block_kernel(DevIndex X, BatchedParams p) {
+  __shared__ uint32_t s_cnt[kWalkTpb / 32], s_base;
+  const uint32_t n = min(*(volatile unsigned int*)p.block_n, p.block_cap);
+  uint32_t sectors = 0;
+  for (uint32_t i0 = blockIdx.x * kWalkTpb; i0 < n; i0 += gridDim.x * kWalkTpb) {
+    const uint32_t i = i0 + threadIdx.x;
+    SpillEntry e{1, 0, 0, 0};
+    uint32_t nk[4], nl[4], ik[4], il[4], mask = 0;  // bit 0 deletion, 1 + b mismatch, 5 + b insertion
+    bool last = false;
+    int end = 0;
+    if (i < n) {
+      e = p.blocks[i];
+      last = ((e.jtype >> 16) & 3u) == kBlkN;
+      const uint32_t strand = e.rs & 1u, d = (last ? 1u : 0u) ^ strand;
+      const OccBlock* occ = d ? X.dir[1].occ : X.dir[0].occ;
+      const uint32_t dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
+      const uint64_t b0 = p.offs[e.rs >> 1];
+      end = (int)(p.offs[(e.rs >> 1) + 1] - b0) - 1;
+      const uint32_t w = (uint32_t)load32(p.packed, (int64_t)b0 + (last ? end : 0)) & 3u;
+      const uint32_t cx = strand ? X.comp_xor : 0u;
+      uint32_t pk[4], pl[4];  // by physical symbol
+      rank_step4(X, occ, dollar, e.k, e.l, pk, pl);
+      if (CENSUS) sectors += (e.k >> 6) == (e.l >> 6) ? 1u : 2u;
+      mask = 1;
+#pragma unroll
+      for (uint32_t b = 0; b < 4; ++b) {
+        nk[b] = sel4(pk, b ^ cx);
+        nl[b] = sel4(pl, b ^ cx);
+        ik[b] = nk[b];
+        il[b] = nl[b];
+        if (nk[b] > nl[b]) continue;
+        if (b != w) mask |= 2u << b;
+        if (CENSUS) sectors += (ik[b] >> 6) == (il[b] >> 6) ? 1u : 2u;
+        rank_step(X, occ, dollar, w ^ cx, ik[b], il[b]);
+        if (ik[b] <= il[b]) mask |= 32u << b;
+      }
+    }
+    uint32_t slot = block_slots<kWalkTpb>((uint32_t)__popc(mask), p.res_total, s_cnt, &s_base);
+    const uint32_t sec = last ? 3u : 1u;
+    if (mask & 1u)
+      write_hit(p, slot++, e.rs, order_key(sec, 0, 0), e.k, e.l, pack_meta(last ? 1 : 0, 1, 1, 0xFF, last ? end : 0));
+    uint32_t bpos = 0;  // the base of the block's last insertion so far
+#pragma unroll
+    for (uint32_t b = 0; b < 4; ++b) {
+      if (mask & (2u << b))
+        write_hit(p, slot++, e.rs, order_key(sec, 0, 1 + 2 * b), nk[b], nl[b],
+                  pack_meta(last ? 1 : 0, 1, 2, b, last ? end : (int)bpos));
+      if (mask & (32u << b)) {
+        write_hit(p, slot++, e.rs, order_key(sec, 0, 2 + 2 * b), ik[b], il[b],
+                  last ? pack_meta(1, 1, 3, b, end) : pack_meta(0, 1, 3, 3, (int)b));
+        bpos = b;
+      }
+    }
     __syncthreads();  // s_cnt and s_base are rewritten next round
   }
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
@@ -974,7 +1059,7 @@ template <bool CENSUS>
 void launch_text_stage(const DevIndex& X, const BatchedParams& p, int num_sms, cudaStream_t s) {
   const uint32_t cap = p.n_reads;
   if (!cap) return;
-  count_launches(6);
+  count_launches(7);
   text_head_kernel<CENSUS><<<dim3((cap + kHeadTpb - 1) / kHeadTpb, 4), kHeadTpb, 0, s>>>(X, p);
   text_read_kernel<<<(cap + kReadTpb - 1) / kReadTpb, kReadTpb, 0, s>>>(X, p);
   int per_sm = 0;
@@ -986,6 +1071,7 @@ void launch_text_stage(const DevIndex& X, const BatchedParams& p, int num_sms, c
   text_rows_kernel<<<(unsigned)(num_sms * std::max(per_sm, 1)), kRowsTpb, 0, s>>>(X, p);
   text_walk_kernel<CENSUS><<<(unsigned)std::min<uint64_t>((4ull * cap + kWalkTpb - 1) / kWalkTpb, 8ull * num_sms),
                              kWalkTpb, 0, s>>>(X, p);
+  text_block_kernel<CENSUS><<<(unsigned)num_sms, kWalkTpb, 0, s>>>(X, p);
 }
 
 }  // namespace
