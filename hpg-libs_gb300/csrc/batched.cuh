@@ -170,6 +170,8 @@ constexpr size_t kTextMaxReads = 1u << 25;
 size_t text_queue_bytes(size_t n_reads, int num_sms);
 void text_queues(BatchedParams& p, void* buffer, size_t n_reads, int num_sms);
 void launch_text_search(const DevIndex& X, const BatchedParams& p, int num_sms, cudaStream_t s);
+// The exact search of both strands with the text: a hit per (read, strand) that matches.
+void launch_text_exact(const DevIndex& X, const BatchedParams& p, cudaStream_t s);
 // The whole search stage of a tuning: the search launches, then (after `mid`,
 // recorded when not null) the drain of queued change points.  `ctr` is the
 // counter block (16 words, zeroed); the warp-cooperative form also needs

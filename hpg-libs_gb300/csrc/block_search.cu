@@ -32,6 +32,7 @@
 
 #include "engine_internal.hpp"
 #include "host_pool.hpp"
+#include "text_dev.cuh"
 
 namespace hpgbwt {
 
@@ -281,7 +282,7 @@ __device__ __forceinline__ View forward_view(uint32_t strand) { return strand ? 
 // bit 0: the anchor was set; bit 1: the block-0 fragment matched (with lists
 // of capacity 0 BWSearchCPU then returns before the last block).
 // The first L steps of an exact search from the full interval over view v, W[from],
-// W[from + dir], ..., by one lookup in the start table (L = X.kmer_len, the
+// W[from + dir], ..., by one lookup in a start table (of L symbols, the
 // table's entries already hold the interval after those steps); true with
 // k, l set when that interval is not empty, else the caller steps from the
 // start (it needs the position where the search failed).  Not in the census
@@ -289,14 +290,16 @@ __device__ __forceinline__ View forward_view(uint32_t strand) { return strand ? 
 template <bool C>
 __device__ __forceinline__ bool start_lookup(const DevIndex& X, View v, const uint8_t* W, int from, int dir, int steps,
                                              uint32_t& k, uint32_t& l) {
-  const uint32_t L = X.kmer_len;
+  // (the text's table where the index has it: longer, and there by default)
+  const uint32_t L = X.text ? X.tmer_len : X.kmer_len;
   if (C || L == 0 || steps < (int)L) return false;
   uint32_t code = 0;
   for (uint32_t j = 0; j < L; ++j) {
     const uint32_t b = W[from + dir * (int)j];
     code = (code << 2) | (v.comp ? sel4(X.comp, b) : b);
   }
-  const uint2 t = __ldg((v.d ? X.kmer[1] : X.kmer[0]) + code);
+  const uint2 t = X.text ? load_row_pair((v.d ? X.tmer[1] : X.tmer[0]) + code)
+                         : __ldg((v.d ? X.kmer[1] : X.kmer[0]) + code);
   if (t.x > t.y) return false;
   k = t.x;
   l = t.y;
@@ -390,7 +393,7 @@ __device__ __forceinline__ void head_start(const DevIndex& X, const HeadWalk& h,
   if (start_lookup<C>(X, h.v, W, h.from, h.dir, steps, k, l)) {
     gk = k;
     gl = l;
-    i = h.from + h.dir * (int)X.kmer_len;
+    i = h.from + h.dir * (int)(X.text ? X.tmer_len : X.kmer_len);
   }
 }
 
@@ -606,14 +609,22 @@ __global__ void __launch_bounds__(kBlockTpb) block_head_kernel(
   queue_append(more, cont, n_cont, it, k, l, (uint32_t)i);
 }
 
+// Block rule below, declared for the one-row blocks.
+__device__ __forceinline__ bool ext_rule_ok(uint32_t part, int pos, int end, int bs);
+
 // The rest of the head walks block_head_kernel compacted: thread g resumes
 // cont[g] at its position with its interval (non-empty, so also the last
 // non-empty one), ends the walk, and appends the blocks that go on to `queue`.
+// With the text on the device (packed given) a walk that has come down to one row
+// ends by comparing the rest of the fragment with the text, and the blocks that go
+// on with one row are appended to `one` as {block, row, text position}.
 template <bool C>
 __global__ void __launch_bounds__(kBlockTpb) block_head_rest_kernel(
     DevIndex X, const uint8_t* __restrict__ codes, const uint64_t* __restrict__ offs, const uint4* __restrict__ cont,
     const uint32_t* __restrict__ n_cont, uint32_t max_results, PartState ps, uint4* __restrict__ queue,
-    uint32_t* __restrict__ n_queue, unsigned long long* census) {
+    uint32_t* __restrict__ n_queue, const uint64_t* __restrict__ packed, uint4* __restrict__ one,
+    uint32_t* __restrict__ n_one, uint4* __restrict__ few_rows, uint32_t* __restrict__ n_few,
+    unsigned long long* census) {
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= *n_cont) return;
   const uint4 q = cont[g];
@@ -632,15 +643,115 @@ __global__ void __launch_bounds__(kBlockTpb) block_head_rest_kernel(
   o.sectors = 0;
   const HeadWalk h = head_walk(len, strand, (int)part);
   int i = (int)q.w;
-  uint32_t k = q.y, l = q.z, gk = q.y, gl = q.z;
-  head_steps<C>(X, h, codes + b0, i, k, l, gk, gl, -1, o.sectors);
+  uint32_t k = q.y, l = q.z, gk = q.y, gl = q.z, P = 0;
+  bool text = false;  // ended by the text, at T_d[P - 1]
+  if (!C && packed) {
+    while (k < l && !head_steps<C>(X, h, codes + b0, i, k, l, gk, gl, 1, o.sectors)) {
+    }
+    const int want = h.dir > 0 ? h.to - i + 1 : i - h.to + 1;
+    if (k == l && want >= 0) {
+      const bool fwd = h.dir > 0;
+      const uint32_t d = h.v.d;
+      P = load_row_word((d ? X.dir[1].sa : X.dir[0].sa) + k);
+      const int m = agree(X, packed, b0, len, fwd, strand, d, fwd ? i : len - 1 - i, P, (int)min((uint32_t)want, P));
+      P -= (uint32_t)m;
+      i += h.dir * m;
+      gk = gl = load_row_word((d ? X.dir[1].isa : X.dir[0].isa) + P);
+      text = m == want;
+      k = text ? gk : 1u;
+      l = text ? gk : 0u;
+    }
+  } else {
+    head_steps<C>(X, h, codes + b0, i, k, l, gk, gl, -1, o.sectors);
+  }
   uint32_t aflag = 0;
   const bool go = head_finish(h, len, o, ps.anchor + it, aflag, i, k, l, gk, gl);
   ps.count[it] = o.n;
   ps.refused[it] = o.refused ? 1 : 0;
   ps.aflag[it] = (uint8_t)aflag;
   if (C) atomicAdd(census, (unsigned long long)o.sectors);
-  queue_append(go, queue, n_queue, it, k, l, 0u);
+  // (a capacity below the 33 branch points that 32 rows can make: the tail counts them)
+  const bool few = go && !text && packed && l - k < 32u && max_results > 32u;
+  queue_append(go && !text && !few, queue, n_queue, it, k, l, 0u);
+  queue_append(go && text, one, n_one, it, k, P, 0u);
+  queue_append(few, few_rows, n_few, it, k, l, 0u);
+}
+
+// A thread per block whose fragment matched on one row.  The walk over the rest of the
+// read changes size only where the row fails, at the one place x that a comparison
+// finds: one branch point, whose extensions are comparisons with the text too, and of
+// its bases only the text's own next symbol c has an interval.  D allows the error
+// there whenever an extension reaches the read's end: every extension ends with
+// W[x+1..] (W[..x-1] backward), so those symbols occur and the restart walk of
+// calculateD* fails once, at x.  Order, the block rule and the mismatch that starts
+// where the insertion's extension ended as in branch_forward / branch_backward.
+__global__ void __launch_bounds__(kBlockTpb)
+    block_one_kernel(DevIndex X, const uint64_t* __restrict__ packed, const uint64_t* __restrict__ offs,
+                     const uint4* __restrict__ one, const uint32_t* __restrict__ n_one, uint32_t max_results,
+                     PartState ps) {
+  const uint32_t n = *n_one;
+  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
+    const uint4 q = one[g];
+    const uint32_t it = q.x, list = it >> 1, part = it & 1u, strand = list & 1u, P = q.z;
+    const uint64_t b0 = offs[list >> 1];
+    const int len = (int)(offs[(list >> 1) + 1] - b0), end = len - 1;
+    int frag = 30;
+    fragments_of(len, frag);
+    ItemOut o;
+    o.slot = ps.slots + (uint64_t)it * kBlockSlots;
+    o.room = kBlockSlots;
+    o.cap = max_results;
+    o.n = 0;
+    o.read = list >> 1;
+    o.strand = strand;
+    o.refused = false;
+    o.sectors = 0;
+    const bool fwd = part == 0;
+    const uint32_t dir = fwd ? 1u : 0u, d = dir ^ strand;
+    const uint32_t* isa = d ? X.dir[1].isa : X.dir[0].isa;
+    const int from = fwd ? frag : len - frag, rest = len - from;  // in search order
+    const int m = agree(X, packed, b0, len, fwd, strand, d, from, P, (int)min((uint32_t)rest, P));
+    const uint32_t Q = P - (uint32_t)m;
+    if (m == rest) {  // the whole read: block 0's complete result
+      if (part == 0) {
+        const uint32_t row = load_row_word(isa + Q);
+        emit(o, 1, 0, 0, 0, 0, row, row);
+      }
+    } else {
+      const int x = from + m;  // the failing symbol
+      const int pos = fwd ? x : len - 1 - x, next = fwd ? pos + 1 : pos - 1;
+      // an extension over the symbols from symbol i on, from text position R: its row's text position, or ~0
+      auto extend = [&](int i, int ext_pos, uint32_t R) -> uint32_t {
+        const int want = len - i;
+        if (!ext_rule_ok(part, ext_pos, end, frag) || R < (uint32_t)want ||
+            agree(X, packed, b0, len, fwd, strand, d, i, R, want) != want)
+          return 0xFFFFFFFFu;
+        return R - (uint32_t)want;
+      };
+      bool room = true;
+      auto result = [&](uint32_t at, uint32_t kind, uint32_t base) {
+        const uint32_t row = load_row_word(isa + at);
+        room = emit(o, dir, 1, kind, base, pos, row, row);
+      };
+      const uint32_t del = extend(x + 1, next, Q);
+      if (del != 0xFFFFFFFFu) result(del, HPG_BWT_DELETION, 0xFF);
+      if (room && Q >= 1) {
+        const uint32_t c = ((uint32_t)text32(X, d, Q, 0) & 3u) ^ (strand ? X.comp_xor : 0u);
+        uint32_t R = Q - 1;
+        const uint32_t ins = extend(x, pos, R);
+        if (ins != 0xFFFFFFFFu) {
+          result(ins, HPG_BWT_INSERTION, c);
+          R = ins;
+        }
+        if (room) {
+          const uint32_t mis = extend(x + 1, next, R);
+          if (mis != 0xFFFFFFFFu) result(mis, HPG_BWT_MISMATCH, c);
+        }
+      }
+    }
+    ps.count[it] = o.n;
+    ps.refused[it] = o.refused ? 1 : 0;
+  }
 }
 
 // BWExactFinalResult{Forward,Backward}'s block rule (search.h:67-155) at the
@@ -662,6 +773,182 @@ __device__ __forceinline__ bool ext_rule_ok(uint32_t part, int pos, int end, int
   return true;
 }
 
+// A lane per row of the blocks whose fragment matched on 2 to 32 rows (and whose result
+// capacity no branch point list of theirs can pass, so that D's restart count matters only
+// where an extension reaches the read's end, and is then one, as for one row).  As
+// text_rows_kernel (text_search.cu): each row's first disagreement te and where its
+// alignment, shifted by one for the deletion and the insertion, begins to agree for good,
+// give the results of every branch point: the changes of the row count, in walk order; at
+// each the deletion, then per base the rows that failed there on that base, inserted and
+// mismatched.  A mismatch whose base's insertion survived starts where that ended
+// (branch_forward), so its rows must agree with the symbols after te once more beyond the
+// read's end.  (1M x 36-150 bp, 100 Mbp: the tail's lanes took 830 us a direction for these
+// blocks, a serial chain of some thousand rank steps in the slowest.)
+struct RowItemsShared {
+  uint4 item[32];
+  uint32_t n, next;
+};
+
+__global__ void __launch_bounds__(kBlockTpb)
+    block_rows_text_kernel(DevIndex X, const uint64_t* __restrict__ packed, const uint64_t* __restrict__ offs,
+                           const uint4* __restrict__ few, const uint32_t* __restrict__ n_few,
+                           uint32_t* __restrict__ head, uint32_t max_results, PartState ps) {
+  constexpr unsigned kFull = 0xFFFFFFFFu;
+  __shared__ RowItemsShared rsh[kBlockTpb / 32];
+  const uint32_t lane = threadIdx.x & 31;
+  RowItemsShared& ws = rsh[threadIdx.x >> 5];
+  const uint32_t n_items = *n_few;
+  const uint32_t per_claim = min(max(n_items / (gridDim.x * (kBlockTpb / 32)), 1u), 8u);
+  if (lane == 0) ws.n = ws.next = 0;
+  __syncwarp();
+  bool exhausted = false;
+  for (;;) {
+    if (ws.next == ws.n) {  // claim the next blocks
+      if (exhausted) break;
+      uint32_t c0 = 0;
+      if (lane == 0) c0 = atomicAdd(head, per_claim);
+      c0 = __shfl_sync(kFull, c0, 0);
+      if (c0 + per_claim >= n_items) exhausted = true;
+      const uint32_t got = c0 < n_items ? min(per_claim, n_items - c0) : 0u;
+      if (lane < got) ws.item[lane] = few[c0 + lane];
+      __syncwarp();
+      if (lane == 0) {
+        ws.n = got;
+        ws.next = 0;
+      }
+      __syncwarp();
+      if (!got) break;
+    }
+    const uint32_t first = ws.next, held = ws.n - first;
+    uint32_t rows = 0;
+    if (lane < held) rows = min(ws.item[first + lane].z - ws.item[first + lane].y + 1u, 32u);
+    uint32_t incl = rows;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(kFull, incl, o);
+      if (lane >= (uint32_t)o) incl += v;
+    }
+    const uint32_t take = (uint32_t)__popc(__ballot_sync(kFull, lane < held && incl <= 32));
+    uint32_t mine = 0xFFFFFFFFu, j = 0;
+    unsigned seg = 0;
+    for (uint32_t i = 0; i < take; ++i) {
+      const uint32_t stop = __shfl_sync(kFull, incl, i), len_i = __shfl_sync(kFull, rows, i);
+      if (lane < stop && lane >= stop - len_i) {
+        mine = i;
+        j = lane - (stop - len_i);
+        seg = (stop == 32 ? kFull : (1u << stop) - 1u) & ~((1u << (stop - len_i)) - 1u);
+      }
+    }
+    uint32_t it = 0, d = 0, P = 0, strand = 0, part = 0;
+    bool fwd = false;
+    int len = 0, from = 0, te = -1, frag = 30, D = 0x7FFFFFFF, I = 0x7FFFFFFF, M = 0x7FFFFFFF;
+    uint64_t b0 = 0;
+    if (mine != 0xFFFFFFFFu) {
+      const uint4 q = ws.item[first + mine];
+      it = q.x;
+      part = it & 1u;
+      strand = (it >> 1) & 1u;
+      fwd = part == 0;
+      d = (fwd ? 1u : 0u) ^ strand;
+      b0 = offs[it >> 2];
+      len = (int)(offs[(it >> 2) + 1] - b0);
+      fragments_of(len, frag);
+      from = fwd ? frag : len - frag;
+      const uint32_t sa = __ldg((d ? X.dir[1].sa : X.dir[0].sa) + q.y + j);
+      P = sa + (uint32_t)from;  // symbol i beside T_d[P - 1 - i]
+      te = from + agree(X, packed, b0, len, fwd, strand, d, from, sa, (int)min((uint32_t)(len - from), sa));
+      auto from_end = [&](int shift) -> int {  // symbols i agree with T(i + shift) down to the returned i, at least `from`
+        if ((int64_t)len + shift > (int64_t)P) return 0x7FFFFFFF;
+        int hi = len;
+        const int lo = shift < 0 ? from + 1 : from;
+        while (hi > lo) {
+          const uint64_t x = rev32(query32(X, packed, b0, len, fwd, strand, hi - 32) ^ text32(X, d, P, hi - 32 + shift));
+          const int same = x ? (__ffsll((long long)x) - 1) >> 1 : 32;
+          hi -= same;
+          if (same < 32) break;
+        }
+        return max(hi, lo);
+      };
+      D = from_end(-1) - 1;
+      I = from_end(1);
+      M = from_end(0);
+    }
+    __syncwarp();
+    if (lane == 0) ws.next = first + take;
+    const uint32_t* isa = d ? X.dir[1].isa : X.dir[0].isa;
+    uint32_t row_d = 0, row_i = 0, row_m = 0, row_2 = 0;
+    bool twice = false;
+    if (mine != 0xFFFFFFFFu) {
+      const int last = min(te, len - 1);
+      if (D <= last) row_d = load_row_word(isa + P - (uint32_t)(len - 1));
+      if (te < len && I <= te) {
+        row_i = load_row_word(isa + P - (uint32_t)(len + 1));
+        const int after = len - 1 - te;
+        const uint32_t R = P - (uint32_t)(len + 1);
+        twice = R >= (uint32_t)after && agree(X, packed, b0, len, fwd, strand, d, te + 1, R, after) == after;
+        if (twice) row_2 = load_row_word(isa + R - (uint32_t)after);
+      }
+      if (te == len || M <= te + 1) row_m = load_row_word(isa + P - (uint32_t)len);
+    }
+    // the chain's results go out through its first lane, in order
+    const bool lead = seg && lane == (uint32_t)__ffs(seg) - 1u;
+    ItemOut o;
+    o.slot = ps.slots + (uint64_t)it * kBlockSlots;
+    o.room = kBlockSlots;
+    o.cap = max_results;
+    o.n = 0;
+    o.read = it >> 2;
+    o.strand = strand;
+    o.refused = false;
+    o.sectors = 0;
+    uint32_t chunk = 0;
+    bool lost = false, room = true;
+    // the interval of the block's lanes with `in`, as every lane of the block sees it
+    auto interval = [&](bool in, uint32_t row, uint32_t& k, uint32_t& l) -> bool {
+      const unsigned m = __ballot_sync(kFull, in) & seg;
+      k = __shfl_sync(kFull, row, m ? __ffs(m) - 1 : (int)lane);
+      l = __shfl_sync(kFull, row, m ? 31 - __clz(m) : (int)lane);
+      return m != 0;
+    };
+    const uint32_t dir = fwd ? 1u : 0u;
+    uint32_t k, l;
+    if (interval(te == len && mine != 0xFFFFFFFFu && part == 0, row_m, k, l) && lead)  // block 0's complete result
+      room = emit_tail(o, ps, it, chunk, lost, 1, 0, 0, 0, 0, k, l);
+    bool todo = mine != 0xFFFFFFFFu && te < len;
+    while (__ballot_sync(kFull, todo)) {
+      int cp = 0x7FFFFFFF;  // the least te left among the block's lanes
+      for (uint32_t i = 0; i < take; ++i) {
+        const int v = __reduce_min_sync(kFull, mine == i && todo ? te : 0x7FFFFFFF);
+        if (mine == i) cp = v;
+      }
+      const bool in = cp != 0x7FFFFFFF && te >= cp, here = cp != 0x7FFFFFFF && te == cp;
+      const int pos = fwd ? cp : len - 1 - cp, next = fwd ? pos + 1 : pos - 1;
+      const bool ok_next = in && ext_rule_ok(part, next, len - 1, frag), ok_pos = in && ext_rule_ok(part, pos, len - 1, frag);
+      uint32_t b = 0xFFu;  // the row's text symbol at cp, as a query base
+      if (here && P > (uint32_t)cp) b = ((uint32_t)text32(X, d, P, cp) & 3u) ^ (strand ? X.comp_xor : 0u);
+      if (interval(in && ok_next && D <= cp, row_d, k, l) && lead && room)
+        room = emit_tail(o, ps, it, chunk, lost, dir, 1, HPG_BWT_DELETION, 0xFF, pos, k, l);
+#pragma unroll
+      for (uint32_t c = 0; c < 4; ++c) {
+        const bool ins = interval(here && ok_pos && b == c && I <= cp, row_i, k, l);
+        if (ins && lead && room) room = emit_tail(o, ps, it, chunk, lost, dir, 1, HPG_BWT_INSERTION, c, pos, k, l);
+        const bool second = interval(here && ok_pos && ok_next && b == c && I <= cp && twice, row_2, k, l);
+        uint32_t k1, l1;
+        const bool plain = interval(here && ok_next && b == c && M <= cp + 1, row_m, k1, l1);
+        if ((ins ? second : plain) && lead && room)
+          room = emit_tail(o, ps, it, chunk, lost, dir, 1, HPG_BWT_MISMATCH, c, pos, ins ? k : k1, ins ? l : l1);
+      }
+      if (here) todo = false;
+    }
+    if (lead) {
+      ps.count[it] = o.n;
+      ps.refused[it] = o.refused ? 1 : 0;
+      ps.lost[it] = lost ? 1 : 0;
+    }
+    __syncwarp();
+  }
+}
+
 // Lane modes of the persistent tail.  The first four make one backward-
 // extension step per loop iteration; the others are transitions between them.
 enum : uint32_t {
@@ -679,8 +966,8 @@ enum : uint32_t {
 };
 enum : uint32_t { kExtDel = 0, kExtIns, kExtMis };
 
-// Tail pass over the queued blocks of one direction, persistent: lane g takes
-// the queued blocks g, g + G, g + 2G, ... (G lanes in the grid; no claim
+// Tail pass over the queued blocks of one direction, persistent: lane i of warp w takes
+// the queued blocks g = i * warps + w, g + G, g + 2G, ... (G lanes in the grid; no claim
 // counter, whose atomics serialised on one address when lanes finished blocks
 // one by one), runs each as a machine that takes one step per loop iteration
 // whatever part of the block it is in (first walk, second walk, a branch
@@ -694,7 +981,9 @@ __global__ void __launch_bounds__(kBlockTpb) block_tail_kernel(
     const uint32_t* __restrict__ n_queue, uint32_t max_results, PartState ps, unsigned long long* census) {
   const uint32_t nq = *n_queue;
   const uint32_t stride = gridDim.x * blockDim.x;
-  uint32_t next = blockIdx.x * blockDim.x + threadIdx.x;
+  // neighbouring blocks go to different warps: with the text on the device only the wide
+  // ones are queued, fewer than lanes, and a warp steps the faster the fewer it holds
+  uint32_t next = (threadIdx.x & 31u) * (stride >> 5) + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   // (register pressure: the block's part, strand and read come from `it`; the
   // interval before a branch point's step lives in a, b while the branch runs)
   const uint8_t* W = nullptr;
@@ -1076,7 +1365,8 @@ int block_search_device(Engine* e, size_t n, uint32_t max_results, uint64_t* tot
       !ensure(e, e->rs_count, T * 4 + 16) || !ensure(e, e->rs_trunc, T + 16) || !ensure(e, e->hit_off, (T + 1) * 8) ||
       !ensure(e, e->scan_part, scan_parts(T) * 8) || !ensure(e, e->vecs, 2 * T * sizeof(hpg_block_anchor_t) + 16) ||
       !ensure(e, e->ovf, T + 16) || !ensure(e, e->census, 16) || !ensure(e, e->rows, P * 4 + 16) ||
-      !ensure(e, e->b_ctr, 64) || !ensure(e, e->b_spill, T * sizeof(uint4) + 16)) {
+      !ensure(e, e->b_ctr, 64) || !ensure(e, e->b_spill, T * sizeof(uint4) + 16) ||
+      (e->X.text && !ensure(e, e->b_one, 2 * T * sizeof(uint4) + 16))) {
     *err = oom_message("block search", P * (kBlockSlots * sizeof(hpg_hit_t) + 2 * sizeof(hpg_block_anchor_t) + 16));
     return -1;
   }
@@ -1126,23 +1416,39 @@ int block_search_device(Engine* e, size_t n, uint32_t max_results, uint64_t* tot
   const unsigned tail_grid = std::max(1u, std::min(grid_of(T), (unsigned)(std::max(per_sm, 1) * e->num_sms)));
   cudaEventRecord(e->cev[0], s);
   uint32_t* n_cont = n_queue + 2;
+  const uint64_t* packed = e->X.text ? ptr<uint64_t>(e->b_packed) + kPackedPad : nullptr;
+  uint4* one = ptr<uint4>(e->b_one);
+  uint4* few = one + T;
+  uint32_t* n_one = ptr<uint32_t>(e->b_ctr) + 9;  // then the blocks of few rows, and those claimed
+  uint32_t* n_few = n_one + 1;
+  uint32_t* few_head = n_one + 2;
   for (uint32_t phys = 0; phys < 2; ++phys) {  // per index direction: head, the heads' rest, tail
     cudaMemsetAsync(n_queue, 0, 4, s);
     cudaMemsetAsync(n_cont, 0, 4, s);
+    cudaMemsetAsync(n_one, 0, 12, s);
     count_launches(3);
     if (census) {
       block_head_kernel<true><<<grid_of(T), kBlockTpb, 0, s>>>(e->X, codes, offs, ok, (uint32_t)T, phys, max_results,
                                                                ps, queue, n_queue, cont, n_cont, census);
-      block_head_rest_kernel<true><<<grid_of(T), kBlockTpb, 0, s>>>(e->X, codes, offs, cont, n_cont, max_results, ps,
-                                                                    queue, n_queue, census);
+      block_head_rest_kernel<true><<<grid_of(T), kBlockTpb, 0, s>>>(
+          e->X, codes, offs, cont, n_cont, max_results, ps, queue, n_queue, nullptr, nullptr, nullptr,
+          nullptr, nullptr, census);
       block_tail_kernel<true><<<tail_grid, kBlockTpb, 0, s>>>(e->X, codes, offs, queue, n_queue, max_results, ps,
                                                               census);
     } else {
       block_head_kernel<false><<<grid_of(T), kBlockTpb, 0, s>>>(e->X, codes, offs, ok, (uint32_t)T, phys,
                                                                 max_results, ps, queue, n_queue, cont, n_cont,
                                                                 nullptr);
-      block_head_rest_kernel<false><<<grid_of(T), kBlockTpb, 0, s>>>(e->X, codes, offs, cont, n_cont, max_results,
-                                                                     ps, queue, n_queue, nullptr);
+      block_head_rest_kernel<false><<<grid_of(T), kBlockTpb, 0, s>>>(
+          e->X, codes, offs, cont, n_cont, max_results, ps, queue, n_queue, packed, one, n_one, few, n_few,
+          nullptr);
+      if (packed) {
+        count_launches(2);
+        block_rows_text_kernel<<<8 * e->num_sms, kBlockTpb, 0, s>>>(e->X, packed, offs, few, n_few, few_head, max_results,
+                                                                   ps);
+        block_one_kernel<<<std::min(grid_of(T), (unsigned)(16 * e->num_sms)), kBlockTpb, 0, s>>>(
+            e->X, packed, offs, one, n_one, max_results, ps);
+      }
       block_tail_kernel<false><<<tail_grid, kBlockTpb, 0, s>>>(e->X, codes, offs, queue, n_queue, max_results, ps,
                                                                nullptr);
     }

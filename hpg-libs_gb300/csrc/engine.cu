@@ -245,7 +245,7 @@ void engine_release_workspace(Engine* e, uint64_t keep_n_cap) {
   DevBuf* bufs[] = {&e->seqs, &e->offs, &e->codes, &e->ok, &e->rs_count, &e->rs_trunc, &e->vecs, &e->slots,
                     &e->ovf, &e->ovf_count, &e->hit_off, &e->scan_part, &e->hits, &e->rows, &e->loc_off, &e->locs,
                     &e->b_res, &e->b_sorted, &e->b_spill, &e->b_arr, &e->b_seg, &e->b_rowhit, &e->b_long,
-                    &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->b_lists, &e->b_bigs, &e->m_hitoff, &e->m_part, &e->m_offs, &e->m_rows, &e->m_pflag,
+                    &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->b_lists, &e->b_bigs, &e->b_one, &e->m_hitoff, &e->m_part, &e->m_offs, &e->m_rows, &e->m_pflag,
                     &e->m_rowoff, &e->m_nrec, &e->m_flags, &e->m_rec};
   for (DevBuf* b : bufs) {
     cudaFree(b->p);
@@ -282,7 +282,7 @@ void engine_destroy(Engine* e) {
   DevBuf* bufs[] = {&e->seqs, &e->offs, &e->codes, &e->ok, &e->rs_count, &e->rs_trunc, &e->vecs, &e->slots,
                     &e->ovf, &e->ovf_count, &e->hit_off, &e->scan_part, &e->hits, &e->rows, &e->loc_off, &e->locs,
                     &e->census, &e->b_ctr, &e->b_res, &e->b_sorted, &e->b_spill, &e->b_arr, &e->b_seg,
-                    &e->b_rowhit, &e->b_long, &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->b_lists, &e->b_bigs, &e->m_hitoff, &e->m_part, &e->m_offs,
+                    &e->b_rowhit, &e->b_long, &e->b_blocks, &e->b_bovf, &e->b_packed, &e->b_text, &e->b_lists, &e->b_bigs, &e->b_one, &e->m_hitoff, &e->m_part, &e->m_offs,
                     &e->m_rows, &e->m_pflag, &e->m_rowoff, &e->m_nrec, &e->m_flags, &e->m_rec};
   for (DevBuf* b : bufs) cudaFree(b->p);
   for (int i = 0; i <= kStageCount; ++i)
@@ -728,24 +728,25 @@ int engine_autotune(Engine* e, const uint8_t* d_seqs, const uint64_t* d_offs, si
 
 namespace {
 
-// Batched form from the captured graph, then the walk-error check every form makes.
+// Batched form from the captured graph (which checks for a corrupt index too).
 int finish_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_t n, uint64_t total,
-                 uint32_t max_results, DeviceResult* out, std::string* err) {
+                 uint32_t max_results, DeviceResult* out, std::string* err, bool exact = false) {
   DeviceResult r;
-  if (run_batched_graph(e, seqs, offs, n, total, max_results, &r, err) != 0) return -1;
-  uint32_t derr = 0;
-  HPG_CUDA(cudaMemcpy(&derr, e->d_err, 4, cudaMemcpyDeviceToHost), "error word");
-  if (derr) {
-    cudaMemset(e->d_err, 0, 4);
-    *err = "corrupt index: suffix-array walk did not reach a sampled row";
-    return -1;
-  }
+  if (run_batched_graph(e, seqs, offs, n, total, max_results, &r, err, exact) != 0) return -1;
   e->last = r;
   *out = r;
   return 0;
 }
 
 }  // namespace
+
+// Whether an exact search of n reads runs from its own captured graph.  What that form
+// refuses (more rows than a batch indexes, offsets that its device check rejects, no room
+// for its pools) runs in the plain form, as every exact search without the text does.
+static bool exact_graph(const Engine* e, int mode, int form, size_t n) {
+  return mode == HPG_BWT_MODE_EXACT && form == kFormBatched && e->use_graph && e->X.text && !e->census_on &&
+         n <= kTextMaxReads;
+}
 
 int engine_set_kmer(Engine* e, int L, std::string* err) {
   if (L < 0 || L > 12) {
@@ -796,6 +797,7 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
     *err = "unknown pipeline form";
     return -1;
   }
+  const bool exact = exact_graph(e, mode, form, n_reads);
   if (form == kFormBatched && mode != HPG_BWT_MODE_SEARCH1) form = kFormPlain;  // exact search has no branches
   if (n_reads >= (1ull << 31)) {
     *err = "too many reads in one batch";
@@ -810,6 +812,10 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
   const uint32_t n = (uint32_t)n_reads;
   const uint32_t len_cap = std::max<uint32_t>(max_len, 3);
   if (form == kFormBatched && e->use_graph) return finish_graph(e, d_seqs, d_offs, n, total_bases, max_results, out, err);
+  if (exact && total_bases <= (1ull << 40)) {
+    std::string why;
+    if (finish_graph(e, d_seqs, d_offs, n, total_bases, max_results, out, &why, true) == 0) return 0;
+  }
 
   if (!ensure(e, e->codes, total_bases + 16) || !ensure(e, e->ok, n + 16) || !ensure(e, e->rs_count, 8ull * n + 16) ||
       !ensure(e, e->rs_trunc, 2ull * n + 16) || !ensure(e, e->census, 16) || !ensure(e, e->ovf_count, 16)) {
@@ -838,14 +844,16 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
 
   cudaEventRecord(e->ev[0], s);
   uint64_t* packed = nullptr;
-  if (form == kFormBatched && text_form(e, n)) {
+  // the plain search counts the reference's steps when asked to (census): rank steps only then
+  const bool plain_text = form == kFormPlain && mode == HPG_BWT_MODE_SEARCH1 && e->X.text && !census;
+  if ((form == kFormBatched && text_form(e, n)) || plain_text) {
     if (!ensure(e, e->b_packed, packed_words(total_bases) * 8)) {
       *err = "out of device memory (packed reads)";
       return -1;
     }
     packed = ptr<uint64_t>(e->b_packed) + kPackedPad;
   }
-  launch_encode(d_seqs, total_bases, d_offs, n, e->d_table, packed ? nullptr : ptr<uint8_t>(e->codes),
+  launch_encode(d_seqs, total_bases, d_offs, n, e->d_table, packed && !plain_text ? nullptr : ptr<uint8_t>(e->codes),
                 ptr<uint8_t>(e->ok), s, packed);
   cudaEventRecord(e->ev[1], s);
 
@@ -892,7 +900,7 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
       launch_plain_search1(e->X, ptr<uint8_t>(e->codes), d_offs, ptr<uint8_t>(e->ok), (uint32_t)r0, nr, max_results,
                            len_cap, ptr<uint2>(e->vecs), ptr<uint4>(e->slots), ptr<OvfEntry>(e->ovf), e->ovf_cap,
                            ptr<uint32_t>(e->ovf_count), ptr<uint32_t>(e->rs_count), ptr<uint8_t>(e->rs_trunc),
-                           census, s);
+                           packed, census, s);
       uint32_t used = 0;
       HPG_CUDA(cudaMemcpyAsync(&used, e->ovf_count.p, 4, cudaMemcpyDeviceToHost, s), "overflow count");
       HPG_CUDA(cudaStreamSynchronize(s), "search kernel");
@@ -1046,6 +1054,11 @@ int engine_search_host_keep(Engine* e, int mode, int form, const char* seqs, con
     static const uint64_t zero = 0;
     return finish_graph(e, seqs + (n_reads ? offs[0] : 0), n_reads ? o : &zero, (uint32_t)n_reads, total,
                         max_results, r, err);
+  }
+  if (exact_graph(e, mode, form, n_reads) && (n_reads == 0 || offs[0] == 0) && total <= (1ull << 40)) {
+    static const uint64_t zero = 0;
+    std::string why;
+    if (finish_graph(e, seqs, n_reads ? offs : &zero, (uint32_t)n_reads, total, max_results, r, &why, true) == 0) return 0;
   }
   uint32_t max_len = 0;
   for (size_t i = 0; i < n_reads; ++i) {

@@ -44,6 +44,7 @@ struct GraphPlan {
   bool skip_locate = false;  // hits only (the alignment-list layer locates the rows it needs)
   uint32_t kmer_len = 0;     // start table captured with the kernels (length and address)
   const void* kmer0 = nullptr;
+  bool exact = false;          // the exact search (slot kExactSlot)
   const void* text = nullptr;  // the packed text the kernels were captured with (null: sampled arrays only)
   // device buffers
   uint8_t* seqs = nullptr;
@@ -82,7 +83,7 @@ struct GraphPlan {
   uint32_t long_cap = 0;
   SpillEntry* blocks = nullptr;   // j = 1 / j = n-1 blocks of the warp-cooperative form (spill_cap entries)
   // pinned host words
-  uint64_t* h_summary = nullptr;  // [0] status | results << 32, [1] spill tail, [2] hits, [3] rows, [4] census
+  uint64_t* h_summary = nullptr;  // [0] status | results << 32, [1] spill tail, [2] hits, [3] rows, [4] census, [5] walk error
   uint32_t* h_hdr = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -118,6 +119,7 @@ struct Engine {
   // batched form
   DevBuf b_ctr, b_res, b_sorted, b_spill, b_arr, b_seg, b_rowhit, b_long, b_blocks, b_lists, b_bigs;
   DevBuf b_packed, b_text;  // text form (text_search.cu)
+  DevBuf b_one;   // block search: blocks whose fragment matched on one row
   DevBuf b_bovf;  // block search: results past a block's slots, in chunks
   // alignment-list records (map_device.cu)
   DevBuf m_hitoff, m_part, m_offs, m_rows, m_pflag, m_rowoff, m_nrec, m_flags, m_rec;
@@ -136,7 +138,7 @@ struct Engine {
   float stage_ms[kStageCount] = {0, 0, 0, 0};
   DeviceResult last;
   // batched form replayed from a captured CUDA graph (graph.cu)
-  GraphPlan** plans = nullptr;  // two per power-of-two read capacity
+  GraphPlan** plans = nullptr;  // three per power-of-two read capacity
   cudaStream_t xs[2] = {nullptr, nullptr};  // host-to-device and device-to-host copy streams (pipelined calls)
   cudaEvent_t pev[3][2];                    // per plan slot: inputs copied, replay done, results copied
   bool pev_made = false;
@@ -198,13 +200,16 @@ inline bool text_form(const Engine* e, uint64_t n) {
   return e->tuning.split == 3 && e->X.text && n <= kTextMaxReads;
 }
 
-// Reads to the engine's device buffers, encoded (codes + validity flags);
+// Reads to the engine's device buffers, encoded (codes + validity flags, and packed
+// codes where the index has its text);
 // offsets may start anywhere (map_device.cu).
 int upload_reads(Engine* e, const char* seqs, const uint64_t* offs, size_t n, std::string* err);
 
 // Graph form of the batched pipeline (graph.cu).
+constexpr int kExactSlot = 2;  // plan slot of the exact search (with the text on the device)
 int run_batched_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_t n, uint64_t total,
-                      uint32_t max_results, DeviceResult* out, std::string* err);
+                      uint32_t max_results, DeviceResult* out, std::string* err, bool exact = false);
+uint64_t graph_plans_bytes(const Engine* e);  // device bytes of all plans
 void graph_plan_destroy(GraphPlan* g);
 void graph_plans_destroy(Engine* e);
 // Free the plans of more than max_n_cap reads (after the streams finish).

@@ -26,16 +26,19 @@ namespace hpgbwt {
 namespace {
 
 constexpr int kMaxPlans = 33;  // one per power-of-two read capacity
-constexpr int kPlanSlots = 2;  // two plans per capacity: chunks of one batch alternate between them
+// Three plans per capacity: 0 and 1 for chunks of one batch, which alternate between them, and
+// kExactSlot the exact search's.
+constexpr int kPlanSlots = 3;
 
 __global__ void graph_summary_kernel(const unsigned* __restrict__ ctr, const uint64_t* __restrict__ n_hits,
                                      const uint64_t* __restrict__ n_locs, const unsigned long long* census,
-                                     uint64_t* __restrict__ out) {
+                                     const uint32_t* __restrict__ walk_err, uint64_t* __restrict__ out) {
   out[0] = (uint64_t)ctr[4] | ((uint64_t)ctr[3] << 32);
   out[1] = ctr[2];
   out[2] = *n_hits;
   out[3] = *n_locs;
   out[4] = census ? *census : 0ull;
+  out[5] = *walk_err;
 }
 
 uint64_t pow2_at_least(uint64_t v, uint64_t lo) {
@@ -80,14 +83,14 @@ void record(cudaEvent_t ev, cudaStream_t s) { cudaEventRecordWithFlags(ev, s, cu
 int capture(Engine* e, GraphPlan* g, std::string* err) {
   const size_t T = 2ull * g->n_cap;
   const size_t parts = scan_parts(T);
-  const bool text = text_form(e, g->n_cap);
+  const bool exact = g->exact, text = exact || text_form(e, g->n_cap);
   if (!grab(g, &g->seqs, g->bases_cap + 64) || !grab(g, &g->offs, ((size_t)g->n_cap + 1) * 8) ||
       !grab(g, &g->hdr, 32) || (!text && !grab(g, &g->codes, g->bases_cap + 64)) || !grab(g, &g->ok, (size_t)g->n_cap + 16) ||
       !grab(g, &g->ctr, 64) || !grab(g, &g->arr, T * 4 + 16) || !grab(g, &g->seg, (T + 1) * 8) ||
       !grab(g, &g->cursor, T * 4 + 16) || !grab(g, &g->kept, T * 4 + 16) || !grab(g, &g->trunc, T + 16) ||
       !grab(g, &g->part, parts * 8) || !grab(g, &g->res, (size_t)g->res_cap * sizeof(PendingHit)) ||
       !grab(g, &g->sorted, (size_t)g->res_cap * sizeof(PendingHit)) ||
-      !grab(g, &g->spill, (size_t)g->spill_cap * sizeof(SpillEntry)) ||
+      (!exact && !grab(g, &g->spill, (size_t)g->spill_cap * sizeof(SpillEntry))) ||
       !grab(g, &g->hits, ((size_t)g->res_cap + 1) * sizeof(hpg_hit_t)) ||
       !grab(g, &g->list_rows, T * 4 + 16) || !grab(g, &g->tiles, finalize_tiles((uint32_t)T) * sizeof(ulonglong2)) ||
       !grab(g, &g->totals, 16) || !grab(g, &g->bigs, big_lists_cap(g->res_cap, g->locs_cap) * sizeof(uint4)) || !grab(g, &g->read_off, ((size_t)g->n_cap + 1) * sizeof(uint2)) ||
@@ -95,9 +98,9 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
       (!e->X.text && !grab(g, &g->items, (g->locs_cap + 1) * locate_row_item_bytes())) ||
       !grab(g, &g->locs, (g->locs_cap + 1) * sizeof(hpg_loc_t)) || !grab(g, &g->census_d, 16) ||
       !grab(g, &g->long_list, (size_t)g->long_cap * 4) || !grab(g, &g->longs, long_lists_cap(g->res_cap) * 4) ||
-      (g->tuning.split == 3 && !grab(g, &g->blocks, (size_t)g->spill_cap * sizeof(SpillEntry))) ||
-      (text && (!grab(g, &g->packed, packed_words(g->bases_cap) * 8) ||
-                !grab(g, &g->queues, text_queue_bytes(g->n_cap, e->num_sms)))) ||
+      (g->tuning.split == 3 && !exact && !grab(g, &g->blocks, (size_t)g->spill_cap * sizeof(SpillEntry))) ||
+      (text && !grab(g, &g->packed, packed_words(g->bases_cap) * 8)) ||
+      (text && !exact && !grab(g, &g->queues, text_queue_bytes(g->n_cap, e->num_sms))) ||
       !grab(g, &g->summary_d, 64)) {
     *err = "out of device memory (graph plan)";
     return -1;
@@ -148,10 +151,15 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
   if (text) {
     p.packed = g->packed + kPackedPad;
     p.packed_len = g->bases_cap;
-    text_queues(p, g->queues, g->n_cap, e->num_sms);
+    if (!exact) text_queues(p, g->queues, g->n_cap, e->num_sms);
   }
-  launch_search_stage(e->X, p, g->tuning, e->num_sms, ctr, g->long_list, g->long_cap, g->blocks,
-                      g->blocks ? g->spill_cap : 0u, g->ev[2], true, s);
+  if (exact) {
+    launch_text_exact(e->X, p, s);
+    record(g->ev[2], s);
+  } else {
+    launch_search_stage(e->X, p, g->tuning, e->num_sms, ctr, g->long_list, g->long_cap, g->blocks,
+                        g->blocks ? g->spill_cap : 0u, g->ev[2], true, s);
+  }
   record(g->ev[3], s);
 
   // ordered finalize over the capacity (lists past the batch are empty)
@@ -188,8 +196,8 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
                              ctr + 5, census, e->num_sms, s, z);
   record(g->ev[5], s);
   count_launches(1);
-  graph_summary_kernel<<<1, 1, 0, s>>>(ctr, z.n_hits, z.n_locs, census, g->summary_d);
-  cudaMemcpyAsync(g->h_summary, g->summary_d, 40, cudaMemcpyDeviceToHost, s);
+  graph_summary_kernel<<<1, 1, 0, s>>>(ctr, z.n_hits, z.n_locs, census, e->d_err, g->summary_d);
+  cudaMemcpyAsync(g->h_summary, g->summary_d, 48, cudaMemcpyDeviceToHost, s);
   const cudaError_t ce = cudaStreamEndCapture(s, &g->graph);
   g->kernels = launch_count() - launches_before;
   uncount_launches(g->kernels);
@@ -253,7 +261,7 @@ GraphPlan* graph_plan_for(Engine* e, uint32_t n, uint64_t total, const GraphPlan
     return nullptr;
   }
   const uint64_t n_cap = pow2_at_least(n, 4096);
-  const int slot = log2_of(n_cap) * kPlanSlots + (pslot & 1);
+  const int slot = log2_of(n_cap) * kPlanSlots + pslot;
   GraphPlan* g = e->plans[slot];
   const uint64_t bases_cap = pow2_at_least(total, n_cap * 128);
   // a plan captured now starts at the per-read rates earlier overflows showed; a
@@ -298,6 +306,7 @@ GraphPlan* graph_plan_for(Engine* e, uint32_t n, uint64_t total, const GraphPlan
   g->kmer_len = e->X.kmer_len;
   g->kmer0 = e->X.kmer[0];
   g->text = e->X.text;
+  g->exact = pslot == kExactSlot;
   if (old) {  // no stream may still read the old plan's buffers
     cudaStreamSynchronize(e->stream);
     for (cudaStream_t x : e->xs)
@@ -383,6 +392,11 @@ int graph_collect(Engine* e, GraphPlan* g, uint32_t n, GraphPlan* grow, DeviceRe
       grow->locs_cap = std::min<uint64_t>(h[3] + h[3] / 4 + 4096, kMaxLocateRows);
     }
     return 1;
+  }
+  if (h[5]) {
+    cudaMemsetAsync(e->d_err, 0, 4, e->stream);
+    *err = "corrupt index: suffix-array walk did not reach a sampled row";
+    return -1;
   }
   e->census_val = g->census ? h[4] : 0;
   float ms = 0;
@@ -592,15 +606,23 @@ int run_graph_pipelined(Engine* e, const char* seqs, const uint64_t* offs, size_
   return 0;
 }
 
+uint64_t graph_plans_bytes(const Engine* e) {
+  uint64_t sum = 0;
+  for (int i = 0; e->plans && i < kMaxPlans * kPlanSlots; ++i)
+    if (e->plans[i]) sum += e->plans[i]->bytes;
+  return sum;
+}
+
 int run_batched_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_t n, uint64_t total,
-                      uint32_t max_results, DeviceResult* out, std::string* err) {
+                      uint32_t max_results, DeviceResult* out, std::string* err, bool exact) {
   cudaStream_t s = e->stream;
   GraphPlan grow;
   const GraphPlan* staged_in = nullptr;  // plan whose own buffers hold the batch
-  int pslot = 0;
+  int pslot = exact ? kExactSlot : 0;
+  if (exact) max_results = 0xFFFFFFFFu;  // one hit a list, never cut
   if (e->plans)
     for (int i = 0; i < kMaxPlans * kPlanSlots; ++i)
-      if (e->plans[i] && seqs == e->plans[i]->seqs && offs == e->plans[i]->offs) {
+      if (!exact && e->plans[i] && seqs == e->plans[i]->seqs && offs == e->plans[i]->offs) {
         staged_in = e->plans[i];
         pslot = i % kPlanSlots;
       }

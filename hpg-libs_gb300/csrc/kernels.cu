@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kTpb) exact_kernel(DevIndex X, const uint8_t* 
   uint32_t cnt = 0, sectors = 0;
   if (ok[read] && len >= 3 && len <= 32767) {
     uint32_t k = 0, l = X.top;
-    if (exact_bwd(X, view_B(strand), codes + b, len - 1, 0, k, l, sectors)) {
+    if (exact_bwd(X, view_B(strand), TextRead{nullptr, 0, 0, 0}, codes + b, len - 1, 0, k, l, sectors)) {
       slots[(size_t)t * kSlotCap] = make_uint4(k, l, pack_meta(0, 0, 0, 0, 0), 0);
       cnt = 1;
     }
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kTpb)
                          uint32_t max_len, uint2* __restrict__ vecs, uint4* __restrict__ slots,
                          OvfEntry* __restrict__ ovf, uint32_t ovf_cap, uint32_t* __restrict__ ovf_count,
                          uint32_t* __restrict__ rs_count, uint8_t* __restrict__ rs_trunc,
-                         unsigned long long* census) {
+                         const uint64_t* __restrict__ packed, unsigned long long* census) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t T = 2 * nr;
   if (t >= T) return;
@@ -222,9 +222,10 @@ __global__ void __launch_bounds__(kTpb)
     const View B = view_B(strand), F = view_F(strand);
     uint2* vB = vecs + t;
     uint2* vF = vecs + (size_t)max_len * T + t;
-    vector_bwd(X, B, W, len, vB, T, sectors);
-    vector_fwd(X, F, W, len, vF, T, sectors);
-    search1_helper(X, W, len, vB, vF, T, B, F, emit, sectors);
+    const TextRead r{packed, b, len, strand};
+    vector_bwd(X, B, r, W, len, vB, T, sectors);
+    vector_fwd(X, F, r, W, len, vF, T, sectors);
+    search1_helper(X, r, W, len, vB, vF, T, B, F, emit, sectors);
   }
   rs_count[2ull * r0 + t] = emit.cnt;
   rs_trunc[2ull * r0 + t] = emit.trunc ? 1 : 0;
@@ -515,12 +516,13 @@ void launch_exact(const DevIndex& X, const uint8_t* codes, const uint64_t* offs,
 void launch_plain_search1(const DevIndex& X, const uint8_t* codes, const uint64_t* offs, const uint8_t* ok,
                           uint32_t r0, uint32_t nr, uint32_t max_results, uint32_t max_len, uint2* vecs,
                           uint4* slots, OvfEntry* ovf, uint32_t ovf_cap, uint32_t* ovf_count,
-                          uint32_t* rs_count, uint8_t* rs_trunc, unsigned long long* census, cudaStream_t s) {
+                          uint32_t* rs_count, uint8_t* rs_trunc, const uint64_t* packed, unsigned long long* census,
+                          cudaStream_t s) {
   if (!nr) return;
   count_launches(1);
   plain_search1_kernel<<<grid_for(2ull * nr, kTpb), kTpb, 0, s>>>(X, codes, offs, ok, r0, nr, max_results, max_len,
                                                                    vecs, slots, ovf, ovf_cap, ovf_count, rs_count,
-                                                                   rs_trunc, census);
+                                                                   rs_trunc, packed, census);
 }
 
 size_t scan_parts(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }

@@ -51,11 +51,14 @@ void launch_exact(const DevIndex& X, const uint8_t* codes, const uint64_t* offs,
                   unsigned long long* census, cudaStream_t s);
 
 // Plain BWSearch1: one thread per (read, strand) runs the two vector searches
-// into `vecs` and then the helper with its continuation searches.
+// into `vecs` and then the helper with its continuation searches.  With `packed` (the
+// bases' packed codes, and the index's text on the device) searches that come down to one
+// row end by comparing the read with the text.
 void launch_plain_search1(const DevIndex& X, const uint8_t* codes, const uint64_t* offs, const uint8_t* ok,
                           uint32_t r0, uint32_t nr, uint32_t max_results, uint32_t max_len, uint2* vecs,
                           uint4* slots, OvfEntry* ovf, uint32_t ovf_cap, uint32_t* ovf_count,
-                          uint32_t* rs_count, uint8_t* rs_trunc, unsigned long long* census, cudaStream_t s);
+                          uint32_t* rs_count, uint8_t* rs_trunc, const uint64_t* packed, unsigned long long* census,
+                          cudaStream_t s);
 
 // Exclusive scan: out[0..n] with out[n] = total.  `part` needs scan_parts(n) entries.
 size_t scan_parts(size_t n);

@@ -221,17 +221,23 @@ int upload_reads(Engine* e, const char* seqs, const uint64_t* offs, size_t n, st
   cudaStream_t s = e->stream;
   const uint64_t total = n ? offs[n] - offs[0] : 0;
   if (!ensure(e, e->seqs, total + 16) || !ensure(e, e->offs, (n + 1) * 8) || !ensure(e, e->codes, total + 16) ||
-      !ensure(e, e->ok, n + 16)) {
+      !ensure(e, e->ok, n + 16) || (e->X.text && !ensure(e, e->b_packed, packed_words(total) * 8))) {
     *err = "out of device memory (reads)";
     return -1;
   }
-  std::vector<uint64_t> rel(n + 1);
-  for (size_t i = 0; i <= n; ++i) rel[i] = n ? offs[i] - offs[0] : 0;
+  static const uint64_t zero = 0;
+  const uint64_t* from = n ? offs : &zero;
+  std::vector<uint64_t> rel;
+  if (from[0]) {  // offsets that start at 0 go as they are
+    rel.resize(n + 1);
+    for (size_t i = 0; i <= n; ++i) rel[i] = offs[i] - offs[0];
+    from = rel.data();
+  }
   if (total) HPG_CUDA(cudaMemcpyAsync(e->seqs.p, seqs + offs[0], total, cudaMemcpyHostToDevice, s), "upload reads");
-  HPG_CUDA(cudaMemcpyAsync(e->offs.p, rel.data(), (n + 1) * 8, cudaMemcpyHostToDevice, s), "upload offsets");
+  HPG_CUDA(cudaMemcpyAsync(e->offs.p, from, (n + 1) * 8, cudaMemcpyHostToDevice, s), "upload offsets");
   launch_encode(ptr<uint8_t>(e->seqs), total, ptr<uint64_t>(e->offs), (uint32_t)n, e->d_table, ptr<uint8_t>(e->codes),
-                ptr<uint8_t>(e->ok), s);
-  HPG_CUDA(cudaStreamSynchronize(s), "encode");  // `rel` is pageable and local
+                ptr<uint8_t>(e->ok), s, e->X.text ? ptr<uint64_t>(e->b_packed) + kPackedPad : nullptr);
+  if (!rel.empty()) HPG_CUDA(cudaStreamSynchronize(s), "encode");  // `rel` is pageable and local
   return 0;
 }
 

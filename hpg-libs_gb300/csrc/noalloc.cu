@@ -76,8 +76,9 @@ __global__ void __launch_bounds__(128)
     const View F = strand ? View{0, 1} : View{1, 0};
     uint2* vB = vecs + t;
     uint2* vF = vecs + (size_t)len_cap * T + t;
-    vector_bwd(X, B, W, len, vB, T, sectors);
-    vector_fwd(X, F, W, len, vF, T, sectors);
+    const TextRead r{nullptr, 0, len, strand};  // (no packed reads here: rank steps)
+    vector_bwd(X, B, r, W, len, vB, T, sectors);
+    vector_fwd(X, F, r, W, len, vF, T, sectors);
     auto emit = [&](const Cursor& c) -> bool {
       if (cnt >= max_results) {
         trunc = true;
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(128)
       ++cnt;
       return true;
     };
-    search1_helper(X, W, len, vB, vF, T, B, F, emit, sectors);
+    search1_helper(X, r, W, len, vB, vF, T, B, F, emit, sectors);
   }
   counts[t] = cnt;
   truncated[t] = trunc ? 1 : 0;

@@ -11,6 +11,7 @@
 #pragma once
 
 #include "fm_device.cuh"
+#include "text_dev.cuh"
 
 namespace hpgbwt {
 
@@ -32,67 +33,116 @@ struct Cursor {
 
 #ifdef __CUDACC__
 
-// Continue a backward search over W[pos..start]; true if the interval survives.
-__device__ __forceinline__ bool exact_bwd(const DevIndex& X, View v, const uint8_t* W, int pos, int start,
-                                          uint32_t& k, uint32_t& l, uint32_t& sectors) {
-  for (int i = pos; i >= start; --i) {
+// Where the read's packed bases are, for searches that finish with the text on the
+// device; packed null: rank steps only.
+struct TextRead {
+  const uint64_t* packed;
+  uint64_t b0;
+  int len;
+  uint32_t strand;
+};
+
+// How far a one-row search at row k agrees with the text over `want` symbols from symbol i of
+// its direction on (search order), and the row it has then.
+__device__ __forceinline__ int text_run(const DevIndex& X, View v, const TextRead& r, bool fwd, int i, int want,
+                                        uint32_t k, uint32_t& row) {
+  const uint32_t P = load_row_word((v.d ? X.dir[1].sa : X.dir[0].sa) + k);
+  const int m = agree(X, r.packed, r.b0, r.len, fwd, r.strand, v.d, i, P, (int)min((uint32_t)want, P));
+  row = load_row_word((v.d ? X.dir[1].isa : X.dir[0].isa) + P - (uint32_t)m);
+  return m;
+}
+
+// Continue a search over `want` bases from W[pos] on (dir -1 or +1); true if the interval
+// survives.  One row that has matched on ends by the text.
+__device__ __forceinline__ bool exact_run(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int pos, int dir,
+                                          int want, uint32_t& k, uint32_t& l, uint32_t& sectors) {
+  for (; want > 0; --want, pos += dir) {
+    const bool one = k == l;
     sectors += ((k >> 6) == (l >> 6)) ? 1u : 2u;
-    bw_step(X, v, W[i], k, l);
+    bw_step(X, v, W[pos], k, l);
     if (k > l) return false;
+    if (one && want > 1 && r.packed) {
+      const int i = dir > 0 ? pos + 1 : r.len - pos;
+      uint32_t row;
+      if (text_run(X, v, r, dir > 0, i, want - 1, k, row) != want - 1) return false;
+      k = l = row;
+      return true;
+    }
   }
   return k <= l;
 }
 
-__device__ __forceinline__ bool exact_fwd(const DevIndex& X, View v, const uint8_t* W, int pos, int end,
+// Continue a backward search over W[pos..start]; true if the interval survives.
+__device__ __forceinline__ bool exact_bwd(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int pos,
+                                          int start, uint32_t& k, uint32_t& l, uint32_t& sectors) {
+  return exact_run(X, v, r, W, pos, -1, pos - start + 1, k, l, sectors);
+}
+
+__device__ __forceinline__ bool exact_fwd(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int pos, int end,
                                           uint32_t& k, uint32_t& l, uint32_t& sectors) {
-  for (int i = pos; i <= end; ++i) {
-    sectors += ((k >> 6) == (l >> 6)) ? 1u : 2u;
-    bw_step(X, v, W[i], k, l);
-    if (k > l) return false;
-  }
-  return k <= l;
+  return exact_run(X, v, r, W, pos, 1, end - pos + 1, k, l, sectors);
 }
 
 __device__ __forceinline__ int64_t isize(uint2 v) { return (int64_t)v.y - (int64_t)v.x; }
 
-// Vector searches; the vector element for read position j lives at vec[j * stride].
-__device__ __forceinline__ void vector_bwd(const DevIndex& X, View v, const uint8_t* W, int len, uint2* vec,
-                                           size_t stride, uint32_t& sectors) {
+// Vector searches; the vector element for read position j lives at vec[j * stride].  The
+// helper reads elements n/2 .. 0 of the backward search and n/2 - 1 .. n of the forward one
+// (n = len - 1), so only those are kept, and a start table of the text's covers steps whose
+// elements are not.  It reads an element's interval only where its size differs from the next
+// one's, so the elements of a run that the text matched keep one row each, and the true one
+// only at the run's end; a failed element is any empty interval (its size is -1 always).
+__device__ __forceinline__ void vector_run(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int len,
+                                           int dir, uint2* vec, size_t stride, uint32_t& sectors) {
   uint32_t k = 0, l = X.top;
-  int i = len - 1;
-  for (; i >= 0; --i) {
-    sectors += ((k >> 6) == (l >> 6)) ? 1u : 2u;
-    bw_step(X, v, W[i], k, l);
-    vec[(size_t)i * stride] = make_uint2(k, l);
-    if (k > l) {
-      --i;
-      break;
+  const int half = (len - 1) / 2, keep = dir > 0 ? half - 1 : len - 1 - half;  // first step whose element is kept
+  int i = dir > 0 ? 0 : len - 1, t = 0;
+  const int L = r.packed ? (int)X.tmer_len : 0;
+  if (L && len >= 2 * L + 2) {
+    const uint64_t q = query32(X, r.packed, r.b0, len, dir > 0, r.strand, 0);
+    const uint32_t c = __brev((uint32_t)q) >> (32 - 2 * L);
+    const uint2 s = load_row_pair((v.d ? X.tmer[1] : X.tmer[0]) + (((c & 0x55555555u) << 1) | ((c >> 1) & 0x55555555u)));
+    k = s.x;
+    l = s.y;
+    t = L;
+    i += dir * L;
+    if (L > keep) vec[(size_t)(i - dir) * stride] = s;  // (the shortest such read's forward search)
+  }
+  for (; t < len; ++t, i += dir) {
+    const bool one = k == l;
+    if (k <= l) {
+      sectors += ((k >> 6) == (l >> 6)) ? 1u : 2u;
+      bw_step(X, v, W[i], k, l);
+    }
+    if (t >= keep) vec[(size_t)i * stride] = make_uint2(k, l);
+    if (one && k == l && t + 1 < len && r.packed) {
+      uint32_t row;
+      const int m = text_run(X, v, r, dir > 0, t + 1, len - t - 1, k, row);
+      for (int q = max(1, keep - t); q <= m; ++q)
+        vec[(size_t)(i + dir * q) * stride] = q == m ? make_uint2(row, row) : make_uint2(k, k);
+      t += m;
+      i += dir * m;
+      k = 1;  // what is left, if anything, has failed
+      l = 0;
     }
   }
-  for (; i >= 0; --i) vec[(size_t)i * stride] = make_uint2(k, l);
 }
 
-__device__ __forceinline__ void vector_fwd(const DevIndex& X, View v, const uint8_t* W, int len, uint2* vec,
-                                           size_t stride, uint32_t& sectors) {
-  uint32_t k = 0, l = X.top;
-  int i = 0;
-  for (; i < len; ++i) {
-    sectors += ((k >> 6) == (l >> 6)) ? 1u : 2u;
-    bw_step(X, v, W[i], k, l);
-    vec[(size_t)i * stride] = make_uint2(k, l);
-    if (k > l) {
-      ++i;
-      break;
-    }
-  }
-  for (; i < len; ++i) vec[(size_t)i * stride] = make_uint2(k, l);
+__device__ __forceinline__ void vector_bwd(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int len,
+                                           uint2* vec, size_t stride, uint32_t& sectors) {
+  vector_run(X, v, r, W, len, -1, vec, stride, sectors);
+}
+
+__device__ __forceinline__ void vector_fwd(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int len,
+                                           uint2* vec, size_t stride, uint32_t& sectors) {
+  vector_run(X, v, r, W, len, 1, vec, stride, sectors);
 }
 
 // The helper for one strand.  `emit(cursor)` appends a hit and returns false
 // when the list is full, which ends the helper (search/results.h:100-101).
 // Returns true on overflow.
 template <typename Emit>
-__device__ bool search1_helper(const DevIndex& X, const uint8_t* W, int len, const uint2* vk, const uint2* vki,
+__device__ bool search1_helper(const DevIndex& X, const TextRead& r, const uint8_t* W, int len, const uint2* vk,
+                               const uint2* vki,
                                size_t stride, View B, View F, Emit& emit, uint32_t& sectors) {
   const int start = 0, end = len - 1;
   const int n = end - start;
@@ -162,7 +212,7 @@ __device__ bool search1_helper(const DevIndex& X, const uint8_t* W, int len, con
     c.err_pos = i - 1;
     {
       uint32_t k = v.x, l = v.y;
-      if (exact_bwd(X, B, W, i - 2, start, k, l, sectors)) {
+      if (exact_bwd(X, B, r, W, i - 2, start, k, l, sectors)) {
         c.k = k;
         c.l = l;
         if (!emit(c)) return true;
@@ -178,7 +228,7 @@ __device__ bool search1_helper(const DevIndex& X, const uint8_t* W, int len, con
       c.base = b;
       {
         uint32_t k = ka, l = la;
-        if (exact_bwd(X, B, W, i - 1, start, k, l, sectors)) {
+        if (exact_bwd(X, B, r, W, i - 1, start, k, l, sectors)) {
           c.k = k;
           c.l = l;
           if (!emit(c)) return true;
@@ -187,7 +237,7 @@ __device__ bool search1_helper(const DevIndex& X, const uint8_t* W, int len, con
       if (b != wi) {
         c.kind = 2;  // MISMATCH
         uint32_t k = ka, l = la;
-        if (exact_bwd(X, B, W, i - 2, start, k, l, sectors)) {
+        if (exact_bwd(X, B, r, W, i - 2, start, k, l, sectors)) {
           c.k = k;
           c.l = l;
           if (!emit(c)) return true;
@@ -245,7 +295,7 @@ __device__ bool search1_helper(const DevIndex& X, const uint8_t* W, int len, con
     c.err_pos = i + 1;
     {
       uint32_t k = v.x, l = v.y;
-      if (exact_fwd(X, F, W, i + 2, end, k, l, sectors)) {
+      if (exact_fwd(X, F, r, W, i + 2, end, k, l, sectors)) {
         c.k = k;
         c.l = l;
         if (!emit(c)) return true;
@@ -261,7 +311,7 @@ __device__ bool search1_helper(const DevIndex& X, const uint8_t* W, int len, con
       c.base = b;
       {
         uint32_t k = ka, l = la;
-        if (exact_fwd(X, F, W, i + 1, end, k, l, sectors)) {
+        if (exact_fwd(X, F, r, W, i + 1, end, k, l, sectors)) {
           c.k = k;
           c.l = l;
           if (!emit(c)) return true;
@@ -270,7 +320,7 @@ __device__ bool search1_helper(const DevIndex& X, const uint8_t* W, int len, con
       if (b != wi) {
         c.kind = 2;
         uint32_t k = ka, l = la;
-        if (exact_fwd(X, F, W, i + 2, end, k, l, sectors)) {
+        if (exact_fwd(X, F, r, W, i + 2, end, k, l, sectors)) {
           c.k = k;
           c.l = l;
           if (!emit(c)) return true;

@@ -462,9 +462,7 @@ struct Server {
       hits_per_read = std::max(hpr, 0.8 * hits_per_read + 0.2 * hpr);
       rows_per_read = std::max(rpr, 0.8 * rows_per_read + 0.2 * rpr);
     }
-    plan_bytes = 0;
-    for (int i = 0; i < 66; ++i)
-      if (e->plans && e->plans[i]) plan_bytes += e->plans[i]->bytes;
+    plan_bytes = graph_plans_bytes(e);
     b->reqs.clear();
     cv_done.notify_all();
     if (timing) {

@@ -52,6 +52,7 @@
 #include "batched.cuh"
 #include "batched_dev.cuh"
 #include "kernels.cuh"
+#include "text_dev.cuh"
 
 namespace hpgbwt {
 
@@ -71,54 +72,6 @@ constexpr uint32_t kRows = 32;       // rows of a chain in the row queue at most
 constexpr uint32_t kAbsent = 0xFFFFFFFFu, kMany = 0xFFFFFFFEu;
 __device__ __forceinline__ bool is_diag(uint32_t x) { return x < kMany; }
 constexpr unsigned kFull = 0xFFFFFFFFu;
-
-// 32 symbols of a 2-bit stream from symbol i on (i may be -31 or reach past the
-// end by as much: the streams are padded), symbol i in the low bits.
-__device__ __forceinline__ uint64_t load32(const uint64_t* s, int64_t i) {
-  const uint64_t* w = s + (i >> 5);
-  const uint32_t sh = ((uint32_t)i & 31u) << 1;
-  return (__ldg(w) >> sh) | ((__ldg(w + 1) << 1) << (63u - sh));
-}
-
-// The 32 symbols in reverse order.
-__device__ __forceinline__ uint64_t rev32(uint64_t x) {
-  const uint64_t r = __brevll(x);
-  return ((r & 0x5555555555555555ull) << 1) | ((r >> 1) & 0x5555555555555555ull);
-}
-
-__device__ __forceinline__ uint64_t comp_word(const DevIndex& X, uint32_t strand) {
-  return strand ? 0x5555555555555555ull * X.comp_xor : 0ull;
-}
-
-// (the words below are selected, not branched on, so that a warp's strands and
-// directions stay together)
-
-// Symbols i .. i+31 of a chain (past the read's end: whatever the stream holds), symbol i in the low bits.
-__device__ __forceinline__ uint64_t query32(const DevIndex& X, const uint64_t* packed, uint64_t b0, int len,
-                                            bool fwd, uint32_t strand, int i) {
-  const uint64_t x = load32(packed, (int64_t)b0 + (fwd ? i : len - 32 - i));
-  const uint64_t r = rev32(x);
-  return (fwd ? x : r) ^ comp_word(X, strand);
-}
-
-// The text read leftwards from position P of physical direction d, from its m-th symbol on:
-// T_d[P-1-m], T_d[P-2-m], ... (past the text's ends: padding).
-__device__ __forceinline__ uint64_t text32(const DevIndex& X, uint32_t d, uint32_t P, int m) {
-  const uint64_t x = load32(X.text, d ? (int64_t)X.top - P + m : (int64_t)P - 32 - m);
-  const uint64_t r = rev32(x);
-  return d ? x : r;
-}
-
-// How many of the symbols i .. i+want-1 of a chain agree with the text read
-// leftwards from position P of physical direction d; want <= P.
-__device__ __forceinline__ int agree(const DevIndex& X, const uint64_t* packed, uint64_t b0, int len, bool fwd,
-                                     uint32_t strand, uint32_t d, int i, uint32_t P, int want) {
-  for (int m = 0; m < want; m += 32) {
-    const uint64_t x = text32(X, d, P, m) ^ query32(X, packed, b0, len, fwd, strand, i + m);
-    if (x) return min(want, m + ((__ffsll((long long)x) - 1) >> 1));
-  }
-  return want;
-}
 
 // One rank step on a physical symbol.
 __device__ __forceinline__ void rank_step(const DevIndex& X, const OccBlock* occ, uint32_t dollar, uint32_t ph,
@@ -1055,6 +1008,67 @@ __global__ void __launch_bounds__(kWalkTpb) text_block_kernel(DevIndex X, Batche
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
 
+// Exact search of both strands (BWExactSearchBackward over backward, '-': over
+// forward_rev; search.h:9-65) with the text: a thread per (read, strand), its start table
+// entry, rank steps until the interval is empty or has stayed one row for a step, then one
+// comparison with the text.  (200k x 100 bp, 4 Mbp: 163 us with rank steps to the end.)
+template <bool CENSUS>
+__global__ void __launch_bounds__(kHeadTpb) text_exact_kernel(DevIndex X, BatchedParams p) {
+  __shared__ uint32_t s_cnt[kHeadTpb / 32], s_base;
+  const uint32_t n_reads = p.n_reads_dev ? *p.n_reads_dev : p.n_reads;
+  if ((uint64_t)blockIdx.x * kHeadTpb >= n_reads) return;
+  const uint32_t read = blockIdx.x * kHeadTpb + threadIdx.x, strand = blockIdx.y, d = strand;
+  uint32_t k = 1, l = 0, sectors = 0, sa1 = 0;
+  if (read < n_reads && p.ok[read]) {
+    const uint64_t b0 = p.offs[read], b1 = p.offs[read + 1];
+    if (b1 >= b0 + 3 && b1 - b0 <= 32767 && b1 <= p.packed_len) {
+      const int len = (int)(b1 - b0);
+      const OccBlock* occ = d ? X.dir[1].occ : X.dir[0].occ;
+      const uint32_t dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
+      uint64_t q = query32(X, p.packed, b0, len, false, strand, 0);
+      int t = 0;
+      k = 0;
+      l = X.top;
+      const int L = (int)X.tmer_len;
+      if (len >= L) {
+        const uint32_t r = __brev((uint32_t)q) >> (32 - 2 * L);
+        const uint2 s = load_row_pair((d ? X.tmer[1] : X.tmer[0]) + (((r & 0x55555555u) << 1) | ((r >> 1) & 0x55555555u)));
+        if (CENSUS) ++sectors;
+        k = s.x;
+        l = s.y;
+        t = L;
+        q >>= 2 * L;
+      }
+      while (k <= l && t < len) {
+        const uint32_t pk = k, pl = l;
+        if (CENSUS) sectors += (k >> 6) == (l >> 6) ? 1u : 2u;
+        rank_step(X, occ, dollar, (uint32_t)q & 3u, k, l);
+        ++t;
+        if ((t & 31) == 0) q = query32(X, p.packed, b0, len, false, strand, t);
+        else q >>= 2;
+        if (k == l && pk == pl && t < len) {
+          const uint32_t P = load_row_word((d ? X.dir[1].sa : X.dir[0].sa) + k);
+          const int left = len - t;
+          if (CENSUS) sectors += 2;
+          if (P >= (uint32_t)left && agree(X, p.packed, b0, len, false, strand, d, t, P, left) == left) {
+            k = l = load_row_word((d ? X.dir[1].isa : X.dir[0].isa) + P - (uint32_t)left);
+            sa1 = P - (uint32_t)left + 1;
+            if (CENSUS) ++sectors;
+          } else {
+            k = 1;
+            l = 0;
+          }
+          break;
+        }
+      }
+    }
+  }
+  const bool hit = k <= l;
+  const uint32_t slot = block_slots<kHeadTpb>(hit ? 1u : 0u, p.res_total, s_cnt, &s_base);
+  if (hit) write_hit(p, slot, (read << 1) | strand, order_key(0, 0, 0), k, l, pack_meta(0, 0, 0, 0, 0), sa1);
+  if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
+}
+
 template <bool CENSUS>
 void launch_text_stage(const DevIndex& X, const BatchedParams& p, int num_sms, cudaStream_t s) {
   const uint32_t cap = p.n_reads;
@@ -1092,6 +1106,14 @@ void text_queues(BatchedParams& p, void* buffer, size_t n_reads, int num_sms) {
   p.walk = p.rest + 4 * n_reads;
   p.walk_cap = (uint32_t)text_walk_cap(n_reads, num_sms);
   p.diag = reinterpret_cast<uint32_t*>(p.walk + p.walk_cap);
+}
+
+void launch_text_exact(const DevIndex& X, const BatchedParams& p, cudaStream_t s) {
+  if (!p.n_reads) return;
+  count_launches(1);
+  const dim3 grid((p.n_reads + kHeadTpb - 1) / kHeadTpb, 2);
+  if (p.census) text_exact_kernel<true><<<grid, kHeadTpb, 0, s>>>(X, p);
+  else text_exact_kernel<false><<<grid, kHeadTpb, 0, s>>>(X, p);
 }
 
 void launch_text_search(const DevIndex& X, const BatchedParams& p, int num_sms, cudaStream_t s) {

@@ -41,6 +41,8 @@ def _check(g: lib.GpuIndex, reads, want, max_results):
             g.set_graph(graph)
             got = g.search(reads, mode=lib.MODE_SEARCH1, form=lib.FORM_BATCHED, max_results=max_results)
             assert got.equal(want), f"full rows {rows}, graph {graph}"
+        got = g.search(reads, mode=lib.MODE_SEARCH1, form=lib.FORM_PLAIN, max_results=max_results)
+        assert got.equal(want), f"plain form, full rows {rows}"
 
 
 @pytest.mark.parametrize("kind,n,chroms", [("iid", 700, 1), ("iid", 30_011, 2), ("repeats", 200_000, 3),
@@ -88,3 +90,25 @@ def test_sampling_ratios(tmp_path, ratio):
     with lib.GpuIndex(str(tmp_path / "idx")) as g:
         assert g.full_rows()
         _check(g, reads, want, 1 << 16)
+
+
+@pytest.mark.parametrize("kind,n", [("iid", 700), ("human_like", 60_000)])
+def test_exact_search_edges(case_factory, kind, n):
+    """The exact search from its graph, from device or host bases, against the oracle and the plain form."""
+    c = case_factory(kind, n, 31, 2)
+    reads = _edge_reads(c.genome, 6)
+    want = PortOracle(c.index).search(reads, mode=lib.MODE_EXACT, max_results=1, threads=8)
+    with lib.GpuIndex(c.index) as g:
+        for rows in (True, False):
+            g.set_full_rows(rows)
+            for max_results in (1, 0):  # an exact list holds one hit whatever the capacity
+                for form in (lib.FORM_BATCHED, lib.FORM_PLAIN):
+                    got = g.search(reads, mode=lib.MODE_EXACT, form=form, max_results=max_results)
+                    assert got.equal(want), f"full rows {rows}, form {form}, capacity {max_results}"
+        g.set_locate_limit(1)
+        a = g.search(reads, mode=lib.MODE_EXACT, form=lib.FORM_BATCHED)
+        assert a.equal(g.search(reads, mode=lib.MODE_EXACT, form=lib.FORM_PLAIN))
+        bad = synth.ReadSet(reads.seq, reads.offsets.copy(), reads.truth_pos, reads.truth_strand, reads.edit)
+        bad.offsets[5] = bad.offsets[7] + np.uint64(1)
+        with pytest.raises(RuntimeError, match="non-decreasing"):
+            g.search(bad, mode=lib.MODE_EXACT, form=lib.FORM_BATCHED)
