@@ -66,7 +66,12 @@ constexpr int kRowsWarps = kRowsTpb / 32;
 // by then (search stage at 4 / 5 / 6 / 8 steps, 2M x 100 bp, 100 Mbp: 899 / 884 / 891 /
 // 901 us; the lanes of the others, some in most warps, would hold their warps longer).
 constexpr int kHeadSteps = 6;
-constexpr uint32_t kRows = 32;       // rows of a chain in the row queue at most
+// Rows of a chain in the row queue at most.  Where the helper does not branch yet a wide
+// chain steps on down to kRowsBefore (2M x 150 bp, 600 Mbp: 4660 us a call at 32, 4560 at
+// 16, 4500 at 8, 4470 at 4, 4450 at 2): a step is two sectors for all its rows, a row in the
+// queue two to three.  Within the branching window every step may queue a change point, and
+// all 32 are taken.
+constexpr uint32_t kRows = 32, kRowsBefore = 4;
 // A chain's entry of `diag` that is no alignment: its first symbols (kHeadSteps past the
 // table at most) do not occur, or it was left to the row queue or the rest list.
 constexpr uint32_t kAbsent = 0xFFFFFFFFu, kMany = 0xFFFFFFFEu;
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, Batched
       while (k <= l) {
         if (t == stop) {
           one = k == l;
-          dest = one ? 0 : (l - k < kRows ? 1 : 2);
+          dest = one ? 0 : (l - k < kRowsBefore ? 1 : 2);
           e = make_uint4(k, l, 0, (uint32_t)t);
           break;
         }
@@ -228,6 +233,44 @@ __global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, Batched
   if (dest == 1) p.rows[s_base[0] + s_cnt[0][warp] + (uint32_t)__popc(m1 & ((1u << lane) - 1u))] = e;
   else if (dest == 2) p.rest[s_base[1] + s_cnt[1][warp] + (uint32_t)__popc(m2 & ((1u << lane) - 1u))] = e;
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
+}
+
+// The least i >= lo from which on symbols i .. len-1 of a chain agree with T(i + shift)
+// beside them, T(i) = T_d[P - 1 - i]; len + shift <= P, and symbol lo inside the text.
+__device__ __forceinline__ int agree_back(const DevIndex& X, const uint64_t* packed, uint64_t b0, int len, bool fwd,
+                                          uint32_t strand, uint32_t d, uint32_t P, int shift, int lo) {
+  int hi = len;  // symbols hi .. len-1 agree
+  while (hi > lo) {
+    // symbols hi-32 .. hi-1 against T(hi-32+shift) .. T(hi-1+shift), the last symbol in the top bits
+    uint64_t qw = fwd ? load32(packed, (int64_t)b0 + hi - 32) : load32(packed, (int64_t)b0 + len - hi);
+    qw ^= comp_word(X, strand);
+    uint64_t tw = d ? load32(X.text, (int64_t)X.top - P + hi - 32 + shift) : load32(X.text, (int64_t)P - hi - shift);
+    if (!fwd) qw = rev32(qw);
+    if (!d) tw = rev32(tw);
+    const uint64_t x = qw ^ tw;
+    const int same = x ? __clzll((long long)x) >> 1 : 32;
+    hi -= same;
+    if (same < 32) break;
+  }
+  return max(hi, lo);
+}
+
+// The first t in ts .. near a wide chain's change points can have hits from (near: none
+// before it), where the strand's other chain has the one alignment `other`: the symbols
+// after a failing one at te < near lie there or nowhere (text_branch_kernel).  So they agree
+// from te + 1 on, and the ones before te agree one place nearer (deletion), there
+// (mismatch, te then the last symbol that disagrees) or one place farther (insertion).
+__device__ __forceinline__ int hits_from(const DevIndex& X, const uint64_t* packed, uint64_t b0, int len, bool fwd,
+                                         uint32_t strand, uint32_t d, uint32_t other, int ts, int near) {
+  const int64_t P64 = (int64_t)X.top + len - other;
+  if (P64 < len || P64 > (int64_t)X.top + 1) return near;
+  const uint32_t P = (uint32_t)P64;
+  const int m = agree_back(X, packed, b0, len, fwd, strand, d, P, 0, ts), te = max(ts, m - 1);
+  if (te >= near) return near;
+  if (agree(X, packed, b0, len, fwd, strand, d, 0, P - 1, te) == te) return te;
+  if (m > ts && P <= X.top && agree(X, packed, b0, len, fwd, strand, d, 0, P, te) == te) return te;
+  if (P < X.top && agree(X, packed, b0, len, fwd, strand, d, 0, P + 1, te) == te) return te;
+  return near;
 }
 
 // The hits of a change point whose interval is one row: with the chain's symbol i
@@ -494,25 +537,10 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
     __syncwarp();
     if (lane == 0) ws.next = first + take;
     if (te >= ts) {  // of use to the helper: where the three shifted alignments begin to agree for good
-      auto from_end = [&](int shift) -> int {  // symbols i agree with T(i + shift) down to the returned i, at least ts
+      auto from_end = [&](int shift) -> int {
         const int64_t need = (int64_t)len + shift;  // text symbols the read takes
         if (need > (int64_t)P) return 0x7FFFFFFF;
-        int hi = len;  // symbols hi .. len-1 agree
-        const int lo = shift < 0 ? ts + 1 : ts;  // the deletion's first symbol is te + 1
-        while (hi > lo) {
-          // symbols hi-32 .. hi-1 against T(hi-32+shift) .. T(hi-1+shift), the last symbol in the top bits
-          uint64_t qw = fwd ? load32(p.packed, (int64_t)b0 + hi - 32) : load32(p.packed, (int64_t)b0 + len - hi);
-          qw ^= comp_word(X, strand);
-          uint64_t tw = d ? load32(X.text, (int64_t)(X.top - P) + hi - 32 + shift)
-                          : load32(X.text, (int64_t)P - hi - shift);
-          if (!fwd) qw = rev32(qw);
-          if (!d) tw = rev32(tw);
-          const uint64_t x = qw ^ tw;
-          const int same = x ? __clzll((long long)x) >> 1 : 32;
-          hi -= same;
-          if (same < 32) break;
-        }
-        return max(hi, lo);
+        return agree_back(X, p.packed, b0, len, fwd, strand, d, P, shift, shift < 0 ? ts + 1 : ts);  // (the deletion's first symbol is te + 1)
       };
       D = from_end(-1) - 1;
       I = from_end(1);
@@ -645,8 +673,13 @@ __global__ void __launch_bounds__(kWideTpb) text_wide_kernel(DevIndex X, Batched
         len = (int)(p.offs[(rs >> 1) + 1] - b0);
         const uint32_t strand = rs & 1u, d = (fwd ? 1u : 0u) ^ strand;
         ts = branch_from(len, fwd);
-        // change points whose remaining symbols hold a head that does not occur have no hits
-        if (other_chain(X, p, rs, d, len, ts + 1) == kAbsent) ts = len - (int)X.tmer_len - kHeadSteps;
+        // change points without hits are not queued: their remaining symbols hold a head that
+        // does not occur, or that occurs once and not where the read's two parts would meet
+        const uint32_t other = other_chain(X, p, rs, d, len, ts + 1);
+        if (other != kMany) {
+          const int near = len - (int)X.tmer_len - kHeadSteps;
+          ts = other == kAbsent ? near : hits_from(X, p.packed, b0, len, fwd, strand, d, other, ts, near);
+        }
         occ = d ? X.dir[1].occ : X.dir[0].occ;
         dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
         q = query32(X, p.packed, b0, len, fwd, strand, t);
@@ -674,7 +707,7 @@ __global__ void __launch_bounds__(kWideTpb) text_wide_kernel(DevIndex X, Batched
     }
     if (k <= l && t + 1 < len) {
       ++t;
-      if (l - k < kRows) {  // few enough rows for a lane each
+      if (l - k < (t < ts ? kRowsBefore : kRows)) {  // few enough rows for a lane each
         p.rows[claim(p.rows_n, 1)] = make_uint4(k, l, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u));
         active = false;
         continue;
