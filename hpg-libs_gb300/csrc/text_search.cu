@@ -778,6 +778,7 @@ __device__ __forceinline__ void rank_step4(const DevIndex& X, const OccBlock* oc
 template <bool CENSUS>
 __global__ void __launch_bounds__(kWideTpb) text_branch_kernel(DevIndex X, BatchedParams p) {
   __shared__ uint32_t c_res[kWideTpb], c_walk[kWideTpb], s_k[4][kWideTpb], s_l[4][kWideTpb];
+  __shared__ uint8_t s_from[kWideTpb];
   const int tid = threadIdx.x;
   const uint32_t lane = tid & 31;
   const uint32_t n_src = min(*(volatile unsigned int*)p.spill_tail, p.spill_cap);
@@ -803,7 +804,38 @@ __global__ void __launch_bounds__(kWideTpb) text_branch_kernel(DevIndex X, Batch
   };
   for (;;) {
     const unsigned idle = __ballot_sync(kFull, !stepping && !todo);  // every lane, every iteration
-    if (!exhausted && (idle == kFull || (uint32_t)__popc(idle) >= bi)) {
+    unsigned give = 0;
+    if (idle != kFull && (uint32_t)__popc(idle) >= bi && (give = __ballot_sync(kFull, stepping && todo)) != 0) {
+      // idle lanes first take a continuation each that another lane of the warp has waiting
+      const unsigned below = (1u << lane) - 1u;
+      const uint32_t n = (uint32_t)min(__popc(idle), __popc(give));
+      const bool giver = ((give >> lane) & 1u) && (uint32_t)__popc(give & below) < n;
+      const bool taker = ((idle >> lane) & 1u) && (uint32_t)__popc(idle & below) < n;
+      uint8_t* from = s_from + (tid & ~31);
+      if (giver) from[__popc(give & below)] = (uint8_t)lane;
+      __syncwarp();
+      const int src = taker ? from[__popc(idle & below)] : (int)lane;
+      const uint32_t item = todo & (0u - todo), b0 = item == 1 ? (uint32_t)(q0 >> 2) & 3u : (uint32_t)(__ffs(item) - 2) & 3u;
+      const uint32_t g_item = __shfl_sync(kFull, item, src), g_b = __shfl_sync(kFull, b0, src);
+      const uint32_t g_rs = __shfl_sync(kFull, rs, src);
+      const uint32_t g_at = __shfl_sync(kFull, (uint32_t)te | (uint32_t)len << 15 | (fwd ? 1u << 31 : 0u), src);
+      const uint64_t g_q = __shfl_sync(kFull, q0, src);
+      if (giver) todo ^= item;
+      if (taker) {
+        todo = g_item;
+        rs = g_rs;
+        te = (int)(g_at & 0x7FFFu);
+        len = (int)((g_at >> 15) & 0x7FFFu);
+        fwd = g_at >> 31;
+        q0 = g_q;
+        s_k[g_b][tid] = s_k[g_b][(tid & ~31) + src];
+        s_l[g_b][tid] = s_l[g_b][(tid & ~31) + src];
+        const uint32_t d = (fwd ? 1u : 0u) ^ (rs & 1u);
+        occ = d ? X.dir[1].occ : X.dir[0].occ;
+        dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
+      }
+      __syncwarp();
+    } else if (!exhausted && (idle == kFull || (uint32_t)__popc(idle) >= bi)) {
       const uint32_t want = (uint32_t)__popc(idle), rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
       uint32_t c0 = 0;
       if (lane == 0) c0 = atomicAdd(p.spill_head, want);
