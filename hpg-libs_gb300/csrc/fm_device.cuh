@@ -135,6 +135,32 @@ __device__ __forceinline__ void load_block_m(const OccBlock* p, uint32_t mode, u
   }
 }
 
+#define HPG_LOAD_PAIR(ld)                                                                                    \
+  asm("{\n .reg .pred two;\n setp.ne.u32 two, %18, 0;\n " ld " {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n @two " ld \
+      " {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n}"                                                          \
+      : "=&r"(cnt0[0]), "=&r"(cnt0[1]), "=&r"(cnt0[2]), "=&r"(cnt0[3]), "=&r"(bits0.x), "=&r"(bits0.y),      \
+        "=&r"(bits0.z), "=&r"(bits0.w), "=&r"(cnt1[0]), "=&r"(cnt1[1]), "=&r"(cnt1[2]), "=&r"(cnt1[3]),      \
+        "=&r"(bits1.x), "=&r"(bits1.y), "=&r"(bits1.z), "=&r"(bits1.w)                                       \
+      : "l"(occ + q0), "l"(occ + q1), "r"(q1 ^ q0))
+
+// Blocks q0 and q1 of a direction, both loads under way together; where q1 == q0 only the
+// first is loaded and cnt1, bits1 are left undefined.
+__device__ __forceinline__ void load_block_pair(const OccBlock* occ, uint32_t q0, uint32_t q1, uint32_t mode,
+                                                uint32_t (&cnt0)[4], uint4& bits0, uint32_t (&cnt1)[4],
+                                                uint4& bits1) {
+  if (mode == 0) {
+    load_block_m(occ + q0, 0, cnt0, bits0);
+    load_block_m(occ + q1, 0, cnt1, bits1);
+  } else if (mode == 1) {
+    HPG_LOAD_PAIR("ld.global.nc.v8.b32");
+  } else if (mode == 2) {
+    HPG_LOAD_PAIR("ld.global.nc.L1::no_allocate.L2::evict_last.v8.b32");
+  } else {
+    HPG_LOAD_PAIR("ld.global.nc.L2::evict_last.v8.b32");
+  }
+}
+#undef HPG_LOAD_PAIR
+
 __device__ __forceinline__ void load_block(const OccBlock* p, uint32_t (&cnt)[4], uint4& bits) {
   load_block_m(p, 0, cnt, bits);
 }
@@ -200,6 +226,31 @@ __device__ __forceinline__ uint64_t row_mask(uint32_t r) {
   uint64_t m;
   asm("shl.b64 %0, %1, %2;" : "=l"(m) : "l"(1ull), "r"(r));
   return m - 1ull;
+}
+
+// One rank step on physical symbol p: [k, l] to C[p] + its occurrences before k, and up to l.
+// An interval over two blocks has both on their way at once (2M x 150 bp, 600 Mbp: 3960 ->
+// 3580 us a call, 1000 reads at 100 Mbp 274 -> 250, against loads one after the other, the
+// second behind the first's use, as bw_step has them: it takes fewer registers, which the
+// kernels that step narrower intervals gain more by, plain search 1198 against 1287 us).
+__device__ __forceinline__ void rank_step(const DevIndex& X, const OccBlock* occ, uint32_t dollar, uint32_t p,
+                                          uint32_t& k, uint32_t& l) {
+  const uint32_t q0 = k >> 6, q1 = l >> 6;
+  uint32_t cnt[4], cnt1[4];
+  uint4 bits, bits1;
+  load_block_pair(occ, q0, q1, X.load_mode, cnt, bits, cnt1, bits1);
+  const bool two = q1 != q0;
+  const uint64_t m0 = match_mask(bits, p), m1 = two ? match_mask(bits1, p) : m0;
+  const uint32_t c0 = sel4(cnt, p), c1 = two ? sel4(cnt1, p) : c0;
+  uint32_t rk = c0 + (uint32_t)__popcll(m0 & row_mask(k & 63));
+  uint32_t rl = c1 + (uint32_t)__popcll(m1 & row_mask((l & 63) + 1));
+  if (p == 0) {  // the '$' row is stored as code 0 in its block
+    if (k > dollar && q0 == (dollar >> 6)) rk -= 1;
+    if (l >= dollar && q1 == (dollar >> 6)) rl -= 1;
+  }
+  const uint32_t c = sel4(X.C, p);  // C1 = C + 1 (checked when the index is loaded)
+  k = c + 1u + rk;
+  l = c + rl;
 }
 
 // BWiteration (search/runtime.h:38-42) over a view, on 32-bit interval ends.

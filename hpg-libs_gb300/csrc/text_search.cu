@@ -72,38 +72,15 @@ constexpr int kHeadSteps = 6;
 // queue two to three.  Within the branching window every step may queue a change point, and
 // all 32 are taken.
 constexpr uint32_t kRows = 32, kRowsBefore = 4;
+// Claims of a warp of the wide and the branch kernel, at least about, where the queues are
+// short (2M x 150 bp, 600 Mbp, a call: 3966 us at 1, 3938 at 4, 3888 at 16, 4585 at 64, where
+// a claim fills half a warp).
+constexpr uint32_t kClaims = 16;
 // A chain's entry of `diag` that is no alignment: its first symbols (kHeadSteps past the
 // table at most) do not occur, or it was left to the row queue or the rest list.
 constexpr uint32_t kAbsent = 0xFFFFFFFFu, kMany = 0xFFFFFFFEu;
 __device__ __forceinline__ bool is_diag(uint32_t x) { return x < kMany; }
 constexpr unsigned kFull = 0xFFFFFFFFu;
-
-// One rank step on a physical symbol.
-__device__ __forceinline__ void rank_step(const DevIndex& X, const OccBlock* occ, uint32_t dollar, uint32_t ph,
-                                          uint32_t& k, uint32_t& l) {
-  const uint32_t q0 = k >> 6, q1 = l >> 6;
-  uint32_t cnt[4];
-  uint4 bits;
-  load_block_m(occ + q0, X.load_mode, cnt, bits);
-  uint64_t mm = match_mask(bits, ph);
-  const uint32_t c0 = sel4(cnt, ph);
-  uint32_t rk = c0 + (uint32_t)__popcll(mm & row_mask(k & 63));
-  uint32_t rl;
-  if (q1 == q0) {
-    rl = c0 + (uint32_t)__popcll(mm & row_mask((l & 63) + 1));
-  } else {
-    load_block_m(occ + q1, X.load_mode, cnt, bits);
-    mm = match_mask(bits, ph);
-    rl = sel4(cnt, ph) + (uint32_t)__popcll(mm & row_mask((l & 63) + 1));
-  }
-  if (ph == 0) {  // the '$' row is stored as code 0 in its block
-    if (k > dollar && q0 == (dollar >> 6)) rk -= 1;
-    if (l >= dollar && q1 == (dollar >> 6)) rl -= 1;
-  }
-  const uint32_t cc = sel4(X.C, ph);  // C1 = C + 1 (checked when the index is loaded)
-  k = cc + 1u + rk;
-  l = cc + rl;
-}
 
 // First t at which the helper branches: J <= n/2 backward, J >= n/2 - 1 forward (n = len - 1).
 __device__ __forceinline__ int branch_from(int len, bool fwd) {
@@ -140,7 +117,7 @@ __device__ __forceinline__ uint32_t branch_meta(bool fwd, int len, int t, uint32
 // 2, 3: those on the forward index ('+' forward, '-' backward), so that the
 // blocks in flight read one direction's table and blocks at a time.
 template <bool CENSUS>
-__global__ void __launch_bounds__(kHeadTpb) text_head_kernel(DevIndex X, BatchedParams p) {
+__global__ void __launch_bounds__(kHeadTpb, 7) text_head_kernel(DevIndex X, BatchedParams p) {
   __shared__ uint32_t s_cnt[2][kHeadTpb / 32], s_base[2];
   const uint32_t n_reads = p.n_reads_dev ? *p.n_reads_dev : p.n_reads;
   if ((uint64_t)blockIdx.x * kHeadTpb >= n_reads) return;
@@ -636,16 +613,38 @@ __device__ __forceinline__ unsigned chunk_slot(unsigned int* ctr, uint32_t cap, 
 
 // Persistent: the chains still more than kRows rows wide, a lane each, one rank
 // step per iteration until they are not (-> row queue); the change points they
-// pass inside the helper's window go to the spill queue.  Idle lanes wait,
-// masked, until `batch_idle` of the warp are idle and claim chains together.
+// pass inside the helper's window go to the spill queue.  A warp prepares 32
+// chains at a time, every lane one (five or six dependent loads), and its lanes
+// take them from shared memory as they run out; what they queue is gathered and written 32
+// at a time.  A lane that fetched its own next chain, and an atomic per entry queued: 1189 us
+// for the wide chains of 2M x 150 bp at 600 Mbp; so: 951, and 773 once an interval's two
+// blocks were loaded together (rank_step).  Latency of the steps, some 130 at most in a row.
+struct WideShared {
+  uint4 chain[32];  // k, l, rs, t | len << 15 | forward << 31
+  uint64_t q[32];
+  int ts[32];
+  uint4 rows[64];         // for the row queue
+  SpillEntry change[64];  // for the spill queue
+};
+
+// Entries a warp takes from a queue at a time: 32, fewer where that would leave warps without.
+__device__ __forceinline__ uint32_t per_claim(uint32_t n, uint32_t warps) {
+  return min(max(n / (kClaims * warps), 1u), 32u);
+}
+
 template <bool CENSUS>
 __global__ void __launch_bounds__(kWideTpb) text_wide_kernel(DevIndex X, BatchedParams p) {
-  __shared__ uint32_t c_res[kWideTpb], c_spl[kWideTpb];
+  __shared__ WideShared wsh[kWideTpb / 32];
+  __shared__ uint32_t c_res[kWideTpb];
   const int tid = threadIdx.x;
   const uint32_t lane = tid & 31;
+  WideShared& ws = wsh[tid >> 5];
   const uint32_t n_src = *(volatile unsigned int*)p.rest_n;
-  c_res[tid] = c_spl[tid] = 0;
+  const uint32_t batch = per_claim(n_src, gridDim.x * (kWideTpb / 32));
+  c_res[tid] = 0;
   bool active = false, exhausted = false;
+  uint32_t ready = 0;  // chains prepared and not taken
+  uint32_t n_rows = 0, n_change = 0;  // entries held for the queues
   uint32_t k = 0, l = 0, rs = 0;
   int t = 0, len = 0, ts = 0;
   bool fwd = false;
@@ -654,86 +653,126 @@ __global__ void __launch_bounds__(kWideTpb) text_wide_kernel(DevIndex X, Batched
   const OccBlock* occ = nullptr;
   uint32_t dollar = 0, sectors = 0;
   const uint32_t bi = p.batch_idle < 1 ? 1u : p.batch_idle;
+  auto flush_rows = [&](uint32_t from, uint32_t n) {
+    __syncwarp();
+    uint32_t c0 = 0;
+    if (lane == 0) c0 = atomicAdd(p.rows_n, n);
+    c0 = __shfl_sync(kFull, c0, 0);
+    if (lane < n) p.rows[c0 + lane] = ws.rows[from + lane];  // (one entry per chain: no bound to check)
+    __syncwarp();
+  };
+  auto flush_change = [&](uint32_t from, uint32_t n) {
+    __syncwarp();
+    uint32_t c0 = 0;
+    if (lane == 0) c0 = atomicAdd(p.spill_tail, n);
+    c0 = __shfl_sync(kFull, c0, 0);
+    if (lane < n) {
+      if (c0 + lane < p.spill_cap) p.spill[c0 + lane] = ws.change[from + lane];
+      else atomicOr(p.status, kStatusSpillFull);
+    }
+    __syncwarp();
+  };
   for (;;) {
     const unsigned idle = __ballot_sync(kFull, !active);  // every lane, every iteration
-    if (!exhausted && (idle == kFull || (uint32_t)__popc(idle) >= bi)) {
-      const uint32_t want = (uint32_t)__popc(idle), rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+    if (!ready && !exhausted && (uint32_t)__popc(idle) >= bi) {
       uint32_t c0 = 0;
-      if (lane == 0) c0 = atomicAdd(p.rest_head, want);
+      if (lane == 0) c0 = atomicAdd(p.rest_head, batch);
       c0 = __shfl_sync(kFull, c0, 0);
-      if (c0 + want >= n_src) exhausted = true;
-      if (!active && c0 + rank < n_src) {
-        const uint4 e = p.rest[c0 + rank];
+      if (c0 + batch >= n_src) exhausted = true;
+      ready = c0 < n_src ? min(batch, n_src - c0) : 0u;
+      if (lane < ready) {
+        const uint4 e = p.rest[c0 + lane];
+        const uint64_t b0 = p.offs[e.z >> 1];
+        const int c_len = (int)(p.offs[(e.z >> 1) + 1] - b0), c_t = (int)(e.w & 0xFFFFu);
+        const bool c_fwd = (e.w >> 16) & 1u;
+        const uint32_t strand = e.z & 1u, d = (c_fwd ? 1u : 0u) ^ strand;
+        int c_ts = branch_from(c_len, c_fwd);
+        // change points without hits are not queued: their remaining symbols hold a head that
+        // does not occur, or that occurs once and not where the read's two parts would meet
+        const uint32_t other = other_chain(X, p, e.z, d, c_len, c_ts + 1);
+        if (other != kMany) {
+          const int near = c_len - (int)X.tmer_len - kHeadSteps;
+          c_ts = other == kAbsent ? near : hits_from(X, p.packed, b0, c_len, c_fwd, strand, d, other, c_ts, near);
+        }
+        ws.chain[lane] = make_uint4(e.x, e.y, e.z, (uint32_t)c_t | (uint32_t)c_len << 15 | (c_fwd ? 1u << 31 : 0u));
+        ws.q[lane] = query32(X, p.packed, b0, c_len, c_fwd, strand, c_t);
+        ws.ts[lane] = c_ts;
+      }
+      __syncwarp();
+    }
+    if (ready) {
+      const uint32_t rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+      if (!active && rank < ready) {
+        const uint32_t i = ready - 1 - rank;
+        const uint4 e = ws.chain[i];
         k = e.x;
         l = e.y;
         rs = e.z;
-        t = (int)(e.w & 0xFFFFu);
-        fwd = (e.w >> 16) & 1u;
-        const uint64_t b0 = p.offs[rs >> 1];
-        len = (int)(p.offs[(rs >> 1) + 1] - b0);
-        const uint32_t strand = rs & 1u, d = (fwd ? 1u : 0u) ^ strand;
-        ts = branch_from(len, fwd);
-        // change points without hits are not queued: their remaining symbols hold a head that
-        // does not occur, or that occurs once and not where the read's two parts would meet
-        const uint32_t other = other_chain(X, p, rs, d, len, ts + 1);
-        if (other != kMany) {
-          const int near = len - (int)X.tmer_len - kHeadSteps;
-          ts = other == kAbsent ? near : hits_from(X, p.packed, b0, len, fwd, strand, d, other, ts, near);
-        }
+        t = (int)(e.w & 0x7FFFu);
+        len = (int)((e.w >> 15) & 0x7FFFu);
+        fwd = e.w >> 31;
+        q = ws.q[i];
+        ts = ws.ts[i];
+        const uint32_t d = (fwd ? 1u : 0u) ^ (rs & 1u);
         occ = d ? X.dir[1].occ : X.dir[0].occ;
         dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
-        q = query32(X, p.packed, b0, len, fwd, strand, t);
         ql = 32;
         active = true;
       }
-      if (__ballot_sync(kFull, active) == 0) break;
+      ready -= min(ready, (uint32_t)__popc(idle));
+      __syncwarp();
     } else if (exhausted && idle == kFull) {
       break;
     }
-    if (!active) continue;
+    bool row = false, change = false;
     const uint32_t pk = k, pl = l;
-    if (CENSUS) sectors += (k >> 6) == (l >> 6) ? 1u : 2u;
-    rank_step(X, occ, dollar, (uint32_t)q & 3u, k, l);
-    if (t >= ts && l - k != pl - pk) {  // a change point
-      if (t == len - 1) {
-        push_block(p, pk, pl, rs, len, fwd);
-      } else {
-        uint32_t cs = c_spl[tid];
-        const unsigned slot = chunk_slot(p.spill_tail, p.spill_cap, cs);
-        c_spl[tid] = cs;
-        if (slot < p.spill_cap) p.spill[slot] = SpillEntry{pk, pl, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u)};
-        else atomicOr(p.status, kStatusSpillFull);
+    const int pt = t;
+    if (active) {
+      if (CENSUS) sectors += (k >> 6) == (l >> 6) ? 1u : 2u;
+      rank_step(X, occ, dollar, (uint32_t)q & 3u, k, l);
+      if (t >= ts && l - k != pl - pk) {  // a change point
+        change = t != len - 1;
+        if (!change) push_block(p, pk, pl, rs, len, fwd);
+      }
+      active = k <= l && t + 1 < len;
+      if (active) {
+        ++t;
+        q >>= 2;
+        row = l - k < (t < ts ? kRowsBefore : kRows);  // few enough rows for a lane each
+        active = !row;
+        if (--ql == 0) {  // 32 symbols on
+          q = query32(X, p.packed, p.offs[rs >> 1], len, fwd, rs & 1u, t);
+          ql = 32;
+        }
+      } else if (k <= l && !fwd) {  // the whole read: the exact hit
+        uint32_t r = c_res[tid];
+        const unsigned slot = res_slot(p, r);
+        c_res[tid] = r;
+        write_hit(p, slot, rs, order_key(0, 0, 0), k, l, pack_meta(0, 0, 0, 0, 0));
       }
     }
-    if (k <= l && t + 1 < len) {
-      ++t;
-      if (l - k < (t < ts ? kRowsBefore : kRows)) {  // few enough rows for a lane each
-        p.rows[claim(p.rows_n, 1)] = make_uint4(k, l, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u));
-        active = false;
-        continue;
-      }
-      q >>= 2;
-      if (--ql == 0) {  // 32 symbols on
-        q = query32(X, p.packed, p.offs[rs >> 1], len, fwd, rs & 1u, t);
-        ql = 32;
-      }
-      continue;
+    // entries for the two queues are written 32 at a time
+    const unsigned mr = __ballot_sync(kFull, row), mc = __ballot_sync(kFull, change);
+    const unsigned below = (1u << lane) - 1u;
+    if (row) ws.rows[n_rows + __popc(mr & below)] = make_uint4(k, l, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u));
+    if (change) ws.change[n_change + __popc(mc & below)] = SpillEntry{pk, pl, rs, (uint32_t)pt | (fwd ? 1u << 16 : 0u)};
+    n_rows += (uint32_t)__popc(mr);
+    n_change += (uint32_t)__popc(mc);
+    if (n_rows >= 32) {
+      n_rows -= 32;
+      flush_rows(n_rows, 32);
     }
-    if (k <= l && !fwd) {  // the whole read: the exact hit
-      uint32_t r = c_res[tid];
-      const unsigned slot = res_slot(p, r);
-      c_res[tid] = r;
-      write_hit(p, slot, rs, order_key(0, 0, 0), k, l, pack_meta(0, 0, 0, 0, 0));
+    if (n_change >= 32) {
+      n_change -= 32;
+      flush_change(n_change, 32);
     }
-    active = false;
   }
-  {  // slots of this lane's last chunks that were reserved but not used
+  if (n_rows) flush_rows(0, n_rows);
+  if (n_change) flush_change(0, n_change);
+  {  // slots of this lane's last chunk that were reserved but not used
     const uint32_t r = c_res[tid];
     for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
       if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-    const uint32_t cs = c_spl[tid];
-    for (unsigned i = 0, left = cs >> 28, s = cs & 0x0FFFFFFFu; i < left; ++i)
-      if (s + i < p.spill_cap) p.spill[s + i].rs = 0xFFFFFFFFu;
   }
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
@@ -742,54 +781,55 @@ __global__ void __launch_bounds__(kWideTpb) text_wide_kernel(DevIndex X, Batched
 __device__ __forceinline__ void rank_step4(const DevIndex& X, const OccBlock* occ, uint32_t dollar, uint32_t k,
                                            uint32_t l, uint32_t (&nk)[4], uint32_t (&nl)[4]) {
   const uint32_t q0 = k >> 6, q1 = l >> 6;
-  uint32_t cnt[4];
-  uint4 bits;
-  load_block_m(occ + q0, X.load_mode, cnt, bits);
+  uint32_t cnt[4], cnt1[4];
+  uint4 bits, bits1;
+  load_block_pair(occ, q0, q1, X.load_mode, cnt, bits, cnt1, bits1);
+  const bool two = q1 != q0;
   const uint64_t mk = row_mask(k & 63), ml = row_mask((l & 63) + 1);
 #pragma unroll
   for (uint32_t b = 0; b < 4; ++b) {
-    const uint64_t mm = match_mask(bits, b);
-    nk[b] = X.C[b] + 1u + cnt[b] + (uint32_t)__popcll(mm & mk);
-    nl[b] = X.C[b] + cnt[b] + (uint32_t)__popcll(mm & ml);
-  }
-  if (q1 != q0) {
-    load_block_m(occ + q1, X.load_mode, cnt, bits);
-#pragma unroll
-    for (uint32_t b = 0; b < 4; ++b)
-      nl[b] = X.C[b] + cnt[b] + (uint32_t)__popcll(match_mask(bits, b) & ml);
+    const uint64_t m0 = match_mask(bits, b), m1 = two ? match_mask(bits1, b) : m0;
+    nk[b] = X.C[b] + 1u + cnt[b] + (uint32_t)__popcll(m0 & mk);
+    nl[b] = X.C[b] + (two ? cnt1[b] : cnt[b]) + (uint32_t)__popcll(m1 & ml);
   }
   // the '$' row is stored as code 0 in its block
   if (k > dollar && q0 == (dollar >> 6)) nk[0] -= 1;
   if (l >= dollar && q1 == (dollar >> 6)) nl[0] -= 1;
 }
 
-// Persistent: a lane per spilled change point.  Its eight continuations begin
-// with one step from the same interval (the deletion with the symbol after the
-// failing one, the insertions and mismatches with b), so one or two blocks give
-// all their first intervals; the lane then runs those that are not empty one
-// after the other, one rank step per iteration, without touching memory between
-// them.  What has narrowed to one row and matched on goes to the walk queue.
+// Persistent: the spilled change points, 32 a warp at a time.  The eight continuations of
+// one begin with one step from the same interval (the deletion with the symbol after the
+// failing one, the insertions and mismatches with b), so one or two blocks give all their
+// first intervals; those that are not empty wait in the lane that holds the change point
+// until a lane of the warp is free to run one, a rank step per iteration, without touching
+// memory between them.  (One lane for all of a change point's: 1246 us on 2M x 150 bp, 600
+// Mbp; the few long ones held their warps.  So: 884, 780 with an interval's two blocks
+// loaded together.)  What has narrowed to one row and matched on goes to the walk queue.
 //
 // Most wide change points lie in tandem runs whose read goes on into sequence that
 // occurs once, or with an error in its head nowhere: there the strand's other chain
-// decides them without a rank step (2M x 150 bp, 600 Mbp with 45 % repeats: 4095 ->
-// 1367 us; about 100 sectors a change point before, its intervals being thousands of
-// rows wide).
+// decides them without a rank step (about 100 sectors a change point otherwise, its
+// intervals being thousands of rows wide), here or, for a chain's leading ones, before
+// they are queued (hits_from).
 template <bool CENSUS>
-__global__ void __launch_bounds__(kWideTpb) text_branch_kernel(DevIndex X, BatchedParams p) {
+__global__ void __launch_bounds__(kWideTpb, 7) text_branch_kernel(DevIndex X, BatchedParams p) {
   __shared__ uint32_t c_res[kWideTpb], c_walk[kWideTpb], s_k[4][kWideTpb], s_l[4][kWideTpb];
   __shared__ uint8_t s_from[kWideTpb];
   const int tid = threadIdx.x;
   const uint32_t lane = tid & 31;
   const uint32_t n_src = min(*(volatile unsigned int*)p.spill_tail, p.spill_cap);
+  const uint32_t batch = per_claim(n_src, gridDim.x * (kWideTpb / 32));
   c_res[tid] = c_walk[tid] = 0;
-  bool exhausted = false, walk_full = false;
-  uint32_t todo = 0;    // continuations left: bit 0 deletion, 1 + b insertion, 5 + b mismatch
-  bool stepping = false;
+  bool exhausted = false, walk_full = false, stepping = false;
+  // the change point this lane holds for the warp
+  uint32_t todo = 0;  // continuations left: bit 0 deletion, 1 + b insertion, 5 + b mismatch
+  uint32_t h_rs = 0, h_at = 0;  // h_at: te | len << 15 | forward << 31
+  uint64_t h_q = 0;   // symbols from te on
+  // the continuation it runs
   uint32_t k = 0, l = 0, rs = 0, key = 0;
   int t = 0, te = 0, len = 0;
   bool fwd = false;
-  uint64_t q0 = 0, q = 0;  // symbols from te on; the next symbols
+  uint64_t q = 0;  // the next symbols
   int ql = 0;
   const OccBlock* occ = nullptr;
   uint32_t dollar = 0, sectors = 0;
@@ -803,63 +843,32 @@ __global__ void __launch_bounds__(kWideTpb) text_branch_kernel(DevIndex X, Batch
               branch_meta(fwd, len, te, s == 0 ? 1u : ((s & 1u) ? 3u : 2u), s == 0 ? 0xFFu : (s - 1) >> 1));
   };
   for (;;) {
-    const unsigned idle = __ballot_sync(kFull, !stepping && !todo);  // every lane, every iteration
-    unsigned give = 0;
-    if (idle != kFull && (uint32_t)__popc(idle) >= bi && (give = __ballot_sync(kFull, stepping && todo)) != 0) {
-      // idle lanes first take a continuation each that another lane of the warp has waiting
-      const unsigned below = (1u << lane) - 1u;
-      const uint32_t n = (uint32_t)min(__popc(idle), __popc(give));
-      const bool giver = ((give >> lane) & 1u) && (uint32_t)__popc(give & below) < n;
-      const bool taker = ((idle >> lane) & 1u) && (uint32_t)__popc(idle & below) < n;
-      uint8_t* from = s_from + (tid & ~31);
-      if (giver) from[__popc(give & below)] = (uint8_t)lane;
-      __syncwarp();
-      const int src = taker ? from[__popc(idle & below)] : (int)lane;
-      const uint32_t item = todo & (0u - todo), b0 = item == 1 ? (uint32_t)(q0 >> 2) & 3u : (uint32_t)(__ffs(item) - 2) & 3u;
-      const uint32_t g_item = __shfl_sync(kFull, item, src), g_b = __shfl_sync(kFull, b0, src);
-      const uint32_t g_rs = __shfl_sync(kFull, rs, src);
-      const uint32_t g_at = __shfl_sync(kFull, (uint32_t)te | (uint32_t)len << 15 | (fwd ? 1u << 31 : 0u), src);
-      const uint64_t g_q = __shfl_sync(kFull, q0, src);
-      if (giver) todo ^= item;
-      if (taker) {
-        todo = g_item;
-        rs = g_rs;
-        te = (int)(g_at & 0x7FFFu);
-        len = (int)((g_at >> 15) & 0x7FFFu);
-        fwd = g_at >> 31;
-        q0 = g_q;
-        s_k[g_b][tid] = s_k[g_b][(tid & ~31) + src];
-        s_l[g_b][tid] = s_l[g_b][(tid & ~31) + src];
-        const uint32_t d = (fwd ? 1u : 0u) ^ (rs & 1u);
-        occ = d ? X.dir[1].occ : X.dir[0].occ;
-        dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
-      }
-      __syncwarp();
-    } else if (!exhausted && (idle == kFull || (uint32_t)__popc(idle) >= bi)) {
-      const uint32_t want = (uint32_t)__popc(idle), rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+    const unsigned idle = __ballot_sync(kFull, !stepping);  // every lane, every iteration
+    unsigned give = idle ? __ballot_sync(kFull, todo != 0) : 0u;
+    if (!give && !exhausted && (uint32_t)__popc(idle) >= bi) {  // the next change points
       uint32_t c0 = 0;
-      if (lane == 0) c0 = atomicAdd(p.spill_head, want);
+      if (lane == 0) c0 = atomicAdd(p.spill_head, batch);
       c0 = __shfl_sync(kFull, c0, 0);
-      if (c0 + want >= n_src) exhausted = true;
-      SpillEntry e{0, 0, 0xFFFFFFFFu, 0};
-      if (!stepping && !todo && c0 + rank < n_src) e = p.spill[c0 + rank];
-      if (e.rs != 0xFFFFFFFFu) {  // (a reserved slot nothing was written to)
-        rs = e.rs;
-        te = (int)(e.jtype & 0xFFFFu);
-        fwd = (e.jtype >> 16) & 1u;
+      if (c0 + batch >= n_src) exhausted = true;
+      if (lane < batch && c0 + lane < n_src) {
+        const SpillEntry e = p.spill[c0 + lane];
+        const uint32_t rs = e.rs;
+        const int te = (int)(e.jtype & 0xFFFFu);
+        const bool fwd = (e.jtype >> 16) & 1u;
         const uint64_t b0 = p.offs[rs >> 1];
-        len = (int)(p.offs[(rs >> 1) + 1] - b0);
+        const int len = (int)(p.offs[(rs >> 1) + 1] - b0);
         const uint32_t strand = rs & 1u, d = (fwd ? 1u : 0u) ^ strand;
-        occ = d ? X.dir[1].occ : X.dir[0].occ;
-        dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
-        q0 = query32(X, p.packed, b0, len, fwd, strand, te);
+        const uint64_t q0 = query32(X, p.packed, b0, len, fwd, strand, te);
         // The symbols after the failing one, read from the other end, begin the strand's
         // other chain.  Where they reach past its head, its one row is the only place a
         // continuation can match, and there is none if the head found it absent.
         const uint32_t other = other_chain(X, p, rs, d, len, te + 1);
         if (other == kMany) {
+          h_rs = rs;
+          h_at = (uint32_t)te | (uint32_t)len << 15 | (fwd ? 1u << 31 : 0u);
+          h_q = q0;
           uint32_t nk[4], nl[4];
-          rank_step4(X, occ, dollar, e.k, e.l, nk, nl);
+          rank_step4(X, d ? X.dir[1].occ : X.dir[0].occ, d ? X.dir[1].dollar : X.dir[0].dollar, e.k, e.l, nk, nl);
           if (CENSUS) sectors += (e.k >> 6) == (e.l >> 6) ? 1u : 2u;
           const uint32_t w = (uint32_t)q0 & 3u, w1 = (uint32_t)(q0 >> 2) & 3u;
 #pragma unroll
@@ -903,33 +912,48 @@ __global__ void __launch_bounds__(kWideTpb) text_branch_kernel(DevIndex X, Batch
           }
         }
       }
-      if (__ballot_sync(kFull, stepping || todo) == 0) {
-        if (exhausted) break;
-        continue;  // holes only
+      __syncwarp();
+      give = __ballot_sync(kFull, todo != 0);
+    }
+    if (give) {  // the i-th idle lane takes a continuation of the i-th lane that holds some
+      const unsigned below = (1u << lane) - 1u;
+      const uint32_t n = (uint32_t)min(__popc(idle), __popc(give));
+      const uint32_t nth = (uint32_t)__popc(give & below);
+      const bool giver = ((give >> lane) & 1u) && nth < n;
+      const bool taker = !stepping && (uint32_t)__popc(idle & below) < n;
+      if (giver) s_from[(tid & ~31) + nth] = (uint8_t)lane;
+      __syncwarp();
+      const int src = taker ? s_from[(tid & ~31) + __popc(idle & below)] : (int)lane;
+      const uint32_t item = (uint32_t)__shfl_sync(kFull, __ffs(todo) - 1, src);
+      const uint32_t g_rs = __shfl_sync(kFull, h_rs, src), g_at = __shfl_sync(kFull, h_at, src);
+      const uint64_t q0 = __shfl_sync(kFull, h_q, src);
+      if (giver) todo &= todo - 1;
+      if (taker) {
+        rs = g_rs;
+        te = (int)(g_at & 0x7FFFu);
+        len = (int)((g_at >> 15) & 0x7FFFu);
+        fwd = g_at >> 31;
+        // the symbol stepped with, as a physical code; the next symbol; the order key's slot
+        const uint32_t b = item == 0 ? (uint32_t)(q0 >> 2) & 3u : (item - 1) & 3u;
+        const int skip = item == 0 ? 2 : (item <= 4 ? 0 : 1);
+        const uint32_t qb = b ^ ((rs & 1u) ? X.comp_xor : 0u);
+        key = order_key(fwd ? 4u : 2u, (uint32_t)(len - te), item == 0 ? 0u : (item <= 4 ? 1 + 2 * qb : 2 + 2 * qb));
+        k = s_k[b][(tid & ~31) + src];
+        l = s_l[b][(tid & ~31) + src];
+        t = te + skip;
+        q = q0 >> (2 * skip);
+        ql = 32 - skip;
+        const uint32_t d = (fwd ? 1u : 0u) ^ (rs & 1u);
+        occ = d ? X.dir[1].occ : X.dir[0].occ;
+        dollar = d ? X.dir[1].dollar : X.dir[0].dollar;
+        if (t == len) hit();  // the deletion of the last symbol but one
+        else stepping = true;
       }
+      __syncwarp();
     } else if (exhausted && idle == kFull) {
       break;
     }
-    if (!stepping) {
-      if (!todo) continue;
-      const uint32_t item = (uint32_t)__ffs(todo) - 1u;
-      todo &= todo - 1;
-      // the symbol stepped with, as a physical code; the next symbol; the order key's slot
-      const uint32_t b = item == 0 ? (uint32_t)(q0 >> 2) & 3u : (item - 1) & 3u;
-      const int skip = item == 0 ? 2 : (item <= 4 ? 0 : 1);
-      const uint32_t qb = b ^ ((rs & 1u) ? X.comp_xor : 0u);
-      key = order_key(fwd ? 4u : 2u, (uint32_t)(len - te), item == 0 ? 0u : (item <= 4 ? 1 + 2 * qb : 2 + 2 * qb));
-      k = s_k[b][tid];
-      l = s_l[b][tid];
-      t = te + skip;
-      if (t == len) {  // the deletion of the last symbol but one
-        hit();
-        continue;
-      }
-      q = q0 >> (2 * skip);
-      ql = 32 - skip;
-      stepping = true;
-    }
+    if (!stepping) continue;
     const bool was_one = k == l;
     if (CENSUS) sectors += (k >> 6) == (l >> 6) ? 1u : 2u;
     rank_step(X, occ, dollar, (uint32_t)q & 3u, k, l);
