@@ -1147,7 +1147,9 @@ __global__ void __launch_bounds__(kBlockTpb) block_tail_kernel(
       y = b;
     }
     const View v = (it & 1u) == 0 ? forward_view((it >> 1) & 1u) : backward_view((it >> 1) & 1u);
-    step<C>(X, v, sym, x, y, o.sectors);
+    if (C) o.sectors += (x >> 6) == (y >> 6) ? 1u : 2u;
+    rank_step(X, v.d ? X.dir[1].occ : X.dir[0].occ, v.d ? X.dir[1].dollar : X.dir[0].dollar,
+              v.comp ? ((X.comp_packed >> (2u * sym)) & 3u) : sym, x, y);
     const int dstep = (it & 1u) == 0 ? 1 : -1;
     if (mode == kFirst) {
       const int64_t before = (int64_t)b - (int64_t)a;
@@ -1365,7 +1367,7 @@ int block_search_device(Engine* e, size_t n, uint32_t max_results, uint64_t* tot
       !ensure(e, e->rs_count, T * 4 + 16) || !ensure(e, e->rs_trunc, T + 16) || !ensure(e, e->hit_off, (T + 1) * 8) ||
       !ensure(e, e->scan_part, scan_parts(T) * 8) || !ensure(e, e->vecs, 2 * T * sizeof(hpg_block_anchor_t) + 16) ||
       !ensure(e, e->ovf, T + 16) || !ensure(e, e->census, 16) || !ensure(e, e->rows, P * 4 + 16) ||
-      !ensure(e, e->b_ctr, 64) || !ensure(e, e->b_spill, T * sizeof(uint4) + 16) ||
+      !ensure(e, e->b_ctr, 64) || !ensure(e, e->b_spill, (e->X.text ? P : T) * sizeof(uint4) + 16) ||
       (e->X.text && !ensure(e, e->b_one, 2 * T * sizeof(uint4) + 16))) {
     *err = oom_message("block search", P * (kBlockSlots * sizeof(hpg_hit_t) + 2 * sizeof(hpg_block_anchor_t) + 16));
     return -1;
@@ -1422,11 +1424,17 @@ int block_search_device(Engine* e, size_t n, uint32_t max_results, uint64_t* tot
   uint32_t* n_one = ptr<uint32_t>(e->b_ctr) + 9;  // then the blocks of few rows, and those claimed
   uint32_t* n_few = n_one + 1;
   uint32_t* few_head = n_one + 2;
+  const bool text_tail = packed && !census;
   for (uint32_t phys = 0; phys < 2; ++phys) {  // per index direction: head, the heads' rest, tail
-    cudaMemsetAsync(n_queue, 0, 4, s);
+    // With the text only the few wide blocks come to the tail, which takes as long as the
+    // longest one's chain of steps: it runs once, for both directions (1M x 36-150 bp, 100
+    // Mbp: 435 us, 467 + 450 a direction at a time).  Without, it is the walks of all blocks,
+    // and one direction's occurrence blocks stay in L2.
+    const bool tail = !text_tail || phys == 1;
+    if (!text_tail || phys == 0) cudaMemsetAsync(n_queue, 0, 4, s);
     cudaMemsetAsync(n_cont, 0, 4, s);
     cudaMemsetAsync(n_one, 0, 12, s);
-    count_launches(3);
+    count_launches(tail ? 3 : 2);
     if (census) {
       block_head_kernel<true><<<grid_of(T), kBlockTpb, 0, s>>>(e->X, codes, offs, ok, (uint32_t)T, phys, max_results,
                                                                ps, queue, n_queue, cont, n_cont, census);
@@ -1449,8 +1457,9 @@ int block_search_device(Engine* e, size_t n, uint32_t max_results, uint64_t* tot
         block_one_kernel<<<std::min(grid_of(T), (unsigned)(16 * e->num_sms)), kBlockTpb, 0, s>>>(
             e->X, packed, offs, one, n_one, max_results, ps);
       }
-      block_tail_kernel<false><<<tail_grid, kBlockTpb, 0, s>>>(e->X, codes, offs, queue, n_queue, max_results, ps,
-                                                               nullptr);
+      if (tail)
+        block_tail_kernel<false><<<tail_grid, kBlockTpb, 0, s>>>(e->X, codes, offs, queue, n_queue, max_results, ps,
+                                                                 nullptr);
     }
   }
   cudaEventRecord(e->cev[1], s);
