@@ -447,8 +447,8 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
   const uint32_t lane = tid & 31;
   RowsShared& ws = rsh[tid >> 5];
   const uint32_t n_items = *(volatile unsigned int*)p.rows_n;
-  // eight chains a claim, fewer when every warp then still has some
-  const uint32_t per_claim = min(max(n_items / (gridDim.x * kRowsWarps), 1u), 8u);
+  // sixteen chains a claim (most have two to five rows), fewer when every warp then still has some
+  const uint32_t batch = min(max(n_items / (gridDim.x * kRowsWarps), 1u), 16u);
   c_res[tid] = 0;
   if (lane == 0) ws.n = ws.next = 0;
   __syncwarp();
@@ -457,10 +457,10 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
     if (ws.next == ws.n) {  // claim the next chains
       if (exhausted) break;
       uint32_t c0 = 0;
-      if (lane == 0) c0 = atomicAdd(p.rows_head, per_claim);
+      if (lane == 0) c0 = atomicAdd(p.rows_head, batch);
       c0 = __shfl_sync(kFull, c0, 0);
-      if (c0 + per_claim >= n_items) exhausted = true;
-      const uint32_t got = c0 < n_items ? min(per_claim, n_items - c0) : 0u;
+      if (c0 + batch >= n_items) exhausted = true;
+      const uint32_t got = c0 < n_items ? min(batch, n_items - c0) : 0u;
       if (lane < got) ws.item[lane] = p.rows[c0 + lane];
       __syncwarp();
       if (lane == 0) {
@@ -476,23 +476,20 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
     if (lane < held) rows = min(ws.item[first + lane].y - ws.item[first + lane].x + 1u, kRows);
     uint32_t incl = rows;
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
+    for (int o = 1; o < 16; o <<= 1) {
       const uint32_t v = __shfl_up_sync(kFull, incl, o);
       if (lane >= (uint32_t)o) incl += v;
     }
     const unsigned fit = __ballot_sync(kFull, lane < held && incl <= 32);
     const uint32_t take = (uint32_t)__popc(fit);  // (sizes are positive: the fitting ones are the first ones)
-    // this lane's chain and its lanes
-    uint32_t mine = 0xFFFFFFFFu, j = 0;
-    unsigned seg = 0;
-    for (uint32_t i = 0; i < take; ++i) {
-      const uint32_t end = __shfl_sync(kFull, incl, i), len_i = __shfl_sync(kFull, rows, i);
-      if (lane < end && lane >= end - len_i) {
-        mine = i;
-        j = lane - (end - len_i);
-        seg = (end == 32 ? kFull : (1u << end) - 1u) & ~((1u << (end - len_i)) - 1u);
-      }
-    }
+    // this lane's chain and its lanes, start .. end-1
+    const uint32_t total = __shfl_sync(kFull, incl, (int)take - 1);
+    const uint32_t widest = __reduce_max_sync(kFull, lane < take ? rows : 0u);
+    const unsigned starts = __reduce_or_sync(kFull, lane < take ? 1u << (incl - rows) : 0u), upto = (2u << lane) - 1u;
+    const uint32_t mine = lane < total ? (uint32_t)__popc(starts & upto) - 1u : 0xFFFFFFFFu;
+    const uint32_t start = lane < total ? 31u - (uint32_t)__clz(starts & upto) : lane, j = lane - start;
+    const uint32_t end = lane < total ? ((starts & ~upto) ? (uint32_t)__ffs(starts & ~upto) - 1u : total) : lane + 1;
+    const unsigned seg = lane < total ? (kFull >> (32u - end)) & (kFull << start) : 0u;
     uint32_t rs = 0, d = 0, P = 0, strand = 0;
     bool fwd = false;
     int len = 0, t0 = 0, ts = 0, te = -1, D = 0x7FFFFFFF, I = 0x7FFFFFFF, M = 0x7FFFFFFF;
@@ -558,11 +555,12 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
     // the other change points, in order
     bool todo = te >= ts && te <= len - 2;
     while (__ballot_sync(kFull, todo)) {
-      int cp = 0x7FFFFFFF;  // the least te left among the chain's lanes
-      for (uint32_t i = 0; i < take; ++i) {
-        const int v = __reduce_min_sync(kFull, mine == i && todo ? te : 0x7FFFFFFF);
-        if (mine == i) cp = v;
+      int cp = todo ? te : 0x7FFFFFFF;  // the least te left among the chain's lanes
+      for (uint32_t o = 1; o < widest; o <<= 1) {
+        const int v = __shfl_down_sync(kFull, cp, o);
+        if (lane + o < end) cp = min(cp, v);
       }
+      cp = __shfl_sync(kFull, cp, (int)start);
       const bool live = cp != 0x7FFFFFFF;
       const bool in = live && te >= cp;
       uint32_t b = 0;  // the row's text symbol at cp, as a query base
@@ -575,14 +573,14 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
       interval(in && D <= cp, row_d, lead, k, l);
       if (lead) emit(order_key(sec, tf, 0), k, l, branch_meta(fwd, len, cp, 1, 0xFFu), at + 1);
       const bool ins = in && I <= cp, mis = in && te == cp && M <= cp + 1;
-      if (__ballot_sync(kFull, ins || mis)) {
-#pragma unroll
-        for (uint32_t v = 0; v < 4; ++v) {
-          interval(ins && b == v, row_i, lead, k, l);
-          if (lead) emit(order_key(sec, tf, 1 + 2 * v), k, l, branch_meta(fwd, len, cp, 3, v), at - 1);
-          interval(mis && b == v, row_m, lead, k, l);
-          if (lead) emit(order_key(sec, tf, 2 + 2 * v), k, l, branch_meta(fwd, len, cp, 2, v), at);
-        }
+      // insertions and mismatches of the bases that occur
+      for (uint32_t some = __reduce_or_sync(kFull, (ins ? 1u << (2 * b) : 0u) | (mis ? 2u << (2 * b) : 0u)); some;
+           some &= some - 1) {
+        const uint32_t item = (uint32_t)__ffs(some) - 1u, v = item >> 1;
+        const bool is_mis = item & 1u;
+        interval((is_mis ? mis : ins) && b == v, is_mis ? row_m : row_i, lead, k, l);
+        if (lead)
+          emit(order_key(sec, tf, 1 + item), k, l, branch_meta(fwd, len, cp, is_mis ? 2 : 3, v), is_mis ? at : at - 1);
       }
       if (te == cp) todo = false;
     }
