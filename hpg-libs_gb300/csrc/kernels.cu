@@ -220,12 +220,10 @@ __global__ void __launch_bounds__(kTpb)
   if (ok[read] && len >= 3 && (uint32_t)len <= max_len) {
     const uint8_t* W = codes + b;
     const View B = view_B(strand), F = view_F(strand);
-    uint2* vB = vecs + t;
-    uint2* vF = vecs + (size_t)max_len * T + t;
     const TextRead r{packed, b, len, strand};
-    vector_bwd(X, B, r, W, len, vB, T, sectors);
-    vector_fwd(X, F, r, W, len, vF, T, sectors);
-    search1_helper(X, r, W, len, vB, vF, T, B, F, emit, sectors);
+    const SearchVector vB = vector_run(X, B, r, W, len, false, vecs + t, T, sectors);
+    const SearchVector vF = vector_run(X, F, r, W, len, true, vecs + (size_t)max_len * T + t, T, sectors);
+    search1_helper(X, r, W, len, vB, vF, B, F, emit, sectors);
   }
   rs_count[2ull * r0 + t] = emit.cnt;
   rs_trunc[2ull * r0 + t] = emit.trunc ? 1 : 0;

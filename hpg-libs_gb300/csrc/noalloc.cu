@@ -74,11 +74,9 @@ __global__ void __launch_bounds__(128)
   if (ok) {
     const View B = strand ? View{1, 1} : View{0, 0};
     const View F = strand ? View{0, 1} : View{1, 0};
-    uint2* vB = vecs + t;
-    uint2* vF = vecs + (size_t)len_cap * T + t;
     const TextRead r{nullptr, 0, len, strand};  // (no packed reads here: rank steps)
-    vector_bwd(X, B, r, W, len, vB, T, sectors);
-    vector_fwd(X, F, r, W, len, vF, T, sectors);
+    const SearchVector vB = vector_run(X, B, r, W, len, false, vecs + t, T, sectors);
+    const SearchVector vF = vector_run(X, F, r, W, len, true, vecs + (size_t)len_cap * T + t, T, sectors);
     auto emit = [&](const Cursor& c) -> bool {
       if (cnt >= max_results) {
         trunc = true;
@@ -101,7 +99,7 @@ __global__ void __launch_bounds__(128)
       ++cnt;
       return true;
     };
-    search1_helper(X, r, W, len, vB, vF, T, B, F, emit, sectors);
+    search1_helper(X, r, W, len, vB, vF, B, F, emit, sectors);
   }
   counts[t] = cnt;
   truncated[t] = trunc ? 1 : 0;

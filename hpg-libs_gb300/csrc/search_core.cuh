@@ -85,20 +85,37 @@ __device__ __forceinline__ bool exact_fwd(const DevIndex& X, View v, const TextR
 
 __device__ __forceinline__ int64_t isize(uint2 v) { return (int64_t)v.y - (int64_t)v.x; }
 
-// Vector searches; the vector element for read position j lives at vec[j * stride].  The
-// helper reads elements n/2 .. 0 of the backward search and n/2 - 1 .. n of the forward one
-// (n = len - 1), so only those are kept, and a start table of the text's covers steps whose
-// elements are not.  It reads an element's interval only where its size differs from the next
-// one's, so the elements of a run that the text matched keep one row each, and the true one
-// only at the run's end; a failed element is any empty interval (its size is -1 always).
-__device__ __forceinline__ void vector_run(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int len,
-                                           int dir, uint2* vec, size_t stride, uint32_t& sectors) {
+// A vector search: the interval of each step t (t + 1 symbols), of which the helper reads
+// those of positions n/2 .. 0 of the backward search and n/2 - 1 .. n of the forward one
+// (n = len - 1), an interval only where its size differs from the next one's.  So only that
+// half is kept in memory, and no element after the search has failed (their size is -1
+// always) nor, but for the last, of a run of one row that the text matched.
+// Plain search of 262,144 reads of 100 bp, 100 Mbp: 1217 us a call with all elements of that
+// half written and read, the kernel bound by them (1.9 GB); 909 so.
+struct SearchVector {
+  uint2* at;      // the element of read position j at at[j * stride]
+  size_t stride;
+  int len;
+  bool fwd;
+  int one_from;   // steps after it and before `last` have one row each
+  int last;       // the last step before the search failed
+  __device__ __forceinline__ uint2 operator[](int j) const {
+    const int t = fwd ? j : len - 1 - j;
+    if (t > last) return make_uint2(1, 0);
+    if (t > one_from && t < last) return make_uint2(0, 0);
+    return at[(size_t)j * stride];
+  }
+};
+
+__device__ __forceinline__ SearchVector vector_run(const DevIndex& X, View v, const TextRead& r, const uint8_t* W,
+                                                   int len, bool fwd, uint2* vec, size_t stride, uint32_t& sectors) {
   uint32_t k = 0, l = X.top;
-  const int half = (len - 1) / 2, keep = dir > 0 ? half - 1 : len - 1 - half;  // first step whose element is kept
-  int i = dir > 0 ? 0 : len - 1, t = 0;
+  const int dir = fwd ? 1 : -1;
+  const int half = (len - 1) / 2, keep = fwd ? half - 1 : len - 1 - half;  // first step whose element is kept
+  int i = fwd ? 0 : len - 1, t = 0;
   const int L = r.packed ? (int)X.tmer_len : 0;
   if (L && len >= 2 * L + 2) {
-    const uint64_t q = query32(X, r.packed, r.b0, len, dir > 0, r.strand, 0);
+    const uint64_t q = query32(X, r.packed, r.b0, len, fwd, r.strand, 0);
     const uint32_t c = __brev((uint32_t)q) >> (32 - 2 * L);
     const uint2 s = load_row_pair((v.d ? X.tmer[1] : X.tmer[0]) + (((c & 0x55555555u) << 1) | ((c >> 1) & 0x55555555u)));
     k = s.x;
@@ -107,43 +124,32 @@ __device__ __forceinline__ void vector_run(const DevIndex& X, View v, const Text
     i += dir * L;
     if (L > keep) vec[(size_t)(i - dir) * stride] = s;  // (the shortest such read's forward search)
   }
-  for (; t < len; ++t, i += dir) {
+  SearchVector out{vec, stride, len, fwd, len, 0};
+  for (; t < len && k <= l; ++t, i += dir) {
     const bool one = k == l;
-    if (k <= l) {
-      sectors += ((k >> 6) == (l >> 6)) ? 1u : 2u;
-      bw_step(X, v, W[i], k, l);
-    }
+    sectors += ((k >> 6) == (l >> 6)) ? 1u : 2u;
+    bw_step(X, v, W[i], k, l);
+    if (k > l) break;
     if (t >= keep) vec[(size_t)i * stride] = make_uint2(k, l);
-    if (one && k == l && t + 1 < len && r.packed) {
+    if (one && t + 1 < len && r.packed) {
       uint32_t row;
-      const int m = text_run(X, v, r, dir > 0, t + 1, len - t - 1, k, row);
-      for (int q = max(1, keep - t); q <= m; ++q)
-        vec[(size_t)(i + dir * q) * stride] = q == m ? make_uint2(row, row) : make_uint2(k, k);
-      t += m;
-      i += dir * m;
-      k = 1;  // what is left, if anything, has failed
-      l = 0;
+      const int m = text_run(X, v, r, fwd, t + 1, len - t - 1, k, row);
+      out.one_from = t;
+      out.last = t + m;
+      if (m && out.last >= keep) vec[(size_t)(i + dir * m) * stride] = make_uint2(row, row);
+      return out;
     }
   }
-}
-
-__device__ __forceinline__ void vector_bwd(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int len,
-                                           uint2* vec, size_t stride, uint32_t& sectors) {
-  vector_run(X, v, r, W, len, -1, vec, stride, sectors);
-}
-
-__device__ __forceinline__ void vector_fwd(const DevIndex& X, View v, const TextRead& r, const uint8_t* W, int len,
-                                           uint2* vec, size_t stride, uint32_t& sectors) {
-  vector_run(X, v, r, W, len, 1, vec, stride, sectors);
+  out.last = t - 1;
+  return out;
 }
 
 // The helper for one strand.  `emit(cursor)` appends a hit and returns false
 // when the list is full, which ends the helper (search/results.h:100-101).
 // Returns true on overflow.
 template <typename Emit>
-__device__ bool search1_helper(const DevIndex& X, const TextRead& r, const uint8_t* W, int len, const uint2* vk,
-                               const uint2* vki,
-                               size_t stride, View B, View F, Emit& emit, uint32_t& sectors) {
+__device__ bool search1_helper(const DevIndex& X, const TextRead& r, const uint8_t* W, int len, const SearchVector& vk,
+                               const SearchVector& vki, View B, View F, Emit& emit, uint32_t& sectors) {
   const int start = 0, end = len - 1;
   const int n = end - start;
   int half = n / 2;
@@ -166,7 +172,7 @@ __device__ bool search1_helper(const DevIndex& X, const TextRead& r, const uint8
   c.err_pos = start;
 
   int64_t res = isize(v0), res_last;
-  uint2 v = vk[1 * stride];
+  uint2 v = vk[1];
   res_last = res;
   res = isize(v);
   if (res != res_last) {
@@ -204,7 +210,7 @@ __device__ bool search1_helper(const DevIndex& X, const TextRead& r, const uint8
 
   for (int i = start + 2, j = 2; j <= half; ++i, ++j) {
     res_last = res;
-    v = vk[(size_t)j * stride];
+    v = vk[j];
     res = isize(v);
     if (res == res_last) continue;
     c.kind = 1;
@@ -248,10 +254,10 @@ __device__ bool search1_helper(const DevIndex& X, const TextRead& r, const uint8
 
   half--;
   c.dir = 1;
-  v = vki[(size_t)n * stride];
+  v = vki[n];
   res = isize(v);
   res_last = res;
-  v = vki[(size_t)(n - 1) * stride];
+  v = vki[n - 1];
   res = isize(v);
   if (res != res_last) {
     c.k = v.x;
@@ -287,7 +293,7 @@ __device__ bool search1_helper(const DevIndex& X, const TextRead& r, const uint8
 
   for (int i = end - 2, j = n - 2; j >= half; --i, --j) {
     res_last = res;
-    v = vki[(size_t)j * stride];
+    v = vki[j];
     res = isize(v);
     if (res == res_last) continue;
     c.kind = 1;
