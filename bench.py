@@ -213,8 +213,9 @@ def make_reads(wl: dict, genome, seed: int):
 class ClockSampler:
     """nvidia-smi samples during the timed region."""
 
-    def __init__(self, device: int):
+    def __init__(self, device: int, ms: int = 100):
         self.device = device
+        self.ms = ms
         self.proc = None
         self.rows: list[list[str]] = []
 
@@ -224,7 +225,7 @@ class ClockSampler:
              "clocks_event_reasons.sw_power_cap")
         try:
             self.proc = subprocess.Popen(["nvidia-smi", "-i", str(self.device), f"--query-gpu={q}",
-                                          "--format=csv,noheader,nounits", "-lms", "100"],
+                                          "--format=csv,noheader,nounits", "-lms", str(self.ms)],
                                          stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.thr = threading.Thread(target=self._read, daemon=True)
             self.thr.start()
@@ -691,7 +692,8 @@ def block_search_leg(gi, reads, log, n_lists: int) -> dict:
         best = dt if best is None else min(best, dt)
         k = gi.block_search_ms()
         kms = k if kms is None else min(kms, k)
-    # one more call with the sector census on (not timed): occupancy-block sectors the kernel reads
+    # one more call with the sector census on (not timed): occurrence-block sectors by rank steps
+    # (the census runs without the text, which the timed calls finish most blocks with)
     gi.set_census(True)
     rs = lib.ResultSetC()
     if gi.lib.bwt_gpu_block_search(gi.handle, seq.ctypes.data, offs.ctypes.data, n, MAX_RESULTS,
@@ -703,7 +705,7 @@ def block_search_leg(gi, reads, log, n_lists: int) -> dict:
     out = {"reads": n, "seconds": round(best, 4), "reads_per_s": round(n / best, 1),
            "kernel_ms": round(kms, 3), "kernel_reads_per_s": round(n / (kms * 1e-3), 1),
            "sectors_per_read": round(sectors / max(1, n), 2),
-           "gather_gsectors_per_s": round(sectors / (kms * 1e-3) / 1e9, 1),
+           "gather_gsectors_per_s": None if gi.full_rows() else round(sectors / (kms * 1e-3) / 1e9, 1),
            "hits_per_read": round(hits / max(1, n), 3), "located_rows_per_read": round(locs / max(1, n), 3),
            "max_results": MAX_RESULTS}
     log(f"[bench] block search: kernel {out['kernel_reads_per_s'] / 1e6:.1f} M reads/s ({kms:.2f} ms), "
@@ -748,20 +750,31 @@ def run_gb300(args, wl: dict, dist: Dist) -> dict | None:
         """census run, W warm-up steps, K timed steps (L2 flushed before each);
         the last timed step's output is copied to the host for the parity check."""
         step = make_step(form)
+        # the plain form's census is of the reference's steps: with the text on the device
+        # it does not take them all, so that run goes without
+        by_steps = form == lib.FORM_PLAIN and gi.full_rows()
+        if by_steps:
+            gi.set_full_rows(False)
         gi.set_census(True)
         rs = step()
         sectors = gi.census()
         gi.set_census(False)
+        if by_steps:
+            gi.set_full_rows(True)
         for _ in range(args.warmup):
             step()
         ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
               for _ in range(args.steps)]
         stage_sum = [0.0, 0.0, 0.0, 0.0, 0.0]
-        dist.barrier()
-        torch.cuda.synchronize()
-        l0 = lib.launch_count()
         last = None
-        with ClockSampler(dev) as clk:
+        with ClockSampler(dev, 20) as clk:
+            # nvidia-smi takes longer to start than the timed steps: more warm-up until it samples
+            until = time.time() + 3
+            while clk.proc and not clk.rows and time.time() < until:
+                step()
+            dist.barrier()
+            torch.cuda.synchronize()
+            l0 = lib.launch_count()
             for i in range(args.steps):
                 flush.fill_(i & 0xFF)
                 torch.cuda.synchronize()
@@ -820,9 +833,9 @@ def run_gb300(args, wl: dict, dist: Dist) -> dict | None:
     ms_max = head["ms"]
     launches = head["launches"]
     clk_summary = head["clocks"]
-    # algorithmic sectors: the census of the plain form, which walks every step
-    # of the reference's searches (a start table in the batched form stands one
-    # lookup for its first steps, so its own census counts fewer sectors)
+    # algorithmic sectors: the census of the plain form by rank steps, which walks every
+    # step of the reference's searches (the batched form's start table and text stand for
+    # most of them, so its own census counts fewer sectors)
     sectors = res["plain"]["sectors"]
     gathered = head["sectors"]
     stage_sum = [x * args.steps for x in head["stages"]]
@@ -864,18 +877,30 @@ def run_gb300(args, wl: dict, dist: Dist) -> dict | None:
     per_step = [x / args.steps for x in stage_sum]
     search_ms = per_step[1]
     peak, peak_kind = measured_peaks()
-    algo_bytes = 32.0 * sectors + total + 16.0 * n_hits
+    text = gi.full_rows() and bool(gi.wave_group())
+    if text:
+        # what the search with the text has to fetch at random, in sectors: a start-table entry per
+        # chain, per hit the suffix array's value, the text beside the read and the inverse's row
+        algo_bytes = 32.0 * 4 * n + n_hits * (32.0 + 32.0 * (1 + total / n / 4 / 32) + 32.0 + 24.0) + total / 4 + 8.0 * n
+        basis = ("bytes the search with the text has to move (a start-table sector per chain; per hit the sectors "
+                 "of the suffix array, the text and its inverse and the pending record; packed bases and offsets) "
+                 "over the search stage's CUDA-event time, against the measured HBM copy bandwidth; random "
+                 "sectors, which DRAM serves at about 38 G/s whatever their size up to 64 bytes")
+        kernel, tuned = "text_search", {}
+    else:
+        algo_bytes = 32.0 * sectors + total + 16.0 * n_hits
+        basis = ("algorithmic bytes (census index sectors of the reference's steps x 32 B + read bytes + "
+                 "16 B per hit) over the search stage's CUDA-event time, against the measured HBM copy "
+                 "bandwidth; the index is mostly served from L2, so this is not DRAM throughput "
+                 "(dram_frac is)")
+        kernel = "wave_search_kernel" if gi.wave_group() else "batched_search_kernel"
+        tuned = {"group": gi.wave_group(), "start_table": gi.start_table(),
+                 "load_mode": gi.load_mode(), "direction_split": gi.direction_split()}
     achieved = algo_bytes / (search_ms * 1e-3) / 1e9
-    kernel = "wave_search_kernel" if gi.wave_group() else "batched_search_kernel"
-    traffic, traffic_src = profiled_traffic(args.workload, kernel,
-                                            {"group": gi.wave_group(), "start_table": gi.start_table(),
-                                             "load_mode": gi.load_mode(), "direction_split": gi.direction_split()})
+    traffic, traffic_src = profiled_traffic(args.workload, kernel, tuned)
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": traffic,
-                "basis": "algorithmic bytes (census index sectors of the reference's steps x 32 B + read bytes + "
-                         "16 B per hit) over the search stage's CUDA-event time, against the measured HBM copy "
-                         "bandwidth; the index is mostly served from L2, so this is not DRAM throughput "
-                         "(dram_frac is)",
+                "basis": basis,
                 "kernel": kernel, "peak_kind": peak_kind,
                 "algorithmic_bytes_per_read": round(algo_bytes / n, 1),
                 "traffic_source": traffic_src,
@@ -898,10 +923,12 @@ def run_gb300(args, wl: dict, dist: Dist) -> dict | None:
             for blocks in (152 * 8, 152 * 16):
                 best = max(best, lib.gather_ceiling(dev, ib, blocks, 1024))
             gather.update({"ceiling_sectors_per_s": round(best, 1), "buffer_bytes": ib,
-                           "frac": round(rate / best, 4), "frac_gathered": round(grate / best, 4),
-                           "basis": "frac: census sectors of the reference's steps (what the plain form "
-                                    "gathers); frac_gathered: sectors the batched form itself gathered (its start "
-                                    "table stands one lookup for a chain's first steps)"})
+                           "frac": None if text else round(rate / best, 4),
+                           "frac_gathered": round(grate / best, 4),
+                           "basis": "frac: census sectors of the reference's steps (what the plain form gathers by "
+                                    "rank steps; the search with the text does not take them: none); frac_gathered: "
+                                    "sectors of start table, occurrence blocks and suffix array the batched form "
+                                    "itself gathered (the text's are not counted)"})
     out = None
     if dist.rank == 0:
         base, parity = (None, None)

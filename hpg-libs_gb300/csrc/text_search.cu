@@ -16,13 +16,14 @@
 //   text_head_kernel    a thread per chain: start table, then rank steps until
 //                       the interval is empty or has stayed one row for a step
 //                       (its SA value, as an alignment, to `diag`), or is still
-//                       several rows where the helper branches or after
-//                       kHeadSteps steps (up to 32 rows -> row queue, else rest list)
+//                       several rows where the helper branches (up to 32: row queue)
+//                       or after kHeadSteps steps (up to 4: row queue); else rest list
 //   text_read_kernel    a thread per read: its one-row chains compared with the
 //                       text, hits
-//   text_wide_kernel    persistent lanes: the chains more than 32 rows wide until
-//                       they are not (-> row queue); their change points queued
-//   text_branch_kernel  persistent lanes: a queued change point's continuations,
+//   text_wide_kernel    persistent warps: the wider chains until they are not (-> row
+//                       queue), one rank step per lane and iteration; their change
+//                       points that can have hits queued
+//   text_branch_kernel  persistent warps: the queued change points' continuations,
 //                       one rank step per lane and iteration; walks that narrow
 //                       to one row -> walk queue
 //   text_rows_kernel    a lane per row of the queued chains, all their change
@@ -39,10 +40,10 @@
 // Bound by random sectors, as rank walks are, but about 20 a read of 100 bp at 100
 // Mbp against 180, and by the latency of some 8 dependent accesses a chain, whatever
 // the read's length.  Search stage, rank walks (wave.cu) -> here:
-//   2M x 100 bp, 100 Mbp                          3704 ->  880 us
-//   4M x 36-250 bp, 100 Mbp                      12570 -> 1965 us
-//   1000 x 50-300 bp, 100 Mbp                      510 ->   92 us
-//   2M x 150 bp, 600 Mbp with 45 % repeats        9809 -> 4087 us
+//   2M x 100 bp, 100 Mbp                          3704 ->  680 us
+//   4M x 36-250 bp, 100 Mbp                      12570 -> 1590 us
+//   1000 x 50-300 bp, 100 Mbp                      510 ->   70 us
+//   2M x 150 bp, 600 Mbp with 45 % repeats        9809 -> 2750 us
 // Indexes without the arrays, and batches above kTextMaxReads (the queues'
 // counters), take the warp-cooperative form.
 #include <cuda_runtime.h>
