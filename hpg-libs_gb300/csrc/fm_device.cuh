@@ -231,8 +231,10 @@ __device__ __forceinline__ uint64_t row_mask(uint32_t r) {
 // One rank step on physical symbol p: [k, l] to C[p] + its occurrences before k, and up to l.
 // An interval over two blocks has both on their way at once (2M x 150 bp, 600 Mbp: 3960 ->
 // 3580 us a call, 1000 reads at 100 Mbp 274 -> 250, against loads one after the other, the
-// second behind the first's use, as bw_step has them: it takes fewer registers, which the
-// kernels that step narrower intervals gain more by, plain search 1198 against 1287 us).
+// second behind the first's use, as bw_step has them: it takes fewer registers and, where both
+// ends share a block, fewer instructions, which the kernels that step narrower intervals gain
+// more by, plain search of 262,144 reads 840 against 912 us; the head is level at 100 Mbp and
+// 579 -> 523 us at 600 Mbp).
 __device__ __forceinline__ void rank_step(const DevIndex& X, const OccBlock* occ, uint32_t dollar, uint32_t p,
                                           uint32_t& k, uint32_t& l) {
   const uint32_t q0 = k >> 6, q1 = l >> 6;
