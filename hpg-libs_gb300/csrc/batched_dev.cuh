@@ -6,6 +6,7 @@
 #include <cooperative_groups.h>
 
 #include "batched.cuh"
+#include "chunk_slots.hpp"
 #include "search_core.cuh"
 
 namespace hpgbwt {
@@ -25,10 +26,9 @@ __device__ __forceinline__ uint32_t order_key(uint32_t section, uint32_t t, uint
   return (section << 28) | (t << 8) | slot;
 }
 
-// Pool slots are reserved per lane in chunks, so an emission normally waits on
-// no atomic: the per-list arrival count is a fire-and-forget reduction and
+// Pool slots are reserved per lane in chunks (chunk_slots.hpp), so an emission normally
+// waits on no atomic: the per-list arrival count is a fire-and-forget reduction and
 // the list position is assigned later by the scatter kernel.
-constexpr unsigned kResChunk = 8;
 
 // sa1: of a one-row hit whose SA value is known, that value plus one.
 __device__ __forceinline__ void write_hit(const BatchedParams& p, unsigned slot, uint32_t rs, uint32_t key,

@@ -594,21 +594,8 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
   }
 }
 
-// A slot of a queue written in per-lane chunks: state = next slot | slots left << 28,
-// counters below 2^28.  Past `cap` the slot is not there: returns cap.
-__device__ __forceinline__ unsigned chunk_slot(unsigned int* ctr, uint32_t cap, uint32_t& state) {
-  if ((state >> 28) == 0) {
-    const unsigned c = claim(ctr, kResChunk);
-    if (c >= (1u << 28) - kResChunk || c + kResChunk > cap) {
-      state = 0;
-      return cap;
-    }
-    state = c | (kResChunk << 28);
-  }
-  const unsigned slot = state & 0x0FFFFFFFu;
-  state = (slot + 1) | (((state >> 28) - 1) << 28);
-  return slot;
-}
+// Marks a slot of the walk queue that holds no walk.
+__device__ __forceinline__ void no_walk(const BatchedParams& p, uint32_t slot) { p.walk[slot].z = 0xFFFFFFFFu; }
 
 // Persistent: the chains still more than kRows rows wide, a lane each, one rank
 // step per iteration until they are not (-> row queue); the change points they
@@ -968,7 +955,8 @@ __global__ void __launch_bounds__(kWideTpb, 7) text_branch_kernel(DevIndex X, Ba
     q >>= 2;
     if (was_one && !walk_full) {  // one row that has matched on: the text tells the rest
       uint32_t cs = c_walk[tid];
-      const unsigned slot = chunk_slot(p.walk_n, p.walk_cap, cs);
+      const unsigned slot = chunk_slot(
+          p.walk_cap, cs, [&](unsigned n) { return claim(p.walk_n, n); }, [&](uint32_t i) { no_walk(p, i); });
       c_walk[tid] = cs;
       if (slot < p.walk_cap) {
         p.walk[slot] = make_uint4(k, key, rs, (uint32_t)t | (fwd ? 1u << 16 : 0u));
@@ -986,9 +974,7 @@ __global__ void __launch_bounds__(kWideTpb, 7) text_branch_kernel(DevIndex X, Ba
     const uint32_t r = c_res[tid];
     for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
       if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-    const uint32_t cw = c_walk[tid];
-    for (unsigned i = 0, left = cw >> 28, s = cw & 0x0FFFFFFFu; i < left; ++i)
-      if (s + i < p.walk_cap) p.walk[s + i].z = 0xFFFFFFFFu;
+    chunk_leave(p.walk_cap, c_walk[tid], [&](uint32_t i) { no_walk(p, i); });
   }
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
@@ -1005,7 +991,7 @@ __global__ void __launch_bounds__(kWalkTpb) text_walk_kernel(DevIndex X, Batched
     uint32_t row = 0, meta = 0, at = 0;
     uint4 e = make_uint4(0, 0, 0xFFFFFFFFu, 0);
     if (i < n) e = __ldcs(p.walk + i);
-    if (e.z != 0xFFFFFFFFu) {  // (a reserved slot nothing was written to)
+    if (e.z != 0xFFFFFFFFu) {  // (no_walk)
       const uint32_t strand = e.z & 1u;
       const bool fwd = (e.w >> 16) & 1u;
       const uint32_t d = (fwd ? 1u : 0u) ^ strand;
