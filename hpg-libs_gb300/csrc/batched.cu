@@ -378,12 +378,7 @@ __global__ void __launch_bounds__(kBlock, MINB) batched_search_kernel(DevIndex X
       mode = kNone;
     }
   }
-  {  // slots of this lane's last chunk that were reserved but not used
-    const uint32_t r = c_res[tid];
-    const unsigned left = r >> 28, slot = r & 0x0FFFFFFFu;
-    for (unsigned i = 0; i < left; ++i)
-      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-  }
+  res_leave(p, c_res[tid]);  // slots of this lane's last chunk that were reserved but not used
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
 
@@ -503,20 +498,7 @@ __global__ void __launch_bounds__(kBlock, MINB) chain_kernel(DevIndex X, Batched
 // flight per lane.  Change points go to the device queue for the drain launch.
 __device__ __forceinline__ void spill_push(const BatchedParams& p, uint32_t& chunk_state, uint32_t a, uint32_t b,
                                            uint32_t rs, uint32_t jt) {
-  unsigned left = chunk_state >> 28;
-  if (left == 0) {
-    chunk_state = claim(p.spill_tail, kResChunk);
-    left = kResChunk;
-    if (chunk_state >= (1u << 28)) {
-      chunk_state = 0;
-      const unsigned s1 = claim(p.spill_tail, 1);
-      if (s1 < p.spill_cap) p.spill[s1] = SpillEntry{a, b, rs, jt};
-      else atomicOr(p.status, kStatusSpillFull);
-      return;
-    }
-  }
-  const unsigned slot = chunk_state & 0x0FFFFFFFu;
-  chunk_state = (slot + 1) | ((left - 1) << 28);
+  const unsigned slot = spill_slot(p, chunk_state);
   if (slot < p.spill_cap) p.spill[slot] = SpillEntry{a, b, rs, jt};
   else atomicOr(p.status, kStatusSpillFull);
 }
@@ -619,12 +601,8 @@ __global__ void __launch_bounds__(kBlock, MINB) chain4_kernel(DevIndex X, Batche
     }
   }
   {  // reserved but unused slots of the last chunks
-    const uint32_t r = c_res[tid];
-    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-    const uint32_t q = c_spill[tid];
-    for (unsigned i = 0, left = q >> 28, slot = q & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.spill_cap) p.spill[slot + i].rs = 0xFFFFFFFFu;
+    res_leave(p, c_res[tid]);
+    spill_leave(p, c_spill[tid]);
   }
 }
 
@@ -737,12 +715,8 @@ __global__ void __launch_bounds__(kBlock, MINB) chain2_kernel(DevIndex X, Batche
     }
   }
   {  // reserved but unused slots of the last chunks
-    const uint32_t r = c_res[tid];
-    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-    const uint32_t q = c_spill[tid];
-    for (unsigned i = 0, left = q >> 28, slot = q & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.spill_cap) p.spill[slot + i].rs = 0xFFFFFFFFu;
+    res_leave(p, c_res[tid]);
+    spill_leave(p, c_spill[tid]);
   }
   if (p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }

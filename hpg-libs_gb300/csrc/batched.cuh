@@ -164,8 +164,9 @@ int wave_max_blocks_per_sm(const BatchedTuning& t);
 void launch_wave_branches(const DevIndex& X, const BatchedParams& p, SpillEntry* blocks, unsigned int* block_n,
                           uint32_t block_cap, int num_sms, cudaStream_t s);
 // The search with the text on the device (text_search.cu); the blocks go to p.blocks.
-// Up to kTextMaxReads reads a batch (the queues' counters and packed chunk states stay below
-// 2^28); text_queue_bytes is what its buffers take for a capacity of n_reads, set by text_queues.
+// Up to kTextMaxReads reads a batch (a few entries a read in the queues, whose counters
+// stay below 2^28; the walk queue is bounded by itself, the result pool past 2^28 by
+// pool_slot); text_queue_bytes is what its buffers take for a capacity of n_reads, set by text_queues.
 constexpr size_t kTextMaxReads = 1u << 25;
 size_t text_queue_bytes(size_t n_reads, int num_sms);
 void text_queues(BatchedParams& p, void* buffer, size_t n_reads, int num_sms);

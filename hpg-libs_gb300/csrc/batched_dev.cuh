@@ -64,20 +64,27 @@ __device__ __forceinline__ unsigned claim(unsigned int* ctr, unsigned n) {
   return g.shfl(base, 0) + g.thread_rank() * n;
 }
 
-// Chunked pool slot for the calling lane (cold state c_res = next slot | left << 28).
+// Chunked slot of the result pool for the calling lane (c_res: its chunk), and the end of
+// the lane's last chunk.
 __device__ __forceinline__ unsigned res_slot(const BatchedParams& p, uint32_t& c_res) {
-  unsigned left = c_res >> 28;
-  if (left == 0) {
-    c_res = claim(p.res_total, kResChunk);
-    left = kResChunk;
-    if (c_res >= (1u << 28)) {  // beyond what the packed form holds: fall back to single slots
-      c_res = 0;
-      return claim(p.res_total, 1) | 0u;
-    }
-  }
-  const unsigned slot = c_res & 0x0FFFFFFFu;
-  c_res = (slot + 1) | ((left - 1) << 28);
-  return slot;
+  return pool_slot(
+      p.res_cap, c_res, [&](unsigned n) { return claim(p.res_total, n); },
+      [&](uint32_t i) { p.res[i].rs = 0xFFFFFFFFu; });
+}
+
+__device__ __forceinline__ void res_leave(const BatchedParams& p, uint32_t c_res) {
+  chunk_leave(p.res_cap, c_res, [&](uint32_t i) { p.res[i].rs = 0xFFFFFFFFu; });
+}
+
+// The same of the queue of change points.
+__device__ __forceinline__ unsigned spill_slot(const BatchedParams& p, uint32_t& c_spill) {
+  return pool_slot(
+      p.spill_cap, c_spill, [&](unsigned n) { return claim(p.spill_tail, n); },
+      [&](uint32_t i) { p.spill[i].rs = 0xFFFFFFFFu; });
+}
+
+__device__ __forceinline__ void spill_leave(const BatchedParams& p, uint32_t c_spill) {
+  chunk_leave(p.spill_cap, c_spill, [&](uint32_t i) { p.spill[i].rs = 0xFFFFFFFFu; });
 }
 
 // Lane modes.

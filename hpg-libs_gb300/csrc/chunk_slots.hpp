@@ -37,6 +37,24 @@ HPG_HD unsigned chunk_slot(uint32_t cap, uint32_t& state, Claim claim, Empty emp
   return slot;
 }
 
+// The next slot of a pool of any size, which may be at or past cap (the caller's
+// overflow).  A chunk that ends past what the state's word holds gives its first slot only.
+template <typename Claim, typename Empty>
+HPG_HD unsigned pool_slot(uint32_t cap, uint32_t& state, Claim claim, Empty empty) {
+  if ((state >> 28) == 0) {
+    const unsigned c = claim(kResChunk);
+    if (c > kChunkSlotMask - kResChunk) {
+      for (unsigned s = c + 1; s < c + kResChunk && s < cap; ++s) empty(s);
+      state = 0;
+      return c;
+    }
+    state = c | (kResChunk << 28);
+  }
+  const unsigned slot = state & kChunkSlotMask;
+  state = (slot + 1) | (((state >> 28) - 1) << 28);
+  return slot;
+}
+
 // Marks what is left of a lane's last chunk.
 template <typename Empty>
 HPG_HD void chunk_leave(uint32_t cap, uint32_t state, Empty empty) {

@@ -587,11 +587,7 @@ __global__ void __launch_bounds__(kRowsTpb) text_rows_kernel(DevIndex X, Batched
     }
     __syncwarp();
   }
-  {
-    const uint32_t r = c_res[tid];
-    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-  }
+  res_leave(p, c_res[tid]);
 }
 
 // Marks a slot of the walk queue that holds no walk.
@@ -755,11 +751,7 @@ __global__ void __launch_bounds__(kWideTpb) text_wide_kernel(DevIndex X, Batched
   }
   if (n_rows) flush_rows(0, n_rows);
   if (n_change) flush_change(0, n_change);
-  {  // slots of this lane's last chunk that were reserved but not used
-    const uint32_t r = c_res[tid];
-    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-  }
+  res_leave(p, c_res[tid]);  // slots of this lane's last chunk that were reserved but not used
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
 
@@ -971,9 +963,7 @@ __global__ void __launch_bounds__(kWideTpb, 7) text_branch_kernel(DevIndex X, Ba
     }
   }
   {  // slots of this lane's last chunks that were reserved but not used
-    const uint32_t r = c_res[tid];
-    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
+    res_leave(p, c_res[tid]);
     chunk_leave(p.walk_cap, c_walk[tid], [&](uint32_t i) { no_walk(p, i); });
   }
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);

@@ -182,20 +182,8 @@ __global__ void __launch_bounds__(kWBlock, MINB) wave_search_kernel(DevIndex X, 
   // A change point for the device queue (wave_branch_kernel), in chunks of slots.
   auto spill_cp = [&](uint32_t a, uint32_t b, uint32_t jt) {
     uint32_t cs = c_spl[tid];
-    unsigned left = cs >> 28;
-    if (left == 0) {
-      cs = claim(p.spill_tail, kResChunk);
-      left = kResChunk;
-      if (cs >= (1u << 28)) {  // beyond what the packed form holds: single slots
-        c_spl[tid] = 0;
-        const unsigned q = claim(p.spill_tail, 1);
-        if (q < p.spill_cap) p.spill[q] = SpillEntry{a, b, rs, jt};
-        else atomicOr(p.status, kStatusSpillFull);
-        return;
-      }
-    }
-    const unsigned q = cs & 0x0FFFFFFFu;
-    c_spl[tid] = (q + 1) | ((left - 1) << 28);
+    const unsigned q = spill_slot(p, cs);
+    c_spl[tid] = cs;
     if (q < p.spill_cap) p.spill[q] = SpillEntry{a, b, rs, jt};
     else atomicOr(p.status, kStatusSpillFull);
   };
@@ -520,12 +508,8 @@ __global__ void __launch_bounds__(kWBlock, MINB) wave_search_kernel(DevIndex X, 
     item_done();
   }
   {  // slots of this lane's last chunks that were reserved but not used
-    const uint32_t r = c_res[tid];
-    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-    const uint32_t cs = c_spl[tid];
-    for (unsigned i = 0, left = cs >> 28, q = cs & 0x0FFFFFFFu; i < left; ++i)
-      if (q + i < p.spill_cap) p.spill[q + i].rs = 0xFFFFFFFFu;
+    res_leave(p, c_res[tid]);
+    spill_leave(p, c_spl[tid]);
   }
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
@@ -704,11 +688,7 @@ __global__ void __launch_bounds__(kWBlock, MINB) wave_branch_kernel(DevIndex X, 
     }
     active = false;
   }
-  {
-    const uint32_t r = c_res[tid];
-    for (unsigned i = 0, left = r >> 28, slot = r & 0x0FFFFFFFu; i < left; ++i)
-      if (slot + i < p.res_cap) p.res[slot + i].rs = 0xFFFFFFFFu;
-  }
+  res_leave(p, c_res[tid]);
   if (CENSUS && p.census) atomicAdd(p.census, (unsigned long long)sectors);
 }
 

@@ -77,3 +77,14 @@ def test_bounded_queue_leaves_no_slot_unwritten(run, cap, entries):
         assert (unwritten, twice, outside) == (0, 0, 0)
         if entries > cap - from_:
             assert refused
+
+
+@pytest.mark.parametrize("cap", [1, 100, 1005, (1 << 28) - 5, 1 << 28, (1 << 28) + 777, (1 << 32) - 17])
+@pytest.mark.parametrize("from_", [0, 3, (1 << 28) - 2000, (1 << 28) - 8, (1 << 28) - 3, 1 << 28, (1 << 31) + 5])
+def test_pool_leaves_no_slot_unwritten(run, cap, from_):
+    """Past 2^28, what a state's word holds, a lane takes one slot a claim."""
+    for lanes, entries in ((1, 9), (13, 3000), (300, 5000)):
+        refused, unwritten, twice, outside = run("pool_slot")(lanes, entries, cap, from_)
+        assert (unwritten, twice, outside) == (0, 0, 0)
+        if cap > from_ + 8 * (entries + lanes):
+            assert refused == 0
