@@ -732,7 +732,7 @@ namespace {
 int finish_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_t n, uint64_t total,
                  uint32_t max_results, DeviceResult* out, std::string* err, bool exact = false) {
   DeviceResult r;
-  if (run_batched_graph(e, seqs, offs, n, total, max_results, &r, err, exact) != 0) return -1;
+  if (const int rc = run_batched_graph(e, seqs, offs, n, total, max_results, &r, err, exact)) return rc;
   e->last = r;
   *out = r;
   return 0;
@@ -741,8 +741,7 @@ int finish_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_t n, 
 }  // namespace
 
 // Whether an exact search of n reads runs from its own captured graph.  What that form
-// refuses (more rows than a batch indexes, offsets that its device check rejects, no room
-// for its pools) runs in the plain form, as every exact search without the text does.
+// refuses (kGraphRefused) runs in the plain form, as every exact search without the text does.
 static bool exact_graph(const Engine* e, int mode, int form, size_t n) {
   return mode == HPG_BWT_MODE_EXACT && form == kFormBatched && e->use_graph && e->X.text && !e->census_on &&
          n <= kTextMaxReads;
@@ -811,10 +810,12 @@ int engine_search_device(Engine* e, int mode, int form, const uint8_t* d_seqs, c
   cudaStream_t s = e->stream;
   const uint32_t n = (uint32_t)n_reads;
   const uint32_t len_cap = std::max<uint32_t>(max_len, 3);
-  if (form == kFormBatched && e->use_graph) return finish_graph(e, d_seqs, d_offs, n, total_bases, max_results, out, err);
+  if (form == kFormBatched && e->use_graph)
+    return finish_graph(e, d_seqs, d_offs, n, total_bases, max_results, out, err) == 0 ? 0 : -1;
   if (exact && total_bases <= (1ull << 40)) {
-    std::string why;
-    if (finish_graph(e, d_seqs, d_offs, n, total_bases, max_results, out, &why, true) == 0) return 0;
+    const int rc = finish_graph(e, d_seqs, d_offs, n, total_bases, max_results, out, err, true);
+    if (rc != kGraphRefused) return rc;
+    err->clear();
   }
 
   if (!ensure(e, e->codes, total_bases + 16) || !ensure(e, e->ok, n + 16) || !ensure(e, e->rs_count, 8ull * n + 16) ||
@@ -1053,12 +1054,14 @@ int engine_search_host_keep(Engine* e, int mode, int form, const char* seqs, con
     }
     static const uint64_t zero = 0;
     return finish_graph(e, seqs + (n_reads ? offs[0] : 0), n_reads ? o : &zero, (uint32_t)n_reads, total,
-                        max_results, r, err);
+                        max_results, r, err) == 0 ? 0 : -1;
   }
   if (exact_graph(e, mode, form, n_reads) && (n_reads == 0 || offs[0] == 0) && total <= (1ull << 40)) {
     static const uint64_t zero = 0;
-    std::string why;
-    if (finish_graph(e, seqs, n_reads ? offs : &zero, (uint32_t)n_reads, total, max_results, r, &why, true) == 0) return 0;
+    const int rc = finish_graph(e, seqs, n_reads ? offs : &zero, (uint32_t)n_reads, total, max_results, r, err, true);
+    if (rc != kGraphRefused) return rc;
+    err->clear();
+    form = kFormPlain;  // refused once, not asked again below
   }
   uint32_t max_len = 0;
   for (size_t i = 0; i < n_reads; ++i) {

@@ -205,18 +205,21 @@ inline bool text_form(const Engine* e, uint64_t n) {
 // offsets may start anywhere (map_device.cu).
 int upload_reads(Engine* e, const char* seqs, const uint64_t* offs, size_t n, std::string* err);
 
-// Graph form of the batched pipeline (graph.cu).
+// Graph form of the batched pipeline (graph.cu).  Returns 0, -1, or kGraphRefused for a
+// batch that this form does not take (more rows than a batch indexes, offsets that its
+// device check rejects, no room for its pools), with the message in err.
 constexpr int kExactSlot = 2;  // plan slot of the exact search (with the text on the device)
+constexpr int kGraphRefused = -2;
 int run_batched_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_t n, uint64_t total,
                       uint32_t max_results, DeviceResult* out, std::string* err, bool exact = false);
 uint64_t graph_plans_bytes(const Engine* e);  // device bytes of all plans
 void graph_plan_destroy(GraphPlan* g);
 void graph_plans_destroy(Engine* e);
-// Free the plans of more than max_n_cap reads (after the streams finish).
+// Free the plans of more than max_n_cap reads, and the exact search's (after the streams finish).
 void graph_plans_drop_above(Engine* e, uint64_t max_n_cap);
 // Free the grow-only workspaces of the direct, plain, block-search and
-// alignment-list calls (they are allocated again on demand) and the plans of
-// more than keep_n_cap reads: a server on the index keeps only what it uses.
+// alignment-list calls (they are allocated again on demand), the plans of
+// more than keep_n_cap reads and the exact search's: a server on the index keeps only what it uses.
 void engine_release_workspace(Engine* e, uint64_t keep_n_cap);
 // Asynchronous halves of run_batched_graph for a batch already staged in the
 // plan's input buffers: launch (header + replay), then collect (synchronize,
@@ -228,9 +231,10 @@ int graph_launch(Engine* e, GraphPlan* g, uint32_t n, uint32_t max_results, std:
                  const void* src = nullptr, uint64_t src_bytes = 0);
 int graph_collect(Engine* e, GraphPlan* g, uint32_t n, GraphPlan* grow, DeviceResult* out, std::string* err);
 // The plan serving batches of n reads and `total` bases (captured on demand).
-// `pslot` (0/1) picks one of the two plans of a capacity class.
+// `pslot` (0/1, or kExactSlot) picks one of the plans of a capacity class.  Null on
+// failure; *no_room then says whether device memory for its buffers was what lacked.
 GraphPlan* graph_plan_for(Engine* e, uint32_t n, uint64_t total, const GraphPlan* grow, bool carry,
-                          std::string* err, int pslot = 0);
+                          std::string* err, int pslot = 0, bool* no_room = nullptr);
 // Recapture, at the per-read pool rates learned so far, every plan of at most
 // max_n_cap reads whose pools are below them, except keep0 and keep1 (plans
 // that hold a batch); for a caller that has just drained its streams after an

@@ -103,7 +103,7 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
       (text && !exact && !grab(g, &g->queues, text_queue_bytes(g->n_cap, e->num_sms))) ||
       !grab(g, &g->summary_d, 64)) {
     *err = "out of device memory (graph plan)";
-    return -1;
+    return kGraphRefused;
   }
   HPG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&g->h_summary), 64, cudaHostAllocDefault), "pinned summary");
   HPG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&g->h_hdr), 32, cudaHostAllocDefault), "pinned header");
@@ -239,7 +239,7 @@ void graph_plans_drop_above(Engine* e, uint64_t max_n_cap) {
   for (cudaStream_t x : e->xs)
     if (x) cudaStreamSynchronize(x);
   for (int i = 0; i < kMaxPlans * kPlanSlots; ++i)
-    if (e->plans[i] && e->plans[i]->n_cap > max_n_cap) {
+    if (e->plans[i] && (e->plans[i]->n_cap > max_n_cap || e->plans[i]->exact)) {
       graph_plan_destroy(e->plans[i]);
       e->plans[i] = nullptr;
     }
@@ -251,7 +251,7 @@ void graph_plans_drop_above(Engine* e, uint64_t max_n_cap) {
 // With `carry` the batch already staged in the old plan's input buffers (n
 // reads, `total` bases) is copied into the new plan's.
 GraphPlan* graph_plan_for(Engine* e, uint32_t n, uint64_t total, const GraphPlan* grow, bool carry,
-                          std::string* err, int pslot) {
+                          std::string* err, int pslot, bool* no_room) {
   if (!e->plans) {
     e->plans = new GraphPlan*[kMaxPlans * kPlanSlots];
     for (int i = 0; i < kMaxPlans * kPlanSlots; ++i) e->plans[i] = nullptr;
@@ -269,8 +269,11 @@ GraphPlan* graph_plan_for(Engine* e, uint32_t n, uint64_t total, const GraphPlan
   // recapture drains every stream, which a serving pipeline should not pay for
   // a batch that fits)
   const double nc = (double)n_cap;
-  const bool fresh = !g || !same_settings(g, e);
-  const double res_rate = fresh ? std::max(4.0, e->res_per_read) : 4.0;
+  // (the exact search has at most one hit a list, and rows a read that say nothing of the
+  // 1-error search's: a plan of its own starts at its first size and grows for its own batches)
+  const bool exact = pslot == kExactSlot;
+  const bool fresh = (!g || !same_settings(g, e)) && !exact;
+  const double res_rate = exact ? 2.0 : (fresh ? std::max(4.0, e->res_per_read) : 4.0);
   const double locs_rate = fresh ? std::max(8.0, e->locs_per_read) : 8.0;
   const double spill_rate = fresh ? e->spill_per_read : 0.0;
   uint32_t res_cap = (uint32_t)std::min<double>(res_rate * nc + 4096, 0xFFFFFFF0u);
@@ -306,13 +309,14 @@ GraphPlan* graph_plan_for(Engine* e, uint32_t n, uint64_t total, const GraphPlan
   g->kmer_len = e->X.kmer_len;
   g->kmer0 = e->X.kmer[0];
   g->text = e->X.text;
-  g->exact = pslot == kExactSlot;
+  g->exact = exact;
   if (old) {  // no stream may still read the old plan's buffers
     cudaStreamSynchronize(e->stream);
     for (cudaStream_t x : e->xs)
       if (x) cudaStreamSynchronize(x);
   }
-  if (capture(e, g, err) != 0) {
+  if (const int rc = capture(e, g, err)) {
+    if (no_room) *no_room = rc == kGraphRefused;
     graph_plan_destroy(g);
     return nullptr;
   }
@@ -333,7 +337,7 @@ int graph_plans_refresh(Engine* e, const GraphPlan* keep0, const GraphPlan* keep
   if (!e->plans) return 0;
   for (int i = 0; i < kMaxPlans * kPlanSlots; ++i) {
     GraphPlan* g = e->plans[i];
-    if (!g || g == keep0 || g == keep1 || g->n_cap > max_n_cap || !same_settings(g, e)) continue;
+    if (!g || g == keep0 || g == keep1 || g->exact || g->n_cap > max_n_cap || !same_settings(g, e)) continue;
     const double nc = (double)g->n_cap;
     GraphPlan grow;
     grow.res_cap = (uint32_t)std::min<double>(std::max(4.0, e->res_per_read) * nc + 4096, 0xFFFFFFF0u);
@@ -366,18 +370,19 @@ int graph_collect(Engine* e, GraphPlan* g, uint32_t n, GraphPlan* grow, DeviceRe
   const uint32_t status = (uint32_t)h[0];
   if (status & kStatusBadInput) {
     *err = "read offsets must be non-decreasing and reads at most 32767 bases";
-    return -1;
+    return kGraphRefused;
   }
   if (status & kStatusWaveAcct) {
     *err = "internal error: inconsistent work counts in the warp-cooperative search";
     return -1;
   }
   if (status) {
-    // the rates this batch needed, with room, for every capacity class from now on
-    const double nr = std::max<double>(n, 1.0);
-    if (status & kStatusResFull) e->res_per_read = std::max(e->res_per_read, 1.5 * (double)(h[0] >> 32) / nr);
-    if (status & kStatusSpillFull) e->spill_per_read = std::max(e->spill_per_read, 1.5 * (double)h[1] / nr);
-    if (status & kStatusLocFull) e->locs_per_read = std::max(e->locs_per_read, 1.25 * (double)h[3] / nr);
+    if (!g->exact) {  // the rates this batch needed, with room, for every capacity class from now on
+      const double nr = std::max<double>(n, 1.0);
+      if (status & kStatusResFull) e->res_per_read = std::max(e->res_per_read, 1.5 * (double)(h[0] >> 32) / nr);
+      if (status & kStatusSpillFull) e->spill_per_read = std::max(e->spill_per_read, 1.5 * (double)h[1] / nr);
+      if (status & kStatusLocFull) e->locs_per_read = std::max(e->locs_per_read, 1.25 * (double)h[3] / nr);
+    }
     grow->res_cap = g->res_cap;
     grow->spill_cap = g->spill_cap;
     grow->locs_cap = g->locs_cap;
@@ -387,7 +392,7 @@ int graph_collect(Engine* e, GraphPlan* g, uint32_t n, GraphPlan* grow, DeviceRe
       if (h[3] > kMaxLocateRows) {
         *err = "too many located rows in one batched call (" + std::to_string(h[3]) + ", limit " +
                std::to_string(kMaxLocateRows) + "): split the batch or use the plain form";
-        return -1;
+        return kGraphRefused;
       }
       grow->locs_cap = std::min<uint64_t>(h[3] + h[3] / 4 + 4096, kMaxLocateRows);
     }
@@ -639,8 +644,10 @@ int run_batched_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_
   // run small batches in a larger class's plan)
   const uint32_t n_plan = staged_in ? std::max<uint32_t>(n, staged_in->n_cap) : n;
   for (int attempt = 0; attempt < 8; ++attempt) {
-    GraphPlan* g = graph_plan_for(e, n_plan, total, attempt ? &grow : nullptr, staged_in != nullptr, err, pslot);
-    if (!g) return -1;
+    bool no_room = false;
+    GraphPlan* g = graph_plan_for(e, n_plan, total, attempt ? &grow : nullptr, staged_in != nullptr, err, pslot,
+                                  &no_room);
+    if (!g) return no_room ? kGraphRefused : -1;
     if (staged_in) {  // follow the batch into a replacement plan
       seqs = g->seqs;
       offs = g->offs;
@@ -652,8 +659,7 @@ int run_batched_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_
       HPG_CUDA(cudaMemcpyAsync(g->offs, offs, ((size_t)n + 1) * 8, cudaMemcpyDefault, s), "read offsets");
     if (graph_launch(e, g, n, max_results, err, in_place ? seqs : nullptr, total) != 0) return -1;
     const int rc = graph_collect(e, g, n, &grow, out, err);
-    if (rc < 0) return -1;
-    if (rc == 0) return 0;
+    if (rc <= 0) return rc;
   }
   *err = "batched search pools kept overflowing";
   return -1;
