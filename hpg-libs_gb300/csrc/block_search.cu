@@ -1518,6 +1518,7 @@ int engine_block_search(Engine* e, const char* seqs, const uint64_t* offs, size_
   out->n_anchors.assign(2 * n, 0);
   out->kernel_ms = 0;
   if (!n) return 0;
+  HostCopies copies(e->stream);
   if (check_block_args(n, err) != 0 || upload_reads(e, seqs, offs, n, err) != 0) return -1;
   uint64_t total = 0;
   if (block_search_device(e, n, max_results, &total, err) != 0) return -1;
@@ -1534,6 +1535,7 @@ int engine_block_search(Engine* e, const char* seqs, const uint64_t* offs, size_
            "block anchors");
   HPG_CUDA(cudaMemcpyAsync(out->n_anchors.data(), e->ovf.p, T, cudaMemcpyDeviceToHost, s), "block anchor counts");
   HPG_CUDA(cudaStreamSynchronize(s), "block search results");
+  copies.waited();
   out->kernel_ms = e->block_ms;
   return 0;
 }
@@ -1546,6 +1548,7 @@ int engine_block_search_result(Engine* e, const char* seqs, const uint64_t* offs
   out->n_reads = n;
   const size_t T = 2 * n;
   uint64_t total = 0;
+  HostCopies copies(e->stream);
   if (n) {
     if (check_block_args(n, err) != 0 || upload_reads(e, seqs, offs, n, err) != 0) return -1;
     if (block_search_device(e, n, max_results, &total, err) != 0) return -1;
@@ -1614,6 +1617,7 @@ int engine_block_search_result(Engine* e, const char* seqs, const uint64_t* offs
     HPG_CUDA(cudaMemcpyAsync(out->locs, e->locs.p, n_rows * sizeof(hpg_loc_t), cudaMemcpyDeviceToHost, s),
              "located rows");
   HPG_CUDA(cudaStreamSynchronize(s), "block search results");
+  copies.waited();
   uint32_t derr = 0;
   HPG_CUDA(cudaMemcpy(&derr, e->d_err, 4, cudaMemcpyDeviceToHost), "error word");
   if (derr) {

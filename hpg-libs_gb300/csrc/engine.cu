@@ -1036,6 +1036,11 @@ int engine_search_host_keep(Engine* e, int mode, int form, const char* seqs, con
   const uint64_t total = n_reads ? offs[n_reads] - offs[0] : 0;
   cudaStream_t s = e->stream;
   std::vector<uint64_t> rel;
+  HostCopies copies(s);
+  auto end = [&](int rc) {  // (a search that succeeds has waited)
+    if (rc == 0) copies.waited();
+    return rc == 0 ? 0 : -1;
+  };
   if (form == kFormBatched && mode == HPG_BWT_MODE_SEARCH1 && e->use_graph) {
     // the graph checks every read's offsets on the device (no host pass over them)
     if (n_reads >= (1ull << 31)) {
@@ -1053,13 +1058,13 @@ int engine_search_host_keep(Engine* e, int mode, int form, const char* seqs, con
       o = rel.data();
     }
     static const uint64_t zero = 0;
-    return finish_graph(e, seqs + (n_reads ? offs[0] : 0), n_reads ? o : &zero, (uint32_t)n_reads, total,
-                        max_results, r, err) == 0 ? 0 : -1;
+    return end(finish_graph(e, seqs + (n_reads ? offs[0] : 0), n_reads ? o : &zero, (uint32_t)n_reads, total,
+                            max_results, r, err));
   }
   if (exact_graph(e, mode, form, n_reads) && (n_reads == 0 || offs[0] == 0) && total <= (1ull << 40)) {
     static const uint64_t zero = 0;
     const int rc = finish_graph(e, seqs, n_reads ? offs : &zero, (uint32_t)n_reads, total, max_results, r, err, true);
-    if (rc != kGraphRefused) return rc;
+    if (rc != kGraphRefused) return end(rc);
     err->clear();
     form = kFormPlain;  // refused once, not asked again below
   }
@@ -1084,8 +1089,8 @@ int engine_search_host_keep(Engine* e, int mode, int form, const char* seqs, con
   for (size_t i = 0; i <= n_reads; ++i) rel[i] = offs[i] - offs[0];
   if (total) HPG_CUDA(cudaMemcpyAsync(e->seqs.p, seqs + offs[0], total, cudaMemcpyHostToDevice, s), "upload reads");
   HPG_CUDA(cudaMemcpyAsync(e->offs.p, rel.data(), (n_reads + 1) * 8, cudaMemcpyHostToDevice, s), "upload offsets");
-  return engine_search_device(e, mode, form, ptr<uint8_t>(e->seqs), ptr<uint64_t>(e->offs), n_reads, total, max_len,
-                              max_results, r, err);
+  return end(engine_search_device(e, mode, form, ptr<uint8_t>(e->seqs), ptr<uint64_t>(e->offs), n_reads, total,
+                                  max_len, max_results, r, err));
 }
 
 int engine_search_host(Engine* e, int mode, int form, const char* seqs, const uint64_t* offs, size_t n_reads,

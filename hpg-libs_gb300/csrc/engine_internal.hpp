@@ -200,9 +200,27 @@ inline bool text_form(const Engine* e, uint64_t n) {
   return e->tuning.split == 3 && e->X.text && n <= kTextMaxReads;
 }
 
+// Copies of a call from its caller's (or its own) host arrays, or to them, which must not
+// outlive it: unless the call says that it has waited for its stream, leaving it waits.
+// So an error between the upload and that wait returns with nothing in flight.
+class HostCopies {
+ public:
+  explicit HostCopies(cudaStream_t s) : s_(s) {}
+  HostCopies(const HostCopies&) = delete;
+  HostCopies& operator=(const HostCopies&) = delete;
+  ~HostCopies() {
+    if (!waited_) cudaStreamSynchronize(s_);
+  }
+  void waited() { waited_ = true; }
+
+ private:
+  cudaStream_t s_;
+  bool waited_ = false;
+};
+
 // Reads to the engine's device buffers, encoded (codes + validity flags, and packed
-// codes where the index has its text);
-// offsets may start anywhere (map_device.cu).
+// codes where the index has its text); offsets may start anywhere (map_device.cu).
+// The copies may still be under way when it returns: the caller holds a HostCopies.
 int upload_reads(Engine* e, const char* seqs, const uint64_t* offs, size_t n, std::string* err);
 
 // Graph form of the batched pipeline (graph.cu).  Returns 0, -1, or kGraphRefused for a

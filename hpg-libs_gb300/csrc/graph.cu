@@ -593,6 +593,10 @@ int run_graph_pipelined(Engine* e, const char* seqs, const uint64_t* offs, size_
     if (rc == 0 && i >= 1) rc = collect(i - 1);
   }
   if (rc == 0) rc = collect(K - 1);
+  if (rc != 0) {  // chunks may still be on their way in
+    cudaStreamSynchronize(h2d);
+    cudaStreamSynchronize(cs);
+  }
   cudaError_t ce = cudaStreamSynchronize(d2h);
   release();
   if (rc != 0) return -1;

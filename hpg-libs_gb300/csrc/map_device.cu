@@ -263,6 +263,7 @@ int engine_exact_api(Engine* e, const char* seqs, const uint64_t* offs, size_t n
     return -1;
   }
   if (!n) return 0;
+  HostCopies copies(e->stream);
   if (upload_reads(e, seqs, offs, n, err) != 0) return -1;
   if (!ensure(e, e->slots, n * sizeof(uint4) + 16)) {
     *err = "out of device memory (exact intervals)";
@@ -274,6 +275,7 @@ int engine_exact_api(Engine* e, const char* seqs, const uint64_t* offs, size_t n
                                                                 ptr<uint8_t>(e->ok), (uint32_t)n, ptr<uint4>(e->slots));
   HPG_CUDA(cudaMemcpyAsync(kl, e->slots.p, n * sizeof(uint4), cudaMemcpyDeviceToHost, s), "exact intervals");
   HPG_CUDA(cudaStreamSynchronize(s), "exact search");
+  copies.waited();
   return 0;
 }
 
@@ -281,6 +283,7 @@ int engine_anchor_scan(Engine* e, const char* seqs, const uint64_t* offs, size_t
                        uint32_t* out, std::string* err) {
   HPG_CUDA(cudaSetDevice(e->device), "cudaSetDevice");
   if (!m) return 0;
+  HostCopies copies(e->stream);
   if (upload_reads(e, seqs, offs, n, err) != 0) return -1;
   if (!ensure(e, e->slots, 4 * m * sizeof(uint4) + 16) || !ensure(e, e->rows, m * 4 + 16)) {
     *err = "out of device memory (anchor scan)";
@@ -295,6 +298,7 @@ int engine_anchor_scan(Engine* e, const char* seqs, const uint64_t* offs, size_t
                                                                       ptr<uint4>(e->slots));
   HPG_CUDA(cudaMemcpyAsync(out, e->slots.p, 4 * m * sizeof(uint4), cudaMemcpyDeviceToHost, s), "anchor scan");
   HPG_CUDA(cudaStreamSynchronize(s), "anchor scan");
+  copies.waited();
   return 0;
 }
 
@@ -311,6 +315,7 @@ int engine_seed_search(Engine* e, const char* seqs, const uint64_t* offs, size_t
       *err = "seed of a read outside the batch";
       return -1;
     }
+  HostCopies copies(e->stream);
   if (upload_reads(e, seqs, offs, n, err) != 0) return -1;
   if (!ensure(e, e->slots, 2 * m * sizeof(uint4) + 16)) {
     *err = "out of device memory (seeds)";
@@ -325,6 +330,7 @@ int engine_seed_search(Engine* e, const char* seqs, const uint64_t* offs, size_t
                                                                   ptr<uint8_t>(e->ok), d_seeds, (uint32_t)m, d_out);
   HPG_CUDA(cudaMemcpyAsync(out, d_out, m * sizeof(uint4), cudaMemcpyDeviceToHost, s), "seed intervals");
   HPG_CUDA(cudaStreamSynchronize(s), "seed search");
+  copies.waited();
   return 0;
 }
 
@@ -352,11 +358,13 @@ int engine_locate_rows(Engine* e, const MapRow* rows, size_t m, hpg_loc_t* out, 
     return -1;
   }
   cudaStream_t s = e->stream;
+  HostCopies copies(s);
   HPG_CUDA(cudaMemcpyAsync(e->b_rowhit.p, items.data(), m * sizeof(RowItem), cudaMemcpyHostToDevice, s), "rows");
   launch_locate_items(e->X, static_cast<const RowItem*>(e->b_rowhit.p), m, ptr<hpg_loc_t>(e->locs),
                       ptr<unsigned int>(e->b_ctr) + 5, e->num_sms, s);
   HPG_CUDA(cudaMemcpyAsync(out, e->locs.p, m * sizeof(hpg_loc_t), cudaMemcpyDeviceToHost, s), "located rows");
   HPG_CUDA(cudaStreamSynchronize(s), "locate rows");
+  copies.waited();
   return check_walk(e, err);
 }
 
@@ -394,6 +402,7 @@ int engine_inexact_records(Engine* e, const char* seqs, const uint64_t* offs, si
   }
   std::vector<uint64_t> rel(n + 1);
   for (size_t i = 0; i <= n; ++i) rel[i] = offs[i] - offs[0];
+  HostCopies copies(s);
   HPG_CUDA(cudaMemcpyAsync(e->m_offs.p, rel.data(), (n + 1) * 8, cudaMemcpyHostToDevice, s), "record offsets");
   launch_scan(r.rs_count, T, ptr<uint64_t>(e->m_hitoff), ptr<uint64_t>(e->m_part), s);
   const unsigned grid = (unsigned)((n + 127) / 128);
@@ -434,6 +443,7 @@ int engine_inexact_records(Engine* e, const char* seqs, const uint64_t* offs, si
     HPG_CUDA(cudaMemcpyAsync(out->rec.data(), e->m_rec.p, rows * sizeof(MapRec), cudaMemcpyDeviceToHost, s),
              "records");
   HPG_CUDA(cudaStreamSynchronize(s), "alignment records");
+  copies.waited();
   return check_walk(e, err);
 }
 
