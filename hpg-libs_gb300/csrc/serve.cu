@@ -107,7 +107,15 @@ struct ResultBuf {
   uint64_t* bounds = nullptr;
   size_t seg_cap = 0;
   int refs = 0;
+  uint64_t last_take = 0;  // the server's count of sets taken when this one was
   cudaEvent_t done = nullptr;
+  size_t bytes() const {
+    return hits_cap * sizeof(hpg_hit_t) + locs_cap * sizeof(hpg_loc_t) + rs_cap * 5 + seg_cap * 8;
+  }
+  // Whether the buffers hold what `want`'s capacities say.
+  bool holds(const ResultBuf& want) const {
+    return hits_cap >= want.hits_cap && locs_cap >= want.locs_cap && rs_cap >= want.rs_cap && seg_cap >= want.seg_cap;
+  }
 };
 
 struct Batch {
@@ -127,6 +135,18 @@ constexpr int kSets = 3;  // result sets a server starts with
 // order before it releases one, and a wait without end here would keep the batch it
 // waits for from ever being published (short batches make that many sets' worth).
 constexpr auto kSetWait = std::chrono::milliseconds(20);
+// The added sets together take at most this much page-locked memory, or as much as the
+// starting ones where that is more.  Past it a batch waits until a set is released: clients
+// that take their results more slowly than they submit hold the server back, not ever
+// more memory.
+constexpr size_t kAddedBytes = (size_t)256 << 20;
+// An added set that was not taken for this many batches is given back, and every idle one
+// when no request came for this long.
+constexpr uint64_t kAddedIdle = 64;
+constexpr auto kIdle = std::chrono::seconds(1);
+// A client's endless wait for a request ends with an error once a batch has waited this
+// long for a set, and no request was released meanwhile: it may be waiting for itself.
+constexpr double kStalledMs = 10000.0;
 
 template <typename T>
 bool pinned_grow(T** p, size_t* cap, size_t want) {
@@ -163,8 +183,14 @@ struct Server {
   bool stop = false;
   std::thread worker;
 
-  std::deque<ResultBuf> sets;  // grown by the worker only, under mu; entries stay where they are
-  int next_set = 0;
+  // grown by the worker only, under mu; entries stay where they are (a set given back is
+  // an entry without buffers).  The first kSets are the starting ones.
+  std::deque<ResultBuf> sets;
+  int next_set = 0;          // of the starting ones
+  uint64_t takes = 0;
+  size_t added_limit = kAddedBytes;
+  size_t set_bytes = 0;      // of all sets, for the statistics
+  double stalled_since = 0;  // a batch waits for a set, and none was released, since then (0: none waits)
   uint64_t* h_offs[2] = {nullptr, nullptr};
   uint32_t* h_seg[2] = {nullptr, nullptr};
   uint32_t* d_seg[2] = {nullptr, nullptr};
@@ -292,18 +318,84 @@ struct Server {
     return 0;
   }
 
+  // (the three below with mu held)
+  size_t added_bytes() const {
+    size_t sum = 0;
+    for (size_t i = kSets; i < sets.size(); ++i) sum += sets[i].bytes();
+    return sum;
+  }
+
+  // A set nobody holds: a starting one, else an added one that holds `want` or may be made
+  // to; -1: none.
+  int free_set(const ResultBuf& want) const {
+    for (int k = 0; k < kSets; ++k)
+      if (sets[(next_set + k) % kSets].refs == 0) return (next_set + k) % kSets;
+    const size_t added = added_bytes();
+    for (size_t i = kSets; i < sets.size(); ++i)
+      if (sets[i].refs == 0 && (sets[i].holds(want) || added - sets[i].bytes() + want.bytes() <= added_limit))
+        return (int)i;
+    return -1;
+  }
+
+  void note_set_bytes() {
+    set_bytes = 0;
+    for (const ResultBuf& rb : sets) set_bytes += rb.bytes();
+  }
+
+  static void drop_buffers(ResultBuf& rb) {
+    cudaFreeHost(rb.hits);
+    cudaFreeHost(rb.locs);
+    cudaFreeHost(rb.cnt);
+    cudaFreeHost(rb.trunc);
+    cudaFreeHost(rb.bounds);
+    rb.hits = nullptr;
+    rb.locs = nullptr;
+    rb.cnt = nullptr;
+    rb.trunc = nullptr;
+    rb.bounds = nullptr;
+    rb.hits_cap = rb.locs_cap = rb.rs_cap = rb.seg_cap = 0;
+  }
+
+  // Gives back the buffers of added sets that nobody holds and that were not taken for
+  // `idle` batches; the worker's, outside mu (nobody but it touches a set without holders).
+  void give_back(uint64_t idle, int keep) {
+    bool any = false;
+    for (size_t i = kSets; i < sets.size(); ++i) {
+      ResultBuf& rb = sets[i];
+      {
+        std::lock_guard<std::mutex> lk(mu);
+        if (rb.refs != 0 || rb.bytes() == 0 || (int)i == keep || takes - rb.last_take < idle) continue;
+      }
+      drop_buffers(rb);
+      any = true;
+    }
+    if (!any) return;
+    std::lock_guard<std::mutex> lk(mu);
+    note_set_bytes();
+  }
+
   ResultBuf* take_set(size_t hits, size_t locs, size_t rs, size_t segs, int* index, std::string* err) {
     int pick = -1;
+    ResultBuf want;
+    want.hits_cap = hits + 1;
+    want.locs_cap = locs + 1;
+    want.rs_cap = rs + 1;
+    want.seg_cap = 2 * segs + 2;
     {
       std::unique_lock<std::mutex> lk(mu);
-      const int n = (int)sets.size();
-      cv_sets.wait_for(lk, kSetWait, [&] {
-        for (int k = 0; k < n; ++k)
-          if (sets[(next_set + k) % n].refs == 0) return true;
-        return false;
-      });
-      for (int k = 0; k < n && pick < 0; ++k)
-        if (sets[(next_set + k) % n].refs == 0) pick = (next_set + k) % n;
+      auto found = [&] { return (pick = free_set(want)) >= 0; };
+      auto go_on = [&] { return found() || stop; };
+      cv_sets.wait_for(lk, kSetWait, go_on);
+      if (pick < 0 && added_bytes() + want.bytes() > added_limit && !stop) {
+        stalled_since = now_ms();
+        cv_done.notify_all();  // (endless waits take note of the time)
+        cv_sets.wait(lk, go_on);
+        stalled_since = 0;
+      }
+      if (pick < 0 && added_bytes() + want.bytes() > added_limit) {
+        *err = "server is stopping while its results are held by requests that were not released";
+        return nullptr;
+      }
       if (pick < 0) {
         ResultBuf more;
         if (cudaEventCreateWithFlags(&more.done, cudaEventDisableTiming) != cudaSuccess) {
@@ -311,27 +403,37 @@ struct Server {
           *err = "out of memory (serving results)";
           return nullptr;
         }
-        pick = n;
+        pick = (int)sets.size();
         sets.push_back(more);
       }
-      next_set = (pick + 1) % (int)sets.size();
+      if (pick < kSets) next_set = (pick + 1) % kSets;
+      sets[pick].last_take = ++takes;
     }
+    give_back(kAddedIdle, pick);
     ResultBuf& rb = sets[pick];
-    if (!pinned_grow(&rb.hits, &rb.hits_cap, hits + 1) || !pinned_grow(&rb.locs, &rb.locs_cap, locs + 1) ||
-        !pinned_grow(&rb.bounds, &rb.seg_cap, 2 * segs + 2)) {
+    const size_t had = rb.bytes();
+    // (an added set takes just what the batch needs, so that the limit holds)
+    if (pick >= kSets && !rb.holds(want)) drop_buffers(rb);
+    const bool ok = pinned_grow(&rb.hits, &rb.hits_cap, want.hits_cap) &&
+                    pinned_grow(&rb.locs, &rb.locs_cap, want.locs_cap) &&
+                    pinned_grow(&rb.bounds, &rb.seg_cap, want.seg_cap) && grow_lists(rb, want.rs_cap);
+    if (rb.bytes() != had) {
+      std::lock_guard<std::mutex> lk(mu);
+      note_set_bytes();
+    }
+    if (!ok) {
       *err = "out of pinned host memory (serving results)";
       return nullptr;
     }
-    if (rs > rb.rs_cap) {
-      size_t c1 = rb.rs_cap, c2 = rb.rs_cap;
-      if (!pinned_grow(&rb.cnt, &c1, rs + 1) || !pinned_grow(&rb.trunc, &c2, rs + 1)) {
-        *err = "out of pinned host memory (serving results)";
-        return nullptr;
-      }
-      rb.rs_cap = std::min(c1, c2);
-    }
     *index = pick;
     return &rb;
+  }
+
+  static bool grow_lists(ResultBuf& rb, size_t rs) {
+    size_t c1 = rb.rs_cap, c2 = rb.rs_cap;
+    const bool ok = pinned_grow(&rb.cnt, &c1, rs) && pinned_grow(&rb.trunc, &c2, rs);
+    rb.rs_cap = std::min(c1, c2);
+    return ok;
   }
 
   void fail(Batch* b, const std::string& why) {
@@ -487,7 +589,13 @@ struct Server {
         Batch* b = &batch[next_obj];
         {
           std::unique_lock<std::mutex> lk(mu);
-          if (may_wait && inflight.empty()) cv_work.wait(lk, [&] { return stop || !queue.empty(); });
+          auto work = [&] { return stop || !queue.empty(); };
+          if (may_wait && inflight.empty() && !cv_work.wait_for(lk, kIdle, work)) {
+            lk.unlock();
+            give_back(0, -1);
+            lk.lock();
+            cv_work.wait(lk, work);
+          }
           if (queue.empty()) return;
           b->slot = slot;
           const double f0 = now_ms();
@@ -581,6 +689,8 @@ Server* server_create(Engine* e, size_t max_batch_reads, uint64_t max_batch_base
          pinned_grow(&rb.cnt, &c1, 2 * max_batch_reads + 1) && pinned_grow(&rb.trunc, &c2, 2 * max_batch_reads + 1);
     rb.rs_cap = std::min(c1, c2);
   }
+  S->note_set_bytes();
+  S->added_limit = std::max(kAddedBytes, S->set_bytes);
   if (!ok) {
     cudaGetLastError();
     *err = "out of memory (serving buffers)";
@@ -626,6 +736,7 @@ void server_destroy(Server* S) {
       S->stop = true;
     }
     S->cv_work.notify_all();
+    S->cv_sets.notify_all();
     S->worker.join();
   }
   cudaStreamSynchronize(S->e->stream);
@@ -646,11 +757,7 @@ void server_destroy(Server* S) {
                  "plan %.3f, result set %.3f; publish to publish %.3f ms\n",
                  S->m_replay, S->m_wait_run, S->m_wait_out, S->m_plan, S->m_take, S->m_cycle);
   for (ResultBuf& rb : S->sets) {
-    cudaFreeHost(rb.hits);
-    cudaFreeHost(rb.locs);
-    cudaFreeHost(rb.cnt);
-    cudaFreeHost(rb.trunc);
-    cudaFreeHost(rb.bounds);
+    Server::drop_buffers(rb);
     if (rb.done) cudaEventDestroy(rb.done);
   }
   for (int k = 0; k < 2; ++k) {
@@ -725,7 +832,18 @@ int server_wait(Server* S, uint64_t ticket, hpg_result_set_t* view, double* late
   ServeReq* q = it->second;
   auto done = [&] { return q->state >= 2; };
   if (timeout_ms < 0) {
-    S->cv_done.wait(lk, done);
+    while (!done()) {
+      if (S->stalled_since == 0) {
+        S->cv_done.wait(lk);
+        continue;
+      }
+      const double left = S->stalled_since + kStalledMs - now_ms();
+      if (left <= 0) {
+        *err = "every result set of the server is held by requests that were not released: release some, then wait again";
+        return -1;
+      }
+      S->cv_done.wait_for(lk, std::chrono::duration<double, std::milli>(left));
+    }
   } else if (!S->cv_done.wait_for(lk, std::chrono::milliseconds(timeout_ms), done)) {
     return 1;
   }
@@ -762,6 +880,7 @@ int server_release(Server* S, uint64_t ticket, std::string* err) {
   if (q->state == 2) S->sets[q->set].refs--;
   S->reqs.erase(it);
   delete q;
+  if (S->stalled_since != 0) S->stalled_since = now_ms();  // a release may be what the worker waits for
   S->cv_sets.notify_all();
   return 0;
 }
@@ -781,7 +900,8 @@ void server_stats(Server* S, double* out, int n) {
                       (double)S->max_batch_reqs,
                       (double)S->queue.size(),
                       S->hits_per_read,
-                      S->rows_per_read};
+                      S->rows_per_read,
+                      (double)S->set_bytes};
   for (int i = 0; i < n && i < (int)(sizeof(v) / sizeof(v[0])); ++i) out[i] = v[i];
 }
 

@@ -534,7 +534,8 @@ class GpuIndex:
 
 
 SERVER_STATS = ("batches", "requests", "reads", "mean_batch_reads", "batch_wall_ms", "regrowths", "plan_bytes",
-                "hbm_budget", "max_batch_reads", "max_batch_requests", "queued", "hits_per_read", "rows_per_read")
+                "hbm_budget", "max_batch_reads", "max_batch_requests", "queued", "hits_per_read", "rows_per_read",
+                "result_bytes")
 
 
 class Server:
@@ -566,8 +567,7 @@ class Server:
         rs = ResultSetC()
         lat = ctypes.c_double()
         rc = self.lib.bwt_gpu_server_wait(self.handle, ticket, ctypes.byref(rs), ctypes.byref(lat), timeout_ms)
-        if rc < 0:
-            self._held.pop(ticket, None)
+        if rc < 0:  # (the request may still be queued: its arrays go with release or close)
             raise RuntimeError(self.lib.bwt_gpu_last_error().decode())
         if rc == 1:
             return None, None

@@ -352,11 +352,16 @@ const char *bwt_gpu_noalloc_last_error(void);
  * until wait returns for the ticket.  wait: 0 done, 1 timed out (timeout_ms
  * >= 0), -1 failed (bwt_gpu_last_error); `view` then points into the server's
  * pinned result buffers, read and hit ids relative to the request, valid until
- * release.  Unreleased requests hold their batch's buffers (three in turn).
+ * release.  Unreleased requests hold their batch's buffers, of which a server has
+ * three; while all are held, batches get further ones (256 MB together, or as
+ * much as the three where that is more), which are given back once they lie
+ * idle.  Past that a batch waits until a request is released; after 10 s without
+ * a release an endless wait fails, its ticket as it was, so that a client which
+ * waits for itself can release and wait again.
  * stats: {batches, requests, reads, mean reads per batch, batch wall ms (sum),
  * pool regrowths, device bytes of the captured plans, HBM budget, largest
  * batch (reads), largest batch (requests), queued requests, hits per read,
- * rows per read}. */
+ * rows per read, bytes of the result buffers}. */
 typedef struct bwt_gpu_server bwt_gpu_server_t;
 bwt_gpu_server_t *bwt_gpu_server_new(bwt_index_t *index, size_t max_batch_reads, uint64_t max_batch_bases,
                                      uint64_t hbm_budget_bytes, uint32_t max_results);
