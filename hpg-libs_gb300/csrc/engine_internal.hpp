@@ -231,6 +231,8 @@ constexpr int kGraphRefused = -2;
 int run_batched_graph(Engine* e, const void* seqs, const uint64_t* offs, uint32_t n, uint64_t total,
                       uint32_t max_results, DeviceResult* out, std::string* err, bool exact = false);
 uint64_t graph_plans_bytes(const Engine* e);  // device bytes of all plans
+// Device bytes that a batch of n reads and `bases` bases holds in its plan, at those rates.
+double graph_batch_bytes(const Engine* e, uint64_t n, uint64_t bases, double hits_per_read, double rows_per_read);
 void graph_plan_destroy(GraphPlan* g);
 void graph_plans_destroy(Engine* e);
 // Free the plans of more than max_n_cap reads, and the exact search's (after the streams finish).

@@ -211,6 +211,20 @@ int capture(Engine* e, GraphPlan* g, std::string* err) {
 
 }  // namespace
 
+// (as capture allocates, without what does not depend on the batch)
+double graph_batch_bytes(const Engine* e, uint64_t n, uint64_t bases, double hits_per_read, double rows_per_read) {
+  const bool text = text_form(e, n), rows = e->X.text != nullptr;
+  const double per_base = 1.0 + (text ? 0.25 : 1.0);
+  // offsets, flags, arrivals, segments, cursors, kept counts, truncation, rows and starts of
+  // the lists; the queue of change points and the blocks; the text form's queues
+  const double per_read = 8 + 1 + 2 * (4 + 8 + 4 + 4 + 1 + 4) + 8 + (e->tuning.split ? 4 : 0.25) * sizeof(SpillEntry) +
+                          (e->tuning.split == 3 ? 4 * sizeof(SpillEntry) : 0) +
+                          (text ? (double)(text_queue_bytes(1u << 20, 0) >> 20) : 0);
+  const double per_hit = 2 * sizeof(PendingHit) + sizeof(hpg_hit_t) + (rows ? 0 : 8);
+  const double per_row = sizeof(hpg_loc_t) + (rows ? 0 : (double)locate_row_item_bytes());
+  return per_base * (double)bases + (per_read + hits_per_read * per_hit + rows_per_read * per_row) * (double)n;
+}
+
 void graph_plan_destroy(GraphPlan* g) {
   if (!g) return;
   if (g->exec) cudaGraphExecDestroy(g->exec);

@@ -222,9 +222,7 @@ struct Server {
 
   // HBM bytes a batch of n reads and `bases` bases is expected to hold.
   double est_bytes(uint64_t n, uint64_t bases) const {
-    const double per_read = 9.0 + 2 * 25.0 + hits_per_read * 1.25 * (2 * 24 + 32 + 4 + 8) +
-                            rows_per_read * 1.25 * (16 + 32) + 4.0;
-    return 2.0 * (double)bases + per_read * (double)n;
+    return graph_batch_bytes(e, n, bases, hits_per_read * 1.25, rows_per_read * 1.25);
   }
 
   // Take waiting requests in arrival order while they fit (called with mu held).
