@@ -362,6 +362,14 @@ int bwt_gpu_full_rows(bwt_index_t* index) {
   return e ? engine_full_rows(e) : 0;
 }
 
+int bwt_gpu_drop_full_rows(bwt_index_t* index) {
+  Engine* e = engine_of(index);
+  if (!e) return fail("bwt_gpu_drop_full_rows: null index");
+  std::string err;
+  if (engine_drop_full_rows(e, &err) != 0) return fail(err);
+  return 0;
+}
+
 void bwt_gpu_set_pipeline_chunk(bwt_index_t* index, size_t reads) {
   Engine* e = engine_of(index);
   if (e) engine_set_pipeline_chunk(e, reads);

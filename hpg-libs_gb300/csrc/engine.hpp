@@ -91,6 +91,8 @@ int engine_set_kmer(Engine* e, int L, std::string* err);
 // default), or the sampled arrays (0); returns what is in use.
 int engine_set_full_rows(Engine* e, int on);
 int engine_full_rows(Engine* e);
+// Frees them, with the plans captured with them and the workspaces only they use.
+int engine_drop_full_rows(Engine* e, std::string* err);
 int engine_kmer(Engine* e);
 // Host-buffer batches of at least two chunks run pipelined; reads per chunk (0 automatic, SIZE_MAX off).
 void engine_set_pipeline_chunk(Engine* e, size_t reads);

@@ -237,6 +237,8 @@ void graph_plan_destroy(GraphPlan* g);
 void graph_plans_destroy(Engine* e);
 // Free the plans of more than max_n_cap reads, and the exact search's (after the streams finish).
 void graph_plans_drop_above(Engine* e, uint64_t max_n_cap);
+// Free the plans captured with the whole suffix arrays and the text.
+void graph_plans_drop_text(Engine* e);
 // Free the grow-only workspaces of the direct, plain, block-search and
 // alignment-list calls (they are allocated again on demand), the plans of
 // more than keep_n_cap reads and the exact search's: a server on the index keeps only what it uses.

@@ -21,8 +21,8 @@
 //
 // They are kept when they take at most a quarter of the device's free memory
 // (several indexes and batch workspaces share the rest) and the derivation
-// proves them consistent with the index; otherwise every path uses the sampled
-// arrays and LF, with the same results.
+// proves them consistent with the index; otherwise, and once a caller has
+// dropped them, every path uses the sampled arrays and LF, with the same results.
 //
 // Derivation: as text_samples.cu, one LF walk from every sampled row to the
 // next, which visits every row once with its SA value v known: SA[row] = v,
@@ -143,6 +143,19 @@ int engine_set_full_rows(Engine* en, int on) {
 }
 
 int engine_full_rows(Engine* en) { return en->X.text ? 1 : 0; }
+
+int engine_drop_full_rows(Engine* en, std::string* err) {
+  HPG_CUDA(cudaSetDevice(en->device), "cudaSetDevice");
+  HPG_CUDA(cudaStreamSynchronize(en->stream), "drop full suffix arrays");
+  graph_plans_drop_text(en);
+  for (DevBuf* b : {&en->b_packed, &en->b_text, &en->b_one}) {
+    cudaFree(b->p);
+    *b = DevBuf();
+  }
+  free_full_rows(en);
+  en->last = DeviceResult();  // may have been in one of the plans
+  return 0;
+}
 
 int build_full_rows(Engine* en, const uint32_t n_samples[2], std::string* err) {
   const size_t n_rows = en->X.walk_mod;

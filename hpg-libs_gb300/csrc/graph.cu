@@ -247,16 +247,25 @@ void graph_plans_destroy(Engine* e) {
   e->plans = nullptr;
 }
 
-void graph_plans_drop_above(Engine* e, uint64_t max_n_cap) {
+template <typename Drop>
+static void plans_drop(Engine* e, Drop drop) {
   if (!e->plans) return;
   cudaStreamSynchronize(e->stream);
   for (cudaStream_t x : e->xs)
     if (x) cudaStreamSynchronize(x);
   for (int i = 0; i < kMaxPlans * kPlanSlots; ++i)
-    if (e->plans[i] && (e->plans[i]->n_cap > max_n_cap || e->plans[i]->exact)) {
+    if (e->plans[i] && drop(*e->plans[i])) {
       graph_plan_destroy(e->plans[i]);
       e->plans[i] = nullptr;
     }
+}
+
+void graph_plans_drop_above(Engine* e, uint64_t max_n_cap) {
+  plans_drop(e, [&](const GraphPlan& g) { return g.n_cap > max_n_cap || g.exact; });
+}
+
+void graph_plans_drop_text(Engine* e) {
+  plans_drop(e, [](const GraphPlan& g) { return g.text != nullptr; });
 }
 
 // The plan for a batch of n reads and `total` bases: one per power-of-two read

@@ -150,6 +150,7 @@ def load() -> ctypes.CDLL:
     lib.bwt_gpu_set_start_table.argtypes = [vp, ctypes.c_int]
     lib.bwt_gpu_set_full_rows.argtypes = [vp, ctypes.c_int]
     lib.bwt_gpu_full_rows.argtypes = [vp]
+    lib.bwt_gpu_drop_full_rows.argtypes = [vp]
     lib.bwt_gpu_set_direction_split.argtypes = [vp, ctypes.c_int]
     lib.bwt_gpu_direction_split.argtypes = [vp]
     lib.bwt_gpu_map_device_seconds.restype = ctypes.c_double
@@ -518,6 +519,10 @@ class GpuIndex:
 
     def full_rows(self) -> bool:
         return bool(self.lib.bwt_gpu_full_rows(self.handle))
+
+    def drop_full_rows(self) -> None:
+        """Gives the memory of the whole suffix arrays and the text back, for good."""
+        self._check(self.lib.bwt_gpu_drop_full_rows(self.handle))
 
     def set_pipeline_chunk(self, reads: int) -> None:
         """Reads per chunk of pipelined host batches (0 or -1: not pipelined, the default)."""

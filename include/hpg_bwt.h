@@ -262,11 +262,15 @@ int bwt_gpu_start_table(bwt_index_t *index);
 /* Whole suffix arrays: an index that finds room (at most a quarter of the
  * device's free memory) keeps the suffix array, its inverse and the packed text
  * beside the sampled arrays, 16.25 bytes per base in all (and start tables of
- * up to 4.3 GB), and locates rows and finishes one-row searches with them.  set: 0 uses the sampled arrays only, 1
- * (the default) the whole ones where the index has them; returns which are in
- * use.  Results are identical. */
+ * up to 4.3 GB), and locates rows and finishes one-row searches with them.
+ * set: 0 uses the sampled arrays only, 1 (the default) the whole ones where the
+ * index has them; returns which are in use.  drop: gives their memory back for
+ * good, with the plans and workspaces that go with them, for a program that
+ * wants the device's memory for itself (not while a server runs on the index;
+ * an index opened again has them again).  Results are identical. */
 int bwt_gpu_set_full_rows(bwt_index_t *index, int on);
 int bwt_gpu_full_rows(bwt_index_t *index);
+int bwt_gpu_drop_full_rows(bwt_index_t *index);
 /* Autotuner: times the batched search on a device-resident read batch for
  * every candidate setting (60 fused, split and lockstep settings, then 12
  * warp-cooperative ones: 8, 16 or 32 reads per warp group x register bound 8
