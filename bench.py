@@ -577,6 +577,15 @@ def served_parity(gi, index_dir: str, pool, rng: np.random.Generator, locate_lim
     return out
 
 
+def tuning_of(gi) -> dict:
+    """The settings that act on the batched search as it runs."""
+    both = {"block_load_mode": gi.load_mode(), "idle_batch": gi.idle_batch()}
+    if gi.full_rows() and gi.wave_group():
+        return dict(both, form="search with the text")
+    return dict(gi.get_tuning(), wave_group=gi.wave_group(), start_table=gi.start_table(),
+                direction_split=gi.direction_split(), **both)
+
+
 def serving_large(dist, log) -> dict:
     """The serving form against the 3.1 Gbp index: the genome of the c4
     workload, indexed on this GPU; requests of log-uniform 1k-256k reads of
@@ -616,9 +625,7 @@ def serving_large(dist, log) -> dict:
                        "1k-256k reads of uniform 50-300 bp at 0.5% per-base substitution (uncapped), <=1 error "
                        "searched; Poisson arrivals at 10-90% of the saturated rate")
     res["genome_and_index_s"] = round(t_index, 1)
-    res["tuning"] = dict(gi.get_tuning(), wave_group=gi.wave_group(), block_load_mode=gi.load_mode(),
-                         start_table=gi.start_table(), direction_split=gi.direction_split(),
-                         tuned_on="held-out pool of 600k request reads (seed 12)")
+    res["tuning"] = dict(tuning_of(gi), tuned_on="held-out pool of 600k request reads (seed 12)")
     gi.close()
     return res
 
@@ -962,8 +969,7 @@ def run_gb300(args, wl: dict, dist: Dist) -> dict | None:
             "cal_generation": cals,
             "alignment_lists": alns,
             "block_search": block,
-            "tuning": dict(gi.get_tuning(), block_load_mode=gi.load_mode(), start_table=gi.start_table(),
-                           direction_split=gi.direction_split(), idle_batch=gi.idle_batch()),
+            "tuning": tuning_of(gi),
             "autotune": ({"settings": len(table), "tuned_on": "held-out batch of the same workload (seed "
                           f"{read_seed(dist.rank) + TUNE_SEED_OFFSET})",
                           "best_search_ms": min(r["search_us"] for r in table) / 1e3,

@@ -538,7 +538,8 @@ int engine_autotune(Engine* e, const uint8_t* d_seqs, const uint64_t* d_offs, si
   static const int cand_minb[] = {1, 10, 12, 16};  // 10: fused form only (the others take 1)
   static const int cand_stack[] = {-1, 0, 2, 4, 8};  // 0: split form, -1: lockstep form
   static const int cand_chunk[] = {1, 2, 4};
-  BatchedTuning best = e->tuning;
+  const BatchedTuning was = e->tuning;
+  BatchedTuning best = was;
   float best_ms = 1e30f;
   int rows = 0;
   DeviceResult r;
@@ -577,7 +578,11 @@ int engine_autotune(Engine* e, const uint8_t* d_seqs, const uint64_t* d_offs, si
       }
   // the warp-cooperative form: reads per warp group (lanes per read = 32 / group)
   // x register bound x one launch per index direction or one for both; rows
-  // carry stack -2 and the group in the chains column
+  // carry stack -2 and the group in the chains column.  With the text on the device
+  // none of them acts (text_search.cu runs in its place): it is timed once, for all
+  // the rows, and the settings stay as they were, for when the arrays are not used.
+  const bool text = e->X.text && n_reads <= kTextMaxReads;
+  float text_ms = 0;
   for (int grp : {8, 16, 32})
     for (int mb : {8, 12})
       for (int ds : {0, 2}) {
@@ -586,13 +591,14 @@ int engine_autotune(Engine* e, const uint8_t* d_seqs, const uint64_t* d_offs, si
         e->tuning.min_blocks = mb;
         e->tuning.group = grp;
         e->tuning.dir_split = ds;
-        float t = 0;
-        for (int rep = 0; rep < 2; ++rep) {
+        float t = text_ms;
+        for (int rep = 0; rep < 2 && text_ms == 0; ++rep) {
           if (engine_search_device(e, HPG_BWT_MODE_SEARCH1, kFormBatched, d_seqs, d_offs, n_reads, total_bases,
                                    max_len, max_results, &r, err) != 0)
             return -1;
           t = e->stage_ms[kStageSearch];
         }
+        if (text) text_ms = t;
         if (table && rows < max_rows) {
           int* row = table + 5 * rows;
           row[0] = mb;
@@ -607,7 +613,8 @@ int engine_autotune(Engine* e, const uint8_t* d_seqs, const uint64_t* d_offs, si
           best = e->tuning;
         }
       }
-  e->tuning = best;
+  const bool text_best = text && best.split == 3;
+  e->tuning = text_best && was.split == 3 ? was : best;
   // then the block-load form, with the chosen setting
   uint32_t best_mode = e->X.load_mode;
   for (int mode = 0; mode < 4; ++mode) {
@@ -667,12 +674,13 @@ int engine_autotune(Engine* e, const uint8_t* d_seqs, const uint64_t* d_offs, si
     best_ms = t_on[best_split];
     e->tuning.dir_split = best_split;
   }
-  // then the start-table length (rows marked by a first column of -100 - L)
+  // then the start-table length (rows marked by a first column of -100 - L); the search
+  // with the text has a table of its own, so none is built or timed for it
   int best_kmer = (int)e->X.kmer_len;
   for (int L : {0, 8, 10, 11, 12}) {
-    if (engine_set_kmer(e, L, err) != 0) return -1;
-    float t = 0;
-    for (int rep = 0; rep < 2; ++rep) {
+    if (!text_best && engine_set_kmer(e, L, err) != 0) return -1;
+    float t = best_ms;
+    for (int rep = 0; rep < 2 && !text_best; ++rep) {
       if (engine_search_device(e, HPG_BWT_MODE_SEARCH1, kFormBatched, d_seqs, d_offs, n_reads, total_bases, max_len,
                                max_results, &r, err) != 0)
         return -1;

@@ -225,7 +225,10 @@ int bwt_gpu_direction_split(bwt_index_t *index);
  * the warp's lanes share the group's chains and one stack of change points.
  * The direction split (0 or 2), register bound (1, 8 or 12 blocks per SM),
  * idle batch, start table and block-load form apply to it as to the fused
- * form.  0 returns to the fused form.  Results are identical. */
+ * form.  0 returns to the fused form.  With the whole suffix arrays in use
+ * (bwt_gpu_full_rows) this form stands for the search with the text, of which
+ * only the idle batch and the block-load form are settings.  Results are
+ * identical. */
 void bwt_gpu_set_wave_group(bwt_index_t *index, int reads);
 /* Reads per warp group of the warp-cooperative form, 0 when another form is selected. */
 int bwt_gpu_wave_group(bwt_index_t *index);
@@ -256,7 +259,8 @@ uint64_t bwt_gpu_locate_limit(bwt_index_t *index);
  * chain of a read of at least 2L+2 bases starts with one lookup of its first L
  * symbols in a table of 4^L intervals per index direction (8 MB each at L = 10)
  * instead of L dependent steps.  0 = no table (the default; the autotuner tries
- * 8, 10, 11, 12), at most 12.  Results are identical. */
+ * 8, 10, 11, 12), at most 12.  The search with the text has a table of its own
+ * and does not read this one.  Results are identical. */
 int bwt_gpu_set_start_table(bwt_index_t *index, int symbols);
 int bwt_gpu_start_table(bwt_index_t *index);
 /* Whole suffix arrays: an index that finds room (at most a quarter of the
@@ -277,7 +281,10 @@ int bwt_gpu_drop_full_rows(bwt_index_t *index);
  * or 12 x direction split 0 or 2), keeps the fastest, then picks the fastest
  * block-load form for it (4 more runs), then the direction split (3 more, fused
  * form only), then the start-table length among 0, 8, 10, 11, 12 (5 more),
- * then the idle-lane batch among 1, 4, 8, 16 (4 more).  Optional table gets
+ * then the idle-lane batch among 1, 4, 8, 16 (4 more).  With the whole suffix
+ * arrays in use the 12 rows are one timing of the search with the text; where
+ * it is the fastest, the warp-cooperative settings and the start table stay as
+ * they were and the 5 rows repeat its time.  Optional table gets
  * rows of {min_blocks (or -1 - load mode, -50 - split, -100 - table length,
  * -200 - idle batch), blocks_per_sm, stack (-2: warp-cooperative),
  * chains_per_claim (reads per warp group), search us}. */
