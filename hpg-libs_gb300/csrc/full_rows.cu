@@ -12,10 +12,10 @@
 // most, per direction (8 bytes an entry): 2.7 GB at 100 Mbp, 54 GB at 3.1 Gbp of
 // the device's 284 GB.  Measured on 2M x 100 bp reads, 100 Mbp: the locate stage
 // takes 406 us per 2M rows with LF walks (16 sectors a row), 80 us with the gather;
-// the search 3704 us with rank steps only, 680 us with the text.
+// the search 3704 us with rank steps only, 700 us with the text.
 //
 // Table length (search stage there / on 2M x 150 bp, 600 Mbp, each before the kernels that
-// took it to 680 / 2750): 11 symbols 903 /
+// took it to 700 / 2760): 11 symbols 903 /
 // 7783 us, 12: 903 / 7570, 13: 891 / 7550, 14: 864 / 7392; a table longer than
 // log4(n) is mostly empty intervals and four times the memory.
 //

@@ -3,13 +3,13 @@
 //
 // Every size the pipeline needs lives in device memory: the read count and
 // max_results in a small header written before each replay, the hit and row
-// totals in the scans' last elements.  Each kernel is captured at a grid sized
+// totals beside the lists.  Each kernel is captured at a grid sized
 // for the plan's capacity (the persistent kernels at one wave) and reads its
 // real extent from device memory, so one capture serves every batch of its
 // capacity class.  The replay is: inputs + header to the device, one
-// cudaGraphLaunch (zeroing, encode, persistent search and drain, ordered
-// finalize, persistent locate, a size summary copied to pinned host memory),
-// one stream synchronize.  A pool that overflows sets a status bit that the
+// cudaGraphLaunch (zeroing, encode, search, ordered finalize, hit records and
+// located rows, a size summary copied to pinned host memory), one stream
+// synchronize.  A pool that overflows sets a status bit that the
 // later stages check; the host then grows that pool, captures again and reruns
 // the batch, so no result is ever dropped.
 #include <cuda_runtime.h>

@@ -2,7 +2,7 @@
 // the plain kernels (one thread per read and strand).
 //
 //   exact_bwd / exact_fwd ....... BWExactSearchBackward/Forward (search/search.h:9-65)
-//   vector_bwd / vector_fwd ..... BWExactSearchVectorBackward/Forward (search/search.c:1407-1489)
+//   vector_run .................. BWExactSearchVectorBackward/Forward (search/search.c:1407-1489)
 //   search1_helper .............. BWSearch1VectorHelper (search/search.c:1491-1709)
 //
 // The helper keeps one mutable result cursor and appends copies of it, as the

@@ -40,10 +40,10 @@
 // Bound by random sectors, as rank walks are, but about 20 a read of 100 bp at 100
 // Mbp against 180, and by the latency of some 8 dependent accesses a chain, whatever
 // the read's length.  Search stage, rank walks (wave.cu) -> here:
-//   2M x 100 bp, 100 Mbp                          3704 ->  680 us
-//   4M x 36-250 bp, 100 Mbp                      12570 -> 1590 us
-//   1000 x 50-300 bp, 100 Mbp                      510 ->   70 us
-//   2M x 150 bp, 600 Mbp with 45 % repeats        9809 -> 2750 us
+//   2M x 100 bp, 100 Mbp                          3704 ->  700 us
+//   4M x 36-250 bp, 100 Mbp                      12570 -> 1610 us
+//   1000 x 50-300 bp, 100 Mbp                      510 ->   80 us
+//   2M x 150 bp, 600 Mbp with 45 % repeats        9809 -> 2760 us
 // Indexes without the arrays, and batches above kTextMaxReads (the queues'
 // counters), take the warp-cooperative form.
 #include <cuda_runtime.h>
