@@ -837,7 +837,19 @@ int server_wait(Server* S, uint64_t ticket, hpg_result_set_t* view, double* late
       }
       const double left = S->stalled_since + kStalledMs - now_ms();
       if (left <= 0) {
-        *err = "every result set of the server is held by requests that were not released: release some, then wait again";
+        *err = "every result set of the server is held by requests that were not released";
+        if (q->state == 0) {  // not in a batch yet: the server lets go of the caller's reads
+          for (auto at = S->queue.begin(); at != S->queue.end(); ++at)
+            if (*at == q) {
+              S->queue.erase(at);
+              break;
+            }
+          q->state = 3;
+          q->err = *err;
+          q->t_done = now_ms();
+        } else {
+          *err += ": release some, then wait again";
+        }
         return -1;
       }
       S->cv_done.wait_for(lk, std::chrono::duration<double, std::milli>(left));

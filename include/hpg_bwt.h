@@ -367,8 +367,9 @@ const char *bwt_gpu_noalloc_last_error(void);
  * three; while all are held, batches get further ones (256 MB together, or as
  * much as the three where that is more), which are given back once they lie
  * idle.  Past that a batch waits until a request is released; after 10 s without
- * a release an endless wait fails, its ticket as it was, so that a client which
- * waits for itself can release and wait again.
+ * a release an endless wait returns -1, so that a client which waits for itself
+ * can release some: a request of a batch that was mapped keeps its ticket, to
+ * be waited for again, and one still queued has failed.
  * stats: {batches, requests, reads, mean reads per batch, batch wall ms (sum),
  * pool regrowths, device bytes of the captured plans, HBM budget, largest
  * batch (reads), largest batch (requests), queued requests, hits per read,

@@ -60,6 +60,11 @@ def test_added_sets_are_bounded_and_given_back(copies):
             with pytest.raises(RuntimeError, match="held by requests"):
                 srv.wait(stuck)
             assert time.time() - t0 < 30
+            queued = srv.submit(reads.seq, reads.offsets)
+            with pytest.raises(RuntimeError, match="held by requests"):
+                srv.wait(queued)
+            assert srv.stats()["queued"] == 0  # its reads are the client's again
+            srv.release(queued)
             srv.release(held.pop())
             rs, _lat = srv.wait(stuck, copy=False)  # the ticket was left as it was
             assert lib.result_from_c(rs, len(reads)).equal(want)
